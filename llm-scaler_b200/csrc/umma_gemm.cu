@@ -320,7 +320,7 @@ umma_wo_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constant__
 
   if (warp == 0) {
     // ---------------- raw weight producer ----------------
-    if (lane == 0) {
+    if (elect_one()) {
       tma_prefetch_desc(&tm_w);
       int grb = 0;                       // raw stages issued so far: ring position and phase carry across segments
       int issued = 0;
@@ -343,7 +343,7 @@ umma_wo_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constant__
     }
   } else if (warp == 2) {
     // ---------------- activation producer ----------------
-    if (lane == 0) {
+    if (elect_one()) {
       tma_prefetch_desc(&tm_x);
       if (!p.tiles) grid_dep_wait();
       int gb = 0, issued = 0;
@@ -362,7 +362,7 @@ umma_wo_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constant__
     }
   } else if (warp == 1 || (Cfg::NMMA == 2 && warp == 3)) {
     // ---------------- MMA issuer(s) ----------------
-    if (lane == 0) {
+    if (elect_one()) {
       constexpr uint32_t idesc = instr_desc(BF16 ? 1u : 0u, BF16 ? 1u : 0u, 128, TOK);
       const int me = warp == 1 ? 0 : 1;
       const uint32_t dacc = tmem + me * Cfg::ACC_COLS;

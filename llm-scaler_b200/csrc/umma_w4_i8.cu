@@ -129,7 +129,7 @@ umma_w4_i8_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constan
 
   if (warp == 0) {
     // ---- raw weight producer: one box of h rows x 128 bytes (256 k) per stage ----
-    if (lane == 0) {
+    if (elect_one()) {
       tma_prefetch_desc(&tm_w);
       int gr = 0;
       bool ok = true;
@@ -147,7 +147,7 @@ umma_w4_i8_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constan
     }
   } else if (warp == 2) {
     // ---- activation producer: the NTOK term rows of one group per stage ----
-    if (lane == 0) {
+    if (elect_one()) {
       tma_prefetch_desc(&tm_x);
       grid_dep_wait();
       int gc = 0;
@@ -166,7 +166,7 @@ umma_w4_i8_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constan
     }
   } else if (warp == 1) {
     // ---- MMA issuer: one group (128 k) = four MMAs into that group's own accumulator ----
-    if (lane == 0) {
+    if (elect_one()) {
       constexpr uint32_t idesc = instr_desc_i8(0u, 1u, 128, NTOK);       // u8 weights x s8 activations -> s32
       int gc = 0;
       bool ok = true;

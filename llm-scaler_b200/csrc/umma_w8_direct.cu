@@ -125,7 +125,7 @@ umma_w8_direct_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_con
 
   if (warp == 0) {
     // ---- weight producer: one 128 x 128 box per stage ----
-    if (lane == 0) {
+    if (elect_one()) {
       tma_prefetch_desc(&tm_w);
       int g = 0;
       bool ok = true;
@@ -143,7 +143,7 @@ umma_w8_direct_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_con
     }
   } else if (warp == 2) {
     // ---- activation producer: the NTOK term rows of the same 128 k ----
-    if (lane == 0) {
+    if (elect_one()) {
       tma_prefetch_desc(&tm_x);
       grid_dep_wait();
       int g = 0;
@@ -162,7 +162,7 @@ umma_w8_direct_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_con
     }
   } else if (warp == 1) {
     // ---- MMA issuer ----
-    if (lane == 0) {
+    if (elect_one()) {
       const uint32_t idesc = instr_desc(p.e5m2 ? 1u : 0u, 0u, 128, NTOK);
       bool ok = true;
       int g = 0, si = 0;

@@ -79,7 +79,7 @@ umma_w8a8_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constant
   const uint32_t tmem = *tmem_slot;
 
   if (warp == 0) {
-    if (lane == 0) {
+    if (elect_one()) {
       tma_prefetch_desc(&tm_w);
       tma_prefetch_desc(&tm_x);
       int kb = 0;
@@ -93,7 +93,7 @@ umma_w8a8_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constant
       if (kb < nkb) drain_issued(full, S, kb);       // gave up: let the copies already issued land first
     }
   } else if (warp == 1) {
-    if (lane == 0) {
+    if (elect_one()) {
       constexpr uint32_t idesc = instr_desc(0u, 0u, 128, TOK);       // e4m3 x e4m3 -> fp32
       for (int kb = 0; kb < nkb; ++kb) {
         const int s = kb % S, b = kb % NBUF;
@@ -239,7 +239,7 @@ umma_w8a8_pair_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_con
 
   if (warp == 0) {
     // ---- producer (both CTAs): own W rows + own half of the token tile; bytes counted on the leader's barrier ----
-    if (lane == 0) {
+    if (elect_one()) {
       tma_prefetch_desc(&tm_w);
       tma_prefetch_desc(&tm_x);
       for (int kb = 0; kb < nkb; ++kb) {
@@ -253,7 +253,7 @@ umma_w8a8_pair_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_con
     }
   } else if (warp == 1) {
     // ---- MMA issuer: the leader's one thread drives both CTAs' tensor cores ----
-    if (lane == 0 && rank == 0) {
+    if (rank == 0 && elect_one()) {
       constexpr uint32_t idesc = instr_desc(0u, 0u, 256, TOK);
       for (int kb = 0; kb < nkb; ++kb) {
         const int s = kb % S, b = kb % NBUF;
