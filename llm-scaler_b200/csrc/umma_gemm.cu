@@ -219,7 +219,7 @@ template <int TOK> struct UmmaCfg {
   // Operand stages (32 columns each) fill the rest of the allocation: a stage is only reusable once
   // the MMAs that read it have completed and signalled, a round trip of a couple of microseconds, so
   // the ring has to be deep for the transform warps to stay busy.
-  static constexpr int S = (TMEM_COLS - A_COL0) / 32 > 12 ? 12 : (TMEM_COLS - A_COL0) / 32;
+  static constexpr int S = ((TMEM_COLS - A_COL0) / 32 > 12 ? 12 : (TMEM_COLS - A_COL0) / 32) & ~1;
 };
 
 // MAGIC: INT4 weights behind the activation pre-pass (fp16 activations in the nibble decode's pair order): its own
@@ -230,7 +230,9 @@ umma_wo_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constant__
   using Cfg = UmmaCfg<TOK>;
   constexpr int S = Cfg::S, RS = Cfg::RS, NG = Cfg::NG, XS = Cfg::XS;
   constexpr int CPR = (WK == WK_W8) ? 2 : 4;          // 64-k chunks per raw stage
-  constexpr int GPR = CPR < NG ? CPR : NG;            // transform groups that touch one raw stage
+  // transform groups that touch one raw stage, and the arrivals each of them makes there and on an operand stage
+  constexpr int GPR = MAGIC ? 2 : (CPR < NG ? CPR : NG);
+  constexpr int GRP_ARRIVALS = MAGIC ? 4 : 128;
   // With equally deep rings chunk g uses operand stage g % S and activation stage g % XS = the same index, and the MMAs
   // that free one free the other: the activation producer waits on the operand stage's barrier, the issuer commits once
   // (MoE pipeline 676 -> 664 us; the decode tiles are indifferent).
@@ -302,9 +304,9 @@ umma_wo_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constant__
   const int64_t sbase = (int64_t)expert * p.s_expert_elems;
 
   if (threadIdx.x == 0) {
-    for (int i = 0; i < S; ++i) { mbar_init(a_full + 8 * i, 128); mbar_init(ab_empty + 8 * i, 1); }
+    for (int i = 0; i < S; ++i) { mbar_init(a_full + 8 * i, GRP_ARRIVALS); mbar_init(ab_empty + 8 * i, 1); }
     for (int i = 0; i < XS; ++i) { mbar_init(x_full + 8 * i, 1); mbar_init(x_empty + 8 * i, 1); }
-    for (int i = 0; i < RS; ++i) { mbar_init(raw_full + 8 * i, 1); mbar_init(raw_empty + 8 * i, GPR * 128); }
+    for (int i = 0; i < RS; ++i) { mbar_init(raw_full + 8 * i, 1); mbar_init(raw_empty + 8 * i, GPR * GRP_ARRIVALS); }
     mbar_init(accum_full, Cfg::NMMA);
     mbar_init(accum_empty, NG * 128);
     mbar_init(fix_bar, NG * 128);
@@ -433,12 +435,6 @@ umma_wo_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constant__
         return __uint_as_float(raw);
       }
     };
-    uint32_t sq0 = chunk_scale_raw(grp), sq1 = chunk_scale_raw(grp + NG), sq2 = chunk_scale_raw(grp + 2 * NG),
-             sq3 = chunk_scale_raw(grp + 3 * NG);
-    uint32_t sn0 = chunk_scale_raw(grp + 4 * NG), sn1 = chunk_scale_raw(grp + 5 * NG), sn2 = chunk_scale_raw(grp + 6 * NG),
-             sn3 = chunk_scale_raw(grp + 7 * NG);
-    int it4 = 0;                                   // position of the current chunk in its set of four
-    int pend = -1;                                 // MAGIC: operand stage whose tensor-memory stores are still in flight
     int saturated = 0;                             // MAGIC: a scale had to be clamped (reported once, behind the loop)
     // fp16 magic route with bf16 / fp32 scales: the group scale is rounded to fp16, whose normal range starts at
     // 6.1e-5.  Every row of a segment therefore carries its own power of two, taken from the scale of the segment's
@@ -458,6 +454,96 @@ umma_wo_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constant__
         }
       }
     }
+    if constexpr (MAGIC) {
+      // One iteration converts one scale group: 128 k of a row = two operand stages of 64 k, half of a raw stage.  The
+      // groups of four warps take the scale groups in turn, so a thread always works on the same half of a raw stage and
+      // every ring position advances by a constant.  What a chunk costs besides its decode (two barrier waits, ring
+      // arithmetic, scale fetch / conversion / range check, arrivals: 265 of 370 issue slots per 64 k when all of it was
+      // done per chunk by division and selection) is most of what this loop cost, so it is paid per 128 k and by counting, and
+      // barriers take one arrival per warp.  Measured: decoder layer at M = 64 299 -> 262 us, MoE pipeline at 4096 tokens
+      // 702 -> 667 us, decoder layer at M = 2048 3138 -> 3072 us.
+      static_assert(!MAGIC || (S % 2 == 0 && NG % 2 == 0 && CPR == 4), "a scale group is two operand stages, half a raw stage");
+      constexpr int RAW_STEP = NG / 2, A_STEP = 2 * NG;
+      const int ngroups = nk >> 1, half = grp & 1;
+      const int raw0 = grb + (grp >> 1), a0 = gb + 2 * grp;
+      int rs = raw0 % RS, as = a0 % S;
+      uint32_t rpar = (uint32_t)(raw0 / RS) & 1u, apar = ((uint32_t)(a0 / S) + 1u) & 1u;
+      const int esz = p.scale_dtype == B2Q_F32 ? 4 : 2;
+      const uint8_t* sp = reinterpret_cast<const uint8_t*>(p.scale) +
+                          (sbase + (int64_t)nrow * p.s_stride_n + (int64_t)((c_begin >> 1) + grp) * p.s_stride_g) * esz;
+      const int64_t sstep = (int64_t)NG * p.s_stride_g * esz;
+      auto next_scale = [&](int gg) -> uint32_t {           // raw bits of group gg's scale; sp walks along with the calls
+        uint32_t v = 0u;
+        if (gg < ngroups) v = esz == 4 ? __ldg(reinterpret_cast<const uint32_t*>(sp)) : (uint32_t)__ldg(reinterpret_cast<const unsigned short*>(sp));
+        sp += sstep;
+        return v;
+      };
+      // two scales in use, two in flight: requested two to three iterations ahead, untouched until their turn
+      uint32_t sq0 = next_scale(grp), sq1 = next_scale(grp + NG), sn0 = next_scale(grp + 2 * NG), sn1 = next_scale(grp + 3 * NG);
+      const uint32_t row0 = raw_smem + (WK == WK_W4N ? t * 128 + (((4 * half) ^ sw) << 4) : t * 4 + half * 16 * 512);
+      const uint32_t ta0 = tmem + ((uint32_t)((warp & 3) * 32) << 16) + Cfg::A_COL0;
+      const bool elected = lane == 0;
+      const MagicConsts mk = p.mk;
+      bool odd = false;
+      int pend = -1;                                 // operand stage whose tensor-memory stores are still in flight
+#pragma unroll 1
+      for (int gg = grp; gg < ngroups; gg += NG) {
+        const uint32_t sr = odd ? sq1 : sq0;
+        if (odd) {
+          sq0 = sn0; sq1 = sn1;
+          sn0 = next_scale(gg + 3 * NG); sn1 = next_scale(gg + 4 * NG);
+        }
+        odd = !odd;
+        float ss = (p.scale_dtype == B2Q_F32 ? __uint_as_float(sr)
+                    : p.scale_dtype == B2Q_BF16 ? __uint_as_float(sr << 16) : __half2float(__ushort_as_half((unsigned short)sr))) * row_mul;
+        if (fabsf(ss) > 8188.f) { ss = copysignf(8188.f, ss); saturated = 1; }   // 8 * scale would leave fp16: saturate, and say so (after the loop)
+        const uint32_t hv = __half_as_ushort(__float2half_rn(ss));
+        const uint32_t m2 = hv | (hv << 16);
+        ok = mbar_wait(raw_full + 8 * rs, rpar, abort_flag, p.status, ST_RAWFULL);
+        if (!ok) break;
+        const uint32_t rowa = row0 + rs * Cfg::RAW_BYTES;
+#pragma unroll
+        for (int q = 0; q < 4; ++q) {                // quarters of 32 k: 16 registers live, half an operand stage
+          uint32_t w0, w1, w2, w3;
+          if constexpr (WK == WK_W4N) {
+            const uint4 rr = lds128(rowa ^ (q << 4));
+            w0 = rr.x; w1 = rr.y; w2 = rr.z; w3 = rr.w;
+          } else {
+            w0 = lds32(rowa + (4 * q + 0) * 512); w1 = lds32(rowa + (4 * q + 1) * 512);
+            w2 = lds32(rowa + (4 * q + 2) * 512); w3 = lds32(rowa + (4 * q + 3) * 512);
+          }
+          if (q == 3) { __syncwarp(); if (elected) mbar_arrive(raw_empty + 8 * rs); }       // last read of this half
+          uint32_t a16[16];
+          { uint32_t o[4]; w4_word_magic(w0, m2, mk, o); a16[0] = o[0]; a16[1] = o[1]; a16[2] = o[2]; a16[3] = o[3]; }
+          { uint32_t o[4]; w4_word_magic(w1, m2, mk, o); a16[4] = o[0]; a16[5] = o[1]; a16[6] = o[2]; a16[7] = o[3]; }
+          { uint32_t o[4]; w4_word_magic(w2, m2, mk, o); a16[8] = o[0]; a16[9] = o[1]; a16[10] = o[2]; a16[11] = o[3]; }
+          { uint32_t o[4]; w4_word_magic(w3, m2, mk, o); a16[12] = o[0]; a16[13] = o[1]; a16[14] = o[2]; a16[15] = o[3]; }
+          if ((q & 1) == 0) {
+            // The previous stage's stores have had this quarter's conversion to complete: only now are they waited for
+            // and the stage handed to the MMA warp.  Waiting right behind the store would leave the warp idle for the
+            // store's whole latency.
+            const int prev = q == 0 ? pend : as;
+            if (q != 0 || prev >= 0) { tmem_st_wait(); tc_fence_before(); __syncwarp(); if (elected) mbar_arrive(a_full + 8 * prev); }
+            // no test for the ring's first round: a wait for the phase before a fresh barrier's first one returns at once
+            ok = mbar_wait(ab_empty + 8 * (as + (q >> 1)), apar, abort_flag, p.status, ST_EMPTY);
+            if (!ok) break;
+            tc_fence_after();
+          }
+          tmem_st16(ta0 + 32 * (as + (q >> 1)) + 16 * (q & 1), a16);
+        }
+        if (!ok) break;
+        pend = as + 1;
+        rs += RAW_STEP; if (rs >= RS) { rs -= RS; rpar ^= 1u; }
+        as += A_STEP % S; apar ^= (uint32_t)(A_STEP / S) & 1u;
+        if (as >= S) { as -= S; apar ^= 1u; }
+      }
+      if (ok && pend >= 0) { tmem_st_wait(); tc_fence_before(); __syncwarp(); if (elected) mbar_arrive(a_full + 8 * pend); }
+    } else {
+    uint32_t sq0 = chunk_scale_raw(grp), sq1 = chunk_scale_raw(grp + NG), sq2 = chunk_scale_raw(grp + 2 * NG),
+             sq3 = chunk_scale_raw(grp + 3 * NG);
+    uint32_t sn0 = chunk_scale_raw(grp + 4 * NG), sn1 = chunk_scale_raw(grp + 5 * NG), sn2 = chunk_scale_raw(grp + 6 * NG),
+             sn3 = chunk_scale_raw(grp + 7 * NG);
+    int it4 = 0;                                   // position of the current chunk in its set of four
     // Position in the raw ring: by counting (this group converts CPG chunks of every raw stage, a segment starts on a
     // stage boundary, jj counts them) or by dividing the chunk number by the stage count for every chunk.  Which is
     // faster is a matter of what the register allocator makes of the loop, measured per tile width on one GPU: the
@@ -495,40 +581,7 @@ umma_wo_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constant__
         { ok = mbar_wait(ab_empty + 8 * s, ((g / S) + 1) & 1, abort_flag, p.status, ST_EMPTY); if (!ok) break; }
         tc_fence_after();
         const uint32_t ta = tmem + ((uint32_t)((warp & 3) * 32) << 16) + Cfg::A_COL0 + 32 * s;
-        if constexpr (MAGIC) {
-          // fp16 magic-number route.  The chunk goes to tensor memory in two halves of 32 k (16 registers each): with
-          // all 64 values of a row live at once the loop ran out of registers, and the decode's masks and fp16
-          // constants were re-created for every use.
-          float ss = sc_cur * row_mul;
-          const bool too_big = fabsf(ss) > 8188.f;            // 8 * scale would leave fp16: saturate, and say so (after the loop)
-          ss = too_big ? copysignf(8188.f, ss) : ss;
-          saturated |= too_big ? 1 : 0;
-          const uint32_t hv = __half_as_ushort(__float2half_rn(ss));
-          const uint32_t m2 = hv | (hv << 16);
-          const MagicConsts mk = p.mk;
-#pragma unroll
-          for (int hf = 0; hf < 2; ++hf) {
-            uint32_t w0, w1, w2, w3;
-            if constexpr (WK == WK_W4N) {
-              const uint4 rr = lds128(rawrow + (((2 * j + hf) ^ sw) << 4));
-              w0 = rr.x; w1 = rr.y; w2 = rr.z; w3 = rr.w;
-            } else {
-              w0 = lds32(rawcol + (8 * j + 4 * hf + 0) * 512); w1 = lds32(rawcol + (8 * j + 4 * hf + 1) * 512);
-              w2 = lds32(rawcol + (8 * j + 4 * hf + 2) * 512); w3 = lds32(rawcol + (8 * j + 4 * hf + 3) * 512);
-            }
-            uint32_t a16[16];
-            { uint32_t o[4]; w4_word_magic(w0, m2, mk, o); a16[0] = o[0]; a16[1] = o[1]; a16[2] = o[2]; a16[3] = o[3]; }
-            { uint32_t o[4]; w4_word_magic(w1, m2, mk, o); a16[4] = o[0]; a16[5] = o[1]; a16[6] = o[2]; a16[7] = o[3]; }
-            { uint32_t o[4]; w4_word_magic(w2, m2, mk, o); a16[8] = o[0]; a16[9] = o[1]; a16[10] = o[2]; a16[11] = o[3]; }
-            { uint32_t o[4]; w4_word_magic(w3, m2, mk, o); a16[12] = o[0]; a16[13] = o[1]; a16[14] = o[2]; a16[15] = o[3]; }
-            // The previous chunk's stores have had this half's conversion to complete: only now are they waited for and
-            // the chunk handed to the MMA warp.  Waiting right behind the store would leave the warp idle for the
-            // store's whole latency, once per chunk.
-            if (hf == 0 && pend >= 0) { tmem_st_wait(); tc_fence_before(); mbar_arrive(a_full + 8 * pend); }
-            tmem_st16(ta + 16 * hf, a16);
-          }
-          pend = s;
-        } else {
+        {
         uint32_t av[32];                         // this row's 64 values of the chunk, two per register, k ascending
         if constexpr (WK == WK_W4N || WK == WK_W4K) {
           uint32_t s2 = 0; float sf = 0.f;
@@ -608,7 +661,7 @@ umma_wo_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constant__
         if (c + NG >= nk || (c + NG) / CPR != c / CPR) mbar_arrive(raw_empty + 8 * rs);
       }
     }
-    if (pend >= 0) { tmem_st_wait(); tc_fence_before(); mbar_arrive(a_full + 8 * pend); pend = -1; }
+    }
     if (saturated) atomicCAS(p.status, 0, ST_SCALERANGE);
     if (!ok) break;
 
