@@ -63,11 +63,17 @@ static inline size_t ws_i8_bytes(int64_t M, int64_t K) {
          align_up((size_t)(K / 128) * 16 * 4, 256) + umma_w4_i8_partial_bytes();
 }
 
+static inline size_t partial_sum_bytes(int64_t M) {
+  const size_t a = umma_balanced_ws_bytes(M), b = umma_w4_partial_bytes(M);
+  return a > b ? a : b;
+}
+
 template <class Args>
 static void give_balanced_scratch(Args& ua, void* workspace, int64_t M, int64_t K) {
-  if (M > 64) return;
+  const size_t bytes = partial_sum_bytes(M);
+  if (!bytes) return;
   ua.sk_ws = reinterpret_cast<uint8_t*>(workspace) + ws_prep_bytes(M, K);
-  ua.sk_ws_bytes = umma_balanced_ws_bytes(M);
+  ua.sk_ws_bytes = bytes;
 }
 
 }  // namespace b2q
@@ -302,7 +308,7 @@ int b2q_linear_int4_allreduce(const void* x, int act_dtype, int64_t ldx, const v
 
 size_t b2q_linear_workspace_bytes(int64_t M, int64_t N, int64_t K) {
   (void)N;
-  const size_t a = ws_prep_bytes(M, K) + umma_balanced_ws_bytes(M), b = ws_i8_bytes(M, K);
+  const size_t a = ws_prep_bytes(M, K) + partial_sum_bytes(M), b = ws_i8_bytes(M, K);
   return a > b ? a : b;
 }
 size_t b2q_linear_fp8_workspace_bytes(int64_t M, int64_t N, int64_t K) {

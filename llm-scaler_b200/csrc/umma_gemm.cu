@@ -30,24 +30,15 @@ namespace b2q {
 using namespace sm100;
 
 __device__ int g_umma_status = 0;
-constexpr int SK_BANKS = 64, SK_MAX_STRIPS = 1024;
+constexpr int SK_BANKS = 64, SK_MAX_STRIPS = UMMA_MAX_CUT_STRIPS;
 __device__ int g_sk_counters[SK_BANKS * SK_MAX_STRIPS];     // arrival counters of cut strips (see "balanced mode" below)
 
 enum { WK_W4N = 0, WK_W4K = 1, WK_W8 = 2 };
-enum { ST_XFULL = 101, ST_AFULL = 102, ST_EMPTY = 103, ST_RAWFULL = 104, ST_RAWEMPTY = 105, ST_ACCUM = 106, ST_ACCEMPTY = 107, ST_FIXUP = 108, ST_SCALERANGE = 109 };
+enum { ST_XFULL = 101, ST_AFULL = 102, ST_EMPTY = 103, ST_RAWFULL = 104, ST_RAWEMPTY = 105, ST_ACCUM = 106, ST_ACCEMPTY = 107, ST_FIXUP = 108 };
 
 // One piece of a CTA's work: 64-k chunks [c_begin, c_begin + nk) of the strip of 128 weight rows at n0.
 // part = the strip's other chunks belong to other CTAs; slot = which of the CTA's two partial-sum slots it uses.
 struct Segment { int n0, c_begin, nk, strip, part, slot; };
-
-// constants of the fp16 magic-number nibble decode, handed to the kernel as parameters (see w4_word_magic)
-struct MagicConsts { uint32_t magic_lo, magic_hi, m72; };
-// twos: the nibbles are two's complement (value, not value + 8).  Flipping their sign bits gives the offset form; the
-// flip is folded into the constant that is merged in: (w & m) ^ (0x6400 ^ flip) is 0x6400 | ((w ^ flip) & m) because
-// the 0x6400 bits and the nibble bits do not overlap.  No extra operation, no branch in the decode.
-__host__ __device__ inline MagicConsts magic_consts(bool twos) {
-  return MagicConsts{0x64006400u ^ (twos ? 0x00080008u : 0u), 0x64006400u ^ (twos ? 0x00800080u : 0u), 0xD480D480u};
-}
 
 struct UmmaWoParams {
   const void* scale; int scale_dtype; int scale_mode;      // scale_mode: B2Q_SCALE_* (fp8) ; ignored for int4
@@ -60,14 +51,12 @@ struct UmmaWoParams {
   int* sk_counters;          // balanced mode: arrivals per strip, zero between launches
   int sk_grid;               // host side only: CTAs of a balanced launch
   int tiles_on_y;            // grouped launches: tile index on blockIdx.y, strip on blockIdx.x (see the kernel)
-  int magic;                 // INT4: fp16 magic-number transform; x was permuted / scaled by the pre-pass
   const int32_t* tiles; const int32_t* expert_offsets; const int32_t* out_map;
   int w_rows_per_expert;     // tensor-map rows per expert: N (N-major) or K/8 (K-major)
   const float* tok_scale;    // optional per-token output multiplier (undoes the activation pre-scale)
   int out_bf16;              // output element type (may differ from the MMA input type)
   int overlap_ok;            // host side only: launch with programmatic stream serialization
   int* status;
-  MagicConsts mk;            // constants of the fp16 magic-number nibble decode (see w4_word_magic)
   int peer_on;               // decode tiles only: the output tile goes to the owner ranks' reduction slots (peer memory)
   PeerEpilogue peer;
 };
@@ -122,18 +111,6 @@ __device__ __forceinline__ void w4_word(uint32_t w, uint32_t s2, float sf, bool 
   }
 }
 
-// fp16 magic-number variant: 0x6400 | q is 1024 + q and 0x6400 | (q << 4) is 1024 + 16 q, so the nibbles at
-// bits 0-3 / 4-7 of each half-word need no shift; one shift by 8 reaches the other four.  The result
-// (q - 8) * s is rounded to fp16 once.  Output pair order: (n0,n4) (n1,n5) (n2,n6) (n3,n7) where n_i is the
-// nibble at bits 4i; the activation pre-pass stores x in the matching order.  Integer work per word: one
-// shift and four LOP3 (the ALU pipe, not the FP pipes, is what bounds the int4 transform).
-// Where the constants live matters more than the arithmetic.  All of them as literals: the compiler folds them into
-// immediates, and since an instruction takes one immediate at most it then spends two logic operations per
-// mask-and-merge and a register move per fused multiply-add (measured: 82 logic operations and 61 moves per 64 k of a
-// row where 32 and a handful are needed).  All of them as kernel parameters: seven registers held through a loop that
-// has none to spare.  Hence one of each instruction's two constants as an immediate, the other in a register
-// (and_xor_lo / and_xor_hi / w4_word_magic below).
-
 // a, b, c or d for i = 0, 1, 2, anything else: three compares and three selects, never a branch (written as a
 // conditional expression the selection of a chunk's prefetched scale became a jump table with a dozen register moves)
 __device__ __forceinline__ uint32_t sel4(int i, uint32_t a, uint32_t b, uint32_t c, uint32_t d) {
@@ -143,33 +120,6 @@ __device__ __forceinline__ uint32_t sel4(int i, uint32_t a, uint32_t b, uint32_t
       : "=&r"(r) : "r"(i), "r"(a), "r"(b), "r"(c), "r"(d));
   return r;
 }
-__device__ __forceinline__ uint32_t and_xor_lo(uint32_t a, uint32_t c) {      // (a & 0x000F000F) ^ c: the mask as an immediate, c in a register
-  uint32_t d;
-  asm("lop3.b32 %0, %1, 0x000F000F, %2, 0x6A;" : "=r"(d) : "r"(a), "r"(c));
-  return d;
-}
-__device__ __forceinline__ uint32_t and_xor_hi(uint32_t a, uint32_t c) {      // (a & 0x00F000F0) ^ c
-  uint32_t d;
-  asm("lop3.b32 %0, %1, 0x00F000F0, %2, 0x6A;" : "=r"(d) : "r"(a), "r"(c));
-  return d;
-}
-// An instruction takes ONE immediate: the masks, 1032 and 1/16 are written as literals, the merge constants (which depend
-// on the nibble encoding) and -72 come in registers.  Three registers of constants instead of seven.
-__device__ __forceinline__ void w4_word_magic(uint32_t w, uint32_t s2, const MagicConsts& k, uint32_t (&o)[4]) {
-  const uint32_t w8 = w >> 8;
-  uint32_t v[4] = {and_xor_lo(w, k.magic_lo), and_xor_hi(w, k.magic_hi), and_xor_lo(w8, k.magic_lo), and_xor_hi(w8, k.magic_hi)};
-  const __half2 sc = *reinterpret_cast<const __half2*>(&s2);
-#pragma unroll
-  for (int i = 0; i < 4; ++i) {
-    __half2 h = *reinterpret_cast<__half2*>(&v[i]);
-    const uint32_t c_r16 = 0x2C002C00u, c_1032 = 0x64086408u;
-    if (i & 1) h = __hfma2(h, *reinterpret_cast<const __half2*>(&c_r16), *reinterpret_cast<const __half2*>(&k.m72));      // h / 16 - 72
-    else h = __hsub2(h, *reinterpret_cast<const __half2*>(&c_1032));                                                     // h - 1032
-    h = __hmul2(h, sc);
-    o[i] = *reinterpret_cast<uint32_t*>(&h);
-  }
-}
-
 // Four fp8 bytes -> four 16-bit values in k order.  SCALED folds an fp32 scale in (one rounding);
 // otherwise bf16 results carry an exact 2^-112 that the epilogue removes.
 template <bool BF16, bool SCALED>
@@ -219,20 +169,16 @@ template <int TOK> struct UmmaCfg {
   // Operand stages (32 columns each) fill the rest of the allocation: a stage is only reusable once
   // the MMAs that read it have completed and signalled, a round trip of a couple of microseconds, so
   // the ring has to be deep for the transform warps to stay busy.
-  static constexpr int S = ((TMEM_COLS - A_COL0) / 32 > 12 ? 12 : (TMEM_COLS - A_COL0) / 32) & ~1;
+  static constexpr int S = (TMEM_COLS - A_COL0) / 32 > 12 ? 12 : (TMEM_COLS - A_COL0) / 32;
 };
 
-// MAGIC: INT4 weights behind the activation pre-pass (fp16 activations in the nibble decode's pair order): its own
-// instantiation so that the decode loop carries none of the other routes' code or registers.
-template <int WK, bool BF16, int TOK, bool FAST, bool MAGIC>
+template <int WK, bool BF16, int TOK, bool FAST>
 __global__ void __launch_bounds__(UmmaCfg<TOK>::THREADS, UmmaCfg<TOK>::CTAS)
 umma_wo_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constant__ CUtensorMap tm_x, const UmmaWoParams p) {
   using Cfg = UmmaCfg<TOK>;
   constexpr int S = Cfg::S, RS = Cfg::RS, NG = Cfg::NG, XS = Cfg::XS;
   constexpr int CPR = (WK == WK_W8) ? 2 : 4;          // 64-k chunks per raw stage
-  // transform groups that touch one raw stage, and the arrivals each of them makes there and on an operand stage
-  constexpr int GPR = MAGIC ? 2 : (CPR < NG ? CPR : NG);
-  constexpr int GRP_ARRIVALS = MAGIC ? 4 : 128;
+  constexpr int GPR = CPR < NG ? CPR : NG;            // transform groups that touch one raw stage
   // With equally deep rings chunk g uses operand stage g % S and activation stage g % XS = the same index, and the MMAs
   // that free one free the other: the activation producer waits on the operand stage's barrier, the issuer commits once
   // (MoE pipeline 676 -> 664 us; the decode tiles are indifferent).
@@ -304,9 +250,9 @@ umma_wo_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constant__
   const int64_t sbase = (int64_t)expert * p.s_expert_elems;
 
   if (threadIdx.x == 0) {
-    for (int i = 0; i < S; ++i) { mbar_init(a_full + 8 * i, GRP_ARRIVALS); mbar_init(ab_empty + 8 * i, 1); }
+    for (int i = 0; i < S; ++i) { mbar_init(a_full + 8 * i, 128); mbar_init(ab_empty + 8 * i, 1); }
     for (int i = 0; i < XS; ++i) { mbar_init(x_full + 8 * i, 1); mbar_init(x_empty + 8 * i, 1); }
-    for (int i = 0; i < RS; ++i) { mbar_init(raw_full + 8 * i, 1); mbar_init(raw_empty + 8 * i, GPR * GRP_ARRIVALS); }
+    for (int i = 0; i < RS; ++i) { mbar_init(raw_full + 8 * i, 1); mbar_init(raw_empty + 8 * i, GPR * 128); }
     mbar_init(accum_full, Cfg::NMMA);
     mbar_init(accum_empty, NG * 128);
     mbar_init(fix_bar, NG * 128);
@@ -435,110 +381,6 @@ umma_wo_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constant__
         return __uint_as_float(raw);
       }
     };
-    int saturated = 0;                             // MAGIC: a scale had to be clamped (reported once, behind the loop)
-    // fp16 magic route with bf16 / fp32 scales: the group scale is rounded to fp16, whose normal range starts at
-    // 6.1e-5.  Every row of a segment therefore carries its own power of two, taken from the scale of the segment's
-    // first group: the row's scales are multiplied by 2^row_e so that this first one lands in [0.5, 1), and the fp32
-    // accumulator row is multiplied by 2^-row_e when it is read ((q - 8) * s needs 11 bits at most, so the fp16
-    // operand stays exact).  Groups within 2^13 of the first one, either way, are exact; one further above would
-    // overflow fp16 and is saturated and reported through the status word (ST_SCALERANGE).
-    float row_mul = 1.f, row_post = 1.f;
-    if constexpr (MAGIC) {
-      if (p.scale_dtype != B2Q_F16) {
-        const int ex = (int)((__float_as_uint(scale_value(chunk_scale_raw(0))) >> 23) & 0xFFu);   // biased exponent; 0 = zero / subnormal, 255 = inf / nan
-        if (ex != 0 && ex != 255) {
-          int k = 126 - ex;
-          k = k > 120 ? 120 : (k < -120 ? -120 : k);
-          row_mul = __uint_as_float((uint32_t)(127 + k) << 23);
-          row_post = __uint_as_float((uint32_t)(127 - k) << 23);
-        }
-      }
-    }
-    if constexpr (MAGIC) {
-      // One iteration converts one scale group: 128 k of a row = two operand stages of 64 k, half of a raw stage.  The
-      // groups of four warps take the scale groups in turn, so a thread always works on the same half of a raw stage and
-      // every ring position advances by a constant.  What a chunk costs besides its decode (two barrier waits, ring
-      // arithmetic, scale fetch / conversion / range check, arrivals: 265 of 370 issue slots per 64 k when all of it was
-      // done per chunk by division and selection) is most of what this loop cost, so it is paid per 128 k and by counting, and
-      // barriers take one arrival per warp.  Measured: decoder layer at M = 64 299 -> 262 us, MoE pipeline at 4096 tokens
-      // 702 -> 667 us, decoder layer at M = 2048 3138 -> 3072 us.
-      static_assert(!MAGIC || (S % 2 == 0 && NG % 2 == 0 && CPR == 4), "a scale group is two operand stages, half a raw stage");
-      constexpr int RAW_STEP = NG / 2, A_STEP = 2 * NG;
-      const int ngroups = nk >> 1, half = grp & 1;
-      const int raw0 = grb + (grp >> 1), a0 = gb + 2 * grp;
-      int rs = raw0 % RS, as = a0 % S;
-      uint32_t rpar = (uint32_t)(raw0 / RS) & 1u, apar = ((uint32_t)(a0 / S) + 1u) & 1u;
-      const int esz = p.scale_dtype == B2Q_F32 ? 4 : 2;
-      const uint8_t* sp = reinterpret_cast<const uint8_t*>(p.scale) +
-                          (sbase + (int64_t)nrow * p.s_stride_n + (int64_t)((c_begin >> 1) + grp) * p.s_stride_g) * esz;
-      const int64_t sstep = (int64_t)NG * p.s_stride_g * esz;
-      auto next_scale = [&](int gg) -> uint32_t {           // raw bits of group gg's scale; sp walks along with the calls
-        uint32_t v = 0u;
-        if (gg < ngroups) v = esz == 4 ? __ldg(reinterpret_cast<const uint32_t*>(sp)) : (uint32_t)__ldg(reinterpret_cast<const unsigned short*>(sp));
-        sp += sstep;
-        return v;
-      };
-      // two scales in use, two in flight: requested two to three iterations ahead, untouched until their turn
-      uint32_t sq0 = next_scale(grp), sq1 = next_scale(grp + NG), sn0 = next_scale(grp + 2 * NG), sn1 = next_scale(grp + 3 * NG);
-      const uint32_t row0 = raw_smem + (WK == WK_W4N ? t * 128 + (((4 * half) ^ sw) << 4) : t * 4 + half * 16 * 512);
-      const uint32_t ta0 = tmem + ((uint32_t)((warp & 3) * 32) << 16) + Cfg::A_COL0;
-      const bool elected = lane == 0;
-      const MagicConsts mk = p.mk;
-      bool odd = false;
-      int pend = -1;                                 // operand stage whose tensor-memory stores are still in flight
-#pragma unroll 1
-      for (int gg = grp; gg < ngroups; gg += NG) {
-        const uint32_t sr = odd ? sq1 : sq0;
-        if (odd) {
-          sq0 = sn0; sq1 = sn1;
-          sn0 = next_scale(gg + 3 * NG); sn1 = next_scale(gg + 4 * NG);
-        }
-        odd = !odd;
-        float ss = (p.scale_dtype == B2Q_F32 ? __uint_as_float(sr)
-                    : p.scale_dtype == B2Q_BF16 ? __uint_as_float(sr << 16) : __half2float(__ushort_as_half((unsigned short)sr))) * row_mul;
-        if (fabsf(ss) > 8188.f) { ss = copysignf(8188.f, ss); saturated = 1; }   // 8 * scale would leave fp16: saturate, and say so (after the loop)
-        const uint32_t hv = __half_as_ushort(__float2half_rn(ss));
-        const uint32_t m2 = hv | (hv << 16);
-        ok = mbar_wait(raw_full + 8 * rs, rpar, abort_flag, p.status, ST_RAWFULL);
-        if (!ok) break;
-        const uint32_t rowa = row0 + rs * Cfg::RAW_BYTES;
-#pragma unroll
-        for (int q = 0; q < 4; ++q) {                // quarters of 32 k: 16 registers live, half an operand stage
-          uint32_t w0, w1, w2, w3;
-          if constexpr (WK == WK_W4N) {
-            const uint4 rr = lds128(rowa ^ (q << 4));
-            w0 = rr.x; w1 = rr.y; w2 = rr.z; w3 = rr.w;
-          } else {
-            w0 = lds32(rowa + (4 * q + 0) * 512); w1 = lds32(rowa + (4 * q + 1) * 512);
-            w2 = lds32(rowa + (4 * q + 2) * 512); w3 = lds32(rowa + (4 * q + 3) * 512);
-          }
-          if (q == 3) { __syncwarp(); if (elected) mbar_arrive(raw_empty + 8 * rs); }       // last read of this half
-          uint32_t a16[16];
-          { uint32_t o[4]; w4_word_magic(w0, m2, mk, o); a16[0] = o[0]; a16[1] = o[1]; a16[2] = o[2]; a16[3] = o[3]; }
-          { uint32_t o[4]; w4_word_magic(w1, m2, mk, o); a16[4] = o[0]; a16[5] = o[1]; a16[6] = o[2]; a16[7] = o[3]; }
-          { uint32_t o[4]; w4_word_magic(w2, m2, mk, o); a16[8] = o[0]; a16[9] = o[1]; a16[10] = o[2]; a16[11] = o[3]; }
-          { uint32_t o[4]; w4_word_magic(w3, m2, mk, o); a16[12] = o[0]; a16[13] = o[1]; a16[14] = o[2]; a16[15] = o[3]; }
-          if ((q & 1) == 0) {
-            // The previous stage's stores have had this quarter's conversion to complete: only now are they waited for
-            // and the stage handed to the MMA warp.  Waiting right behind the store would leave the warp idle for the
-            // store's whole latency.
-            const int prev = q == 0 ? pend : as;
-            if (q != 0 || prev >= 0) { tmem_st_wait(); tc_fence_before(); __syncwarp(); if (elected) mbar_arrive(a_full + 8 * prev); }
-            // no test for the ring's first round: a wait for the phase before a fresh barrier's first one returns at once
-            ok = mbar_wait(ab_empty + 8 * (as + (q >> 1)), apar, abort_flag, p.status, ST_EMPTY);
-            if (!ok) break;
-            tc_fence_after();
-          }
-          tmem_st16(ta0 + 32 * (as + (q >> 1)) + 16 * (q & 1), a16);
-        }
-        if (!ok) break;
-        pend = as + 1;
-        rs += RAW_STEP; if (rs >= RS) { rs -= RS; rpar ^= 1u; }
-        as += A_STEP % S; apar ^= (uint32_t)(A_STEP / S) & 1u;
-        if (as >= S) { as -= S; apar ^= 1u; }
-      }
-      if (ok && pend >= 0) { tmem_st_wait(); tc_fence_before(); __syncwarp(); if (elected) mbar_arrive(a_full + 8 * pend); }
-    } else {
     uint32_t sq0 = chunk_scale_raw(grp), sq1 = chunk_scale_raw(grp + NG), sq2 = chunk_scale_raw(grp + 2 * NG),
              sq3 = chunk_scale_raw(grp + 3 * NG);
     uint32_t sn0 = chunk_scale_raw(grp + 4 * NG), sn1 = chunk_scale_raw(grp + 5 * NG), sn2 = chunk_scale_raw(grp + 6 * NG),
@@ -587,7 +429,8 @@ umma_wo_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constant__
           uint32_t s2 = 0; float sf = 0.f;
           if constexpr (FAST) {
             // the scale has the activation's 16-bit type here, so float -> 16 bit gives back its stored bits
-            if (!p.magic) { const uint32_t sv = BF16 ? __bfloat16_as_ushort(__float2bfloat16_rn(sc_cur)) : __half_as_ushort(__float2half_rn(sc_cur)); s2 = sv | (sv << 16); }
+            const uint32_t sv = BF16 ? __bfloat16_as_ushort(__float2bfloat16_rn(sc_cur)) : __half_as_ushort(__float2half_rn(sc_cur));
+            s2 = sv | (sv << 16);
           } else sf = sc_cur;
           uint32_t ww[8];
           bool marlin = false;
@@ -661,8 +504,6 @@ umma_wo_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constant__
         if (c + NG >= nk || (c + NG) / CPR != c / CPR) mbar_arrive(raw_empty + 8 * rs);
       }
     }
-    }
-    if (saturated) atomicCAS(p.status, 0, ST_SCALERANGE);
     if (!ok) break;
 
     // ---------------- epilogue of this segment ----------------
@@ -736,12 +577,6 @@ umma_wo_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constant__
         tmem_ld_wait();
 #pragma unroll
         for (int i = 0; i < CB; ++i) r[i] = __float_as_uint(__uint_as_float(r[i]) + __uint_as_float(q[i]));
-      }
-      if constexpr (MAGIC) {
-        if (row_post != 1.f) {
-#pragma unroll
-          for (int i = 0; i < CB; ++i) r[i] = __float_as_uint(__uint_as_float(r[i]) * row_post);
-        }
       }
       // balanced mode has one column block per thread at most: the accumulators are free for the next segment now
       if (BAL && balanced && !freed) { tc_fence_before(); mbar_arrive(accum_empty); freed = true; }
@@ -867,6 +702,8 @@ static int* status_ptr() {
   return ptr[dev];
 }
 
+int* umma_status_ptr() { return status_ptr(); }
+
 // Self-test of the bounded-wait machinery: one CTA waits on an mbarrier that nobody ever arrives on, with a limit of
 // about a millisecond instead of two seconds.  The wait must give up, record `code` in the status word and return;
 // the context stays usable.  Nothing here faults or spins without bound.
@@ -945,6 +782,8 @@ static int* sk_counter_bank() {
   return basep[dev] + (size_t)(next_bank.fetch_add(1, std::memory_order_relaxed) % SK_BANKS) * SK_MAX_STRIPS;
 }
 
+int* umma_strip_counters() { return sk_counter_bank(); }
+
 static int device_slots() {
   static thread_local int sms[16] = {0};
   int dev = 0;
@@ -987,12 +826,12 @@ static int plan_balanced(UmmaWoParams& p, const UmmaGroupArgs& a, int M, int N, 
 
 static int pick_tok(int m) { return m <= 16 ? 16 : (m <= 32 ? 32 : (m <= 64 ? 64 : (m <= 128 ? 128 : 256))); }
 
-template <int WK, bool BF16, int TOK, bool FAST, bool MAGIC>
+template <int WK, bool BF16, int TOK, bool FAST>
 static int launch_one(const CUtensorMap& tw, const CUtensorMap& tx, const UmmaWoParams& p_in, int token_tiles, cudaStream_t st) {
   UmmaWoParams p = p_in;
   p.tiles_on_y = (p.tiles && token_tiles <= 65535) ? 1 : 0;      // gridDim.y is limited to 65535
   using Cfg = UmmaCfg<TOK>;
-  auto kern = umma_wo_kernel<WK, BF16, TOK, FAST, MAGIC>;
+  auto kern = umma_wo_kernel<WK, BF16, TOK, FAST>;
   static thread_local bool configured[16] = {false};
   int dev = 0;
   cudaGetDevice(&dev);
@@ -1009,14 +848,14 @@ static int launch_one(const CUtensorMap& tw, const CUtensorMap& tx, const UmmaWo
   return launch_status();
 }
 
-template <int WK, bool BF16, bool FAST, bool MAGIC = false>
+template <int WK, bool BF16, bool FAST>
 static int launch_tok(int tok, const CUtensorMap& tw, const CUtensorMap& tx, const UmmaWoParams& p, int tiles, cudaStream_t st) {
   switch (tok) {
-    case 16: return launch_one<WK, BF16, 16, FAST, MAGIC>(tw, tx, p, tiles, st);
-    case 32: return launch_one<WK, BF16, 32, FAST, MAGIC>(tw, tx, p, tiles, st);
-    case 64: return launch_one<WK, BF16, 64, FAST, MAGIC>(tw, tx, p, tiles, st);
-    case 128: return launch_one<WK, BF16, 128, FAST, MAGIC>(tw, tx, p, tiles, st);
-    default: return launch_one<WK, BF16, 256, FAST, MAGIC>(tw, tx, p, tiles, st);
+    case 16: return launch_one<WK, BF16, 16, FAST>(tw, tx, p, tiles, st);
+    case 32: return launch_one<WK, BF16, 32, FAST>(tw, tx, p, tiles, st);
+    case 64: return launch_one<WK, BF16, 64, FAST>(tw, tx, p, tiles, st);
+    case 128: return launch_one<WK, BF16, 128, FAST>(tw, tx, p, tiles, st);
+    default: return launch_one<WK, BF16, 256, FAST>(tw, tx, p, tiles, st);
   }
 }
 
@@ -1041,12 +880,16 @@ bool umma_w4_supported(const UmmaW4Args& a) {
   if (a.row_map) return false;                             // rows are gathered by the caller first
   return tensor_map_encoder() != nullptr && status_ptr() != nullptr;
 }
-int umma_w4_token_tile(const UmmaW4Args& a) { return a.expert_offsets ? grouped_tok(a.M, a.E) : pick_tok(a.M); }
+int umma_w4_token_tile(const UmmaW4Args& a) {
+  if (a.magic) return umma_w4_prep_token_tile(a);
+  return a.expert_offsets ? grouped_tok(a.M, a.E) : pick_tok(a.M);
+}
 
 int umma_w4_linear(const UmmaW4Args& a, cudaStream_t st) {
   const bool kmajor = a.layout == B2Q_W4_KMAJOR || a.layout == B2Q_W4_KMAJOR_MARLIN;
   const bool grouped = a.expert_offsets != nullptr;
   const int E = grouped ? a.E : 1;
+  if (a.magic) return umma_w4_prep_linear(a, st);
   const int tok = umma_w4_token_tile(a);
   CUtensorMap tw, tx;
   int rc;
@@ -1068,8 +911,7 @@ int umma_w4_linear(const UmmaW4Args& a, cudaStream_t st) {
   p.marlin = a.layout == B2Q_W4_KMAJOR_MARLIN; p.xor_mask = a.layout == B2Q_W4_NMAJOR_S4 ? 0x88888888u : 0u;
   p.tiles = grouped ? a.tiles : nullptr; p.expert_offsets = a.expert_offsets; p.out_map = a.out_map;
   p.w_rows_per_expert = kmajor ? a.K / 8 : a.N;
-  p.tok_scale = a.tok_scale; p.out_bf16 = a.out_bf16 ? 1 : 0; p.magic = a.magic ? 1 : 0;
-  p.mk = magic_consts(p.xor_mask != 0);
+  p.tok_scale = a.tok_scale; p.out_bf16 = a.out_bf16 ? 1 : 0;
   p.status = status_ptr();
   p.overlap_ok = (a.after_prep || tls().overlap_mode == 2) ? 1 : 0;
   p.sk_grid = plan_balanced(p, a, a.M, a.N, a.K, 4, tok);
@@ -1077,13 +919,8 @@ int umma_w4_linear(const UmmaW4Args& a, cudaStream_t st) {
     if (tok > 64 || grouped || (a.N % 128) != 0 || (a.peer->slice % 128) != 0 || a.peer->M != a.M) return B2Q_ERR_UNSUPPORTED;
     p.peer_on = 1; p.peer = *a.peer;
   }
-  const bool fast = a.magic || (a.scale_dtype == (a.bf16 ? B2Q_BF16 : B2Q_F16));
+  const bool fast = a.scale_dtype == (a.bf16 ? B2Q_BF16 : B2Q_F16);
   const int tiles = grouped ? a.tile_cap : (a.M + tok - 1) / tok;
-  if (a.magic) {
-    if (a.bf16) return B2Q_ERR_UNSUPPORTED;       // the pre-pass always hands over fp16
-    return kmajor ? launch_tok<WK_W4K, false, true, true>(tok, tw, tx, p, tiles, st)
-                  : launch_tok<WK_W4N, false, true, true>(tok, tw, tx, p, tiles, st);
-  }
   return kmajor ? launch_wk<WK_W4K>(a.bf16, fast, tok, tw, tx, p, tiles, st)
                 : launch_wk<WK_W4N>(a.bf16, fast, tok, tw, tx, p, tiles, st);
 }

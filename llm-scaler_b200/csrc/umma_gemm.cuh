@@ -79,6 +79,16 @@ bool umma_w4_supported(const UmmaW4Args& a);
 int umma_w4_token_tile(const UmmaW4Args& a);
 int umma_w4_linear(const UmmaW4Args& a, cudaStream_t st);
 
+// umma_w4.cu: the INT4 GEMM behind the activation pre-pass (a.magic), and its scratch for partial sums (a.sk_ws)
+int umma_w4_prep_token_tile(const UmmaW4Args& a);
+int umma_w4_prep_linear(const UmmaW4Args& a, cudaStream_t st);
+size_t umma_w4_partial_bytes(int64_t M);
+
+// shared by the weight-only kernels: the device's status word, and a bank of zeroed arrival counters for cut strips
+constexpr int UMMA_MAX_CUT_STRIPS = 1024;
+int* umma_status_ptr();
+int* umma_strip_counters();
+
 bool umma_w8_supported(const UmmaW8Args& a);
 int umma_w8_token_tile(const UmmaW8Args& a);
 int umma_w8_linear(const UmmaW8Args& a, cudaStream_t st);

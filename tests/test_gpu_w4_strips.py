@@ -1,0 +1,71 @@
+"""The persistent INT4 tcgen05 GEMM at the sizes where its division of work can go wrong: token-tile edges, ragged strips,
+a scale-group count that fills no whole raw stage, strips cut between CTAs (several segments per CTA), tall strips, and
+the three scale types through both ways of fetching them.
+
+Tolerance: the output is rounded to bf16 once (relative 2^-9 of every element) and every weight (q - 8) * s to fp16 once
+(2^-12, independent, so at most that in the 2-norm of a column); column by column the 2-norm error of the result is
+therefore below 2^-9 + 2^-11, while one lost or repeated group of 128 k is an error of 1 / sqrt(K / 128)."""
+import pytest
+import torch
+
+from gpu_util import DEV
+
+pytestmark = pytest.mark.gpu
+TOL = 2.0 ** -9 + 2.0 ** -11
+
+
+@pytest.fixture(scope="module")
+def e():
+    import custom_esimd_kernels_vllm as pkg
+    pkg.set_force_kernel(2)
+    yield pkg
+    pkg.set_force_kernel(0)
+
+
+def _case(M, N, K, scale_dtype, seed):
+    g = torch.Generator(device=DEV).manual_seed(seed)
+    w = torch.randint(-2 ** 31, 2 ** 31 - 1, (N, K // 8), generator=g, device=DEV, dtype=torch.int64).to(torch.int32)
+    s = ((0.5 + torch.rand(N, K // 128, generator=g, device=DEV)) * 0.01).to(scale_dtype)
+    x = torch.randn(M, K, generator=g, device=DEV).to(torch.bfloat16)
+    shifts = torch.arange(0, 32, 4, device=DEV, dtype=torch.int32)
+    q = ((w.unsqueeze(-1) >> shifts) & 15).reshape(N, K // 128, 128).double() - 8
+    ref = x.double() @ (q * s.double().unsqueeze(-1)).view(N, K).T
+    return x, w, s, ref
+
+
+def _check(out, ref, what):
+    err = (out.double() - ref).norm(dim=0) / ref.norm(dim=0)
+    assert float(err.max()) < TOL, (what, float(err.max()), int(err.argmax()))
+
+
+@pytest.mark.parametrize("scale_dtype", [torch.bfloat16, torch.float16, torch.float32])
+@pytest.mark.parametrize("M,N,K", [
+    (1, 128, 128), (16, 136, 384), (17, 1000, 1024),     # one tile; ragged strip; odd group count; aligned scale fetch
+    (33, 520, 2560), (64, 2048, 4096),                   # 64-token tile, cut strips
+    (65, 300, 1280), (128, 1032, 2048),                  # 128-token tile, one of them
+    (129, 384, 640), (400, 2184, 1152),                  # several token tiles, odd group counts
+])
+def test_tile_and_group_edges(e, M, N, K, scale_dtype):
+    x, w, s, ref = _case(M, N, K, scale_dtype, M + N + K)
+    out = torch.full((M, N), float("nan"), dtype=torch.bfloat16, device=DEV)
+    e.esimd_gemm_int4_pgrp(x, w, s, out)
+    _check(out, ref, (M, N, K))
+    kmaj = torch.full_like(out, float("nan"))
+    if N % 4 == 0:
+        e.esimd_gemm_int4_pgrp(x, w.t().contiguous(), s.t().contiguous(), kmaj)
+        _check(kmaj, ref, ("k-major", M, N, K))
+    assert e._lib.device_status() == 0
+
+
+@pytest.mark.parametrize("M,N,K", [(16, 8192, 14336), (64, 8192, 14336), (64, 38016, 2048), (100, 10240, 8192), (700, 8192, 2048)])
+def test_many_segments_repeat_bit_for_bit(e, M, N, K):
+    x, w, s, ref = _case(M, N, K, torch.bfloat16, 7)
+    first = None
+    for _ in range(8):
+        out = torch.full((M, N), float("nan"), dtype=torch.bfloat16, device=DEV)
+        e.esimd_gemm_int4_pgrp(x, w, s, out)
+        if first is None:
+            first = out
+            _check(out, ref, (M, N, K))
+        assert torch.equal(out, first)
+    assert e._lib.device_status() == 0
