@@ -63,14 +63,15 @@ template <int TOK, int R> struct Cfg {
   static constexpr int SCS = 4, SC_GROUPS = 8, SC_BYTES = SC_GROUPS * ROWS * 2;   // scale slots: [row][group] 16-bit
   static constexpr int POST_RING = 16;                       // row exponents per segment, read by the epilogue
   static constexpr int POST_BYTES = POST_RING * ROWS;
+  static constexpr int STAGE_OUT = EW * 1024;                // 16 tokens x 32 columns of output per epilogue warp
   static constexpr int BUDGET = 232448 - 1024 /*align*/ - 1024 /*barriers*/;
-  static constexpr int RS_FIT = (BUDGET - XS * X_BYTES - SCS * SC_BYTES - POST_BYTES) / RAW_BYTES;
+  static constexpr int RS_FIT = (BUDGET - XS * X_BYTES - SCS * SC_BYTES - POST_BYTES - STAGE_OUT) / RAW_BYTES;
   // Raw and operand stages always belong to the same transform group(s), whatever segment they are in: a wait tells a
   // phase from the one after it, not from the one after that, so nobody may wait for a stage whose previous use was
   // somebody else's.  Hence ring depths in multiples of a round of the groups.
   static constexpr int RAW_ROUND = KG / 2, A_ROUND = KG;
   static constexpr int RS = (RS_FIT > 12 ? 12 : RS_FIT) / RAW_ROUND * RAW_ROUND;
-  static constexpr int SMEM = XS * X_BYTES + RS * RAW_BYTES + SCS * SC_BYTES + POST_BYTES + 1024 + 1024;
+  static constexpr int SMEM = XS * X_BYTES + RS * RAW_BYTES + SCS * SC_BYTES + POST_BYTES + STAGE_OUT + 1024 + 1024;
   static constexpr int ACC_COLS = TOK < 32 ? 32 : TOK;
   static constexpr int NBUF = 2 * R * ACC_COLS <= 256 ? 2 : 1;   // accumulator sets
   static constexpr int A_COL0 = NBUF * R * ACC_COLS;
@@ -84,6 +85,7 @@ struct W4Params {
   const void* scale; int scale_dtype; int64_t s_stride_n, s_stride_g, s_expert_elems;
   int scale_vec8;            // eight consecutive groups of a row are one aligned 16-byte load
   void* out; int64_t ldo; int out_bf16;
+  int vec_out;               // rows of out are 16-byte aligned
   int M, N, K;
   int nk;                    // 64-k chunks of a whole strip, rounded up to whole raw stages (what lies beyond K multiplies by zero)
   int strips, tiles_n;       // strips of R * 128 rows; token tiles of a dense launch
@@ -231,7 +233,7 @@ umma_w4_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constant__
   const uint32_t raw_smem = base, x_smem = base + RS * C::RAW_BYTES, sc_smem = x_smem + XS * C::X_BYTES;
   const uint32_t post_off = RS * C::RAW_BYTES + XS * C::X_BYTES + C::SCS * C::SC_BYTES;
   int8_t* post_exp = reinterpret_cast<int8_t*>(gen + post_off);
-  const uint32_t bar = base + post_off + C::POST_BYTES;
+  const uint32_t out_smem = base + post_off + C::POST_BYTES, bar = out_smem + C::STAGE_OUT;
   // barrier map (8 bytes each)
   const uint32_t raw_full = bar, raw_empty = raw_full + 8 * RS, x_full = raw_empty + 8 * RS, x_empty = x_full + 8 * XS;
   const uint32_t a_full = x_empty + 8 * XS, a_empty = a_full + 8 * S, sc_full = a_empty + 8 * S, sc_empty = sc_full + 8 * C::SCS;
@@ -461,6 +463,35 @@ umma_w4_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constant__
         if (lane < CB && lane < left) ts_lane = __ldcg(p.tok_scale + sg.xrow0 + sg.tok0 + cb + lane);
         int map_lane = 0;
         if (p.out_map && lane < CB && lane < left) map_lane = __ldcg(p.out_map + sg.xrow0 + sg.tok0 + cb + lane);
+        if (p.vec_out && nb + quad * 32 + 32 <= p.N && !(TOK <= 64 && p.peer_on)) {
+          // Through shared memory, sixteen tokens at a time, so that a lane stores 16 bytes of a row instead of 2: with
+          // 2-byte stores draining a 256 x 128 tile took 16,000 cycles in which the MMAs of the next one had to wait.
+          const uint32_t st = out_smem + (warp - C::CW) * 1024;
+#pragma unroll
+          for (int h = 0; h < CB; h += 16) {
+            __syncwarp();
+#pragma unroll
+            for (int i = 0; i < 16; i += 2) {
+              const float v0 = r[h + i] * __shfl_sync(0xffffffffu, ts_lane, h + i), v1 = r[h + i + 1] * __shfl_sync(0xffffffffu, ts_lane, h + i + 1);
+              uint32_t pk;
+              if (p.out_bf16) asm("cvt.rn.bf16x2.f32 %0, %1, %2;" : "=r"(pk) : "f"(v1), "f"(v0));
+              else asm("cvt.rn.f16x2.f32 %0, %1, %2;" : "=r"(pk) : "f"(v1), "f"(v0));
+              asm volatile("st.shared.u16 [%0], %1;" ::"r"(st + i * 64 + lane * 2), "h"((unsigned short)pk) : "memory");
+              asm volatile("st.shared.u16 [%0], %1;" ::"r"(st + i * 64 + 64 + lane * 2), "h"((unsigned short)(pk >> 16)) : "memory");
+            }
+            __syncwarp();
+#pragma unroll
+            for (int j = 0; j < 2; ++j) {
+              const int tk = h + j * 8 + (lane >> 2);
+              const uint4 v = lds128(st + j * 512 + lane * 16);
+              int64_t orow = sg.xrow0 + sg.tok0 + cb + tk;
+              if (p.out_map) orow = __shfl_sync(0xffffffffu, map_lane, tk);
+              if (tk < left)
+                *reinterpret_cast<uint4*>(reinterpret_cast<uint16_t*>(p.out) + orow * p.ldo + nb + quad * 32 + (lane & 3) * 8) = v;
+            }
+          }
+          return;
+        }
 #pragma unroll
         for (int i = 0; i < CB; ++i) {
           const float v = r[i] * __shfl_sync(0xffffffffu, ts_lane, i);
@@ -766,7 +797,9 @@ int umma_w4_prep_linear(const UmmaW4Args& a, cudaStream_t st) {
   p.scale = a.scale; p.scale_dtype = a.scale_dtype; p.s_stride_n = a.s_stride_n; p.s_stride_g = a.s_stride_g;
   p.s_expert_elems = (int64_t)a.N * (a.K / 128);
   p.scale_vec8 = a.scale_dtype != B2Q_F32 && a.s_stride_g == 1 && (a.s_stride_n % 8) == 0 && (a.K % 1024) == 0 && aligned16(a.scale);
-  p.out = a.out; p.ldo = a.ldo; p.out_bf16 = a.out_bf16 ? 1 : 0; p.M = a.M; p.N = a.N; p.K = a.K; p.nk = ((a.K >> 6) + 3) & ~3;
+  p.out = a.out; p.ldo = a.ldo; p.out_bf16 = a.out_bf16 ? 1 : 0;
+  p.vec_out = aligned16(a.out) && (a.ldo % 8) == 0;
+  p.M = a.M; p.N = a.N; p.K = a.K; p.nk = ((a.K >> 6) + 3) & ~3;
   p.tiles = grouped ? a.tiles : nullptr; p.expert_offsets = a.expert_offsets; p.out_map = a.out_map;
   p.w_rows_per_expert = kmajor ? a.K / 8 : a.N;
   p.tok_scale = a.tok_scale;
