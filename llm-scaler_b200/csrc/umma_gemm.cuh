@@ -83,6 +83,8 @@ int umma_w4_linear(const UmmaW4Args& a, cudaStream_t st);
 int umma_w4_prep_token_tile(const UmmaW4Args& a);
 int umma_w4_prep_linear(const UmmaW4Args& a, cudaStream_t st);
 size_t umma_w4_partial_bytes(int64_t M);
+// block-scaled e4m3 weights, fp16 activations, M <= 64 (B2Q_ERR_UNSUPPORTED otherwise)
+int umma_w8_strip_linear(const UmmaW8Args& a, cudaStream_t st);
 
 // shared by the weight-only kernels: the device's status word, and a bank of zeroed arrival counters for cut strips
 constexpr int UMMA_MAX_CUT_STRIPS = 1024;

@@ -1,4 +1,5 @@
-// INT4 (group 128) weight-only GEMM on tcgen05 behind the activation pre-pass: out[tok, n] = sum_k x[tok, k] * W[n, k].
+// Weight-only GEMM on tcgen05 for fp16 activations: out[tok, n] = sum_k x[tok, k] * W[n, k], W INT4 (group 128, behind the
+// activation pre-pass) or, for decode tiles, block-scaled e4m3.
 //
 // Swap-AB: strips of R x 128 weight rows are the MMA's M dimension, a tile of TOK tokens its N dimension.  The nibbles are
 // decoded to fp16 in registers and written straight into tensor memory as the MMA's A operand (no trip back through
@@ -46,7 +47,9 @@ inline MagicConsts magic_consts(bool twos) {
   return MagicConsts{0x64006400u ^ (twos ? 0x00080008u : 0u), 0x64006400u ^ (twos ? 0x00800080u : 0u), 0xD480D480u};
 }
 
-template <int TOK, int R> struct Cfg {
+enum { WT_W4N = 0, WT_W4K = 1, WT_W8 = 2 };          // N-major nibbles, K-major nibbles, e4m3 with a scale per 128 x 128 block
+
+template <int WT, int TOK, int R> struct Cfg {
   static constexpr int NG = 4, KG = NG / R;                  // transform groups of four warps; of these, groups along k
   static constexpr int EW = TOK >= 64 ? 8 : 4;               // epilogue warps
   static constexpr int CW = 4;                               // control warps
@@ -56,9 +59,10 @@ template <int TOK, int R> struct Cfg {
   // (clock() around them): with operand and activation stages of 64 k it spent 490 cycles per 64 k of a 128-row strip,
   // and the transform warps waited two thirds of their time for it.  So an operand stage is a whole scale group (128 k)
   // and an activation stage 256 k where shared memory allows.
-  static constexpr int XC = (R == 1 && TOK <= 64) ? 4 : 2;   // 64-k chunks per activation stage
+  static constexpr int GPS = WT == WT_W8 ? 1 : 2;            // scale groups (128 k) per raw stage of 128 bytes a row
+  static constexpr int XC = (R == 1 && TOK <= 64) ? 2 * GPS : 2;   // 64-k chunks per activation stage
   static constexpr int X_BYTES = TOK * 128 * XC;
-  static constexpr int XS = TOK == 128 ? 3 : (R == 2 ? 6 : (TOK == 64 ? 3 : 4));
+  static constexpr int XS = TOK == 128 ? 3 : (R == 2 ? 6 : (TOK == 64 ? 6 : 8) / GPS);
   static constexpr int RAW_BYTES = R * 16384;
   static constexpr int SCS = 4, SC_GROUPS = 8, SC_BYTES = SC_GROUPS * ROWS * 2;   // scale slots: [row][group] 16-bit
   static constexpr int POST_RING = 16;                       // row exponents per segment, read by the epilogue
@@ -69,7 +73,7 @@ template <int TOK, int R> struct Cfg {
   // Raw and operand stages always belong to the same transform group(s), whatever segment they are in: a wait tells a
   // phase from the one after it, not from the one after that, so nobody may wait for a stage whose previous use was
   // somebody else's.  Hence ring depths in multiples of a round of the groups.
-  static constexpr int RAW_ROUND = KG / 2, A_ROUND = KG;
+  static constexpr int RAW_ROUND = KG / GPS, A_ROUND = KG;
   static constexpr int RS = (RS_FIT > 12 ? 12 : RS_FIT) / RAW_ROUND * RAW_ROUND;
   static constexpr int SMEM = XS * X_BYTES + RS * RAW_BYTES + SCS * SC_BYTES + POST_BYTES + STAGE_OUT + 1024 + 1024;
   static constexpr int ACC_COLS = TOK < 32 ? 32 : TOK;
@@ -158,6 +162,14 @@ __device__ __forceinline__ void w4_word_magic(uint32_t w, uint32_t s2, const Mag
   }
 }
 
+// Four e4m3 bytes -> four fp16 values in k order, each times the block's fp32 scale with one rounding.
+__device__ __forceinline__ void e4m3_word(uint32_t w, float sf, uint32_t* o) {
+  uint32_t h0 = fp8x2_to_act<false, false>(w), h1 = fp8x2_to_act<false, false>(w >> 16);
+  const float2 f0 = __half22float2(*reinterpret_cast<__half2*>(&h0)), f1 = __half22float2(*reinterpret_cast<__half2*>(&h1));
+  asm("cvt.rn.f16x2.f32 %0, %1, %2;" : "=r"(o[0]) : "f"(f0.y * sf), "f"(f0.x * sf));
+  asm("cvt.rn.f16x2.f32 %0, %1, %2;" : "=r"(o[1]) : "f"(f1.y * sf), "f"(f1.x * sf));
+}
+
 // One piece of a CTA's work: 64-k chunks [c_begin, c_begin + nk) of the strip of weight rows at n0, for the token tile
 // at tok0.  part = the strip's other chunks belong to other CTAs; slot = which of the CTA's two partial-sum slots it uses.
 struct Segment { int n0, c_begin, nk, strip, part, slot, tok0, xrow0, M, expert; };
@@ -166,8 +178,9 @@ struct Segment { int n0, c_begin, nk, strip, part, slot, tok0, xrow0, M, expert;
 // units of one raw stage and CTA b takes the units [b U / G, (b + 1) U / G): up to two partial strips around any number
 // of whole ones.  Otherwise whole (tile, strip) pairs in steps of the grid, ordered so that CTAs running at the same time
 // share what does not fit in L2 twice: dense launches the weight strip, grouped launches an expert's activation rows.
-template <int ROWS, int TOK> struct Cursor {
+template <int ROWS, int TOK, int GPS> struct Cursor {
   int u, u0, u1;
+  int block_row, block_col;          // 128 x 128 block the last segment of next_nk began with
   __device__ __forceinline__ void init(const W4Params& p, int total) {
     if (p.units > 0) {
       u0 = (int)((int64_t)blockIdx.x * p.units / gridDim.x);
@@ -183,10 +196,12 @@ template <int ROWS, int TOK> struct Cursor {
     if (u >= u1) return 0;
     if (p.units > 0) {
       const int r0 = u % p.sps, take = min(p.sps - r0, u1 - u);
-      if (off) *off = (2 * r0) & 7;
+      if (off) *off = (GPS * r0) & 7;
+      block_row = u / p.sps * (ROWS / 128); block_col = GPS * r0;
       u += take;
-      return take * 4;
+      return take * 2 * GPS;
     }
+    block_row = (p.tiles ? 0 : u / p.tiles_n) * (ROWS / 128); block_col = 0;
     u += gridDim.x;
     return p.nk;
   }
@@ -196,7 +211,7 @@ template <int ROWS, int TOK> struct Cursor {
     if (p.units > 0) {
       const int strip = u / p.sps, r0 = u - strip * p.sps;
       const int take = min(p.sps - r0, u1 - u);
-      sg.n0 = strip * ROWS; sg.c_begin = r0 * 4; sg.nk = take * 4; sg.strip = strip;
+      sg.n0 = strip * ROWS; sg.c_begin = r0 * 2 * GPS; sg.nk = take * 2 * GPS; sg.strip = strip;
       sg.part = take != p.sps; sg.slot = (u == u0) ? 0 : 1;
       u += take;
       return true;
@@ -220,11 +235,12 @@ template <int ROWS, int TOK> struct Cursor {
 };
 }  // namespace w4
 
-template <bool KMAJOR, int TOK, int R>
-__global__ void __launch_bounds__(w4::Cfg<TOK, R>::THREADS, 1)
+template <int WT, int TOK, int R>
+__global__ void __launch_bounds__(w4::Cfg<WT, TOK, R>::THREADS, 1)
 umma_w4_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constant__ CUtensorMap tm_x, const W4Params p) {
   using namespace w4;
-  using C = Cfg<TOK, R>;
+  using C = Cfg<WT, TOK, R>;
+  constexpr bool KMAJOR = WT == WT_W4K;
   constexpr int S = C::S, RS = C::RS, XS = C::XS, KG = C::KG, NBUF = C::NBUF, ROWS = C::ROWS;
 
   extern __shared__ uint8_t smem_raw[];
@@ -250,12 +266,12 @@ umma_w4_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constant__
   grid_dep_release();
   int total = p.strips * p.tiles_n;
   if (p.tiles) { grid_dep_wait(); total = __ldcg(p.tiles) * p.strips; }
-  Cursor<ROWS, TOK> cur;
+  Cursor<ROWS, TOK, C::GPS> cur;
   cur.init(p, total);
   if (cur.u >= cur.u1) return;                       // the whole CTA: fewer pieces of work than CTAs
 
   if (threadIdx.x == 0) {
-    for (int i = 0; i < RS; ++i) { mbar_init(raw_full + 8 * i, 1); mbar_init(raw_empty + 8 * i, 8 * R); }
+    for (int i = 0; i < RS; ++i) { mbar_init(raw_full + 8 * i, 1); mbar_init(raw_empty + 8 * i, 4 * C::GPS * R); }
     for (int i = 0; i < XS; ++i) { mbar_init(x_full + 8 * i, 1); mbar_init(x_empty + 8 * i, 1); }
     for (int i = 0; i < S; ++i) { mbar_init(a_full + 8 * i, 4 * R); mbar_init(a_empty + 8 * i, 1); }
     for (int i = 0; i < C::SCS; ++i) { mbar_init(sc_full + 8 * i, 32); mbar_init(sc_empty + 8 * i, 16); }
@@ -279,7 +295,7 @@ umma_w4_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constant__
       uint32_t par = 1u;                       // parity of the phase before the ring's current round
       bool ok = true;
       while (ok && cur.next(p, sg)) {
-        const int nraw = sg.nk >> 2;
+        const int nraw = sg.nk / (2 * C::GPS);
         for (int r = 0; r < nraw; ++r) {
           ok = mbar_wait(raw_empty + 8 * rs, par, abort_flag, p.status, ST_RAWEMPTY);
           if (!ok) break;
@@ -289,9 +305,9 @@ umma_w4_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constant__
           for (int rb = 0; rb < R; ++rb) {
             const uint32_t dst = raw_smem + rs * C::RAW_BYTES + rb * 16384;
             if constexpr (KMAJOR)
-              tma_load_2d(dst, &tm_w, sg.n0 + rb * 128, sg.expert * p.w_rows_per_expert + (sg.c_begin / 4 + r) * 32, raw_full + 8 * rs);
+              tma_load_2d(dst, &tm_w, sg.n0 + rb * 128, sg.expert * p.w_rows_per_expert + (sg.c_begin / (2 * C::GPS) + r) * 32, raw_full + 8 * rs);
             else
-              tma_load_2d(dst, &tm_w, (sg.c_begin / 4 + r) * 128, sg.expert * p.w_rows_per_expert + sg.n0 + rb * 128, raw_full + 8 * rs);
+              tma_load_2d(dst, &tm_w, (sg.c_begin / (2 * C::GPS) + r) * 128, sg.expert * p.w_rows_per_expert + sg.n0 + rb * 128, raw_full + 8 * rs);
           }
           if (++rs == RS) { rs = 0; par ^= 1u; }
         }
@@ -375,7 +391,7 @@ umma_w4_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constant__
     bool ok = true;
     const bool f32 = p.scale_dtype == B2Q_F32;
     const int esz = f32 ? 4 : 2;
-    while (ok && cur.next(p, sg)) {
+    while (WT != WT_W8 && ok && cur.next(p, sg)) {
       const int gs = sg.c_begin >> 1, npad = sg.nk >> 1, off = gs & 7, nslot = (off + npad + 7) >> 3;
       const int ngroups = min(npad, (p.K >> 7) - gs);
       const uint8_t* sbase = reinterpret_cast<const uint8_t*>(p.scale) +
@@ -460,7 +476,7 @@ umma_w4_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constant__
         // call's scales at this address), handed round the warp by shuffle
         const int left = sg.M - (sg.tok0 + cb);
         float ts_lane = 1.f;
-        if (lane < CB && lane < left) ts_lane = __ldcg(p.tok_scale + sg.xrow0 + sg.tok0 + cb + lane);
+        if (p.tok_scale && lane < CB && lane < left) ts_lane = __ldcg(p.tok_scale + sg.xrow0 + sg.tok0 + cb + lane);
         int map_lane = 0;
         if (p.out_map && lane < CB && lane < left) map_lane = __ldcg(p.out_map + sg.xrow0 + sg.tok0 + cb + lane);
         if (p.vec_out && nb + quad * 32 + 32 <= p.N && !(TOK <= 64 && p.peer_on)) {
@@ -527,7 +543,7 @@ umma_w4_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constant__
           const uint32_t ta = tmem + lane_base + (b * R + rb) * C::ACC_COLS + cb;
           if constexpr (CB == 32) tmem_ld32(ta, q); else tmem_ld16(ta, q);
           tmem_ld_wait();
-          const float pm = __uint_as_float((uint32_t)(127 + post[rb * 128 + quad * 32 + lane]) << 23);
+          const float pm = WT == WT_W8 ? 1.f : __uint_as_float((uint32_t)(127 + post[rb * 128 + quad * 32 + lane]) << 23);
 #pragma unroll
           for (int i = 0; i < CB; ++i) r[i] = __uint_as_float(q[i]) * pm;
         }
@@ -621,7 +637,7 @@ umma_w4_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constant__
     const int quad = warp & 3, grp = (warp - C::CW - C::EW) >> 2;
     const int t = quad * 32 + lane;                // row of the block == tensor-memory lane this thread may write
     const int rb = R == 2 ? (grp & 1) : 0, kq = R == 2 ? (grp >> 1) : grp;
-    const int half = kq & 1;
+    const int half = C::GPS == 2 ? (kq & 1) : 0;
     const uint32_t row0 = raw_smem + rb * 16384 + (KMAJOR ? t * 4 + half * 16 * 512 : t * 128 + (((4 * half) ^ (t & 7)) << 4));
     const uint32_t ta0 = tmem + ((uint32_t)(quad * 32) << 16) + C::A_COL0 + rb * 64;
     const uint32_t sc0 = sc_smem + (rb * 128 + t) * 16;
@@ -634,16 +650,20 @@ umma_w4_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constant__
       const int ngroups = nk >> 1, nslot = (off + ngroups + 7) >> 3;
       // first group of this segment that is this transform group's in the count over all segments
       int gg = (kq - (gb >> 1)) & (KG - 1);
-      const int g0 = (gb >> 1) + gg, raw0 = g0 >> 1;
+      const int g0 = (gb >> 1) + gg, raw0 = g0 / C::GPS;
       int rs = raw0 % RS, as = g0 % S;
       uint32_t rpar = (uint32_t)(raw0 / RS) & 1u, apar = ((uint32_t)(g0 / S) + 1u) & 1u;
       float row_mul = 1.f;
+      // e4m3: one fp32 scale per block, the same for the whole CTA, requested an iteration ahead
+      const float* block_scale = reinterpret_cast<const float*>(p.scale) + (cur.block_row + rb) * (int64_t)(p.K >> 7) + cur.block_col;
+      float sf_next = 0.f;
+      if (WT == WT_W8 && gg < ngroups) sf_next = __ldg(block_scale + gg);
 #pragma unroll 1
       for (int sl = 0; sl < nslot; ++sl) {
-        ok = wait_converged(sc_full + 8 * ss, spar, abort_flag, p.status, ST_SCFULL);
+        if (WT != WT_W8) ok = wait_converged(sc_full + 8 * ss, spar, abort_flag, p.status, ST_SCFULL);
         if (!ok) break;
         const uint32_t sca = sc0 + ss * C::SC_BYTES;
-        if (sl == 0 && p.scale_dtype != B2Q_F32) {
+        if (WT != WT_W8 && sl == 0 && p.scale_dtype != B2Q_F32) {
           const int k = bf16_scale ? row_exponent(__uint_as_float(lds_u16(sca + 2 * off) << 16)) : 0;
           row_mul = __uint_as_float((uint32_t)(127 + k) << 23);
           // told to the epilogue by the group that converts the segment's first 128 k: before these are handed over
@@ -652,8 +672,11 @@ umma_w4_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constant__
         const int gend = min(8 * sl + 8 - off, ngroups);
 #pragma unroll 1
         for (; gg < gend; gg += KG) {
-          uint32_t hv = lds_u16(sca + 2 * ((gg + off) & 7));
-          if (bf16_scale) hv = fp16_factor(__uint_as_float(hv << 16) * row_mul, saturated);
+          uint32_t hv = WT == WT_W8 ? 0u : lds_u16(sca + 2 * ((gg + off) & 7));
+          const float sf = sf_next;
+          if (WT == WT_W8 && gg + KG < ngroups) sf_next = __ldg(block_scale + gg + KG);
+          if (WT == WT_W8) {}
+          else if (bf16_scale) hv = fp16_factor(__uint_as_float(hv << 16) * row_mul, saturated);
           else if ((hv & 0x7FFFu) - 0x7000u <= 0x0C00u) { hv = (hv & 0x8000u) | 0x6FFFu; saturated = 1; }     // above 8188, NaN stays
           const uint32_t m2 = hv | (hv << 16);
           ok = wait_converged(raw_full + 8 * rs, rpar, abort_flag, p.status, ST_RAWFULL);
@@ -663,16 +686,25 @@ umma_w4_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constant__
 #pragma unroll
           for (int q = 0; q < 4; ++q) {            // quarters of 32 k: 16 registers live
             uint32_t w0, w1, w2, w3;
-            if constexpr (!KMAJOR) {
+            uint32_t a16[16];
+            if constexpr (WT == WT_W8) {
+#pragma unroll
+              for (int z = 0; z < 2; ++z) {
+                const uint4 rr = lds128(rowa ^ ((2 * q + z) << 4));
+                e4m3_word(rr.x, sf, a16 + 8 * z); e4m3_word(rr.y, sf, a16 + 8 * z + 2);
+                e4m3_word(rr.z, sf, a16 + 8 * z + 4); e4m3_word(rr.w, sf, a16 + 8 * z + 6);
+              }
+            } else if constexpr (!KMAJOR) {
               const uint4 rr = lds128(rowa ^ (q << 4));
               w0 = rr.x; w1 = rr.y; w2 = rr.z; w3 = rr.w;
             } else {
               w0 = lds32(rowa + (4 * q + 0) * 512); w1 = lds32(rowa + (4 * q + 1) * 512);
               w2 = lds32(rowa + (4 * q + 2) * 512); w3 = lds32(rowa + (4 * q + 3) * 512);
             }
-            uint32_t a16[16];
-            w4_word_magic(w0, m2, mk, a16); w4_word_magic(w1, m2, mk, a16 + 4);
-            w4_word_magic(w2, m2, mk, a16 + 8); w4_word_magic(w3, m2, mk, a16 + 12);
+            if constexpr (WT != WT_W8) {
+              w4_word_magic(w0, m2, mk, a16); w4_word_magic(w1, m2, mk, a16 + 4);
+              w4_word_magic(w2, m2, mk, a16 + 8); w4_word_magic(w3, m2, mk, a16 + 12);
+            }
             if (q == 0) {                          // the first quarter is converted while the stage is still being read
               ok = wait_converged(a_empty + 8 * as, apar, abort_flag, p.status, ST_EMPTY);
               if (!ok) break;
@@ -691,7 +723,7 @@ umma_w4_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constant__
         }
         if (!ok) break;
         __syncwarp();
-        if (elected) mbar_arrive(sc_empty + 8 * ss);
+        if (WT != WT_W8 && elected) mbar_arrive(sc_empty + 8 * ss);
         __syncwarp();
         if (++ss == C::SCS) { ss = 0; spar ^= 1u; }
       }
@@ -733,10 +765,10 @@ size_t umma_w4_partial_bytes(int64_t M) {
   return (size_t)2 * sm_count() * (tok >= 64 ? 256 : 128) * tok * sizeof(float);
 }
 
-template <bool KMAJOR, int TOK, int R>
+template <int WT, int TOK, int R>
 static int launch_w4(const CUtensorMap& tw, const CUtensorMap& tx, const W4Params& p, int grid, bool overlap, cudaStream_t st) {
-  using C = w4::Cfg<TOK, R>;
-  auto kern = umma_w4_kernel<KMAJOR, TOK, R>;
+  using C = w4::Cfg<WT, TOK, R>;
+  auto kern = umma_w4_kernel<WT, TOK, R>;
   static thread_local bool configured[16] = {false};
   int dev = 0;
   cudaGetDevice(&dev);
@@ -749,13 +781,28 @@ static int launch_w4(const CUtensorMap& tw, const CUtensorMap& tx, const W4Param
   return launch_status();
 }
 
-template <bool KMAJOR>
+template <int WT>
 static int launch_w4_tile(int tok, int R, const CUtensorMap& tw, const CUtensorMap& tx, const W4Params& p, int grid, bool overlap,
                           cudaStream_t st) {
-  if (tok == 16) return launch_w4<KMAJOR, 16, 1>(tw, tx, p, grid, overlap, st);
-  if (tok == 32) return launch_w4<KMAJOR, 32, 1>(tw, tx, p, grid, overlap, st);
-  if (tok == 64) return R == 2 ? launch_w4<KMAJOR, 64, 2>(tw, tx, p, grid, overlap, st) : launch_w4<KMAJOR, 64, 1>(tw, tx, p, grid, overlap, st);
-  return R == 2 ? launch_w4<KMAJOR, 128, 2>(tw, tx, p, grid, overlap, st) : launch_w4<KMAJOR, 128, 1>(tw, tx, p, grid, overlap, st);
+  if (tok == 16) return launch_w4<WT, 16, 1>(tw, tx, p, grid, overlap, st);
+  if (tok == 32) return launch_w4<WT, 32, 1>(tw, tx, p, grid, overlap, st);
+  if (tok == 64) return R == 2 ? launch_w4<WT, 64, 2>(tw, tx, p, grid, overlap, st) : launch_w4<WT, 64, 1>(tw, tx, p, grid, overlap, st);
+  return R == 2 ? launch_w4<WT, 128, 2>(tw, tx, p, grid, overlap, st) : launch_w4<WT, 128, 1>(tw, tx, p, grid, overlap, st);
+}
+
+// Cuts the strips along k, raw stage by raw stage, when whole ones would leave more than a twentieth of the machine idle in
+// the last round (one token tile only).
+template <class Args>
+static int cut_strips(W4Params& p, const Args& a, int sms, int stages_per_strip) {
+  if (p.strips > UMMA_MAX_CUT_STRIPS || !a.sk_ws || !aligned16(a.sk_ws) || a.sk_ws_bytes < umma_w4_partial_bytes(a.M) || tls().force_kernel == 4)
+    return B2Q_OK;
+  const double eff = (double)p.strips / ((double)((p.strips + sms - 1) / sms) * sms);
+  const int64_t units = (int64_t)p.strips * stages_per_strip;
+  if (eff > 0.95 || units > INT32_MAX) return B2Q_OK;
+  p.counters = umma_strip_counters();
+  if (!p.counters) return B2Q_ERR_CUDA;
+  p.sps = stages_per_strip; p.units = (int)units; p.partials = reinterpret_cast<float*>(a.sk_ws);
+  return B2Q_OK;
 }
 
 int umma_w4_prep_token_tile(const UmmaW4Args& a) { return a.expert_offsets ? grouped_tok(a.M, a.E) : dense_tok(a.M); }
@@ -808,17 +855,10 @@ int umma_w4_prep_linear(const UmmaW4Args& a, cudaStream_t st) {
   if (!p.status) return B2Q_ERR_CUDA;
   p.strips = R == 2 ? strips2 : strips1; p.tiles_n = tiles;
   int64_t work = (int64_t)p.strips * tiles;
-  // Cut strips along k when whole ones would leave more than a twentieth of the machine idle in the last round.
-  if (!grouped && tiles == 1 && (a.K % 256) == 0 && p.strips <= UMMA_MAX_CUT_STRIPS && a.sk_ws && aligned16(a.sk_ws) &&
-      a.sk_ws_bytes >= umma_w4_partial_bytes(a.M) && tls().force_kernel != 4) {
-    const double eff = (double)p.strips / ((double)((p.strips + sms - 1) / sms) * sms);
-    const int64_t units = (int64_t)p.strips * (a.K / 256);
-    if (eff <= 0.95 && units <= INT32_MAX) {
-      p.counters = umma_strip_counters();
-      if (!p.counters) return B2Q_ERR_CUDA;
-      p.sps = a.K / 256; p.units = (int)units; p.partials = reinterpret_cast<float*>(a.sk_ws);
-      work = units;
-    }
+  if (!grouped && tiles == 1 && (a.K % 256) == 0) {
+    rc = cut_strips(p, a, sms, a.K / 256);
+    if (rc) return rc;
+    if (p.units > 0) work = p.units;
   }
   if (work > INT32_MAX) return B2Q_ERR_LIMIT;
   if (a.peer) {
@@ -827,7 +867,36 @@ int umma_w4_prep_linear(const UmmaW4Args& a, cudaStream_t st) {
   }
   const int grid = (int)(work < sms ? work : sms);
   const bool overlap = tls().overlap_mode > 0 && (a.after_prep || tls().overlap_mode == 2);
-  return kmajor ? launch_w4_tile<true>(tok, R, tw, tx, p, grid, overlap, st) : launch_w4_tile<false>(tok, R, tw, tx, p, grid, overlap, st);
+  return kmajor ? launch_w4_tile<w4::WT_W4K>(tok, R, tw, tx, p, grid, overlap, st)
+                : launch_w4_tile<w4::WT_W4N>(tok, R, tw, tx, p, grid, overlap, st);
+}
+
+// Block-scaled e4m3 weights on fp16 activations, decode tiles.
+int umma_w8_strip_linear(const UmmaW8Args& a, cudaStream_t st) {
+  const int sms = sm_count(), tok = dense_tok(a.M);
+  if (a.bf16 || a.expert_offsets || a.scale_mode != B2Q_SCALE_BLOCK128 || a.fmt != B2Q_E4M3 || a.M > 64 || (a.K % 128) != 0)
+    return B2Q_ERR_UNSUPPORTED;
+  CUtensorMap tw, tx;
+  int rc = make_tmap_2d(&tw, CU_TENSOR_MAP_DATA_TYPE_UINT8, 1, a.w, a.N, a.K, (uint64_t)a.K, 128, 128, CU_TENSOR_MAP_SWIZZLE_128B);
+  if (rc) return rc;
+  rc = make_tmap_2d(&tx, CU_TENSOR_MAP_DATA_TYPE_FLOAT16, 2, a.x, a.M, a.K, (uint64_t)a.ldx * 2, tok, 64, CU_TENSOR_MAP_SWIZZLE_128B);
+  if (rc) return rc;
+  W4Params p{};
+  p.scale = a.scale; p.scale_dtype = B2Q_F32;
+  p.out = a.out; p.ldo = a.ldo; p.out_bf16 = a.out_bf16 ? 1 : 0;
+  p.vec_out = aligned16(a.out) && (a.ldo % 8) == 0;
+  p.M = a.M; p.N = a.N; p.K = a.K; p.nk = a.K >> 6;
+  p.tok_scale = a.tok_scale;
+  p.status = umma_status_ptr();
+  if (!p.status) return B2Q_ERR_CUDA;
+  p.strips = (a.N + 127) / 128; p.tiles_n = 1;
+  rc = cut_strips(p, a, sms, a.K / 128);
+  if (rc) return rc;
+  const int work = p.units > 0 ? p.units : p.strips, grid = work < sms ? work : sms;
+  const bool overlap = tls().overlap_mode > 0 && (a.after_prep || tls().overlap_mode == 2);
+  if (tok == 16) return launch_w4<w4::WT_W8, 16, 1>(tw, tx, p, grid, overlap, st);
+  if (tok == 32) return launch_w4<w4::WT_W8, 32, 1>(tw, tx, p, grid, overlap, st);
+  return launch_w4<w4::WT_W8, 64, 1>(tw, tx, p, grid, overlap, st);
 }
 
 }  // namespace b2q

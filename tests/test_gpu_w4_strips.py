@@ -70,3 +70,25 @@ def test_many_segments_repeat_bit_for_bit(e, M, N, K):
             _check(out, ref, (M, N, K))
         assert torch.equal(out, first)
     assert e._lib.device_status() == 0
+
+
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16])
+@pytest.mark.parametrize("M,N,K", [(1, 128, 128), (16, 200, 384), (17, 1032, 640), (33, 2048, 1152), (64, 8192, 5120), (27, 17408, 5120)])
+def test_block_scaled_fp8_strips(e, M, N, K, dtype):
+    """The e4m3 form of the kernel: a weight times its fp32 block scale is rounded to fp16 once, as above; with fp16
+    output the tolerance is 2^-11 for the output's rounding and the same 2^-9 of a typical column for the weights'."""
+    g = torch.Generator(device=DEV).manual_seed(M + N + K)
+    w = (torch.randn(N, K, generator=g, device=DEV) * 96).clamp_(-448, 448).to(torch.float8_e4m3fn)
+    s = (0.5 + torch.rand((N + 127) // 128, K // 128, generator=g, device=DEV)) / 4096
+    x = torch.randn(M, K, generator=g, device=DEV).to(dtype)
+    full = s.double().repeat_interleave(128, 0)[:N].repeat_interleave(128, 1)
+    ref = x.double() @ (w.double() * full).T
+    first = None
+    for _ in range(3):
+        out = torch.full((M, N), float("nan"), dtype=dtype, device=DEV)
+        e.esimd_gemm_fp8_blockscale(x, w, s, out)
+        if first is None:
+            first = out
+            _check(out, ref, (M, N, K))
+        assert torch.equal(out, first)
+    assert e._lib.device_status() == 0
