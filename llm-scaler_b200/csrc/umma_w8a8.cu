@@ -41,6 +41,7 @@ template <int TOK> struct Cfg {
 struct W8A8Params {
   const float* xs; const float* ws;     // [M, K/128], [ceil(N/128), K/128]
   void* out; int64_t ldo; int out_bf16;
+  int vec_out;                          // rows of out are 16-byte aligned
   int M, N, K;
   int* status;
 };
@@ -164,7 +165,29 @@ umma_w8a8_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constant
     }
     if (ok) {
       const int n = n0 + quad * 32 + lane;
-      if (n < p.N) {
+      if (p.vec_out && n0 + quad * 32 + 32 <= p.N) {
+        // Turned round in shared memory (all MMAs of the CTA are done: the operand stages are free), so that a lane
+        // stores 16 bytes of a row instead of 2.
+        const uint32_t st = base + (warp - 2) * 2048;
+#pragma unroll
+        for (int h = 0; h < CPT; h += 32) {
+          __syncwarp();
+#pragma unroll
+          for (int i = 0; i < 32; ++i) {
+            const unsigned short v = p.out_bf16 ? __bfloat16_as_ushort(__float2bfloat16_rn(acc[h + i])) : __half_as_ushort(__float2half_rn(acc[h + i]));
+            asm volatile("st.shared.u16 [%0], %1;" ::"r"(st + i * 64 + lane * 2), "h"(v) : "memory");
+          }
+          __syncwarp();
+#pragma unroll
+          for (int i = 0; i < 4; ++i) {
+            const int tok = tok0 + col0 + h + i * 8 + (lane >> 2);
+            uint4 v;
+            asm volatile("ld.shared.v4.u32 {%0,%1,%2,%3}, [%4];" : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w) : "r"(st + i * 512 + lane * 16));
+            if (tok < p.M)
+              *reinterpret_cast<uint4*>(reinterpret_cast<uint16_t*>(p.out) + (int64_t)tok * p.ldo + n0 + quad * 32 + (lane & 3) * 8) = v;
+          }
+        }
+      } else if (n < p.N) {
         uint16_t* outp = reinterpret_cast<uint16_t*>(p.out);
 #pragma unroll
         for (int i = 0; i < CPT; ++i) {
@@ -390,6 +413,7 @@ int umma_w8a8_block(const UmmaW8A8Args& a, cudaStream_t st) {
   if (!tensor_map_encoder()) return B2Q_ERR_CUDA;
   W8A8Params p{};
   p.xs = a.xs; p.ws = a.ws; p.out = a.out; p.ldo = a.ldo; p.out_bf16 = a.bf16 ? 1 : 0;
+  p.vec_out = aligned16(a.out) && (a.ldo % 8) == 0;
   p.M = a.M; p.N = a.N; p.K = a.K;
   void* sym = nullptr;
   if (cudaGetSymbolAddress(&sym, g_w8a8_status) != cudaSuccess) return B2Q_ERR_CUDA;
