@@ -936,7 +936,7 @@ int umma_w8_token_tile(const UmmaW8Args& a) { return a.expert_offsets ? grouped_
 
 int umma_w8_linear(const UmmaW8Args& a, cudaStream_t st) {
   const bool grouped = a.expert_offsets != nullptr;
-  if (!grouped && a.scale_mode == B2Q_SCALE_BLOCK128 && !a.bf16 && a.M <= 64) return umma_w8_strip_linear(a, st);
+  if (umma_w8_strip_supported(a)) return umma_w8_strip_linear(a, st);
   const int E = grouped ? a.E : 1;
   const int tok = umma_w8_token_tile(a);
   CUtensorMap tw, tx;

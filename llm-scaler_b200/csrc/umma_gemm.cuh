@@ -83,7 +83,8 @@ int umma_w4_linear(const UmmaW4Args& a, cudaStream_t st);
 int umma_w4_prep_token_tile(const UmmaW4Args& a);
 int umma_w4_prep_linear(const UmmaW4Args& a, cudaStream_t st);
 size_t umma_w4_partial_bytes(int64_t M);
-// block-scaled e4m3 weights, fp16 activations, M <= 64 (B2Q_ERR_UNSUPPORTED otherwise)
+// the same kernel for e4m3 weights and fp16 activations, up to 64 tokens per tile
+bool umma_w8_strip_supported(const UmmaW8Args& a);
 int umma_w8_strip_linear(const UmmaW8Args& a, cudaStream_t st);
 
 // shared by the weight-only kernels: the device's status word, and a bank of zeroed arrival counters for cut strips

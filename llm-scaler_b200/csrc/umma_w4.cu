@@ -87,6 +87,7 @@ template <int WT, int TOK, int R> struct Cfg {
 
 struct W4Params {
   const void* scale; int scale_dtype; int64_t s_stride_n, s_stride_g, s_expert_elems;
+  int scale_mode;            // e4m3 weights: B2Q_SCALE_*; without blocks the epilogue multiplies by the scale
   int scale_vec8;            // eight consecutive groups of a row are one aligned 16-byte load
   void* out; int64_t ldo; int out_bf16;
   int vec_out;               // rows of out are 16-byte aligned
@@ -543,7 +544,13 @@ umma_w4_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constant__
           const uint32_t ta = tmem + lane_base + (b * R + rb) * C::ACC_COLS + cb;
           if constexpr (CB == 32) tmem_ld32(ta, q); else tmem_ld16(ta, q);
           tmem_ld_wait();
-          const float pm = WT == WT_W8 ? 1.f : __uint_as_float((uint32_t)(127 + post[rb * 128 + quad * 32 + lane]) << 23);
+          float pm;
+          if constexpr (WT == WT_W8) {
+            pm = 1.f;
+            if (p.scale_mode != B2Q_SCALE_BLOCK128)
+              pm = load_scalar(p.scale, sg.expert * p.s_expert_elems +
+                                            (p.scale_mode == B2Q_SCALE_CHANNEL ? min(sg.n0 + rb * 128 + quad * 32 + lane, p.N - 1) : 0), p.scale_dtype);
+          } else pm = __uint_as_float((uint32_t)(127 + post[rb * 128 + quad * 32 + lane]) << 23);
 #pragma unroll
           for (int i = 0; i < CB; ++i) r[i] = __uint_as_float(q[i]) * pm;
         }
@@ -656,8 +663,9 @@ umma_w4_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constant__
       float row_mul = 1.f;
       // e4m3: one fp32 scale per block, the same for the whole CTA, requested an iteration ahead
       const float* block_scale = reinterpret_cast<const float*>(p.scale) + (cur.block_row + rb) * (int64_t)(p.K >> 7) + cur.block_col;
-      float sf_next = 0.f;
-      if (WT == WT_W8 && gg < ngroups) sf_next = __ldg(block_scale + gg);
+      const bool blocks = WT == WT_W8 && p.scale_mode == B2Q_SCALE_BLOCK128;
+      float sf_next = 1.f;
+      if (blocks && gg < ngroups) sf_next = __ldg(block_scale + gg);
 #pragma unroll 1
       for (int sl = 0; sl < nslot; ++sl) {
         if (WT != WT_W8) ok = wait_converged(sc_full + 8 * ss, spar, abort_flag, p.status, ST_SCFULL);
@@ -674,7 +682,7 @@ umma_w4_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constant__
         for (; gg < gend; gg += KG) {
           uint32_t hv = WT == WT_W8 ? 0u : lds_u16(sca + 2 * ((gg + off) & 7));
           const float sf = sf_next;
-          if (WT == WT_W8 && gg + KG < ngroups) sf_next = __ldg(block_scale + gg + KG);
+          if (blocks && gg + KG < ngroups) sf_next = __ldg(block_scale + gg + KG);
           if (WT == WT_W8) {}
           else if (bf16_scale) hv = fp16_factor(__uint_as_float(hv << 16) * row_mul, saturated);
           else if ((hv & 0x7FFFu) - 0x7000u <= 0x0C00u) { hv = (hv & 0x8000u) | 0x6FFFu; saturated = 1; }     // above 8188, NaN stays
@@ -871,28 +879,37 @@ int umma_w4_prep_linear(const UmmaW4Args& a, cudaStream_t st) {
                 : launch_w4_tile<w4::WT_W4N>(tok, R, tw, tx, p, grid, overlap, st);
 }
 
-// Block-scaled e4m3 weights on fp16 activations, decode tiles.
+// e4m3 weights on fp16 activations, up to 64 tokens per tile: dense with block scales, grouped with one scale per channel or
+// tensor (whose transform multiplies by 1).
+bool umma_w8_strip_supported(const UmmaW8Args& a) {
+  if (a.bf16 || a.fmt != B2Q_E4M3 || (a.K % 128) != 0) return false;
+  if (a.expert_offsets) return a.scale_mode != B2Q_SCALE_BLOCK128 && grouped_tok(a.M, a.E) <= 64;
+  return a.scale_mode == B2Q_SCALE_BLOCK128 && a.M <= 64;
+}
+
 int umma_w8_strip_linear(const UmmaW8Args& a, cudaStream_t st) {
-  const int sms = sm_count(), tok = dense_tok(a.M);
-  if (a.bf16 || a.expert_offsets || a.scale_mode != B2Q_SCALE_BLOCK128 || a.fmt != B2Q_E4M3 || a.M > 64 || (a.K % 128) != 0)
-    return B2Q_ERR_UNSUPPORTED;
+  const bool grouped = a.expert_offsets != nullptr;
+  const int sms = sm_count(), tok = grouped ? grouped_tok(a.M, a.E) : dense_tok(a.M);
   CUtensorMap tw, tx;
-  int rc = make_tmap_2d(&tw, CU_TENSOR_MAP_DATA_TYPE_UINT8, 1, a.w, a.N, a.K, (uint64_t)a.K, 128, 128, CU_TENSOR_MAP_SWIZZLE_128B);
+  int rc = make_tmap_2d(&tw, CU_TENSOR_MAP_DATA_TYPE_UINT8, 1, a.w, (uint64_t)(grouped ? a.E : 1) * a.N, a.K, (uint64_t)a.K, 128, 128,
+                        CU_TENSOR_MAP_SWIZZLE_128B);
   if (rc) return rc;
   rc = make_tmap_2d(&tx, CU_TENSOR_MAP_DATA_TYPE_FLOAT16, 2, a.x, a.M, a.K, (uint64_t)a.ldx * 2, tok, 64, CU_TENSOR_MAP_SWIZZLE_128B);
   if (rc) return rc;
   W4Params p{};
-  p.scale = a.scale; p.scale_dtype = B2Q_F32;
+  p.scale = a.scale; p.scale_dtype = a.scale_dtype; p.scale_mode = a.scale_mode; p.s_expert_elems = a.s_expert_elems;
+  p.tiles = grouped ? a.tiles : nullptr; p.expert_offsets = a.expert_offsets; p.out_map = a.out_map; p.w_rows_per_expert = a.N;
   p.out = a.out; p.ldo = a.ldo; p.out_bf16 = a.out_bf16 ? 1 : 0;
   p.vec_out = aligned16(a.out) && (a.ldo % 8) == 0;
   p.M = a.M; p.N = a.N; p.K = a.K; p.nk = a.K >> 6;
   p.tok_scale = a.tok_scale;
   p.status = umma_status_ptr();
   if (!p.status) return B2Q_ERR_CUDA;
-  p.strips = (a.N + 127) / 128; p.tiles_n = 1;
-  rc = cut_strips(p, a, sms, a.K / 128);
-  if (rc) return rc;
-  const int work = p.units > 0 ? p.units : p.strips, grid = work < sms ? work : sms;
+  p.strips = (a.N + 127) / 128; p.tiles_n = grouped ? a.tile_cap : 1;
+  if (!grouped) { rc = cut_strips(p, a, sms, a.K / 128); if (rc) return rc; }
+  const int64_t work = p.units > 0 ? p.units : (int64_t)p.strips * p.tiles_n;
+  if (work > INT32_MAX) return B2Q_ERR_LIMIT;
+  const int grid = (int)(work < sms ? work : sms);
   const bool overlap = tls().overlap_mode > 0 && (a.after_prep || tls().overlap_mode == 2);
   if (tok == 16) return launch_w4<w4::WT_W8, 16, 1>(tw, tx, p, grid, overlap, st);
   if (tok == 32) return launch_w4<w4::WT_W8, 32, 1>(tw, tx, p, grid, overlap, st);
