@@ -68,14 +68,15 @@ template <int WT, int TOK, int R> struct Cfg {
   static constexpr int POST_RING = 16;                       // row exponents per segment, read by the epilogue
   static constexpr int POST_BYTES = POST_RING * ROWS;
   static constexpr int STAGE_OUT = EW * 1024;                // 16 tokens x 32 columns of output per epilogue warp
-  static constexpr int BUDGET = 232448 - 1024 /*align*/ - 1024 /*barriers*/;
+  static constexpr int TILE_TABLE = 32;                      // segments of a grouped launch whose tile every role finds in shared memory
+  static constexpr int BUDGET = 232448 - 1024 /*align*/ - 1024 /*barriers*/ - TILE_TABLE * 16;
   static constexpr int RS_FIT = (BUDGET - XS * X_BYTES - SCS * SC_BYTES - POST_BYTES - STAGE_OUT) / RAW_BYTES;
   // Raw and operand stages always belong to the same transform group(s), whatever segment they are in: a wait tells a
   // phase from the one after it, not from the one after that, so nobody may wait for a stage whose previous use was
   // somebody else's.  Hence ring depths in multiples of a round of the groups.
   static constexpr int RAW_ROUND = KG / GPS, A_ROUND = KG;
   static constexpr int RS = (RS_FIT > 12 ? 12 : RS_FIT) / RAW_ROUND * RAW_ROUND;
-  static constexpr int SMEM = XS * X_BYTES + RS * RAW_BYTES + SCS * SC_BYTES + POST_BYTES + STAGE_OUT + 1024 + 1024;
+  static constexpr int SMEM = XS * X_BYTES + RS * RAW_BYTES + SCS * SC_BYTES + POST_BYTES + STAGE_OUT + 1024 + 1024 + TILE_TABLE * 16;
   static constexpr int ACC_COLS = TOK < 32 ? 32 : TOK;
   static constexpr int NBUF = 2 * R * ACC_COLS <= 256 ? 2 : 1;   // accumulator sets
   static constexpr int A_COL0 = NBUF * R * ACC_COLS;
@@ -88,7 +89,7 @@ template <int WT, int TOK, int R> struct Cfg {
 struct W4Params {
   const void* scale; int scale_dtype; int64_t s_stride_n, s_stride_g, s_expert_elems;
   int scale_mode;            // e4m3 weights: B2Q_SCALE_*; without blocks the epilogue multiplies by the scale
-  int scale_vec8;            // eight consecutive groups of a row are one aligned 16-byte load
+  int scale_vec;             // a row's 16-bit scales can be fetched eight groups (8) or two groups (2) per aligned load; else 1
   void* out; int64_t ldo; int out_bf16;
   int vec_out;               // rows of out are 16-byte aligned
   int M, N, K;
@@ -179,8 +180,9 @@ struct Segment { int n0, c_begin, nk, strip, part, slot, tok0, xrow0, M, expert;
 // units of one raw stage and CTA b takes the units [b U / G, (b + 1) U / G): up to two partial strips around any number
 // of whole ones.  Otherwise whole (tile, strip) pairs in steps of the grid, ordered so that CTAs running at the same time
 // share what does not fit in L2 twice: dense launches the weight strip, grouped launches an expert's activation rows.
-template <int ROWS, int TOK, int GPS> struct Cursor {
+template <int ROWS, int TOK, int GPS, int TABLE> struct Cursor {
   int u, u0, u1;
+  int it; uint32_t table;            // segments handed out so far; tile table in shared memory (grouped launches)
   int block_row, block_col;          // 128 x 128 block the last segment of next_nk began with
   __device__ __forceinline__ void init(const W4Params& p, int total) {
     if (p.units > 0) {
@@ -189,7 +191,13 @@ template <int ROWS, int TOK, int GPS> struct Cursor {
     } else {
       u0 = blockIdx.x; u1 = total;
     }
-    u = u0;
+    u = u0; it = 0;
+  }
+  // {expert, first row in it, its first row, its rows} of a tile of a grouped launch
+  static __device__ __forceinline__ int4 tile_info(const W4Params& p, int tile) {
+    const int2 td = __ldcg(reinterpret_cast<const int2*>(p.tiles + 4) + tile);
+    const int x0 = __ldcg(p.expert_offsets + td.x);
+    return make_int4(td.x, td.y, x0, __ldcg(p.expert_offsets + td.x + 1) - x0);
   }
   // only the number of 64-k chunks and where in a run of eight scale groups they begin (for the roles that need no more)
   __device__ __forceinline__ int next_nk(const W4Params& p, int* off = nullptr) {
@@ -221,10 +229,11 @@ template <int ROWS, int TOK, int GPS> struct Cursor {
     if (p.tiles) {
       const int tile = u / p.strips;
       sg.strip = u - tile * p.strips;
-      const int2 td = __ldcg(reinterpret_cast<const int2*>(p.tiles + 4) + tile);
-      sg.expert = td.x; sg.tok0 = td.y;
-      sg.xrow0 = __ldcg(p.expert_offsets + td.x);
-      sg.M = __ldcg(p.expert_offsets + td.x + 1) - sg.xrow0;
+      int4 ti;
+      if (it < TABLE) asm volatile("ld.shared.v4.u32 {%0,%1,%2,%3}, [%4];" : "=r"(ti.x), "=r"(ti.y), "=r"(ti.z), "=r"(ti.w) : "r"(table + 16 * it));
+      else ti = tile_info(p, tile);
+      ++it;
+      sg.expert = ti.x; sg.tok0 = ti.y; sg.xrow0 = ti.z; sg.M = ti.w;
     } else {
       sg.strip = u / p.tiles_n;
       sg.tok0 = (u - sg.strip * p.tiles_n) * TOK;
@@ -250,7 +259,7 @@ umma_w4_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constant__
   const uint32_t raw_smem = base, x_smem = base + RS * C::RAW_BYTES, sc_smem = x_smem + XS * C::X_BYTES;
   const uint32_t post_off = RS * C::RAW_BYTES + XS * C::X_BYTES + C::SCS * C::SC_BYTES;
   int8_t* post_exp = reinterpret_cast<int8_t*>(gen + post_off);
-  const uint32_t out_smem = base + post_off + C::POST_BYTES, bar = out_smem + C::STAGE_OUT;
+  const uint32_t out_smem = base + post_off + C::POST_BYTES, tile_table = out_smem + C::STAGE_OUT, bar = tile_table + C::TILE_TABLE * 16;
   // barrier map (8 bytes each)
   const uint32_t raw_full = bar, raw_empty = raw_full + 8 * RS, x_full = raw_empty + 8 * RS, x_empty = x_full + 8 * XS;
   const uint32_t a_full = x_empty + 8 * XS, a_empty = a_full + 8 * S, sc_full = a_empty + 8 * S, sc_empty = sc_full + 8 * C::SCS;
@@ -267,8 +276,10 @@ umma_w4_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constant__
   grid_dep_release();
   int total = p.strips * p.tiles_n;
   if (p.tiles) { grid_dep_wait(); total = __ldcg(p.tiles) * p.strips; }
-  Cursor<ROWS, TOK, C::GPS> cur;
+  using Cur = Cursor<ROWS, TOK, C::GPS, C::TILE_TABLE>;
+  Cur cur;
   cur.init(p, total);
+  cur.table = tile_table;
   if (cur.u >= cur.u1) return;                       // the whole CTA: fewer pieces of work than CTAs
 
   if (threadIdx.x == 0) {
@@ -280,6 +291,15 @@ umma_w4_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constant__
     mbar_init(fix_bar, C::EW);
     *abort_flag = 0;
     fence_barrier_init();
+  }
+  // Every role needs a segment's tile; two dependent loads each, once per segment and role, cost short segments (768 k: six
+  // scale groups) more than their work.  One thread per segment fetches them all at once.
+  if (p.tiles && warp == 2) {
+    const int64_t su = (int64_t)blockIdx.x + (int64_t)lane * gridDim.x;
+    if (lane < C::TILE_TABLE && su < total) {
+      const int4 ti = Cur::tile_info(p, (int)(su / p.strips));
+      asm volatile("st.shared.v4.u32 [%0], {%1,%2,%3,%4};" ::"r"(tile_table + 16 * lane), "r"(ti.x), "r"(ti.y), "r"(ti.z), "r"(ti.w) : "memory");
+    }
   }
   if (warp == 1) { tmem_alloc(smem_u32(const_cast<uint32_t*>(tmem_slot)), 512); tmem_relinquish(); }
   tc_fence_before();
@@ -401,14 +421,24 @@ umma_w4_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constant__
       for (int sl = 0; sl < nslot; ++sl) {
         const uint32_t dst = sc_smem + ss * C::SC_BYTES + lane * 16;
         uint4 v[RI];
-        if (p.scale_vec8) {                            // requested before the slot is free
+        if (p.scale_vec == 8) {                        // requested before the slot is free
 #pragma unroll
           for (int i = 0; i < RI; ++i)
             v[i] = __ldg(reinterpret_cast<const uint4*>(sbase + ((int64_t)min(sg.n0 + lane + 32 * i, p.N - 1) * p.s_stride_n + 8 * sl) * 2));
+        } else if (p.scale_vec == 2) {                 // off, npad and ngroups are even then
+#pragma unroll
+          for (int i = 0; i < RI; ++i) {
+            const uint32_t* rp = reinterpret_cast<const uint32_t*>(sbase + ((int64_t)min(sg.n0 + lane + 32 * i, p.N - 1) * p.s_stride_n + 8 * sl) * 2);
+            const int g = 8 * sl - off;
+            v[i].x = (g >= 0 && g < ngroups) ? __ldg(rp) : 0u;
+            v[i].y = (g + 2 >= 0 && g + 2 < ngroups) ? __ldg(rp + 1) : 0u;
+            v[i].z = (g + 4 >= 0 && g + 4 < ngroups) ? __ldg(rp + 2) : 0u;
+            v[i].w = (g + 6 >= 0 && g + 6 < ngroups) ? __ldg(rp + 3) : 0u;
+          }
         }
         ok = wait_converged(sc_empty + 8 * ss, par, abort_flag, p.status, ST_SCEMPTY);
         if (!ok) break;
-        if (!p.scale_vec8) {
+        if (p.scale_vec == 1) {
 #pragma unroll
           for (int i = 0; i < RI; ++i) {
             const uint8_t* rp = sbase + ((int64_t)min(sg.n0 + lane + 32 * i, p.N - 1) * p.s_stride_n + (int64_t)(8 * sl) * p.s_stride_g) * esz;
@@ -851,7 +881,11 @@ int umma_w4_prep_linear(const UmmaW4Args& a, cudaStream_t st) {
   W4Params p{};
   p.scale = a.scale; p.scale_dtype = a.scale_dtype; p.s_stride_n = a.s_stride_n; p.s_stride_g = a.s_stride_g;
   p.s_expert_elems = (int64_t)a.N * (a.K / 128);
-  p.scale_vec8 = a.scale_dtype != B2Q_F32 && a.s_stride_g == 1 && (a.s_stride_n % 8) == 0 && (a.K % 1024) == 0 && aligned16(a.scale);
+  p.scale_vec = 1;
+  if (a.scale_dtype != B2Q_F32 && a.s_stride_g == 1) {
+    if ((a.s_stride_n % 8) == 0 && (a.K % 1024) == 0 && aligned16(a.scale)) p.scale_vec = 8;
+    else if ((a.s_stride_n % 2) == 0 && (a.K % 256) == 0 && (reinterpret_cast<uintptr_t>(a.scale) & 3u) == 0) p.scale_vec = 2;
+  }
   p.out = a.out; p.ldo = a.ldo; p.out_bf16 = a.out_bf16 ? 1 : 0;
   p.vec_out = aligned16(a.out) && (a.ldo % 8) == 0;
   p.M = a.M; p.N = a.N; p.K = a.K; p.nk = ((a.K >> 6) + 3) & ~3;
