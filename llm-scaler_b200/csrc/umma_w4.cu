@@ -122,6 +122,13 @@ __device__ __forceinline__ uint32_t lds_u16(uint32_t addr) {
   asm volatile("ld.shared.u16 %0, [%1];" : "=h"(v) : "r"(addr));
   return v;
 }
+__device__ __forceinline__ void cp_async4(uint32_t dst, const void* src, int src_bytes) {       // the rest of the four bytes is zeroed
+  asm volatile("cp.async.ca.shared.global [%0], [%1], 4, %2;" ::"r"(dst), "l"(src), "r"(src_bytes) : "memory");
+}
+// One arrival on the barrier when all copies this thread has issued have landed.
+__device__ __forceinline__ void cp_async_arrive(uint32_t bar) {
+  asm volatile("cp.async.mbarrier.arrive.noinc.shared::cta.b64 [%0];" ::"r"(bar) : "memory");
+}
 // Power of two that brings a scale into [0.5, 1) (0 for zero, subnormal, infinite and NaN scales).
 __device__ __forceinline__ int row_exponent(float first) {
   const int ex = (int)((__float_as_uint(first) >> 23) & 0xFFu);
@@ -420,25 +427,27 @@ umma_w4_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constant__
       float mul[RI];
       for (int sl = 0; sl < nslot; ++sl) {
         const uint32_t dst = sc_smem + ss * C::SC_BYTES + lane * 16;
-        uint4 v[RI];
-        if (p.scale_vec == 8) {                        // requested before the slot is free
-#pragma unroll
-          for (int i = 0; i < RI; ++i)
-            v[i] = __ldg(reinterpret_cast<const uint4*>(sbase + ((int64_t)min(sg.n0 + lane + 32 * i, p.N - 1) * p.s_stride_n + 8 * sl) * 2));
-        } else if (p.scale_vec == 2) {                 // off, npad and ngroups are even then
-#pragma unroll
-          for (int i = 0; i < RI; ++i) {
-            const uint32_t* rp = reinterpret_cast<const uint32_t*>(sbase + ((int64_t)min(sg.n0 + lane + 32 * i, p.N - 1) * p.s_stride_n + 8 * sl) * 2);
-            const int g = 8 * sl - off;
-            v[i].x = (g >= 0 && g < ngroups) ? __ldg(rp) : 0u;
-            v[i].y = (g + 2 >= 0 && g + 2 < ngroups) ? __ldg(rp + 1) : 0u;
-            v[i].z = (g + 4 >= 0 && g + 4 < ngroups) ? __ldg(rp + 2) : 0u;
-            v[i].w = (g + 6 >= 0 && g + 6 < ngroups) ? __ldg(rp + 3) : 0u;
-          }
-        }
         ok = wait_converged(sc_empty + 8 * ss, par, abort_flag, p.status, ST_SCEMPTY);
         if (!ok) break;
-        if (p.scale_vec == 1) {
+        if (p.scale_vec > 1) {
+          // Asynchronous copies, up to SCS slots ahead: a scale comes from DRAM, and with loads through registers the
+          // transform warps waited about 500 cycles per scale group for this warp (64 tokens, 256-row strips).
+#pragma unroll
+          for (int i = 0; i < RI; ++i) {
+            const uint8_t* rp = sbase + (int64_t)min(sg.n0 + lane + 32 * i, p.N - 1) * p.s_stride_n * 2;
+            if (p.scale_vec == 8) {
+              cp_async16(dst + 512 * i, rp + 16 * sl, 16);
+            } else {
+#pragma unroll
+              for (int j = 0; j < 8; j += 2) {           // off, npad and ngroups are even then
+                const int g = 8 * sl - off + j;
+                const bool in = g >= 0 && g < ngroups;
+                cp_async4(dst + 512 * i + 2 * j, in ? rp + 2 * (8 * sl + j) : rp + 2 * off, in ? 4 : 0);
+              }
+            }
+          }
+          cp_async_arrive(sc_full + 8 * ss);               // every lane for its own rows, once they have landed
+        } else {
 #pragma unroll
           for (int i = 0; i < RI; ++i) {
             const uint8_t* rp = sbase + ((int64_t)min(sg.n0 + lane + 32 * i, p.N - 1) * p.s_stride_n + (int64_t)(8 * sl) * p.s_stride_g) * esz;
@@ -459,13 +468,11 @@ umma_w4_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constant__
 #pragma unroll
               for (int j = 0; j < 8; ++j) e[j] = fp16_factor(__uint_as_float(e[j]) * mul[i], saturated);
             }
-            v[i] = make_uint4(e[0] | (e[1] << 16), e[2] | (e[3] << 16), e[4] | (e[5] << 16), e[6] | (e[7] << 16));
+            asm volatile("st.shared.v4.u32 [%0], {%1,%2,%3,%4};" ::"r"(dst + 512 * i), "r"(e[0] | (e[1] << 16)), "r"(e[2] | (e[3] << 16)),
+                         "r"(e[4] | (e[5] << 16)), "r"(e[6] | (e[7] << 16)) : "memory");
           }
+          mbar_arrive(sc_full + 8 * ss);
         }
-#pragma unroll
-        for (int i = 0; i < RI; ++i)
-          asm volatile("st.shared.v4.u32 [%0], {%1,%2,%3,%4};" ::"r"(dst + 512 * i), "r"(v[i].x), "r"(v[i].y), "r"(v[i].z), "r"(v[i].w) : "memory");
-        mbar_arrive(sc_full + 8 * ss);                 // every lane for its own rows
         if (++ss == C::SCS) { ss = 0; par ^= 1u; }
       }
       ++segno;
