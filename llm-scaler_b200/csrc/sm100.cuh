@@ -67,12 +67,28 @@ __device__ __forceinline__ bool mbar_try_wait(uint32_t bar, uint32_t parity) {
   return ok != 0;
 }
 
+// One look, without suspending the thread.
+__device__ __forceinline__ bool mbar_test(uint32_t bar, uint32_t parity) {
+  uint32_t ok;
+  asm volatile(
+      "{\n\t.reg .pred p;\n\t"
+      "mbarrier.test_wait.parity.shared::cta.b64 p, [%1], %2;\n\t"
+      "selp.u32 %0, 1, 0, p;\n\t}"
+      : "=r"(ok)
+      : "r"(bar), "r"(parity)
+      : "memory");
+  return ok != 0;
+}
+
 // Bounded wait.  `abort_flag` is a shared-memory word every role polls, so one role's
 // timeout releases all the others; `status` is a global word the host can read.  The clock
 // and the abort flag are looked at once every 128 polls so the spin itself stays two
-// instructions long.
+// instructions long.  A plain test comes before the first suspending one: where the phase is already over it is the cheaper
+// (W8A8 4096 x 17408 x 5120 566 -> 548 us; INT4 decoder layer at M = 2048 3073 -> 3014 us, at M = 64 209.4 -> 206.1 us;
+// INT4 MoE pipeline at 4096 tokens 583 -> 573 us; the other kernels are indifferent).
 __device__ __forceinline__ bool mbar_wait(uint32_t bar, uint32_t parity, volatile int* abort_flag, int* status, int code,
                                           long long limit_ticks = WAIT_LIMIT_TICKS) {
+  if (mbar_test(bar, parity)) return true;
   if (mbar_try_wait(bar, parity)) return true;
   const long long t0 = clock64();
   for (;;) {

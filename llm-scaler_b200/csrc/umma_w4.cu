@@ -108,8 +108,10 @@ struct W4Params {
 
 namespace w4 {
 // Wait of a whole warp.  The lanes leave the polling loop one by one, and what follows (tcgen05.ld / st, shuffles) wants
-// all of them together: the vote brings them back together and gives every lane the same answer.
+// all of them together: the vote brings them back together and gives every lane the same answer.  A plain test goes first,
+// for the warp as a whole: most waits of the transform warps are for a phase already over.
 __device__ __forceinline__ bool wait_converged(uint32_t bar, uint32_t parity, volatile int* abort_flag, int* status, int code) {
+  if (__all_sync(0xffffffffu, mbar_test(bar, parity))) return true;
   return __all_sync(0xffffffffu, mbar_wait(bar, parity, abort_flag, status, code)) != 0;
 }
 __device__ __forceinline__ uint32_t lds32(uint32_t addr) {

@@ -15,8 +15,9 @@
 // Work is shared out like in umma_w8_direct.cu: one CTA per strip of h <= 128 rows, h chosen for equal load
 // per SM, or, when there are few strips, strips cut along k with ordered partial sums.
 //
-// Status: measured on B200 it streams 1.2-1.9 TB/s, on a level with the two 16-bit kernels and ahead of them only
-// for few rows and a long k ([8192 x 28672] at M <= 8), which is where it is dispatched (umma_w4_i8_preferred): with
+// Status: measured on B200 it streams 1.2-1.9 TB/s, ahead of smallm_kernel for few rows and a long k ([8192 x 28672] at
+// M <= 8, 59 against 65 us), which is where it is dispatched (umma_w4_i8_preferred).  umma_w4.cu needs 43 us there, but
+// rounds (q - 8) * s to fp16, which these shapes have never had done to them.  With
 // one accumulator per group of 128 k, only four groups (32 KB of weights) fit in a CTA's tensor memory between the
 // transform and the promotion warps, and the barrier hand-offs along that chain, not arithmetic, set the pace.
 // b2q_set_force_kernel(5) selects it for every decode shape.
