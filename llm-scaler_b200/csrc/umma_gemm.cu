@@ -2,7 +2,8 @@
 //
 // The 128 weight rows of a CTA's strip are the MMA's M dimension and the tokens its N
 // dimension ("swap-AB"), so one kernel serves decode (16..64 tokens) and prefill (256-token
-// tiles).  Warp roles, one CTA of 11 to 19 warps per output tile:
+// tiles).  FP8 weights with more than 64 tokens, and whatever comes without scratch or with bf16 operands; INT4 behind the
+// pre-pass and FP8 decode tiles run on umma_w4.cu.  Warp roles, one CTA of 11 to 19 warps per output tile:
 //   warp 0     TMA producer of raw quantised weight tiles (runs up to RS stages ahead: this
 //              is the HBM stream)
 //   warp 1     tensor-memory owner and the single thread that issues tcgen05.mma
