@@ -159,10 +159,12 @@ B2Q_API int b2q_quantize_fp8(const void* w, int w_dtype, int64_t ldw, void* wq, 
  * works on and taken out of the fp32 accumulator again.  Groups within 2^13 of that first one, either
  * way, are exact; a group further below loses bits, one further above is saturated and reported
  * through b2q_device_status (code 109).
- * Without scratch the weight is rounded exactly as the torch reference rounds it.  For M <= 64
- * the scratch also holds partial sums: layers with few output rows are cut along K over several CTAs
- * per strip of rows so that they still occupy every SM; the partial sums are added in a fixed order,
- * so results are bit-reproducible from run to run.                                              */
+ * Without scratch the weight is rounded exactly as the torch reference rounds it.  For M <= 128
+ * the scratch also holds partial sums where they are used: layers with few output rows are cut along K
+ * over several CTAs per strip of rows so that they still occupy every SM; the partial sums are added in
+ * a fixed order, so results are bit-reproducible from run to run.  Scratch that holds the rewritten
+ * activations (M * K * 2 + M * 4 bytes, each part rounded up to 256) but not the partial sums keeps the
+ * pre-pass; strips then stay whole.                                                              */
 B2Q_API size_t b2q_linear_workspace_bytes(int64_t M, int64_t N, int64_t K);
 B2Q_API int b2q_linear_int4(const void* x, int act_dtype, int64_t ldx,
                     const void* w, int w_layout,
@@ -184,7 +186,8 @@ B2Q_API int b2q_linear_int4(const void* x, int act_dtype, int64_t ldx,
  *    (fp16) e4m3 terms, which reproduces it exactly (elements more than 2^14 below their row maximum
  *    lose low bits);
  *  - otherwise bf16 activations are rewritten as fp16 times a per-token power of two (exact for every
- *    element within 2^-31 of its row maximum), which makes the in-kernel fp8 decode four times cheaper. */
+ *    element within 2^-31 of its row maximum), which makes the in-kernel fp8 decode four times cheaper;
+ *    M <= 64 with block scales also keeps partial sums there, as above.                             */
 B2Q_API size_t b2q_linear_fp8_workspace_bytes(int64_t M, int64_t N, int64_t K);
 B2Q_API int b2q_linear_fp8(const void* x, int act_dtype, int64_t ldx,
                    const void* w, int fp8_format,

@@ -44,7 +44,7 @@ static inline size_t tile_list_bytes(int64_t rows, int E, int tile) {
   return align_up(16 + 8 * (size_t)((rows + tile - 1) / tile + E), 256);
 }
 
-// [pre-passed activations M x K fp16] [per-token scales] [partial sums of the balanced decode mode]
+// [pre-passed activations M x K fp16] [per-token scales] [partial sums of cut strips]
 static inline size_t ws_prep_bytes(int64_t M, int64_t K) {
   return align_up((size_t)M * (size_t)K * 2, 256) + align_up((size_t)M * 4, 256);
 }
@@ -63,17 +63,13 @@ static inline size_t ws_i8_bytes(int64_t M, int64_t K) {
          align_up((size_t)(K / 128) * 16 * 4, 256) + umma_w4_i8_partial_bytes();
 }
 
-static inline size_t partial_sum_bytes(int64_t M) {
-  const size_t a = umma_balanced_ws_bytes(M), b = umma_w4_partial_bytes(M);
-  return a > b ? a : b;
-}
-
+// What of the caller's scratch is left behind the pre-pass's part may hold partial sums; the GEMM decides whether it is enough.
 template <class Args>
-static void give_balanced_scratch(Args& ua, void* workspace, int64_t M, int64_t K) {
-  const size_t bytes = partial_sum_bytes(M);
-  if (!bytes) return;
-  ua.sk_ws = reinterpret_cast<uint8_t*>(workspace) + ws_prep_bytes(M, K);
-  ua.sk_ws_bytes = bytes;
+static void give_partial_sum_scratch(Args& ua, void* workspace, size_t workspace_bytes, int64_t M, int64_t K) {
+  const size_t front = ws_prep_bytes(M, K);
+  if (workspace_bytes <= front) return;
+  ua.sk_ws = reinterpret_cast<uint8_t*>(workspace) + front;
+  ua.sk_ws_bytes = workspace_bytes - front;
 }
 
 }  // namespace b2q
@@ -227,7 +223,7 @@ static int linear_int4_core(const void* x, int act_dtype, int64_t ldx, const voi
   // the int8 tensor-core path (umma_w4_i8.cu): decode shapes, N-major nibbles, scratch available; on request, or
   // where it measured fastest
   if (!peer && (force == 5 || (force == 0 && umma_w4_i8_preferred(M, N, K))) && umma_ok && !kmajor && M <= 16 && workspace && aligned16(workspace) &&
-      workspace_bytes >= b2q_linear_workspace_bytes(M, N, K)) {
+      workspace_bytes >= ws_i8_bytes(M, K)) {
     uint8_t* wsb = reinterpret_cast<uint8_t*>(workspace);
     float* inv = reinterpret_cast<float*>(wsb + align_up((size_t)umma_w4_i8_rows(M) * (size_t)K, 256));
     float* xsum = reinterpret_cast<float*>(reinterpret_cast<uint8_t*>(inv) + align_up((size_t)M * 4, 256));
@@ -250,8 +246,8 @@ static int linear_int4_core(const void* x, int act_dtype, int64_t ldx, const voi
   if (umma_ok && want_umma) {
     // With scratch, activations go through the pre-pass (fp16, per-token power-of-two scale, pair order of
     // the magic-number transform) and the transform's integer work drops from 12 to 5 operations per word.
-    const bool prep = workspace && aligned16(workspace) && workspace_bytes >= b2q_linear_workspace_bytes(M, N, K) &&
-                      force != 3;
+    // The pre-pass asks for its own part only: scratch that a caller sized for another M or N still gets it.
+    const bool prep = workspace && aligned16(workspace) && workspace_bytes >= ws_prep_bytes(M, K) && force != 3;
     ua.out_bf16 = ua.bf16;
     if (prep) {
       float* inv = reinterpret_cast<float*>(reinterpret_cast<uint8_t*>(workspace) + align_up((size_t)M * (size_t)K * 2, 256));
@@ -259,7 +255,7 @@ static int linear_int4_core(const void* x, int act_dtype, int64_t ldx, const voi
       int rc = act_prep(x, act_dtype == B2Q_BF16, false, ldx, nullptr, 1, workspace, inv, M, (int)K, perm, st);
       if (rc) return rc;
       ua.x = workspace; ua.ldx = K; ua.bf16 = false; ua.tok_scale = inv; ua.magic = true; ua.after_prep = true;
-      give_balanced_scratch(ua, workspace, M, K);
+      give_partial_sum_scratch(ua, workspace, workspace_bytes, M, K);
     }
     return umma_w4_linear(ua, st);
   }
@@ -307,12 +303,11 @@ int b2q_linear_int4_allreduce(const void* x, int act_dtype, int64_t ldx, const v
 }
 
 size_t b2q_linear_workspace_bytes(int64_t M, int64_t N, int64_t K) {
-  (void)N;
-  const size_t a = ws_prep_bytes(M, K) + partial_sum_bytes(M), b = ws_i8_bytes(M, K);
+  const size_t a = ws_prep_bytes(M, K) + umma_w4_partial_bytes(M, N, K), b = ws_i8_bytes(M, K);
   return a > b ? a : b;
 }
 size_t b2q_linear_fp8_workspace_bytes(int64_t M, int64_t N, int64_t K) {
-  const size_t a = b2q_linear_workspace_bytes(M, N, K), b = ws_direct_bytes(M, K);
+  const size_t a = ws_prep_bytes(M, K) + umma_w8_strip_partial_bytes(M, N, K), b = ws_direct_bytes(M, K);
   return a > b ? a : b;
 }
 
@@ -344,11 +339,10 @@ static int linear_fp8_core(const void* x, int act_dtype, int64_t ldx, const void
   ua.out = out; ua.ldo = ldo; ua.M = (int)M; ua.N = (int)N; ua.K = (int)K;
   const bool umma_ok = umma_w8_supported(ua);
   // bf16 activations + scratch: convert them once to per-token-scaled fp16 so the weight decode is one cvt per pair
-  const bool have_ws = workspace && aligned16(workspace) && workspace_bytes >= b2q_linear_fp8_workspace_bytes(M, N, K) &&
-                       force != 3;
+  const bool have_ws = workspace && aligned16(workspace) && force != 3;
   // decode shapes with one scale per row or per tensor: weights stay e4m3 all the way into the 8-bit MMA, the
   // activations are split into e4m3 terms instead (exact), see umma_w8_direct.cu
-  if (force == 0 && have_ws && M <= 64 && scale_mode != B2Q_SCALE_BLOCK128 && umma_ok) {
+  if (force == 0 && have_ws && M <= 64 && workspace_bytes >= ws_direct_bytes(M, K) && scale_mode != B2Q_SCALE_BLOCK128 && umma_ok) {
     float* inv = reinterpret_cast<float*>(reinterpret_cast<uint8_t*>(workspace) +
                                           align_up((size_t)umma_w8_direct_rows(M, false) * (size_t)K, 256));
     // with a norm front end, ONE pre-pass launch does residual add, RMSNorm (normed_out = x) and the term split
@@ -369,7 +363,7 @@ static int linear_fp8_core(const void* x, int act_dtype, int64_t ldx, const void
                             act_dtype == B2Q_BF16, M, (int)K, nf->eps, nf->scalar, st);
     if (rc) return rc;
   }
-  const bool prep = act_dtype == B2Q_BF16 && have_ws && (K % 8) == 0;
+  const bool prep = act_dtype == B2Q_BF16 && have_ws && workspace_bytes >= ws_prep_bytes(M, K) && (K % 8) == 0;
   const bool want_umma = force >= 2 || (force == 0 && (M > 4 || prep || act_dtype == B2Q_F16));
   if (umma_ok && want_umma) {
     if (prep) {
@@ -378,7 +372,7 @@ static int linear_fp8_core(const void* x, int act_dtype, int64_t ldx, const void
       if (rc) return rc;
       ua.x = workspace; ua.ldx = K; ua.bf16 = false; ua.out_bf16 = true; ua.tok_scale = inv; ua.after_prep = true;
     }
-    if (have_ws) give_balanced_scratch(ua, workspace, M, K);
+    if (have_ws) give_partial_sum_scratch(ua, workspace, workspace_bytes, M, K);
     return umma_w8_linear(ua, st);
   }
 

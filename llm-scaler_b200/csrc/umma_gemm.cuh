@@ -14,8 +14,7 @@ struct UmmaGroupArgs {
   const int32_t* tiles = nullptr;           // device tile list {n, pad3, int2...}
   int tile_cap = 0;
   int64_t s_expert_elems = 0;
-  // scratch for the balanced decode mode (partial sums of strips cut between CTAs), umma_balanced_ws_bytes(M)
-  // bytes; without it every strip is one CTA's job
+  // scratch for the partial sums of strips cut between CTAs; where it is too small every strip is one CTA's job
   void* sk_ws = nullptr; size_t sk_ws_bytes = 0;
   // the activation pre-pass of the same call was launched directly before this GEMM: everything older on the
   // stream is then known to be complete, so the weight stream may start before the pre-pass has finished
@@ -82,10 +81,11 @@ int umma_w4_linear(const UmmaW4Args& a, cudaStream_t st);
 // umma_w4.cu: the INT4 GEMM behind the activation pre-pass (a.magic), and its scratch for partial sums (a.sk_ws)
 int umma_w4_prep_token_tile(const UmmaW4Args& a);
 int umma_w4_prep_linear(const UmmaW4Args& a, cudaStream_t st);
-size_t umma_w4_partial_bytes(int64_t M);
+size_t umma_w4_partial_bytes(int64_t M, int64_t N, int64_t K);
 // the same kernel for e4m3 weights and fp16 activations, up to 64 tokens per tile
 bool umma_w8_strip_supported(const UmmaW8Args& a);
 int umma_w8_strip_linear(const UmmaW8Args& a, cudaStream_t st);
+size_t umma_w8_strip_partial_bytes(int64_t M, int64_t N, int64_t K);
 
 // shared by the weight-only kernels: the device's status word, and a bank of zeroed arrival counters for cut strips
 constexpr int UMMA_MAX_CUT_STRIPS = 1024;

@@ -805,12 +805,29 @@ static int grouped_tok(int rows, int E) {
   return avg <= 16 ? 16 : (avg <= 32 ? 32 : (avg <= 96 ? 64 : 128));
 }
 
-// Scratch for the partial sums of cut strips: two slots per CTA of 128 rows (256 where the tall strip is possible) x tokens.
-size_t umma_w4_partial_bytes(int64_t M) {
-  if (M > 128) return 0;
-  const int tok = dense_tok(M);
-  return (size_t)2 * sm_count() * (tok >= 64 ? 256 : 128) * tok * sizeof(float);
+// How one token tile of a dense launch is shared out: strips of R x 128 rows, cut along k, raw stage by raw stage, when whole
+// ones would leave more than a twentieth of the machine idle in the last round.
+struct StripPlan { int R, strips, sps, units, grid; size_t partial_bytes; };      // sps, units: raw stages per strip and in total, 0 = whole strips
+static StripPlan plan_strips(int64_t M, int64_t N, int64_t K, int k_per_stage, bool tall) {
+  StripPlan pl{};
+  const int sms = sm_count(), tok = dense_tok(M);
+  const int64_t strips2 = (N + 255) / 256;
+  pl.R = tall && tok >= 64 && strips2 >= sms ? 2 : 1;          // the tall strip where it still gives every SM one
+  const int64_t strips = pl.R == 2 ? strips2 : (N + 127) / 128, units = strips * (K / k_per_stage);
+  pl.strips = (int)strips;
+  pl.grid = (int)(strips < sms ? strips : sms);
+  if (M > tok || (K % k_per_stage) != 0 || strips > UMMA_MAX_CUT_STRIPS || units > INT32_MAX) return pl;
+  if ((double)strips / ((double)((strips + sms - 1) / sms) * sms) > 0.95) return pl;
+  pl.sps = (int)(K / k_per_stage); pl.units = (int)units;
+  pl.grid = (int)(units < sms ? units : sms);
+  pl.partial_bytes = (size_t)2 * pl.grid * pl.R * 128 * tok * sizeof(float);       // two slots per CTA
+  return pl;
 }
+static StripPlan plan_w4(int64_t M, int64_t N, int64_t K) { return plan_strips(M, N, K, 256, true); }
+static StripPlan plan_w8(int64_t M, int64_t N, int64_t K) { return plan_strips(M, N, K, 128, false); }
+
+size_t umma_w4_partial_bytes(int64_t M, int64_t N, int64_t K) { return M > 0 && N > 0 ? plan_w4(M, N, K).partial_bytes : 0; }
+size_t umma_w8_strip_partial_bytes(int64_t M, int64_t N, int64_t K) { return M > 0 && M <= 64 && N > 0 ? plan_w8(M, N, K).partial_bytes : 0; }
 
 template <int WT, int TOK, int R>
 static int launch_w4(const CUtensorMap& tw, const CUtensorMap& tx, const W4Params& p, int grid, bool overlap, cudaStream_t st) {
@@ -837,18 +854,13 @@ static int launch_w4_tile(int tok, int R, const CUtensorMap& tw, const CUtensorM
   return R == 2 ? launch_w4<WT, 128, 2>(tw, tx, p, grid, overlap, st) : launch_w4<WT, 128, 1>(tw, tx, p, grid, overlap, st);
 }
 
-// Cuts the strips along k, raw stage by raw stage, when whole ones would leave more than a twentieth of the machine idle in
-// the last round (one token tile only).
+// Takes the plan's cut over where the caller's scratch holds its partial sums; without it every strip stays whole.
 template <class Args>
-static int cut_strips(W4Params& p, const Args& a, int sms, int stages_per_strip) {
-  if (p.strips > UMMA_MAX_CUT_STRIPS || !a.sk_ws || !aligned16(a.sk_ws) || a.sk_ws_bytes < umma_w4_partial_bytes(a.M) || tls().force_kernel == 4)
-    return B2Q_OK;
-  const double eff = (double)p.strips / ((double)((p.strips + sms - 1) / sms) * sms);
-  const int64_t units = (int64_t)p.strips * stages_per_strip;
-  if (eff > 0.95 || units > INT32_MAX) return B2Q_OK;
+static int cut_strips(W4Params& p, const Args& a, const StripPlan& pl) {
+  if (!pl.units || !a.sk_ws || !aligned16(a.sk_ws) || a.sk_ws_bytes < pl.partial_bytes || tls().force_kernel == 4) return B2Q_OK;
   p.counters = umma_strip_counters();
   if (!p.counters) return B2Q_ERR_CUDA;
-  p.sps = stages_per_strip; p.units = (int)units; p.partials = reinterpret_cast<float*>(a.sk_ws);
+  p.sps = pl.sps; p.units = pl.units; p.partials = reinterpret_cast<float*>(a.sk_ws);
   return B2Q_OK;
 }
 
@@ -863,14 +875,15 @@ int umma_w4_prep_linear(const UmmaW4Args& a, cudaStream_t st) {
   const int tiles = grouped ? a.tile_cap : (a.M + tok - 1) / tok;
   const int strips1 = (a.N + 127) / 128, strips2 = (a.N + 255) / 256;
   // 256-row strips move fewer bytes per flop, 128-row strips give twice the pieces of work.  A single token tile takes the
-  // tall strip when that still gives every SM one; several weigh the rounds over the SMs against 1.3 times the time per
-  // row block of the short strip.
+  // tall strip when that still gives every SM one (plan_strips); several weigh the rounds over the SMs against 1.3 times the
+  // time per row block of the short strip.
+  const StripPlan pl = grouped || tiles > 1 ? StripPlan{} : plan_w4(a.M, a.N, a.K);
   int R = 1;
   if (tok >= 64) {
     if (grouped) {
       R = a.N >= 256 ? 2 : 1;
     } else if (tiles == 1) {
-      R = strips2 >= sms ? 2 : 1;
+      R = pl.R;
     } else {
       const int64_t r1 = ((int64_t)strips1 * tiles + sms - 1) / sms, r2 = ((int64_t)strips2 * tiles + sms - 1) / sms;
       R = 20 * r2 <= 13 * r1 ? 2 : 1;
@@ -906,11 +919,9 @@ int umma_w4_prep_linear(const UmmaW4Args& a, cudaStream_t st) {
   if (!p.status) return B2Q_ERR_CUDA;
   p.strips = R == 2 ? strips2 : strips1; p.tiles_n = tiles;
   int64_t work = (int64_t)p.strips * tiles;
-  if (!grouped && tiles == 1 && (a.K % 256) == 0) {
-    rc = cut_strips(p, a, sms, a.K / 256);
-    if (rc) return rc;
-    if (p.units > 0) work = p.units;
-  }
+  rc = cut_strips(p, a, pl);
+  if (rc) return rc;
+  if (p.units > 0) work = p.units;
   if (work > INT32_MAX) return B2Q_ERR_LIMIT;
   if (a.peer) {
     if (tok > 64 || grouped || (a.N % 128) != 0 || (a.peer->slice % 128) != 0 || a.peer->M != a.M) return B2Q_ERR_UNSUPPORTED;
@@ -949,7 +960,7 @@ int umma_w8_strip_linear(const UmmaW8Args& a, cudaStream_t st) {
   p.status = umma_status_ptr();
   if (!p.status) return B2Q_ERR_CUDA;
   p.strips = (a.N + 127) / 128; p.tiles_n = grouped ? a.tile_cap : 1;
-  if (!grouped) { rc = cut_strips(p, a, sms, a.K / 128); if (rc) return rc; }
+  if (!grouped) { rc = cut_strips(p, a, plan_w8(a.M, a.N, a.K)); if (rc) return rc; }
   const int64_t work = p.units > 0 ? p.units : (int64_t)p.strips * p.tiles_n;
   if (work > INT32_MAX) return B2Q_ERR_LIMIT;
   const int grid = (int)(work < sms ? work : sms);

@@ -111,3 +111,21 @@ def test_grouped_fp8_per_expert_scale(e, rows, N, K):
     err = (out.double() - ref).norm() / ref.norm()
     assert float(err) < 2.0 ** -11, float(err)
     assert e._lib.device_status() == 0
+
+
+@pytest.mark.parametrize("M,N,K", [(100, 2048, 2048), (64, 2048, 4096), (100, 5120, 8192)])
+def test_scratch_without_room_for_partial_sums_keeps_the_pre_pass(e, M, N, K):
+    """Scratch that a caller sized for another M: the activations are rewritten as ever (two launches), strips stay whole.
+    The sums differ from those of cut strips in their order alone, so both stay within the tolerance."""
+    L = e._lib
+    x, w, s, ref = _case(M, N, K, torch.bfloat16, 11)
+    up = lambda n: (n + 255) // 256 * 256
+    for size in (up(2 * M * K) + up(4 * M), 2 * (up(2 * M * K) + up(4 * M))):
+        ws = torch.empty(size, dtype=torch.uint8, device=DEV)
+        out = torch.full((M, N), float("nan"), dtype=torch.bfloat16, device=DEV)
+        before = e.launch_count()
+        L.check(L.lib.b2q_linear_int4(x.data_ptr(), L.BF16, K, w.data_ptr(), L.W4_NMAJOR, s.data_ptr(), L.BF16, K // 128, 1,
+                                      out.data_ptr(), N, M, N, K, 128, ws.data_ptr(), size, torch.cuda.current_stream().cuda_stream))
+        assert e.launch_count() - before == 2
+        _check(out, ref, (M, N, K, size))
+    assert e._lib.device_status() == 0
