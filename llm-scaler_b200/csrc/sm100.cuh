@@ -119,17 +119,13 @@ __device__ __forceinline__ void drain_issued(uint32_t full0, int depth, int issu
   }
 }
 
-// Whole-warp wait: lane 0 spins, the other lanes park at the shuffle, then every lane observes
-// the completed phase itself (one try_wait that succeeds at once) so each has its own acquire.
+// Wait of a whole warp, for every role that is not one elected thread.  The lanes leave the polling loop of mbar_wait one by
+// one and may give up one by one, and what follows such a wait (tcgen05.ld / st, shuffles, __syncwarp) wants all of them
+// together and of one mind: the vote brings them back together and gives every lane the same answer.  A plain test goes
+// first, for the warp as a whole: most waits of the transform and promotion warps are for a phase already over.
 __device__ __forceinline__ bool mbar_wait_warp(uint32_t bar, uint32_t parity, volatile int* abort_flag, int* status, int code) {
-  int ok = 1;
-  if ((threadIdx.x & 31) == 0) ok = mbar_wait(bar, parity, abort_flag, status, code) ? 1 : 0;
-  ok = __shfl_sync(0xffffffffu, ok, 0);
-  if (ok) {
-    int guard = 0;
-    while (!mbar_try_wait(bar, parity) && ++guard < 1024) {}
-  }
-  return ok != 0;
+  if (__all_sync(0xffffffffu, mbar_test(bar, parity))) return true;
+  return __all_sync(0xffffffffu, mbar_wait(bar, parity, abort_flag, status, code)) != 0;
 }
 
 // ---- TMA: 2-D tiled load global -> shared, completion on an mbarrier -------------------

@@ -413,7 +413,7 @@ umma_wo_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constant__
         const int gr = grb + c / CPR;
         j = c % CPR; rs = gr % RS; rpar = (uint32_t)(gr / RS) & 1u;
       }
-      ok = mbar_wait(raw_full + 8 * rs, rpar, abort_flag, p.status, ST_RAWFULL);
+      ok = mbar_wait_warp(raw_full + 8 * rs, rpar, abort_flag, p.status, ST_RAWFULL);
       if (!ok) break;
       const float sc_cur = scale_value(sr_cur);
       const uint32_t rawrow = raw_smem + rs * Cfg::RAW_BYTES + t * 128;     // N-major / fp8: this thread's row
@@ -421,7 +421,7 @@ umma_wo_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constant__
       {
         const int g = gb + c, s = g % S;
         // no test for the ring's first round: a wait for the phase before a fresh barrier's first one returns at once
-        { ok = mbar_wait(ab_empty + 8 * s, ((g / S) + 1) & 1, abort_flag, p.status, ST_EMPTY); if (!ok) break; }
+        { ok = mbar_wait_warp(ab_empty + 8 * s, ((g / S) + 1) & 1, abort_flag, p.status, ST_EMPTY); if (!ok) break; }
         tc_fence_after();
         const uint32_t ta = tmem + ((uint32_t)((warp & 3) * 32) << 16) + Cfg::A_COL0 + 32 * s;
         {
@@ -508,7 +508,7 @@ umma_wo_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constant__
     if (!ok) break;
 
     // ---------------- epilogue of this segment ----------------
-    { ok = mbar_wait(accum_full, si & 1, abort_flag, p.status, ST_ACCUM); }
+    { ok = mbar_wait_warp(accum_full, si & 1, abort_flag, p.status, ST_ACCUM); }
     if (!ok) break;
     tc_fence_after();
     const int quad = warp & 3;                   // tensor-memory lane quadrant this warp may read
@@ -563,6 +563,7 @@ umma_wo_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constant__
 #pragma unroll 1
     for (int cb = cgrp * CB; cb < TOK; cb += NG * CB) {
       if (tok0 + cb >= M) break;
+      __syncwarp();                              // the stores of the last block were per lane
       uint32_t r[32];
       if constexpr (CB == 32) tmem_ld32(tmem + ((uint32_t)(quad * 32) << 16) + cb, r);
       else { uint32_t r16[16]; tmem_ld16(tmem + ((uint32_t)(quad * 32) << 16) + cb, r16);
@@ -594,7 +595,7 @@ umma_wo_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constant__
       if (peer_flag && !sg.part) {
         // all epilogue threads have issued their stores of this strip; one of them publishes it
         mbar_arrive(fix_bar);
-        ok = mbar_wait(fix_bar, fixn & 1, abort_flag, p.status, ST_FIXUP); ++fixn;
+        ok = mbar_wait_warp(fix_bar, fixn & 1, abort_flag, p.status, ST_FIXUP); ++fixn;
         if (!ok) break;
         if (threadIdx.x == Cfg::CW * 32) {
           __threadfence_system();
@@ -612,7 +613,7 @@ umma_wo_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constant__
       // device-scope fence then orders all of them before the count.  A fence per thread in front of the barrier adds
       // nothing to that and cost 0.7 % of a decode layer.
       mbar_arrive(fix_bar);
-      ok = mbar_wait(fix_bar, fixn & 1, abort_flag, p.status, ST_FIXUP); ++fixn;
+      ok = mbar_wait_warp(fix_bar, fixn & 1, abort_flag, p.status, ST_FIXUP); ++fixn;
       if (!ok) break;
       if (threadIdx.x == Cfg::CW * 32) {
         __threadfence();                               // orders the partial sums of all epilogue threads before the count
@@ -622,7 +623,7 @@ umma_wo_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constant__
         *last_flag = last;
       }
       mbar_arrive(fix_bar);
-      ok = mbar_wait(fix_bar, fixn & 1, abort_flag, p.status, ST_FIXUP); ++fixn;
+      ok = mbar_wait_warp(fix_bar, fixn & 1, abort_flag, p.status, ST_FIXUP); ++fixn;
       if (!ok) break;
       const int cb = cgrp * CB;
       if (*last_flag && cb < TOK && cb < M) {
@@ -641,7 +642,7 @@ umma_wo_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constant__
       }
       if (*last_flag && peer_flag) {
         mbar_arrive(fix_bar);
-        ok = mbar_wait(fix_bar, fixn & 1, abort_flag, p.status, ST_FIXUP); ++fixn;
+        ok = mbar_wait_warp(fix_bar, fixn & 1, abort_flag, p.status, ST_FIXUP); ++fixn;
         if (!ok) break;
         if (threadIdx.x == Cfg::CW * 32) {
           __threadfence_system();

@@ -107,13 +107,6 @@ struct W4Params {
 };
 
 namespace w4 {
-// Wait of a whole warp.  The lanes leave the polling loop one by one, and what follows (tcgen05.ld / st, shuffles) wants
-// all of them together: the vote brings them back together and gives every lane the same answer.  A plain test goes first,
-// for the warp as a whole: most waits of the transform warps are for a phase already over.
-__device__ __forceinline__ bool wait_converged(uint32_t bar, uint32_t parity, volatile int* abort_flag, int* status, int code) {
-  if (__all_sync(0xffffffffu, mbar_test(bar, parity))) return true;
-  return __all_sync(0xffffffffu, mbar_wait(bar, parity, abort_flag, status, code)) != 0;
-}
 __device__ __forceinline__ uint32_t lds32(uint32_t addr) {
   uint32_t v;
   asm volatile("ld.shared.u32 %0, [%1];" : "=r"(v) : "r"(addr));
@@ -429,7 +422,7 @@ umma_w4_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constant__
       float mul[RI];
       for (int sl = 0; sl < nslot; ++sl) {
         const uint32_t dst = sc_smem + ss * C::SC_BYTES + lane * 16;
-        ok = wait_converged(sc_empty + 8 * ss, par, abort_flag, p.status, ST_SCEMPTY);
+        ok = mbar_wait_warp(sc_empty + 8 * ss, par, abort_flag, p.status, ST_SCEMPTY);
         if (!ok) break;
         if (p.scale_vec > 1) {
           // Asynchronous copies, up to SCS slots ahead: a scale comes from DRAM, and with loads through registers the
@@ -492,7 +485,7 @@ umma_w4_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constant__
     int segno = 0, fixn = 0, b = 0;
     uint32_t bpar = 0u;
     while (ok && cur.next(p, sg)) {
-      ok = wait_converged(acc_full + 8 * b, bpar, abort_flag, p.status, ST_ACCUM);
+      ok = mbar_wait_warp(acc_full + 8 * b, bpar, abort_flag, p.status, ST_ACCUM);
       if (!ok) break;
       tc_fence_after();
       const int8_t* post = post_exp + (segno % C::POST_RING) * ROWS;
@@ -577,6 +570,7 @@ umma_w4_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constant__
       for (int rc = cgrp; rc < BLOCKS; rc += CG) {
         const int rb = rc / (TOK / CB), cb = (rc % (TOK / CB)) * CB;
         if (sg.tok0 + cb >= sg.M) continue;
+        __syncwarp();                              // the stores of the last block were per lane
         float r[CB];
         {
           uint32_t q[CB];
@@ -610,7 +604,7 @@ umma_w4_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constant__
       auto all_epilogue_warps = [&]() -> bool {
         __syncwarp();
         if (lane == 0) mbar_arrive(fix_bar);
-        const bool r = wait_converged(fix_bar, fixn & 1, abort_flag, p.status, ST_FIXUP);
+        const bool r = mbar_wait_warp(fix_bar, fixn & 1, abort_flag, p.status, ST_FIXUP);
         ++fixn;
         return r;
       };
@@ -707,7 +701,7 @@ umma_w4_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constant__
       if (blocks && gg < ngroups) sf_next = __ldg(block_scale + gg);
 #pragma unroll 1
       for (int sl = 0; sl < nslot; ++sl) {
-        if (WT != WT_W8) ok = wait_converged(sc_full + 8 * ss, spar, abort_flag, p.status, ST_SCFULL);
+        if (WT != WT_W8) ok = mbar_wait_warp(sc_full + 8 * ss, spar, abort_flag, p.status, ST_SCFULL);
         if (!ok) break;
         const uint32_t sca = sc0 + ss * C::SC_BYTES;
         if (WT != WT_W8 && sl == 0 && p.scale_dtype != B2Q_F32) {
@@ -726,7 +720,7 @@ umma_w4_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constant__
           else if (bf16_scale) hv = fp16_factor(__uint_as_float(hv << 16) * row_mul, saturated);
           else if ((hv & 0x7FFFu) - 0x7000u <= 0x0C00u) { hv = (hv & 0x8000u) | 0x6FFFu; saturated = 1; }     // above 8188, NaN stays
           const uint32_t m2 = hv | (hv << 16);
-          ok = wait_converged(raw_full + 8 * rs, rpar, abort_flag, p.status, ST_RAWFULL);
+          ok = mbar_wait_warp(raw_full + 8 * rs, rpar, abort_flag, p.status, ST_RAWFULL);
           if (!ok) break;
           const uint32_t rowa = row0 + rs * C::RAW_BYTES;
           const uint32_t ta = ta0 + 64 * R * as;
@@ -753,7 +747,7 @@ umma_w4_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constant__
               w4_word_magic(w2, m2, mk, a16 + 8); w4_word_magic(w3, m2, mk, a16 + 12);
             }
             if (q == 0) {                          // the first quarter is converted while the stage is still being read
-              ok = wait_converged(a_empty + 8 * as, apar, abort_flag, p.status, ST_EMPTY);
+              ok = mbar_wait_warp(a_empty + 8 * as, apar, abort_flag, p.status, ST_EMPTY);
               if (!ok) break;
               tc_fence_after();
             }

@@ -207,10 +207,10 @@ umma_w4_i8_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constan
         const int c = gc + j, r = gr + (j >> 1), rs = r % RS;
         const bool mine = (j & 1) == team;
         if (mine) {
-          { ok = mbar_wait(raw_full + 8 * rs, (r / RS) & 1, abort_flag, p.status, ST_RAWFULL); }
+          { ok = mbar_wait_warp(raw_full + 8 * rs, (r / RS) & 1, abort_flag, p.status, ST_RAWFULL); }
           if (!ok) break;
           const int sa = c % SA;
-          if (c >= SA) { ok = mbar_wait(a_empty + 8 * sa, ((c / SA) - 1) & 1, abort_flag, p.status, ST_AEMPTY); if (!ok) break; }
+          if (c >= SA) { ok = mbar_wait_warp(a_empty + 8 * sa, ((c / SA) - 1) & 1, abort_flag, p.status, ST_AEMPTY); if (!ok) break; }
           tc_fence_after();
           const uint32_t rawrow = raw_smem + rs * C::RAW_BYTES + t * 128;
 #pragma unroll
@@ -291,7 +291,7 @@ umma_w4_i8_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constan
                 xv[mb * 8 + 4] = x1.x; xv[mb * 8 + 5] = x1.y; xv[mb * 8 + 6] = x1.z; xv[mb * 8 + 7] = x1.w;
               }
             }
-            { ok = mbar_wait(acc_full + 8 * nb, (gc / NB) & 1, abort_flag, p.status, ST_ACCFULL); }
+            { ok = mbar_wait_warp(acc_full + 8 * nb, (gc / NB) & 1, abort_flag, p.status, ST_ACCFULL); }
             if (ok) {
               tc_fence_after();
               const float scj = scalar_from_raw(sc_raw[j], p.scale_dtype);
@@ -340,7 +340,7 @@ umma_w4_i8_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constan
         const int64_t us = (int64_t)sg.strip * p.sps, ue = us + p.sps - 1;
         const int b_lo = (int)(((us + 1) * G + U - 1) / U) - 1, b_hi = (int)(((ue + 1) * G + U - 1) / U) - 1;
         mbar_arrive(fix_bar);          // hands this thread's partial sums to the leader, whose fence orders them before the count
-        ok = mbar_wait(fix_bar, fixn & 1, abort_flag, p.status, ST_FIXUP); ++fixn;
+        ok = mbar_wait_warp(fix_bar, fixn & 1, abort_flag, p.status, ST_FIXUP); ++fixn;
         if (!ok) break;
         if (threadIdx.x == 4 * 32) {
           __threadfence();
@@ -350,7 +350,7 @@ umma_w4_i8_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constan
           *last_flag = last;
         }
         mbar_arrive(fix_bar);
-        ok = mbar_wait(fix_bar, fixn & 1, abort_flag, p.status, ST_FIXUP); ++fixn;
+        ok = mbar_wait_warp(fix_bar, fixn & 1, abort_flag, p.status, ST_FIXUP); ++fixn;
         if (!ok) break;
         if (*last_flag) {
           __threadfence();

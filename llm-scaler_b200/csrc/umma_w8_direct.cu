@@ -196,7 +196,7 @@ umma_w8_direct_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_con
     int si = 0, fixn = 0;
     while (ok && next_segment(sg)) {
       const int buf = si & 1;
-      ok = mbar_wait(accum_full + 8 * buf, (si >> 1) & 1, abort_flag, p.status, ST_ACCUM);
+      ok = mbar_wait_warp(accum_full + 8 * buf, (si >> 1) & 1, abort_flag, p.status, ST_ACCUM);
       if (!ok) break;
       tc_fence_after();
       const int n = sg.n0 + rowi;
@@ -221,6 +221,7 @@ umma_w8_direct_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_con
       };
 #pragma unroll 1
       for (int m0 = 0; m0 < p.M; m0 += 8) {
+        __syncwarp();                              // the stores of the last block were per lane
         uint32_t a[8], b[8], c[8];
         tmem_ld8(trow + m0, a);
         tmem_ld8(trow + p.Mp + m0, b);
@@ -246,7 +247,7 @@ umma_w8_direct_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_con
         const int64_t us = (int64_t)sg.strip * p.sps, ue = us + p.sps - 1;
         const int b_lo = (int)(((us + 1) * G + U - 1) / U) - 1, b_hi = (int)(((ue + 1) * G + U - 1) / U) - 1;
         mbar_arrive(fix_bar);          // hands this thread's partial sums to the leader, whose fence orders them before the count
-        ok = mbar_wait(fix_bar, fixn & 1, abort_flag, p.status, ST_FIXUP); ++fixn;
+        ok = mbar_wait_warp(fix_bar, fixn & 1, abort_flag, p.status, ST_FIXUP); ++fixn;
         if (!ok) break;
         if (threadIdx.x == 3 * 32) {
           __threadfence();                             // orders the partial sums of all 128 threads before the count
@@ -256,7 +257,7 @@ umma_w8_direct_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_con
           *last_flag = last;
         }
         mbar_arrive(fix_bar);
-        ok = mbar_wait(fix_bar, fixn & 1, abort_flag, p.status, ST_FIXUP); ++fixn;
+        ok = mbar_wait_warp(fix_bar, fixn & 1, abort_flag, p.status, ST_FIXUP); ++fixn;
         if (!ok) break;
         if (*last_flag) {
           __threadfence();

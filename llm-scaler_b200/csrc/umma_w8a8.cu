@@ -138,7 +138,7 @@ umma_w8a8_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constant
 #pragma unroll 1
     for (int kb = 0; kb < nkb; ++kb) {
       const int b = kb % NBUF;
-      ok = mbar_wait(acc_full + 8 * b, (kb / NBUF) & 1, abort_flag, p.status, ST_ACCFULL);
+      ok = mbar_wait_warp(acc_full + 8 * b, (kb / NBUF) & 1, abort_flag, p.status, ST_ACCFULL);
       if (!ok) break;
       tc_fence_after();
 #pragma unroll
@@ -316,7 +316,7 @@ umma_w8a8_pair_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_con
 #pragma unroll 1
     for (int kb = 0; kb < nkb; ++kb) {
       const int b = kb % NBUF;
-      ok = mbar_wait(acc_full + 8 * b, (kb / NBUF) & 1, abort_flag, p.status, ST_ACCFULL);
+      ok = mbar_wait_warp(acc_full + 8 * b, (kb / NBUF) & 1, abort_flag, p.status, ST_ACCFULL);
       if (!ok) break;
       tc_fence_after();
       uint32_t r0[32];

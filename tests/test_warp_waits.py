@@ -1,0 +1,41 @@
+"""Every barrier wait of a whole warp brings its lanes back together.
+
+tcgen05.ld / st, shuffles and __syncwarp need all lanes of a warp at the same instruction, and mbar_wait() lets them leave, or
+give up, one by one.  Only the branch of one elected thread may call it; everything else goes through mbar_wait_warp().
+Undefined behaviour cannot be shown by running it, so this reads the sources."""
+import os
+import re
+
+import pytest
+
+CSRC = os.path.join(os.path.dirname(os.path.dirname(os.path.abspath(__file__))), "llm-scaler_b200", "csrc")
+KERNELS = sorted(f for f in os.listdir(CSRC) if f.startswith("umma_") and f.endswith(".cu"))
+
+
+def _per_lane_waits(text):
+    """Line numbers of mbar_wait() calls that no enclosing block's head restricts to one thread."""
+    text = re.sub(r"//[^\n]*", "", text)
+    heads, start, found = [], 0, []
+    for m in re.finditer(r"[{};]|\bmbar_wait\(", text):
+        tok = m.group()
+        if tok == "{":
+            heads.append(text[start:m.start()])
+        elif tok == "}":
+            heads.pop()
+        elif tok != ";":
+            if not any(re.search(r"elect_one\(\)|_selftest_kernel", h) for h in heads):
+                found.append(text.count("\n", 0, m.start()) + 1)
+            continue
+        start = m.end()
+    return found
+
+
+def test_the_reader_sees_both_forms():
+    assert _per_lane_waits("if (elect_one()) { while (x) { if (!mbar_wait(a)) break; } }") == []
+    assert _per_lane_waits("if (lane == 0) {\n mbar_wait(a);\n}\nelse { ok = mbar_wait_warp(b); }") == [2]
+
+
+@pytest.mark.parametrize("name", KERNELS)
+def test_whole_warps_wait_together(name):
+    with open(os.path.join(CSRC, name)) as f:
+        assert _per_lane_waits(f.read()) == []
