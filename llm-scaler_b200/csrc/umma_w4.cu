@@ -799,8 +799,26 @@ static int grouped_tok(int rows, int E) {
   return avg <= 16 ? 16 : (avg <= 32 ? 32 : (avg <= 96 ? 64 : 128));
 }
 
+// CTAs among which strips of n raw stages are best cut for a 128-token tile; 0 = whole strips.  Every contributor to a strip adds
+// 64 KB of partial sums that one CTA reads back, so here a cut has to be weighed, and into few and equal pieces where
+// possible.  Fitted over N = 512 .. 12288 x K = 1024 .. 28672 at 65, 96 and 128 tokens (0.3 % above the best of seven divisions
+// on average, 6 % at most): 0.8 us per stage of a strip, and for cut strips 4 us, 2 us per contributor, and 1.2 us more where
+// the pieces do not line up with the strips, which then have one contributor more; 256-row strips take twice of each.  In
+// half stages below.  Against cutting over the whole grid: 128 x 2048 x 2048 25.9 -> 11.7 us, 128 x 4096 x 4096 35.0 -> 18.1,
+// 128 x 4096 x 14336 37.8 -> 32.1, 128 x 24576 x 4096 34.2 -> 31.3; unchanged 128 x 8192 x 28672, 64 us (97 with whole strips).
+static int cut_grid_128(int64_t strips, int64_t n, int sms) {
+  int64_t best = 2 * ((strips + sms - 1) / sms) * n, grid = 0;
+  for (int64_t p = 2; p <= n && p * strips <= sms; ++p) {
+    const int64_t t = 2 * ((n + p - 1) / p) + 10 + 5 * p;
+    if (t < best) { best = t; grid = p * strips; }
+  }
+  const int64_t g = strips * n < sms ? strips * n : sms, pieces = (g + strips - 1) / strips;
+  if (g % strips != 0 && 2 * ((strips * n + g - 1) / g) + 13 + 5 * (pieces + 1) < best) grid = g;
+  return (int)grid;
+}
+
 // How one token tile of a dense launch is shared out: strips of R x 128 rows, cut along k, raw stage by raw stage, when whole
-// ones would leave more than a twentieth of the machine idle in the last round.
+// ones would leave more than a twentieth of the machine idle in the last round (128-token tiles: cut_grid_128).
 struct StripPlan { int R, strips, sps, units, grid; size_t partial_bytes; };      // sps, units: raw stages per strip and in total, 0 = whole strips
 static StripPlan plan_strips(int64_t M, int64_t N, int64_t K, int k_per_stage, bool tall) {
   StripPlan pl{};
@@ -812,8 +830,9 @@ static StripPlan plan_strips(int64_t M, int64_t N, int64_t K, int k_per_stage, b
   pl.grid = (int)(strips < sms ? strips : sms);
   if (M > tok || (K % k_per_stage) != 0 || strips > UMMA_MAX_CUT_STRIPS || units > INT32_MAX) return pl;
   if ((double)strips / ((double)((strips + sms - 1) / sms) * sms) > 0.95) return pl;
-  pl.sps = (int)(K / k_per_stage); pl.units = (int)units;
-  pl.grid = (int)(units < sms ? units : sms);
+  const int grid = tok == 128 ? cut_grid_128(strips, K / k_per_stage, sms) : (int)(units < sms ? units : sms);
+  if (!grid) return pl;
+  pl.sps = (int)(K / k_per_stage); pl.units = (int)units; pl.grid = grid;
   pl.partial_bytes = (size_t)2 * pl.grid * pl.R * 128 * tok * sizeof(float);       // two slots per CTA
   return pl;
 }
@@ -915,7 +934,7 @@ int umma_w4_prep_linear(const UmmaW4Args& a, cudaStream_t st) {
   int64_t work = (int64_t)p.strips * tiles;
   rc = cut_strips(p, a, pl);
   if (rc) return rc;
-  if (p.units > 0) work = p.units;
+  if (p.units > 0) work = pl.grid;
   if (work > INT32_MAX) return B2Q_ERR_LIMIT;
   if (a.peer) {
     if (tok > 64 || grouped || (a.N % 128) != 0 || (a.peer->slice % 128) != 0 || a.peer->M != a.M) return B2Q_ERR_UNSUPPORTED;

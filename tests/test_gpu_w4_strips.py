@@ -58,7 +58,8 @@ def test_tile_and_group_edges(e, M, N, K, scale_dtype):
     assert e._lib.device_status() == 0
 
 
-@pytest.mark.parametrize("M,N,K", [(16, 8192, 14336), (64, 8192, 14336), (64, 38016, 2048), (100, 10240, 8192), (700, 8192, 2048)])
+@pytest.mark.parametrize("M,N,K", [(16, 8192, 14336), (64, 8192, 14336), (64, 38016, 2048), (100, 10240, 8192), (700, 8192, 2048),
+                                   (100, 4096, 14336), (128, 12288, 14336), (96, 520, 8192)])    # 128-token tiles cut into equal pieces, over the whole grid, ragged
 def test_many_segments_repeat_bit_for_bit(e, M, N, K):
     x, w, s, ref = _case(M, N, K, torch.bfloat16, 7)
     first = None

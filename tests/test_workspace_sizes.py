@@ -42,3 +42,14 @@ def test_int4_no_partial_sums_where_nothing_is_cut(lib):
                     (64, 128 * SMS, 4096),         # a whole strip for every SM
                     (129, 2048, 2048)):            # two token tiles
         assert lib.b2q_linear_workspace_bytes(M, N, K) == _prep(M, K)
+
+
+def test_int4_short_k_is_not_cut_for_128_token_tiles(lib):
+    """Cutting costs a 128-token tile 4 us and 2 us per contributor, a stage of 256 k 0.8 us: up to K = 4096 no cut of less
+    than one round of strips pays, and none ever has more pieces than stages or SMs."""
+    for M in (65, 128):
+        for N in (512, 2048, 4096, 12288):
+            for K in (1024, 2048, 4096):
+                assert lib.b2q_linear_workspace_bytes(M, N, K) == _prep(M, K)
+        assert lib.b2q_linear_workspace_bytes(M, 4096, 14336) - _prep(M, 14336) == 2 * 4 * 32 * 128 * 128 * 4      # four equal pieces
+        assert lib.b2q_linear_workspace_bytes(M, 8192, 28672) - _prep(M, 28672) == 2 * SMS * 128 * 128 * 4         # the whole grid
