@@ -130,3 +130,34 @@ def test_scratch_without_room_for_partial_sums_keeps_the_pre_pass(e, M, N, K):
         assert e.launch_count() - before == 2
         _check(out, ref, (M, N, K, size))
     assert e._lib.device_status() == 0
+
+
+@pytest.mark.parametrize("E,rows,N,K", [
+    (3, (60, 0, 33), 1096, 640),                       # 64-token tiles, short strips: few pieces
+    (2, (129, 200), 520, 1152),                        # 128-token tiles, short strips
+    (64, (1, 40, 65, 54), 2048, 256),                  # 64-token tiles, tall strips: many rounds
+    (16, (97, 128, 1, 160), 3072, 4096),               # 128-token tiles, tall strips: long k
+    (80, (1, 16, 7, 3), 8192, 128),                    # more pieces per CTA than the table of tiles holds
+])
+def test_grouped_int4_strip_heights(e, E, rows, N, K):
+    """Grouped INT4 over the strip heights and tile sizes it chooses between.  fp16 throughout: the output is rounded once (at
+    most 2^-11 of it) and every weight once (at most 2^-11, spread evenly), together below 2^-10 in the 2-norm; one lost tile
+    of n is 1 / sqrt(n)."""
+    from custom_esimd_kernels_vllm import _impl
+    rows = [rows[i % len(rows)] for i in range(E)]
+    M = sum(rows)
+    g = torch.Generator(device=DEV).manual_seed(E + N + K)
+    w = torch.randint(-2 ** 31, 2 ** 31 - 1, (E, N, K // 8), generator=g, device=DEV, dtype=torch.int64).to(torch.int32)
+    s = ((0.5 + torch.rand(E, N, K // 128, generator=g, device=DEV)) * 0.01).to(torch.float16)
+    x = torch.randn(M, K, generator=g, device=DEV).to(torch.float16)
+    off = torch.tensor([0] + rows, device=DEV).cumsum(0).to(torch.int32)
+    shifts = torch.arange(0, 32, 4, device=DEV, dtype=torch.int32)
+    parts = []
+    for i in range(E):
+        q = ((w[i].unsqueeze(-1) >> shifts) & 15).reshape(N, K // 128, 128).double() - 8
+        parts.append(x[off[i]:off[i + 1]].double() @ (q * s[i].double().unsqueeze(-1)).view(N, K).T)
+    ref = torch.cat(parts)
+    out = _impl.moe_gemm_int4(x, w, s, off, M)
+    err = (out.double() - ref).norm() / ref.norm()
+    assert float(err) < 2.0 ** -10, float(err)
+    assert e._lib.device_status() == 0
