@@ -441,7 +441,7 @@ B2Q_API void b2q_set_force_kernel(int which);
  *      fully ordered in every mode.                                             */
 B2Q_API void b2q_set_overlap_mode(int mode);
 /* Name of the kernel family the last b2q_linear_* / b2q_moe_gemm_* call on this
- * thread launched ("smallm", "umma", ...).                                    */
+ * thread launched ("smallm", "umma_w4", "umma_wo", "umma_w8_direct", ...).    */
 B2Q_API const char* b2q_last_kernel(void);
 /* Number of kernel launches issued by this library on this thread so far.     */
 B2Q_API uint64_t b2q_launch_count(void);

@@ -854,7 +854,7 @@ static int launch_w4(const CUtensorMap& tw, const CUtensorMap& tx, const W4Param
     if (dev < 16) configured[dev] = true;
   }
   if (launch_overlapped(kern, dim3(grid), dim3(C::THREADS), C::SMEM, st, overlap, tw, tx, p) != cudaSuccess) return B2Q_ERR_CUDA;
-  note_launch("umma_wo");
+  note_launch("umma_w4");
   return launch_status();
 }
 

@@ -155,6 +155,6 @@ def test_int4_scales_outside_fp16_range(e, scale_dtype, magnitude):
     x = torch.randn(M, K, generator=g).to(torch.bfloat16)
     out = torch.empty(M, N, dtype=torch.bfloat16, device=DEV)
     e.esimd_gemm_int4_pgrp(x.to(DEV), int4.pack_nmajor_i32(q).to(DEV), s.to(DEV), out)
-    assert e.last_kernel() == "umma_wo"
+    assert e.last_kernel() == "umma_w4"
     ref = x.float() @ ((q.float() - 8.0) * s.float().repeat_interleave(128, dim=1)).T       # unrounded weights
     _gate(slices.errors(out, ref.to(torch.bfloat16)), f"scales ~{magnitude} {scale_dtype}")

@@ -50,10 +50,12 @@ def test_tile_and_group_edges(e, M, N, K, scale_dtype):
     x, w, s, ref = _case(M, N, K, scale_dtype, M + N + K)
     out = torch.full((M, N), float("nan"), dtype=torch.bfloat16, device=DEV)
     e.esimd_gemm_int4_pgrp(x, w, s, out)
+    assert e.last_kernel() == "umma_w4"
     _check(out, ref, (M, N, K))
     kmaj = torch.full_like(out, float("nan"))
     if N % 4 == 0:
         e.esimd_gemm_int4_pgrp(x, w.t().contiguous(), s.t().contiguous(), kmaj)
+        assert e.last_kernel() == "umma_w4"
         _check(kmaj, ref, ("k-major", M, N, K))
     assert e._lib.device_status() == 0
 
@@ -66,6 +68,7 @@ def test_many_segments_repeat_bit_for_bit(e, M, N, K):
     for _ in range(8):
         out = torch.full((M, N), float("nan"), dtype=torch.bfloat16, device=DEV)
         e.esimd_gemm_int4_pgrp(x, w, s, out)
+        assert e.last_kernel() == "umma_w4"
         if first is None:
             first = out
             _check(out, ref, (M, N, K))
@@ -88,6 +91,7 @@ def test_block_scaled_fp8_strips(e, M, N, K, dtype):
     for _ in range(3):
         out = torch.full((M, N), float("nan"), dtype=dtype, device=DEV)
         e.esimd_gemm_fp8_blockscale(x, w, s, out)
+        assert e.last_kernel() == "umma_w4"
         if first is None:
             first = out
             _check(out, ref, (M, N, K))
@@ -109,6 +113,7 @@ def test_grouped_fp8_per_expert_scale(e, rows, N, K):
     ref = torch.cat([x[off[i]:off[i + 1]].double() @ (w[i].double() * float(s[i])).T for i in range(E)])
     out = torch.full((M, N), float("nan"), dtype=torch.float16, device=DEV)
     e.esimd_moe_gemm_fp8_pert(x, w, s, out, off, N, K, E, M)
+    assert e.last_kernel() == "umma_w4"
     err = (out.double() - ref).norm() / ref.norm()
     assert float(err) < 2.0 ** -11, float(err)
     assert e._lib.device_status() == 0
@@ -127,7 +132,7 @@ def test_scratch_without_room_for_partial_sums_keeps_the_pre_pass(e, M, N, K):
         before = e.launch_count()
         L.check(L.lib.b2q_linear_int4(x.data_ptr(), L.BF16, K, w.data_ptr(), L.W4_NMAJOR, s.data_ptr(), L.BF16, K // 128, 1,
                                       out.data_ptr(), N, M, N, K, 128, ws.data_ptr(), size, torch.cuda.current_stream().cuda_stream))
-        assert e.launch_count() - before == 2
+        assert e.launch_count() - before == 2 and e.last_kernel() == "umma_w4"
         _check(out, ref, (M, N, K, size))
     assert e._lib.device_status() == 0
 
@@ -158,6 +163,7 @@ def test_grouped_int4_strip_heights(e, E, rows, N, K):
         parts.append(x[off[i]:off[i + 1]].double() @ (q * s[i].double().unsqueeze(-1)).view(N, K).T)
     ref = torch.cat(parts)
     out = _impl.moe_gemm_int4(x, w, s, off, M)
+    assert e.last_kernel() == "umma_w4"
     err = (out.double() - ref).norm() / ref.norm()
     assert float(err) < 2.0 ** -10, float(err)
     assert e._lib.device_status() == 0
