@@ -868,11 +868,6 @@ static int launch_wk(bool bf16, bool fast, int tok, const CUtensorMap& tw, const
   return fast ? launch_tok<WK, false, true>(tok, tw, tx, p, tiles, st) : launch_tok<WK, false, false>(tok, tw, tx, p, tiles, st);
 }
 
-static int grouped_tok(int rows, int E) {
-  const int avg = E > 0 ? (rows + E - 1) / E : rows;
-  return avg <= 16 ? 16 : (avg <= 32 ? 32 : (avg <= 96 ? 64 : 128));
-}
-
 bool umma_w4_supported(const UmmaW4Args& a) {
   if (a.K % 128 != 0 || a.K < 64) return false;
   if (!aligned16(a.x) || !aligned16(a.w) || ((a.ldx * 2) & 15)) return false;

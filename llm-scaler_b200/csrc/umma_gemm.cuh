@@ -74,6 +74,13 @@ bool umma_w4_i8_preferred(int64_t M, int64_t N, int64_t K);
 size_t umma_w4_i8_partial_bytes();
 int umma_w4_i8_linear(const UmmaW4I8Args& a, cudaStream_t st);
 
+// Token-tile height of grouped launches, from the mean rows per expert.  The tile list is built with it and every kernel
+// that reads the list takes it from here.
+inline int grouped_tok(int rows, int E) {
+  const int avg = E > 0 ? (rows + E - 1) / E : rows;
+  return avg <= 16 ? 16 : (avg <= 32 ? 32 : (avg <= 96 ? 64 : 128));
+}
+
 bool umma_w4_supported(const UmmaW4Args& a);
 int umma_w4_token_tile(const UmmaW4Args& a);
 int umma_w4_linear(const UmmaW4Args& a, cudaStream_t st);

@@ -794,10 +794,6 @@ static int sm_count() {
 }
 
 static int dense_tok(int64_t M) { return M <= 16 ? 16 : (M <= 32 ? 32 : (M <= 64 ? 64 : 128)); }
-static int grouped_tok(int rows, int E) {
-  const int avg = E > 0 ? (rows + E - 1) / E : rows;
-  return avg <= 16 ? 16 : (avg <= 32 ? 32 : (avg <= 96 ? 64 : 128));
-}
 
 // CTAs among which strips of n raw stages are best cut for a 128-token tile; 0 = whole strips.  Every contributor to a strip adds
 // 64 KB of partial sums that one CTA reads back, so here a cut has to be weighed, and into few and equal pieces where
