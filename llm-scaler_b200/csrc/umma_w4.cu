@@ -962,7 +962,15 @@ int umma_w4_prep_linear(const UmmaW4Args& a, cudaStream_t st) {
 // tensor (whose transform multiplies by 1).
 bool umma_w8_strip_supported(const UmmaW8Args& a) {
   if (a.bf16 || a.fmt != B2Q_E4M3 || (a.K % 128) != 0) return false;
-  if (a.expert_offsets) return a.scale_mode != B2Q_SCALE_BLOCK128 && grouped_tok(a.M, a.E) <= 64;
+  if (a.expert_offsets) {
+    const int tok = grouped_tok(a.M, a.E);
+    if (a.scale_mode == B2Q_SCALE_BLOCK128 || tok > 64) return false;
+    // 64-token tiles in two rounds over the SMs go through umma_gemm.cu's kernel in one, with two CTAs on each: 8 experts x 80
+    // rows, 2048 x 2048, 21.6 against 24.8 us, 2 x 80, 8192 x 2048, 21.7 against 25.2.  One round (2 x 40, 8192 x 2048, 19.4 against
+    // 18.1 us), more than two (4 x 60, 8192 x 2048, 35.4 against 33.9; 64 x 40, 2048 x 1024, 56.4 against 40.9) and 32-token tiles (8 x 24,
+    // 4096 x 2048, 27.6 against 22.4) are faster here.
+    return tok < 64 || grouped_rounds(a.M, a.E, (a.N + 127) / 128, tok, sm_count()) != 2;
+  }
   return a.scale_mode == B2Q_SCALE_BLOCK128 && a.M <= 64;
 }
 

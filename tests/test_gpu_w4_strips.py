@@ -119,6 +119,28 @@ def test_grouped_fp8_per_expert_scale(e, rows, N, K):
     assert e._lib.device_status() == 0
 
 
+@pytest.mark.parametrize("E,avg,N,kernel", [(8, 40, 1024, "umma_w4"), (8, 80, 2048, "umma_wo"), (12, 40, 2000, "umma_wo"), (8, 60, 4096, "umma_w4"),
+                                            (16, 24, 2048, "umma_w4")])
+def test_grouped_fp8_route_by_rounds(e, E, avg, N, kernel):
+    """64-token tiles in one round over the SMs, in two, in more, and 32-token tiles: which kernel serves them, and that both of
+    them give the same product (tolerance as above)."""
+    K = 512
+    rows = [avg + (avg // 3 if i % 2 else -(avg // 3)) for i in range(E)]
+    M = sum(rows)
+    g = torch.Generator(device=DEV).manual_seed(M + N)
+    w = (torch.randn(E, N, K, generator=g, device=DEV) * 96).clamp_(-448, 448).to(torch.float8_e4m3fn)
+    s = (0.5 + torch.rand(E, generator=g, device=DEV)) / 4096
+    x = torch.randn(M, K, generator=g, device=DEV).to(torch.float16)
+    off = torch.tensor([0] + rows, device=DEV).cumsum(0).to(torch.int32)
+    ref = torch.cat([x[off[i]:off[i + 1]].double() @ (w[i].double() * float(s[i])).T for i in range(E)])
+    out = torch.full((M, N), float("nan"), dtype=torch.float16, device=DEV)
+    e.esimd_moe_gemm_fp8_pert(x, w, s, out, off, N, K, E, M)
+    assert e.last_kernel() == kernel
+    err = (out.double() - ref).norm() / ref.norm()
+    assert float(err) < 2.0 ** -11, float(err)
+    assert e._lib.device_status() == 0
+
+
 @pytest.mark.parametrize("M,N,K", [(100, 2048, 2048), (64, 2048, 4096), (100, 5120, 8192)])
 def test_scratch_without_room_for_partial_sums_keeps_the_pre_pass(e, M, N, K):
     """Scratch that a caller sized for another M: the activations are rewritten as ever (two launches), strips stay whole.
