@@ -187,7 +187,10 @@ B2Q_API int b2q_linear_int4(const void* x, int act_dtype, int64_t ldx,
  *    lose low bits);
  *  - otherwise bf16 activations are rewritten as fp16 times a per-token power of two (exact for every
  *    element within 2^-31 of its row maximum), which makes the in-kernel fp8 decode four times cheaper;
- *    M <= 64 with block scales also keeps partial sums there, as above.                             */
+ *    M <= 64 with block scales also keeps partial sums there, as above.
+ * With block scales and fp16 operands (fp16 activations, or bf16 ones with scratch) a weight times its scale
+ * is rounded once to fp16, after a power of two that brings the largest scale of its strip of 128 rows
+ * into range: any magnitude of scale is safe, and blocks down to 2^-11 of the largest keep all bits.   */
 B2Q_API size_t b2q_linear_fp8_workspace_bytes(int64_t M, int64_t N, int64_t K);
 B2Q_API int b2q_linear_fp8(const void* x, int act_dtype, int64_t ldx,
                    const void* w, int fp8_format,

@@ -387,6 +387,14 @@ umma_wo_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constant__
     uint32_t sn0 = chunk_scale_raw(grp + 4 * NG), sn1 = chunk_scale_raw(grp + 5 * NG), sn2 = chunk_scale_raw(grp + 6 * NG),
              sn3 = chunk_scale_raw(grp + 7 * NG);
     int it4 = 0;                                   // position of the current chunk in its set of four
+    // fp16 operands: the block scales of this strip, brought into range together (see block_scale_exponent)
+    float blk_mul = 1.f, blk_post = 1.f;
+    if constexpr (WK == WK_W8 && !BF16) {
+      if (blockscale) {
+        const int k = block_scale_exponent(reinterpret_cast<const float*>(p.scale) + sbase + (int64_t)(n0 >> 7) * kblocks + (c_begin >> 1), (nk + 1) >> 1);
+        blk_mul = pow2(k); blk_post = pow2(-k);
+      }
+    }
     // Position in the raw ring: by counting (this group converts CPG chunks of every raw stage, a segment starts on a
     // stage boundary, jj counts them) or by dividing the chunk number by the stage count for every chunk.  Which is
     // faster is a matter of what the register allocator makes of the loop, measured per tile width on one GPU: the
@@ -459,7 +467,7 @@ umma_wo_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constant__
           for (int c4 = 0; c4 < 4; ++c4) rv[c4] = lds128(rawrow + (((4 * j + c4) ^ sw) << 4));
           uint32_t (&o)[32] = av;
           if (blockscale) {
-            const float sf = sc_cur;
+            const float sf = sc_cur * blk_mul;
 #pragma unroll
             for (int c4 = 0; c4 < 4; ++c4) {
               w8_word<BF16, true>(rv[c4].x, p.e5m2, sf, o[8 * c4 + 0], o[8 * c4 + 1]);
@@ -514,7 +522,7 @@ umma_wo_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constant__
     const int quad = warp & 3;                   // tensor-memory lane quadrant this warp may read
     const int cgrp = (warp - Cfg::CW) >> 2;      // the NG warps of a quadrant take column blocks in turn
     const int n = n0 + quad * 32 + lane;
-    float post = 1.f;
+    float post = blk_post;
     if constexpr (WK == WK_W8) {
       if (p.scale_mode != B2Q_SCALE_BLOCK128) {
         post = (BF16 ? 5192296858534827628530496329220096.0f : 1.0f);   // 2^112 undoes the bf16 bit trick

@@ -4,6 +4,22 @@
 
 namespace b2q {
 
+#ifdef __CUDACC__
+// Power of two (its exponent) that brings the largest of n block scales into [64, 128).  Weight kernels that fold the block scale
+// into an fp16 operand multiply it in and take it out of the fp32 accumulator again: 448 times the largest scale then stays
+// below fp16's 65504, and blocks down to 2^-11 of it keep every e4m3 value in fp16's normal range.  Smaller blocks lose bits
+// that are below 2^-24 of the strip's largest product.  For a whole warp; 0 if a scale is infinite or NaN.
+__device__ __forceinline__ int block_scale_exponent(const float* s, int n) {
+  uint32_t m = 0;
+#pragma unroll 4
+  for (int i = threadIdx.x & 31; i < n; i += 32) m = max(m, __float_as_uint(__ldg(s + i)) & 0x7FFFFFFFu);
+  m = __reduce_max_sync(0xffffffffu, m);       // positive floats order as their bits
+  const int ex = (int)(m >> 23);
+  return ex == 255 ? 0 : max(-120, min(120, 133 - ex));
+}
+__device__ __forceinline__ float pow2(int k) { return __uint_as_float((uint32_t)(127 + k) << 23); }      // |k| < 127
+#endif
+
 // Common tail of the argument blocks: optional grouped (MoE) mode.
 struct UmmaGroupArgs {
   const int32_t* expert_offsets = nullptr;  // [E+1]; nullptr = dense

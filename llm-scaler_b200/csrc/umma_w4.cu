@@ -457,7 +457,7 @@ umma_w4_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constant__
             if (f32) {
               if (sl == 0) {
                 const int k = row_exponent(__uint_as_float(off == 0 ? e[0] : (off == 2 ? e[2] : (off == 4 ? e[4] : e[6]))));   // off is even
-                mul[i] = __uint_as_float((uint32_t)(127 + k) << 23);
+                mul[i] = pow2(k);
                 post_exp[(segno % C::POST_RING) * ROWS + lane + 32 * i] = (int8_t)-k;
               }
 #pragma unroll
@@ -578,12 +578,10 @@ umma_w4_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constant__
           if constexpr (CB == 32) tmem_ld32(ta, q); else tmem_ld16(ta, q);
           tmem_ld_wait();
           float pm;
-          if constexpr (WT == WT_W8) {
-            pm = 1.f;
-            if (p.scale_mode != B2Q_SCALE_BLOCK128)
-              pm = load_scalar(p.scale, sg.expert * p.s_expert_elems +
-                                            (p.scale_mode == B2Q_SCALE_CHANNEL ? min(sg.n0 + rb * 128 + quad * 32 + lane, p.N - 1) : 0), p.scale_dtype);
-          } else pm = __uint_as_float((uint32_t)(127 + post[rb * 128 + quad * 32 + lane]) << 23);
+          if (WT == WT_W8 && p.scale_mode != B2Q_SCALE_BLOCK128)
+            pm = load_scalar(p.scale, sg.expert * p.s_expert_elems +
+                                          (p.scale_mode == B2Q_SCALE_CHANNEL ? min(sg.n0 + rb * 128 + quad * 32 + lane, p.N - 1) : 0), p.scale_dtype);
+          else pm = pow2(post[rb * 128 + quad * 32 + lane]);
 #pragma unroll
           for (int i = 0; i < CB; ++i) r[i] = __uint_as_float(q[i]) * pm;
         }
@@ -694,11 +692,17 @@ umma_w4_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constant__
       int rs = raw0 % RS, as = g0 % S;
       uint32_t rpar = (uint32_t)(raw0 / RS) & 1u, apar = ((uint32_t)(g0 / S) + 1u) & 1u;
       float row_mul = 1.f;
-      // e4m3: one fp32 scale per block, the same for the whole CTA, requested an iteration ahead
+      // e4m3: one fp32 scale per block, the same for the whole CTA, requested an iteration ahead; one power of two per segment
+      // brings them into fp16's range (see block_scale_exponent)
       const float* block_scale = reinterpret_cast<const float*>(p.scale) + (cur.block_row + rb) * (int64_t)(p.K >> 7) + cur.block_col;
       const bool blocks = WT == WT_W8 && p.scale_mode == B2Q_SCALE_BLOCK128;
       float sf_next = 1.f;
-      if (blocks && gg < ngroups) sf_next = __ldg(block_scale + gg);
+      if (blocks) {
+        if (gg < ngroups) sf_next = __ldg(block_scale + gg);
+        const int k = block_scale_exponent(block_scale, ngroups);
+        row_mul = pow2(k);
+        if (gg == 0) post_exp[(segno % C::POST_RING) * ROWS + rb * 128 + t] = (int8_t)-k;
+      }
 #pragma unroll 1
       for (int sl = 0; sl < nslot; ++sl) {
         if (WT != WT_W8) ok = mbar_wait_warp(sc_full + 8 * ss, spar, abort_flag, p.status, ST_SCFULL);
@@ -706,7 +710,7 @@ umma_w4_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constant__
         const uint32_t sca = sc0 + ss * C::SC_BYTES;
         if (WT != WT_W8 && sl == 0 && p.scale_dtype != B2Q_F32) {
           const int k = bf16_scale ? row_exponent(__uint_as_float(lds_u16(sca + 2 * off) << 16)) : 0;
-          row_mul = __uint_as_float((uint32_t)(127 + k) << 23);
+          row_mul = pow2(k);
           // told to the epilogue by the group that converts the segment's first 128 k: before these are handed over
           if (gg == 0) post_exp[(segno % C::POST_RING) * ROWS + rb * 128 + t] = (int8_t)-k;
         }
@@ -714,7 +718,7 @@ umma_w4_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constant__
 #pragma unroll 1
         for (; gg < gend; gg += KG) {
           uint32_t hv = WT == WT_W8 ? 0u : lds_u16(sca + 2 * ((gg + off) & 7));
-          const float sf = sf_next;
+          const float sf = sf_next * row_mul;
           if (blocks && gg + KG < ngroups) sf_next = __ldg(block_scale + gg + KG);
           if (WT == WT_W8) {}
           else if (bf16_scale) hv = fp16_factor(__uint_as_float(hv << 16) * row_mul, saturated);

@@ -33,9 +33,9 @@ def _case(M, N, K, scale_dtype, seed):
     return x, w, s, ref
 
 
-def _check(out, ref, what):
+def _check(out, ref, what, rounding=2.0 ** -8):
     norms = ref.norm(dim=0)
-    err = (out.double() - ref).norm(dim=0) / (2.0 ** -8 * norms + 2.0 ** -9 * norms.pow(2).mean().sqrt())
+    err = (out.double() - ref).norm(dim=0) / (rounding * norms + 2.0 ** -9 * norms.pow(2).mean().sqrt())
     assert float(err.max()) < 1.0, (what, float(err.max()), int(err.argmax()))       # also false for NaN
 
 
@@ -188,4 +188,44 @@ def test_grouped_int4_strip_heights(e, E, rows, N, K):
     assert e.last_kernel() == "umma_w4"
     err = (out.double() - ref).norm() / ref.norm()
     assert float(err) < 2.0 ** -10, float(err)
+    assert e._lib.device_status() == 0
+
+
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16])
+@pytest.mark.parametrize("M", [16, 64, 300])
+@pytest.mark.parametrize("unit,spread", [(1e3, 0), (1e-6, 0), (1e-8, 0), (1e-3, 24), (300.0, 24)])
+def test_block_scales_outside_fp16_range(e, dtype, M, unit, spread):
+    """Block scales whose product with an e4m3 value overflows fp16 or falls among its subnormals, and scales up to 2^24 apart in one
+    row, an all but vanishing one first: weights are rounded to fp16 once, relative to the largest block of their strip.
+    The activations keep the output within fp16's range; the tolerance is that of the other block-scaled cases."""
+    N, K = 520, 1152
+    g = torch.Generator(device=DEV).manual_seed(M + spread)
+    w = (torch.randn(N, K, generator=g, device=DEV) * 96).clamp_(-448, 448).to(torch.float8_e4m3fn)
+    s = (0.5 + torch.rand((N + 127) // 128, K // 128, generator=g, device=DEV)) * unit
+    if spread:
+        s = s * torch.exp2(-torch.randint(0, spread + 1, s.shape, generator=g, device=DEV).float())
+        s[:, 0] = 1e-20
+        s[:, 3] = unit
+    x = (torch.randn(M, K, generator=g, device=DEV) * min(2.0 ** 11, 2.0 ** -11 / unit)).to(dtype)
+    full = s.double().repeat_interleave(128, 0)[:N].repeat_interleave(128, 1)
+    ref = x.double() @ (w.double() * full).T
+    out = torch.full((M, N), float("nan"), dtype=dtype, device=DEV)
+    e.esimd_gemm_fp8_blockscale(x, w, s, out)
+    _check(out, ref, (M, unit, spread), 2.0 ** -8 if dtype == torch.bfloat16 else 2.0 ** -11)
+    assert e._lib.device_status() == 0
+
+
+@pytest.mark.parametrize("unit", [1e3, 1e-8])
+def test_grouped_block_scales_outside_fp16_range(e, unit):
+    E, rows, N, K = 2, (40, 90), 256, 512
+    g = torch.Generator(device=DEV).manual_seed(3)
+    w = (torch.randn(E, N, K, generator=g, device=DEV) * 96).clamp_(-448, 448).to(torch.float8_e4m3fn)
+    s = (0.5 + torch.rand(E, N // 128, K // 128, generator=g, device=DEV)) * unit
+    x = (torch.randn(sum(rows), K, generator=g, device=DEV) * min(2.0 ** 11, 2.0 ** -11 / unit)).to(torch.float16)
+    off = torch.tensor([0, rows[0], sum(rows)], dtype=torch.int32, device=DEV)
+    full = s.double().repeat_interleave(128, 1).repeat_interleave(128, 2)
+    ref = torch.cat([x[off[i]:off[i + 1]].double() @ (w[i].double() * full[i]).T for i in range(E)])
+    out = torch.full((sum(rows), N), float("nan"), dtype=torch.float16, device=DEV)
+    e.esimd_moe_gemm_fp8_blockscale(x, w, s, out, off, N, K, E)
+    _check(out, ref, unit, 2.0 ** -11)
     assert e._lib.device_status() == 0
