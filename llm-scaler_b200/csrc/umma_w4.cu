@@ -124,6 +124,8 @@ __device__ __forceinline__ void cp_async4(uint32_t dst, const void* src, int src
 __device__ __forceinline__ void cp_async_arrive(uint32_t bar) {
   asm volatile("cp.async.mbarrier.arrive.noinc.shared::cta.b64 [%0];" ::"r"(bar) : "memory");
 }
+// Waits for every copy this thread has issued.
+__device__ __forceinline__ void cp_async_wait_all() { asm volatile("cp.async.wait_all;" ::: "memory"); }
 // Power of two that brings a scale into [0.5, 1) (0 for zero, subnormal, infinite and NaN scales).
 __device__ __forceinline__ int row_exponent(float first) {
   const int ex = (int)((__float_as_uint(first) >> 23) & 0xFFu);
@@ -472,6 +474,7 @@ umma_w4_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constant__
       }
       ++segno;
     }
+    cp_async_wait_all();             // after a give-up copies may still be on their way; otherwise all have landed
     if (saturated) atomicCAS(p.status, 0, ST_SCALERANGE);
   } else if (warp < C::CW + C::EW) {
     // ---------------- epilogue ----------------

@@ -265,7 +265,8 @@ umma_w8a8_pair_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_con
     if (elect_one()) {
       tma_prefetch_desc(&tm_w);
       tma_prefetch_desc(&tm_x);
-      for (int kb = 0; kb < nkb; ++kb) {
+      int kb = 0;
+      for (; kb < nkb; ++kb) {
         const int s = kb % S;
         if (kb >= S && !mbar_wait(empty + 8 * s, ((kb / S) - 1) & 1, abort_flag, p.status, ST_EMPTY)) break;
         const uint32_t lead_full = map_to_cta(full + 8 * s, 0);
@@ -273,6 +274,8 @@ umma_w8a8_pair_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_con
         tma_load_2d_pair(base + s * PAIR_STAGE, &tm_w, kb * 128, n0, lead_full);
         tma_load_2d_pair(base + s * PAIR_STAGE + 16384, &tm_x, kb * 128, tok0 + (int)rank * 64, lead_full);
       }
+      // gave up: the leader's barriers count both CTAs' copies, and the peer does not leave before the leader
+      if (kb < nkb && rank == 0) drain_issued(full, S, kb);
     }
   } else if (warp == 1) {
     // ---- MMA issuer: the leader's one thread drives both CTAs' tensor cores ----

@@ -1,8 +1,10 @@
-"""Every barrier wait of a whole warp brings its lanes back together.
+"""What the tensor-core kernels' barrier waits have to keep to, read from the sources: neither undefined behaviour nor a CTA that
+leaves too early can be shown by running them.
 
 tcgen05.ld / st, shuffles and __syncwarp need all lanes of a warp at the same instruction, and mbar_wait() lets them leave, or
 give up, one by one.  Only the branch of one elected thread may call it; everything else goes through mbar_wait_warp().
-Undefined behaviour cannot be shown by running it, so this reads the sources."""
+
+A role that has given up waits for the copies it has issued before the CTA frees its memory."""
 import os
 import re
 
@@ -39,3 +41,14 @@ def test_the_reader_sees_both_forms():
 def test_whole_warps_wait_together(name):
     with open(os.path.join(CSRC, name)) as f:
         assert _per_lane_waits(f.read()) == []
+
+
+@pytest.mark.parametrize("name", KERNELS)
+def test_copies_in_flight_are_waited_for(name):
+    with open(os.path.join(CSRC, name)) as f:
+        kernels = f.read().split("__global__ ")[1:]
+    for text in kernels:
+        # one drain per elected producer, one wait behind asynchronous copies that arrive on a barrier
+        producers = sum(bool(re.search(r"\btma_load_2d(_pair)?\(", part)) for part in text.split("if (elect_one()) {")[1:])
+        assert text.count("drain_issued(") == producers
+        assert ("cp_async_arrive(" in text) == ("cp_async_wait_all()" in text)
