@@ -126,3 +126,43 @@ def test_rejects_shapes_outside_the_contract(L):
             ranks.reduce(big)                                                    # more rows than the communicator was made for
     finally:
         ranks.close()
+
+
+@pytest.mark.parametrize("M,N,K,kmajor", [
+    (64, 2048, 4096, False), (16, 8192, 14336, False), (40, 5120, 2560, True),     # strips cut along k: partial sums, then delivery
+    (33, 18944, 512, False),                                                       # one whole strip per SM
+    (64, 37888, 512, False), (48, 40960, 768, False),                              # 256-row strips, whole and cut
+])
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16])
+def test_gemm_epilogue_delivers_its_strips(L, M, N, K, kmajor, dtype):
+    """b2q_linear_int4_allreduce with ONE rank: the GEMM's epilogue stores its strips into the rank's own reduction slots and
+    raises their flags, and the reduction kernel, an ordinary launch behind it, finds every flag raised.  A sum over one rank
+    is the linear itself, bit for bit; `partial` stays untouched where the epilogue delivers.  Several calls: epochs advance, the
+    result areas alternate."""
+    g = torch.Generator(device=DEV).manual_seed(M + N)
+    w = torch.randint(-2 ** 31, 2 ** 31 - 1, (N, K // 8), generator=g, device=DEV, dtype=torch.int64).to(torch.int32)
+    s = ((0.5 + torch.rand(N, K // 128, generator=g, device=DEV)) * 0.01).to(dtype)
+    sn, sg, layout = K // 128, 1, L.W4_NMAJOR
+    if kmajor:
+        w, s, sn, sg, layout = w.t().contiguous(), s.t().contiguous(), 1, N, L.W4_KMAJOR
+    wsb = L.lib.b2q_linear_workspace_bytes(M, N, K)
+    ws = torch.empty(wsb, dtype=torch.uint8, device=DEV)
+    comm = C.c_void_p()
+    L.check(L.lib.b2q_comm_create_mode(0, 1, M, N, 2, C.byref(comm), None))
+    try:
+        for call in range(3):
+            x = torch.randn(M, K, generator=g, device=DEV).to(dtype)
+            ref, partial = torch.empty(M, N, dtype=dtype, device=DEV), torch.full((M, N), 7.0, dtype=dtype, device=DEV)
+            st = torch.cuda.current_stream().cuda_stream
+            args = (x.data_ptr(), L.dt(x), K, w.data_ptr(), layout, s.data_ptr(), L.dt(s), sn, sg)
+            L.check(L.lib.b2q_linear_int4(*args, ref.data_ptr(), N, M, N, K, 128, ws.data_ptr(), wsb, st))
+            out = C.c_void_p()
+            L.check(L.lib.b2q_linear_int4_allreduce(*args, partial.data_ptr(), N, M, N, K, 128, ws.data_ptr(), wsb, comm, C.c_double(500.0),
+                                                    C.byref(out), st))
+            assert torch.equal(L.view_as_tensor(out.value, (M, N), dtype, ref.device), ref), call
+            assert bool((partial == 7.0).all())
+        v = C.c_int(0)
+        L.check(L.lib.b2q_comm_status(comm, C.byref(v)))
+        assert v.value == 0 and L.device_status() == 0
+    finally:
+        L.lib.b2q_comm_destroy(comm)

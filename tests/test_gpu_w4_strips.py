@@ -94,25 +94,26 @@ def test_block_scaled_fp8_strips(e, M, N, K, dtype):
         assert e.last_kernel() == "umma_w4"
         if first is None:
             first = out
-            _check(out, ref, (M, N, K))
+            _check(out, ref, (M, N, K), 2.0 ** -8 if dtype == torch.bfloat16 else 2.0 ** -11)
         assert torch.equal(out, first)
     assert e._lib.device_status() == 0
 
 
 @pytest.mark.parametrize("rows", [(1, 0, 3, 16, 2), (40, 17, 0, 31, 33), (64, 65, 130, 1, 40)])
 @pytest.mark.parametrize("N,K", [(256, 128), (1032, 1152)])
-def test_grouped_fp8_per_expert_scale(e, rows, N, K):
-    """Grouped e4m3 with one scale per expert on fp16 activations: the weights are exact, so only the output's rounding
-    (2^-11) and the fp32 sums remain; experts without rows, ragged strips, 16- / 32- / 64-token tiles."""
+@pytest.mark.parametrize("channel", [False, True])
+def test_grouped_fp8_scale_per_expert_or_channel(e, rows, N, K, channel):
+    """Grouped e4m3 with one scale per expert or per output channel on fp16 activations: the weights are exact, so only the
+    output's rounding (2^-11) and the fp32 sums remain; experts without rows, ragged strips, 16- / 32- / 64-token tiles."""
     E, M = len(rows), sum(rows)
     g = torch.Generator(device=DEV).manual_seed(M + N + K)
     w = (torch.randn(E, N, K, generator=g, device=DEV) * 96).clamp_(-448, 448).to(torch.float8_e4m3fn)
-    s = (0.5 + torch.rand(E, generator=g, device=DEV)) / 4096
+    s = (0.5 + torch.rand(*((E, N) if channel else (E,)), generator=g, device=DEV)) / 4096
     x = torch.randn(M, K, generator=g, device=DEV).to(torch.float16)
     off = torch.tensor([0] + list(rows), device=DEV).cumsum(0).to(torch.int32)
-    ref = torch.cat([x[off[i]:off[i + 1]].double() @ (w[i].double() * float(s[i])).T for i in range(E)])
+    ref = torch.cat([x[off[i]:off[i + 1]].double() @ (w[i].double() * s[i].double().reshape(-1, 1)).T for i in range(E)])
     out = torch.full((M, N), float("nan"), dtype=torch.float16, device=DEV)
-    e.esimd_moe_gemm_fp8_pert(x, w, s, out, off, N, K, E, M)
+    (e.esimd_moe_gemm_fp8 if channel else e.esimd_moe_gemm_fp8_pert)(x, w, s, out, off, N, K, E, M)
     assert e.last_kernel() == "umma_w4"
     err = (out.double() - ref).norm() / ref.norm()
     assert float(err) < 2.0 ** -11, float(err)
