@@ -32,14 +32,10 @@ using namespace sm100;
 
 __device__ int g_umma_status = 0;
 constexpr int SK_BANKS = 64, SK_MAX_STRIPS = UMMA_MAX_CUT_STRIPS;
-__device__ int g_sk_counters[SK_BANKS * SK_MAX_STRIPS];     // arrival counters of cut strips (see "balanced mode" below)
+__device__ int g_sk_counters[SK_BANKS * SK_MAX_STRIPS];     // arrival counters of cut strips (see umma_strip_counters)
 
 enum { WK_W4N = 0, WK_W4K = 1, WK_W8 = 2 };
-enum { ST_XFULL = 101, ST_AFULL = 102, ST_EMPTY = 103, ST_RAWFULL = 104, ST_RAWEMPTY = 105, ST_ACCUM = 106, ST_ACCEMPTY = 107, ST_FIXUP = 108 };
-
-// One piece of a CTA's work: 64-k chunks [c_begin, c_begin + nk) of the strip of 128 weight rows at n0.
-// part = the strip's other chunks belong to other CTAs; slot = which of the CTA's two partial-sum slots it uses.
-struct Segment { int n0, c_begin, nk, strip, part, slot; };
+enum { ST_XFULL = 101, ST_AFULL = 102, ST_EMPTY = 103, ST_RAWFULL = 104, ST_RAWEMPTY = 105, ST_ACCUM = 106, ST_FIXUP = 108 };
 
 struct UmmaWoParams {
   const void* scale; int scale_dtype; int scale_mode;      // scale_mode: B2Q_SCALE_* (fp8) ; ignored for int4
@@ -47,10 +43,6 @@ struct UmmaWoParams {
   void* out; int64_t ldo;
   int M, N, K;
   int marlin; uint32_t xor_mask; int e5m2;
-  int sk_sps, sk_units;      // balanced mode: raw stages per strip and in total (0 = one CTA per token tile and strip)
-  float* sk_partials;        // balanced mode: [2 * grid][TOK][128] fp32 partial sums of cut strips
-  int* sk_counters;          // balanced mode: arrivals per strip, zero between launches
-  int sk_grid;               // host side only: CTAs of a balanced launch
   int tiles_on_y;            // grouped launches: tile index on blockIdx.y, strip on blockIdx.x (see the kernel)
   const int32_t* tiles; const int32_t* expert_offsets; const int32_t* out_map;
   int w_rows_per_expert;     // tensor-map rows per expert: N (N-major) or K/8 (K-major)
@@ -146,7 +138,7 @@ template <int TOK> struct UmmaCfg {
   // read once by the transform) and the activation tiles, i.e. about twice the HBM traffic instead
   // of six (fp8) to ten (int4) times, which is what capped the shared-memory variant near 3 TB/s.
   // transform groups of 4 warps.  The 256-token tile runs one CTA per SM: four groups give it the sixteen converting
-  // warps the narrower tiles get from two CTAs (prefill layer -3.4 %, FP8 block GEMM -2.7 %).
+  // warps the narrower tiles get from two CTAs (FP8 block GEMM -2.7 %).
   static constexpr int NG = TOK == 256 ? 4 : 2;
   static constexpr int CTAS = TOK <= 128 ? 2 : 1;                    // two CTAs per SM except for the 256-token prefill tile: a second CTA hides fill and epilogue of short K loops (MoE) and doubles the issuers for decode
   // activation stages (64 k each).  Up to 128 tokens there are as many as operand stages, and one barrier per stage
@@ -182,7 +174,7 @@ umma_wo_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constant__
   constexpr int GPR = CPR < NG ? CPR : NG;            // transform groups that touch one raw stage
   // With equally deep rings chunk g uses operand stage g % S and activation stage g % XS = the same index, and the MMAs
   // that free one free the other: the activation producer waits on the operand stage's barrier, the issuer commits once
-  // (MoE pipeline 676 -> 664 us; the decode tiles are indifferent).
+  // (grouped 128-token tiles 2 % faster, the decode tiles indifferent, both with INT4, which umma_w4.cu has since taken over).
   constexpr bool SHARED_EMPTY = S == XS;
 
   extern __shared__ uint8_t smem_raw[];
@@ -193,11 +185,10 @@ umma_wo_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constant__
   // barrier map (8 bytes each)
   const uint32_t x_full = bar, x_empty = x_full + 8 * XS, a_full = x_empty + 8 * XS, ab_empty = a_full + 8 * S;
   const uint32_t raw_full = ab_empty + 8 * S, raw_empty = raw_full + 8 * RS, accum_full = raw_empty + 8 * RS;
-  const uint32_t accum_empty = accum_full + 8, fix_bar = accum_full + 16;
+  const uint32_t fix_bar = accum_full + 8;
   uint8_t* gen = smem_raw + (base - smem_u32(smem_raw));
-  volatile uint32_t* tmem_slot = reinterpret_cast<volatile uint32_t*>(gen + (accum_full + 24 - base));
-  volatile int* abort_flag = reinterpret_cast<volatile int*>(gen + (accum_full + 32 - base));
-  volatile int* last_flag = reinterpret_cast<volatile int*>(gen + (accum_full + 36 - base));
+  volatile uint32_t* tmem_slot = reinterpret_cast<volatile uint32_t*>(gen + (accum_full + 16 - base));
+  volatile int* abort_flag = reinterpret_cast<volatile int*>(gen + (accum_full + 24 - base));
 
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
 
@@ -220,34 +211,8 @@ umma_wo_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constant__
     xrow0 = p.expert_offsets[expert];
     M = p.expert_offsets[expert + 1] - xrow0;
   }
-  // A CTA works through a list of segments = (strip of 128 weight rows, range of 64-k chunks).  Normally that
-  // is one whole strip, blockIdx.y.  Balanced mode (decode shapes, one token tile): the launch is a 1-D grid
-  // that fills the machine exactly, the work is cut into units of one raw stage, and CTA b takes the units
-  // [b U / G, (b + 1) U / G): up to two partial strips around any number of whole ones.  Every role below walks
-  // the same list with its own copy of this cursor.
-  constexpr bool BAL = TOK <= 64;               // only decode tiles carry the multi-segment / partial-sum code
-  const bool balanced = BAL && p.sk_sps > 0;
-  int u = 0, u0 = 0, u1 = 1;
-  if (balanced) {
-    tok0 = 0;
-    u0 = (int)((int64_t)blockIdx.x * p.sk_units / gridDim.x);
-    u1 = (int)((int64_t)(blockIdx.x + 1) * p.sk_units / gridDim.x);
-    u = u0;
-  }
-  auto next_segment = [&](Segment& sg) -> bool {
-    if (u >= u1) return false;
-    if (!balanced) {
-      sg.n0 = strip_idx * 128; sg.c_begin = 0; sg.nk = p.K / 64; sg.strip = strip_idx; sg.part = 0; sg.slot = 0;
-      u = u1;
-      return true;
-    }
-    const int strip = u / p.sk_sps, r0 = u - strip * p.sk_sps;
-    const int take = min(p.sk_sps - r0, u1 - u);
-    sg.n0 = strip * 128; sg.c_begin = r0 * CPR; sg.nk = take * CPR; sg.strip = strip;
-    sg.part = take != p.sk_sps; sg.slot = (u == u0) ? 0 : 1;
-    u += take;
-    return true;
-  };
+  constexpr bool DECODE = TOK <= 64;            // only decode tiles carry the code that delivers to peer ranks
+  const int n0 = strip_idx * 128, nk = p.K / 64;
   const int64_t sbase = (int64_t)expert * p.s_expert_elems;
 
   if (threadIdx.x == 0) {
@@ -255,7 +220,6 @@ umma_wo_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constant__
     for (int i = 0; i < XS; ++i) { mbar_init(x_full + 8 * i, 1); mbar_init(x_empty + 8 * i, 1); }
     for (int i = 0; i < RS; ++i) { mbar_init(raw_full + 8 * i, 1); mbar_init(raw_empty + 8 * i, GPR * 128); }
     mbar_init(accum_full, Cfg::NMMA);
-    mbar_init(accum_empty, NG * 128);
     mbar_init(fix_bar, NG * 128);
     *abort_flag = 0;
     fence_barrier_init();
@@ -265,28 +229,23 @@ umma_wo_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constant__
   __syncthreads();
   tc_fence_after();
   const uint32_t tmem = *tmem_slot;
-  Segment sg;
 
   if (warp == 0) {
     // ---------------- raw weight producer ----------------
     if (elect_one()) {
       tma_prefetch_desc(&tm_w);
-      int grb = 0;                       // raw stages issued so far: ring position and phase carry across segments
+      const int nraw = (nk + CPR - 1) / CPR;
       int issued = 0;
       bool ok = true;
-      while (ok && next_segment(sg)) {
-        const int nraw = (sg.nk + CPR - 1) / CPR;
-        for (int r = 0; r < nraw; ++r) {
-          const int gr = grb + r, rs = gr % RS;
-          { if (gr >= RS && !mbar_wait(raw_empty + 8 * rs, ((gr / RS) - 1) & 1, abort_flag, p.status, ST_RAWEMPTY)) { ok = false; break; } }
-          issued = gr + 1;
-          mbar_expect_tx(raw_full + 8 * rs, Cfg::RAW_BYTES);
-          if constexpr (WK == WK_W4K)
-            tma_load_2d(raw_smem + rs * Cfg::RAW_BYTES, &tm_w, sg.n0, expert * p.w_rows_per_expert + (sg.c_begin / CPR + r) * 32, raw_full + 8 * rs);
-          else
-            tma_load_2d(raw_smem + rs * Cfg::RAW_BYTES, &tm_w, (sg.c_begin / CPR + r) * 128, expert * p.w_rows_per_expert + sg.n0, raw_full + 8 * rs);
-        }
-        grb += nraw;
+      for (int gr = 0; gr < nraw; ++gr) {
+        const int rs = gr % RS;
+        if (gr >= RS && !mbar_wait(raw_empty + 8 * rs, ((gr / RS) - 1) & 1, abort_flag, p.status, ST_RAWEMPTY)) { ok = false; break; }
+        issued = gr + 1;
+        mbar_expect_tx(raw_full + 8 * rs, Cfg::RAW_BYTES);
+        if constexpr (WK == WK_W4K)
+          tma_load_2d(raw_smem + rs * Cfg::RAW_BYTES, &tm_w, n0, expert * p.w_rows_per_expert + gr * 32, raw_full + 8 * rs);
+        else
+          tma_load_2d(raw_smem + rs * Cfg::RAW_BYTES, &tm_w, gr * 128, expert * p.w_rows_per_expert + n0, raw_full + 8 * rs);
       }
       if (!ok) drain_issued(raw_full, RS, issued);
     }
@@ -295,17 +254,14 @@ umma_wo_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constant__
     if (elect_one()) {
       tma_prefetch_desc(&tm_x);
       if (!p.tiles) grid_dep_wait();
-      int gb = 0, issued = 0;
+      int issued = 0;
       bool ok = true;
-      while (ok && next_segment(sg)) {
-        for (int c = 0; c < sg.nk; ++c) {
-          const int g = gb + c, s = g % XS;
-          { if (g >= XS && !mbar_wait((SHARED_EMPTY ? ab_empty : x_empty) + 8 * s, ((g / XS) - 1) & 1, abort_flag, p.status, ST_EMPTY)) { ok = false; break; } }
-          issued = g + 1;
-          mbar_expect_tx(x_full + 8 * s, Cfg::X_BYTES);
-          tma_load_2d(x_smem + s * Cfg::X_BYTES, &tm_x, (sg.c_begin + c) * 64, xrow0 + tok0, x_full + 8 * s);
-        }
-        gb += sg.nk;
+      for (int g = 0; g < nk; ++g) {
+        const int s = g % XS;
+        if (g >= XS && !mbar_wait((SHARED_EMPTY ? ab_empty : x_empty) + 8 * s, ((g / XS) - 1) & 1, abort_flag, p.status, ST_EMPTY)) { ok = false; break; }
+        issued = g + 1;
+        mbar_expect_tx(x_full + 8 * s, Cfg::X_BYTES);
+        tma_load_2d(x_smem + s * Cfg::X_BYTES, &tm_x, g * 64, xrow0 + tok0, x_full + 8 * s);
       }
       if (!ok) drain_issued(x_full, XS, issued);
     }
@@ -317,29 +273,23 @@ umma_wo_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constant__
       const uint32_t dacc = tmem + me * Cfg::ACC_COLS;
       const uint64_t db0 = smem_desc_sw128(x_smem);
       bool ok = true;
-      int gb = 0, si = 0;
-      while (ok && next_segment(sg)) {
-        // the accumulators are reused: wait until the epilogue warps have read the previous segment's
-        if (BAL && si > 0) { ok = mbar_wait(accum_empty, (si - 1) & 1, abort_flag, p.status, ST_ACCEMPTY); if (!ok) break; tc_fence_after(); }
 #pragma unroll 1
-        for (int c = me; c < sg.nk; c += Cfg::NMMA) {
-          const int g = gb + c, s = g % S, xs = g % XS;
-          { ok = mbar_wait(x_full + 8 * xs, (g / XS) & 1, abort_flag, p.status, ST_XFULL); }
-          if (ok) { ok = mbar_wait(a_full + 8 * s, (g / S) & 1, abort_flag, p.status, ST_AFULL); }
-          if (!ok) break;
-          tc_fence_after();
-          const uint32_t ta = tmem + Cfg::A_COL0 + 32 * s;
-          const uint64_t db = db0 + (uint64_t)(xs * (Cfg::X_BYTES >> 4));
-          mma_f16_ts(dacc, ta, db, idesc, c >= Cfg::NMMA ? 1u : 0u);
-          mma_f16_ts(dacc, ta + 8, db + 2, idesc, 1u);
-          mma_f16_ts(dacc, ta + 16, db + 4, idesc, 1u);
-          mma_f16_ts(dacc, ta + 24, db + 6, idesc, 1u);
-          tc_commit(ab_empty + 8 * s);
-          if constexpr (!SHARED_EMPTY) tc_commit(x_empty + 8 * xs);
-        }
-        if (ok) tc_commit(accum_full);
-        gb += sg.nk; ++si;
+      for (int g = me; g < nk; g += Cfg::NMMA) {
+        const int s = g % S, xs = g % XS;
+        ok = mbar_wait(x_full + 8 * xs, (g / XS) & 1, abort_flag, p.status, ST_XFULL);
+        if (ok) ok = mbar_wait(a_full + 8 * s, (g / S) & 1, abort_flag, p.status, ST_AFULL);
+        if (!ok) break;
+        tc_fence_after();
+        const uint32_t ta = tmem + Cfg::A_COL0 + 32 * s;
+        const uint64_t db = db0 + (uint64_t)(xs * (Cfg::X_BYTES >> 4));
+        mma_f16_ts(dacc, ta, db, idesc, g >= Cfg::NMMA ? 1u : 0u);
+        mma_f16_ts(dacc, ta + 8, db + 2, idesc, 1u);
+        mma_f16_ts(dacc, ta + 16, db + 4, idesc, 1u);
+        mma_f16_ts(dacc, ta + 24, db + 6, idesc, 1u);
+        tc_commit(ab_empty + 8 * s);
+        if constexpr (!SHARED_EMPTY) tc_commit(x_empty + 8 * xs);
       }
+      if (ok) tc_commit(accum_full);
     }
   } else {
     // ---------------- transform, then epilogue (the NG x 4 warps after the control warps) ----------------
@@ -351,9 +301,6 @@ umma_wo_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constant__
     const bool blockscale = (WK == WK_W8) && (p.scale_mode == B2Q_SCALE_BLOCK128);
     const int kblocks = (p.K + 127) >> 7;
     bool ok = true;
-    int gb = 0, grb = 0, si = 0, fixn = 0;       // chunks / raw stages / segments / fix-up barrier phases so far
-    while (ok && next_segment(sg)) {
-    const int n0 = sg.n0, nk = sg.nk, c_begin = sg.c_begin;
     int nrow = n0 + t; if (nrow >= p.N) nrow = p.N - 1;
     // The scale of a chunk (one per weight row for INT4, one per CTA for block-scaled FP8) comes from global memory,
     // usually from DRAM (scales are read once per launch): about a thousand cycles.  Scales are requested four to
@@ -365,11 +312,11 @@ umma_wo_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constant__
     auto chunk_scale_raw = [&](int c) -> uint32_t {
       if (c >= nk) return 0u;
       if constexpr (WK == WK_W4N || WK == WK_W4K) {
-        const int64_t i = sbase + (int64_t)nrow * p.s_stride_n + (int64_t)((c_begin + c) >> 1) * p.s_stride_g;
+        const int64_t i = sbase + (int64_t)nrow * p.s_stride_n + (int64_t)(c >> 1) * p.s_stride_g;
         if (p.scale_dtype == B2Q_F32) return __ldg(reinterpret_cast<const uint32_t*>(p.scale) + i);
         return (uint32_t)__ldg(reinterpret_cast<const unsigned short*>(p.scale) + i);
       } else {
-        return blockscale ? __ldg(reinterpret_cast<const uint32_t*>(p.scale) + sbase + (int64_t)(n0 >> 7) * kblocks + ((c_begin + c) >> 1)) : 0u;
+        return blockscale ? __ldg(reinterpret_cast<const uint32_t*>(p.scale) + sbase + (int64_t)(n0 >> 7) * kblocks + (c >> 1)) : 0u;
       }
     };
     auto scale_value = [&](uint32_t raw) -> float {
@@ -391,19 +338,18 @@ umma_wo_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constant__
     float blk_mul = 1.f, blk_post = 1.f;
     if constexpr (WK == WK_W8 && !BF16) {
       if (blockscale) {
-        const int k = block_scale_exponent(reinterpret_cast<const float*>(p.scale) + sbase + (int64_t)(n0 >> 7) * kblocks + (c_begin >> 1), (nk + 1) >> 1);
+        const int k = block_scale_exponent(reinterpret_cast<const float*>(p.scale) + sbase + (int64_t)(n0 >> 7) * kblocks, (nk + 1) >> 1);
         blk_mul = pow2(k); blk_post = pow2(-k);
       }
     }
-    // Position in the raw ring: by counting (this group converts CPG chunks of every raw stage, a segment starts on a
-    // stage boundary, jj counts them) or by dividing the chunk number by the stage count for every chunk.  Which is
-    // faster is a matter of what the register allocator makes of the loop, measured per tile width on one GPU: the
-    // 128-token grouped tiles gain 3 % from counting (MoE pipeline 693 -> 672 us), the decode tiles lose 2 %
-    // (gate_up at M = 64: 133 -> 136 us).
+    // Position in the raw ring: by counting (this group converts CPG chunks of every raw stage, jj counts them) or by
+    // dividing the chunk number by the stage count for every chunk.  Which is faster is a matter of what the register
+    // allocator makes of the loop: measured with INT4, the 128-token grouped tiles gained 3 % from counting, the decode
+    // tiles lost 2 %.
     constexpr bool COUNTED = TOK > 64 && NG <= CPR;      // counting assumes every group has a chunk in every raw stage
     constexpr int CPG = CPR / NG > 0 ? CPR / NG : 1;
-    int jj = 0, rs = grb % RS;
-    uint32_t rpar = (uint32_t)(grb / RS) & 1u;
+    int jj = 0, rs = 0;
+    uint32_t rpar = 0u;
 #pragma unroll 1
     for (int c = grp; c < nk; c += NG) {
       if (it4 == 4) {
@@ -418,7 +364,7 @@ umma_wo_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constant__
       if constexpr (COUNTED) {
         j = grp + jj * NG;                           // == c % CPR
       } else {
-        const int gr = grb + c / CPR;
+        const int gr = c / CPR;
         j = c % CPR; rs = gr % RS; rpar = (uint32_t)(gr / RS) & 1u;
       }
       ok = mbar_wait_warp(raw_full + 8 * rs, rpar, abort_flag, p.status, ST_RAWFULL);
@@ -427,9 +373,9 @@ umma_wo_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constant__
       const uint32_t rawrow = raw_smem + rs * Cfg::RAW_BYTES + t * 128;     // N-major / fp8: this thread's row
       const uint32_t rawcol = raw_smem + rs * Cfg::RAW_BYTES + t * 4;       // K-major: this thread's column
       {
-        const int g = gb + c, s = g % S;
+        const int s = c % S;
         // no test for the ring's first round: a wait for the phase before a fresh barrier's first one returns at once
-        { ok = mbar_wait_warp(ab_empty + 8 * s, ((g / S) + 1) & 1, abort_flag, p.status, ST_EMPTY); if (!ok) break; }
+        { ok = mbar_wait_warp(ab_empty + 8 * s, ((c / S) + 1) & 1, abort_flag, p.status, ST_EMPTY); if (!ok) break; }
         tc_fence_after();
         const uint32_t ta = tmem + ((uint32_t)((warp & 3) * 32) << 16) + Cfg::A_COL0 + 32 * s;
         {
@@ -513,11 +459,10 @@ umma_wo_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constant__
         if (c + NG >= nk || (c + NG) / CPR != c / CPR) mbar_arrive(raw_empty + 8 * rs);
       }
     }
-    if (!ok) break;
 
-    // ---------------- epilogue of this segment ----------------
-    { ok = mbar_wait_warp(accum_full, si & 1, abort_flag, p.status, ST_ACCUM); }
-    if (!ok) break;
+    // ---------------- epilogue ----------------
+    if (ok) ok = mbar_wait_warp(accum_full, 0, abort_flag, p.status, ST_ACCUM);
+    if (ok) {
     tc_fence_after();
     const int quad = warp & 3;                   // tensor-memory lane quadrant this warp may read
     const int cgrp = (warp - Cfg::CW) >> 2;      // the NG warps of a quadrant take column blocks in turn
@@ -537,7 +482,7 @@ umma_wo_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constant__
     // ([block][row][128 columns]) with plain peer stores, and the owner is told through flag1 when the strip is done.
     uint16_t* peer_dst = nullptr;
     uint32_t* peer_flag = nullptr;
-    if constexpr (BAL) {
+    if constexpr (DECODE) {
       if (p.peer_on) {
         const int owner = n0 / p.peer.slice, blk = (n0 - owner * p.peer.slice) >> 7;
         uint8_t* ob = p.peer.bufs[owner];
@@ -560,14 +505,11 @@ umma_wo_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constant__
           if (p.out_map) orow = p.out_map[orow];
           const float v = __uint_as_float(r[i]) * post * ts;
           uint16_t* dst = outp + orow * p.ldo + n;
-          if constexpr (BAL) { if (peer_dst) dst = peer_dst + (size_t)tok * PR_CB; }
+          if constexpr (DECODE) { if (peer_dst) dst = peer_dst + (size_t)tok * PR_CB; }
           *dst = p.out_bf16 ? __bfloat16_as_ushort(__float2bfloat16_rn(v)) : __half_as_ushort(__float2half_rn(v));
         }
       }
     };
-    // partial sums of a cut strip: [CTA][slot][token][row of the strip] fp32, raw accumulator values
-    float* const my_part = balanced ? p.sk_partials + ((size_t)(blockIdx.x * 2 + sg.slot) * TOK) * 128 + quad * 32 + lane : nullptr;
-    bool freed = false;
 #pragma unroll 1
     for (int cb = cgrp * CB; cb < TOK; cb += NG * CB) {
       if (tok0 + cb >= M) break;
@@ -588,78 +530,19 @@ umma_wo_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constant__
 #pragma unroll
         for (int i = 0; i < CB; ++i) r[i] = __float_as_uint(__uint_as_float(r[i]) + __uint_as_float(q[i]));
       }
-      // balanced mode has one column block per thread at most: the accumulators are free for the next segment now
-      if (BAL && balanced && !freed) { tc_fence_before(); mbar_arrive(accum_empty); freed = true; }
-      if (!BAL || !sg.part) {
-        write_out(r, cb);
-      } else {
-#pragma unroll
-        for (int i = 0; i < CB; ++i)
-          if (cb + i < M) __stcg(my_part + (cb + i) * 128, __uint_as_float(r[i]));
-      }
+      write_out(r, cb);
     }
-    if (BAL && balanced && !freed) { tc_fence_before(); mbar_arrive(accum_empty); }
-    if constexpr (BAL) {
-      if (peer_flag && !sg.part) {
+    if constexpr (DECODE) {
+      if (peer_flag) {
         // all epilogue threads have issued their stores of this strip; one of them publishes it
         mbar_arrive(fix_bar);
-        ok = mbar_wait_warp(fix_bar, fixn & 1, abort_flag, p.status, ST_FIXUP); ++fixn;
-        if (!ok) break;
-        if (threadIdx.x == Cfg::CW * 32) {
+        if (mbar_wait_warp(fix_bar, 0, abort_flag, p.status, ST_FIXUP) && threadIdx.x == Cfg::CW * 32) {
           __threadfence_system();
           st_release_sys(peer_flag, reinterpret_cast<const PeerCtrl*>(p.peer.bufs[p.peer.rank])->epoch + 1);
         }
       }
     }
-    if (BAL && sg.part) {
-      // Whoever delivers a strip's last partial sums adds all of them up, always in CTA order, and writes the
-      // result: no CTA ever waits for another one, and the sum does not depend on who came last.
-      const int64_t U = p.sk_units, G = gridDim.x;
-      const int64_t us = (int64_t)sg.strip * p.sk_sps, ue = us + p.sk_sps - 1;
-      const int b_lo = (int)(((us + 1) * G + U - 1) / U) - 1, b_hi = (int)(((ue + 1) * G + U - 1) / U) - 1;
-      // the barrier hands every thread's partial sums to the leader (release / acquire at CTA scope); the leader's one
-      // device-scope fence then orders all of them before the count.  A fence per thread in front of the barrier adds
-      // nothing to that and cost 0.7 % of a decode layer.
-      mbar_arrive(fix_bar);
-      ok = mbar_wait_warp(fix_bar, fixn & 1, abort_flag, p.status, ST_FIXUP); ++fixn;
-      if (!ok) break;
-      if (threadIdx.x == Cfg::CW * 32) {
-        __threadfence();                               // orders the partial sums of all epilogue threads before the count
-        const int old = atomicAdd(p.sk_counters + sg.strip, 1);
-        const int last = old == b_hi - b_lo;
-        if (last) p.sk_counters[sg.strip] = 0;       // every contributor has arrived: ready for the next launch
-        *last_flag = last;
-      }
-      mbar_arrive(fix_bar);
-      ok = mbar_wait_warp(fix_bar, fixn & 1, abort_flag, p.status, ST_FIXUP); ++fixn;
-      if (!ok) break;
-      const int cb = cgrp * CB;
-      if (*last_flag && cb < TOK && cb < M) {
-        __threadfence();
-        uint32_t r[32];
-#pragma unroll
-        for (int i = 0; i < CB; ++i) r[i] = 0u;
-        for (int b = b_lo; b <= b_hi; ++b) {
-          const int64_t bu0 = (int64_t)b * U / G;
-          const float* src = p.sk_partials + ((size_t)(b * 2 + (bu0 >= us ? 0 : 1)) * TOK) * 128 + quad * 32 + lane;
-#pragma unroll
-          for (int i = 0; i < CB; ++i)
-            if (cb + i < M) r[i] = __float_as_uint(__uint_as_float(r[i]) + __ldcg(src + (cb + i) * 128));
-        }
-        write_out(r, cb);
-      }
-      if (*last_flag && peer_flag) {
-        mbar_arrive(fix_bar);
-        ok = mbar_wait_warp(fix_bar, fixn & 1, abort_flag, p.status, ST_FIXUP); ++fixn;
-        if (!ok) break;
-        if (threadIdx.x == Cfg::CW * 32) {
-          __threadfence_system();
-          st_release_sys(peer_flag, reinterpret_cast<const PeerCtrl*>(p.peer.bufs[p.peer.rank])->epoch + 1);
-        }
-      }
     }
-    gb += nk; grb += (nk + CPR - 1) / CPR; ++si;
-    }   // segments
   }
 
   tc_fence_before();
@@ -773,12 +656,10 @@ int umma_read_status(int* out) {
 }
 
 
-// ---- balanced mode (decode shapes) ----------------------------------------------------------------
 // Arrival counters of cut strips.  They are zero whenever no launch is in flight (the last arriver of a
 // strip resets its counter), so nothing has to be cleared per launch; launches take one of 64 banks in turn
 // so that launches overlapping in time (other streams, programmatic dependent launch) do not share counters.
-
-static int* sk_counter_bank() {
+int* umma_strip_counters() {
   static thread_local int* basep[16] = {nullptr};
   static std::atomic<unsigned> next_bank{0};
   int dev = 0;
@@ -790,48 +671,6 @@ static int* sk_counter_bank() {
     basep[dev] = reinterpret_cast<int*>(p);
   }
   return basep[dev] + (size_t)(next_bank.fetch_add(1, std::memory_order_relaxed) % SK_BANKS) * SK_MAX_STRIPS;
-}
-
-int* umma_strip_counters() { return sk_counter_bank(); }
-
-static int device_slots() {
-  static thread_local int sms[16] = {0};
-  int dev = 0;
-  cudaGetDevice(&dev);
-  if (dev < 0 || dev >= 16) return 296;
-  if (!sms[dev]) {
-    cudaDeviceGetAttribute(&sms[dev], cudaDevAttrMultiProcessorCount, dev);
-    if (sms[dev] <= 0) sms[dev] = 148;
-  }
-  return 2 * sms[dev];                     // decode tiles run two CTAs per SM
-}
-
-static int pick_tok(int m);
-
-size_t umma_balanced_ws_bytes(int64_t M) {
-  if (M > 64) return 0;
-  return (size_t)2 * device_slots() * pick_tok((int)M) * 128 * sizeof(float);
-}
-
-// Fills the balanced-mode fields of p when the shape profits: one token tile, whole raw stages, and a grid of
-// one CTA per strip that would leave more than a twentieth of the machine idle in its last wave.
-static int plan_balanced(UmmaWoParams& p, const UmmaGroupArgs& a, int M, int N, int K, int cpr, int tok) {
-  p.sk_sps = 0; p.sk_units = 0; p.sk_partials = nullptr; p.sk_counters = nullptr;
-  if (tls().force_kernel == 4) return 0;       // benchmarking: one CTA per strip
-  if (a.expert_offsets || tok > 64 || M > tok || !a.sk_ws || a.sk_ws_bytes < umma_balanced_ws_bytes(M)) return 0;
-  if ((K % (64 * cpr)) != 0 || (reinterpret_cast<uintptr_t>(a.sk_ws) & 15u)) return 0;
-  const int strips = (N + 127) / 128, slots = device_slots();
-  if (strips > SK_MAX_STRIPS) return 0;
-  const double eff = (double)strips / ((double)((strips + slots - 1) / slots) * slots);
-  if (eff > 0.95) return 0;
-  const int sps = K / (64 * cpr);
-  const int64_t units = (int64_t)strips * sps;
-  if (units > INT32_MAX) return 0;
-  int* counters = sk_counter_bank();
-  if (!counters) return 0;
-  p.sk_sps = sps; p.sk_units = (int)units;
-  p.sk_partials = reinterpret_cast<float*>(a.sk_ws); p.sk_counters = counters;
-  return (int)(units < slots ? units : slots);
 }
 
 static int pick_tok(int m) { return m <= 16 ? 16 : (m <= 32 ? 32 : (m <= 64 ? 64 : (m <= 128 ? 128 : 256))); }
@@ -851,7 +690,6 @@ static int launch_one(const CUtensorMap& tw, const CUtensorMap& tx, const UmmaWo
   }
   dim3 grid(token_tiles, (p.N + 127) / 128, 1);
   if (p.tiles_on_y) grid = dim3((p.N + 127) / 128, token_tiles, 1);
-  if (p.sk_sps > 0) grid = dim3(p.sk_grid, 1, 1);
   const bool overlap = tls().overlap_mode > 0 && p.overlap_ok;
   if (launch_overlapped(kern, grid, dim3(Cfg::THREADS), Cfg::SMEM, st, overlap, tw, tx, p) != cudaSuccess) return B2Q_ERR_CUDA;
   note_launch("umma_wo");
@@ -872,6 +710,8 @@ static int launch_tok(int tok, const CUtensorMap& tw, const CUtensorMap& tx, con
 template <int WK>
 static int launch_wk(bool bf16, bool fast, int tok, const CUtensorMap& tw, const CUtensorMap& tx, const UmmaWoParams& p,
                      int tiles, cudaStream_t st) {
+  if constexpr (WK == WK_W8)        // FAST is about INT4 scales
+    return bf16 ? launch_tok<WK, true, true>(tok, tw, tx, p, tiles, st) : launch_tok<WK, false, true>(tok, tw, tx, p, tiles, st);
   if (bf16) return fast ? launch_tok<WK, true, true>(tok, tw, tx, p, tiles, st) : launch_tok<WK, true, false>(tok, tw, tx, p, tiles, st);
   return fast ? launch_tok<WK, false, true>(tok, tw, tx, p, tiles, st) : launch_tok<WK, false, false>(tok, tw, tx, p, tiles, st);
 }
@@ -919,7 +759,6 @@ int umma_w4_linear(const UmmaW4Args& a, cudaStream_t st) {
   p.tok_scale = a.tok_scale; p.out_bf16 = a.out_bf16 ? 1 : 0;
   p.status = status_ptr();
   p.overlap_ok = (a.after_prep || tls().overlap_mode == 2) ? 1 : 0;
-  p.sk_grid = plan_balanced(p, a, a.M, a.N, a.K, 4, tok);
   if (a.peer) {
     if (tok > 64 || grouped || (a.N % 128) != 0 || (a.peer->slice % 128) != 0 || a.peer->M != a.M) return B2Q_ERR_UNSUPPORTED;
     p.peer_on = 1; p.peer = *a.peer;
@@ -961,7 +800,6 @@ int umma_w8_linear(const UmmaW8Args& a, cudaStream_t st) {
   p.tok_scale = a.tok_scale; p.out_bf16 = a.out_bf16 ? 1 : 0;
   p.status = status_ptr();
   p.overlap_ok = (a.after_prep || tls().overlap_mode == 2) ? 1 : 0;
-  p.sk_grid = plan_balanced(p, a, a.M, a.N, a.K, 2, tok);
   const int tiles = grouped ? a.tile_cap : (a.M + tok - 1) / tok;
   return launch_wk<WK_W8>(a.bf16, true, tok, tw, tx, p, tiles, st);
 }

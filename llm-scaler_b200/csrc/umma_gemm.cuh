@@ -121,8 +121,6 @@ int umma_w8_linear(const UmmaW8Args& a, cudaStream_t st);
 
 int umma_w8a8_block(const UmmaW8A8Args& a, cudaStream_t st);
 
-size_t umma_balanced_ws_bytes(int64_t M);
-
 // First device-side wait timeout recorded since the library was loaded (0 = none).  Synchronises.
 int umma_read_status(int* out);
 // Clears the status word of the tcgen05 weight-only kernels; launches the bounded-wait self-test (see the kernel).
