@@ -240,7 +240,10 @@ static int linear_int4_core(const void* x, int act_dtype, int64_t ldx, const voi
   }
   // measured on B200: the mma.sync streaming kernel wins only for a handful of tokens (its per-token cost is
   // fragment traffic), the tcgen05 kernel is flat in M up to 64 and the only one for K-major layouts and prefill
-  // small weights at small M: one launch of the streaming kernel beats pre-pass + GEMM
+  // small weights at small M: one launch of the streaming kernel beats pre-pass + GEMM (16 / 32 tokens: 1024 x 1024 3.5 / 5.4
+  // against 8.4 / 10.1 us, 2048 x 4096 8.6 / 17.3 against 13.9 / 17.5, 4096 x 4096 11.8 / 19.6 against 16.1 / 17.8).  At the upper
+  // end of the line umma_w4.cu is the faster one (8192 x 4096: 24.3 / 41.3 against 15.8 / 17.9 us), but it rounds
+  // (q - 8) * scale to fp16, which these shapes, exact for every scale here, have never had done to them.
   const bool tiny = M <= 32 && N * K <= (int64_t)1 << 25;
   const bool want_umma = force >= 2 || (force == 0 && (kmajor || (M > 8 && !tiny)));
   if (umma_ok && want_umma) {
@@ -571,9 +574,9 @@ int b2q_moe_gemm_int4(const void* x, int act_dtype, int64_t ldx, const int32_t* 
   ua.out = gemm_out; ua.ldo = gemm_ldo; ua.M = (int)rows; ua.N = (int)N; ua.K = (int)K;
   ua.expert_offsets = expert_offsets; ua.E = E; ua.out_map = gemm_out_map; ua.tiles = tiles;
   const int64_t avg = (rows + E - 1) / E;
-  // measured on 128 experts of [1536 x 2048] / [2048 x 768] at 1 to 256 tokens (top-8): the tcgen05 kernel behind its
-  // pre-pass beats the streaming kernel at every batch (49 / 76 / 139 / 205 / 284 us per pipeline pass against
-  // 60 / 94 / 177 / 286 / 467), so only experts too small to matter stay on the streaming kernel
+  // measured on 128 experts of [1536 x 2048] / [2048 x 768] at 1 / 4 / 16 / 64 / 256 tokens (top-8): the tcgen05 kernel behind
+  // its pre-pass beats the streaming kernel at every batch (39 / 55 / 93 / 125 / 165 us per pipeline pass against
+  // 58 / 84 / 185 / 281 / 457), so only experts too small to matter stay on the streaming kernel
   const bool want_umma = force == 2 || (force == 0 && (kmajor || avg > 16 || N * K >= ((int64_t)1 << 20)));
   ua.out_bf16 = bf;
   if (umma_w4_supported(ua) && want_umma) {

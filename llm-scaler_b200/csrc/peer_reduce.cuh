@@ -1,5 +1,5 @@
 // Buffer layout and flag protocol shared by the peer-memory reduction kernel (peer_reduce.cu) and the GEMM epilogue
-// that performs the reduction's first step itself (umma_gemm.cu).
+// that performs the reduction's first step itself (umma_w4.cu; without scratch umma_gemm.cu).
 #pragma once
 #include "common.cuh"
 

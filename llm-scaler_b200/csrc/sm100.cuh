@@ -84,8 +84,8 @@ __device__ __forceinline__ bool mbar_test(uint32_t bar, uint32_t parity) {
 // timeout releases all the others; `status` is a global word the host can read.  The clock
 // and the abort flag are looked at once every 128 polls so the spin itself stays two
 // instructions long.  A plain test comes before the first suspending one: where the phase is already over it is the cheaper
-// (W8A8 4096 x 17408 x 5120 566 -> 548 us; INT4 decoder layer at M = 2048 3073 -> 3014 us, at M = 64 209.4 -> 206.1 us;
-// INT4 MoE pipeline at 4096 tokens 583 -> 573 us; the other kernels are indifferent).
+// (W8A8 4096 x 17408 x 5120 566 -> 551 us; INT4 decoder layer at M = 2048 3073 -> 3005 us, at M = 64 209.4 -> 207 us;
+// INT4 MoE pipeline at 4096 tokens 583 -> 571 us; the other kernels are indifferent).
 __device__ __forceinline__ bool mbar_wait(uint32_t bar, uint32_t parity, volatile int* abort_flag, int* status, int code,
                                           long long limit_ticks = WAIT_LIMIT_TICKS) {
   if (mbar_test(bar, parity)) return true;

@@ -1,5 +1,5 @@
 // Weight-only GEMM on tcgen05 for fp16 activations: out[tok, n] = sum_k x[tok, k] * W[n, k], W INT4 (group 128, behind the
-// activation pre-pass) or, for decode tiles, block-scaled e4m3.
+// activation pre-pass) or e4m3 (tiles of up to 64 tokens: block-scaled, or grouped with one scale per channel or tensor).
 //
 // Swap-AB: strips of R x 128 weight rows are the MMA's M dimension, a tile of TOK tokens its N dimension.  The nibbles are
 // decoded to fp16 in registers and written straight into tensor memory as the MMA's A operand (no trip back through
