@@ -127,6 +127,15 @@ __device__ __forceinline__ bool mbar_wait_warp(uint32_t bar, uint32_t parity, vo
   if (__all_sync(0xffffffffu, mbar_test(bar, parity))) return true;
   return __all_sync(0xffffffffu, mbar_wait(bar, parity, abort_flag, status, code)) != 0;
 }
+// Two waits of a whole warp, one vote where both phases are over (block-scaled FP8 128 x 17408 x 5120: 51.2 us with a vote each,
+// 50.6 with one, 50.1 with none).
+__device__ __forceinline__ bool mbar_wait_warp2(uint32_t bar, uint32_t parity, int code, uint32_t bar2, uint32_t parity2, int code2,
+                                                volatile int* abort_flag, int* status) {
+  if (__all_sync(0xffffffffu, mbar_test(bar, parity) && mbar_test(bar2, parity2))) return true;
+  bool ok = mbar_wait(bar, parity, abort_flag, status, code);
+  if (ok) ok = mbar_wait(bar2, parity2, abort_flag, status, code2);
+  return __all_sync(0xffffffffu, ok) != 0;
+}
 
 // ---- TMA: 2-D tiled load global -> shared, completion on an mbarrier -------------------
 // The innermost coordinate times the element size must be a multiple of 16 bytes.

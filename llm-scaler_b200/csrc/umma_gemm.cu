@@ -367,15 +367,14 @@ umma_wo_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constant__
         const int gr = c / CPR;
         j = c % CPR; rs = gr % RS; rpar = (uint32_t)(gr / RS) & 1u;
       }
-      ok = mbar_wait_warp(raw_full + 8 * rs, rpar, abort_flag, p.status, ST_RAWFULL);
+      const int s = c % S;
+      // no test for the ring's first round: a wait for the phase before a fresh barrier's first one returns at once
+      ok = mbar_wait_warp2(raw_full + 8 * rs, rpar, ST_RAWFULL, ab_empty + 8 * s, ((c / S) + 1) & 1, ST_EMPTY, abort_flag, p.status);
       if (!ok) break;
       const float sc_cur = scale_value(sr_cur);
       const uint32_t rawrow = raw_smem + rs * Cfg::RAW_BYTES + t * 128;     // N-major / fp8: this thread's row
       const uint32_t rawcol = raw_smem + rs * Cfg::RAW_BYTES + t * 4;       // K-major: this thread's column
       {
-        const int s = c % S;
-        // no test for the ring's first round: a wait for the phase before a fresh barrier's first one returns at once
-        { ok = mbar_wait_warp(ab_empty + 8 * s, ((c / S) + 1) & 1, abort_flag, p.status, ST_EMPTY); if (!ok) break; }
         tc_fence_after();
         const uint32_t ta = tmem + ((uint32_t)((warp & 3) * 32) << 16) + Cfg::A_COL0 + 32 * s;
         {
