@@ -134,7 +134,8 @@ def test_rejects_shapes_outside_the_contract(L):
     (64, 37888, 512, False), (48, 40960, 768, False),                              # 256-row strips, whole and cut
 ])
 @pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16])
-def test_gemm_epilogue_delivers_its_strips(L, M, N, K, kmajor, dtype):
+@pytest.mark.parametrize("scratch", [True, False])                                 # without it the two-CTA kernel delivers
+def test_gemm_epilogue_delivers_its_strips(L, M, N, K, kmajor, dtype, scratch):
     """b2q_linear_int4_allreduce with ONE rank: the GEMM's epilogue stores its strips into the rank's own reduction slots and
     raises their flags, and the reduction kernel, an ordinary launch behind it, finds every flag raised.  A sum over one rank
     is the linear itself, bit for bit; `partial` stays untouched where the epilogue delivers.  Several calls: epochs advance, the
@@ -145,8 +146,9 @@ def test_gemm_epilogue_delivers_its_strips(L, M, N, K, kmajor, dtype):
     sn, sg, layout = K // 128, 1, L.W4_NMAJOR
     if kmajor:
         w, s, sn, sg, layout = w.t().contiguous(), s.t().contiguous(), 1, N, L.W4_KMAJOR
-    wsb = L.lib.b2q_linear_workspace_bytes(M, N, K)
+    wsb = L.lib.b2q_linear_workspace_bytes(M, N, K) if scratch else 0
     ws = torch.empty(wsb, dtype=torch.uint8, device=DEV)
+    wsp = ws.data_ptr() if scratch else None
     comm = C.c_void_p()
     L.check(L.lib.b2q_comm_create_mode(0, 1, M, N, 2, C.byref(comm), None))
     try:
@@ -155,9 +157,9 @@ def test_gemm_epilogue_delivers_its_strips(L, M, N, K, kmajor, dtype):
             ref, partial = torch.empty(M, N, dtype=dtype, device=DEV), torch.full((M, N), 7.0, dtype=dtype, device=DEV)
             st = torch.cuda.current_stream().cuda_stream
             args = (x.data_ptr(), L.dt(x), K, w.data_ptr(), layout, s.data_ptr(), L.dt(s), sn, sg)
-            L.check(L.lib.b2q_linear_int4(*args, ref.data_ptr(), N, M, N, K, 128, ws.data_ptr(), wsb, st))
+            L.check(L.lib.b2q_linear_int4(*args, ref.data_ptr(), N, M, N, K, 128, wsp, wsb, st))
             out = C.c_void_p()
-            L.check(L.lib.b2q_linear_int4_allreduce(*args, partial.data_ptr(), N, M, N, K, 128, ws.data_ptr(), wsb, comm, C.c_double(500.0),
+            L.check(L.lib.b2q_linear_int4_allreduce(*args, partial.data_ptr(), N, M, N, K, 128, wsp, wsb, comm, C.c_double(500.0),
                                                     C.byref(out), st))
             assert torch.equal(L.view_as_tensor(out.value, (M, N), dtype, ref.device), ref), call
             assert bool((partial == 7.0).all())

@@ -160,6 +160,27 @@ def test_scratch_without_room_for_partial_sums_keeps_the_pre_pass(e, M, N, K):
     assert e._lib.device_status() == 0
 
 
+@pytest.mark.parametrize("M,kernel", [(33, "umma_w4"), (100, "umma_wo")])
+def test_fp8_scratch_for_the_pre_pass_alone(e, M, kernel):
+    """Block-scaled FP8, the same: bf16 activations are rewritten with scratch that holds nothing else."""
+    N, K = 2048, 2048
+    L = e._lib
+    g = torch.Generator(device=DEV).manual_seed(M)
+    w = (torch.randn(N, K, generator=g, device=DEV) * 96).clamp_(-448, 448).to(torch.float8_e4m3fn)
+    s = (0.5 + torch.rand(N // 128, K // 128, generator=g, device=DEV)) / 4096
+    x = torch.randn(M, K, generator=g, device=DEV).to(torch.bfloat16)
+    ref = x.double() @ (w.double() * s.double().repeat_interleave(128, 0).repeat_interleave(128, 1)).T
+    size = (2 * M * K + 255) // 256 * 256 + (4 * M + 255) // 256 * 256
+    ws = torch.empty(size, dtype=torch.uint8, device=DEV)
+    out = torch.full((M, N), float("nan"), dtype=torch.bfloat16, device=DEV)
+    before = e.launch_count()
+    L.check(L.lib.b2q_linear_fp8(x.data_ptr(), L.BF16, K, w.data_ptr(), L.E4M3, s.data_ptr(), L.F32, L.SCALE_BLOCK128, out.data_ptr(), N, M, N, K,
+                                 ws.data_ptr(), size, torch.cuda.current_stream().cuda_stream))
+    assert e.launch_count() - before == 2 and e.last_kernel() == kernel
+    _check(out, ref, M)
+    assert e._lib.device_status() == 0
+
+
 @pytest.mark.parametrize("E,rows,N,K", [
     (3, (60, 0, 33), 1096, 640),                       # 64-token tiles, short strips: few pieces
     (2, (129, 200), 520, 1152),                        # 128-token tiles, short strips
