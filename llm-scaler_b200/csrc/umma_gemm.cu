@@ -143,7 +143,7 @@ template <int TOK> struct UmmaCfg {
   static constexpr int CTAS = TOK <= 128 ? 2 : 1;                    // two CTAs per SM except for the 256-token prefill tile: a second CTA hides fill and epilogue of short K loops (MoE) and doubles the issuers for decode
   // activation stages (64 k each).  Up to 128 tokens there are as many as operand stages, and one barrier per stage
   // releases both (see SHARED_EMPTY in the kernel): one tcgen05.commit less per chunk for the issuing thread.
-  static constexpr int XS = TOK <= 128 ? 4 : 5;
+  static constexpr int XS = 4;
   // Issuing tcgen05.mma is a serial job of one thread and costs it several hundred cycles per 64-k
   // chunk regardless of the tile width; decode tiles therefore use two issuer warps on alternate
   // chunks, each with its own accumulator (summed in the epilogue).
@@ -154,7 +154,12 @@ template <int TOK> struct UmmaCfg {
   static constexpr int RAW_BYTES = 16384;
   static constexpr int SMEM_BUDGET = CTAS == 2 ? 114688 : 230400;    // per CTA, leaving room for the driver's reserve
   static constexpr int RS_FIT = (SMEM_BUDGET - 1536 - XS * X_BYTES) / RAW_BYTES;
-  static constexpr int RS = RS_FIT > 8 ? 8 : RS_FIT;                 // raw weight stages (16 KB each)
+  // Raw weight stages (16 KB each, two 64-k chunks of FP8).  A stage must always belong to the same transform groups: a parity
+  // wait cannot tell the phase it waits for from the one two before it, so a group that waits for a stage whose last use was
+  // another group's passes while that use is still under way, converts what happens to lie there and releases the stage for
+  // it.  Hence whole rounds of the groups.
+  static constexpr int RAW_ROUND = NG / 2;
+  static constexpr int RS = (RS_FIT > 8 ? 8 : RS_FIT) / RAW_ROUND * RAW_ROUND;
   static constexpr int SMEM = XS * X_BYTES + RS * RAW_BYTES + 1024 /*align*/ + 512 /*barriers*/;
   static constexpr int ACC_COLS = TOK < 32 ? 32 : TOK;               // fp32 accumulator columns
   static constexpr int A_COL0 = NMMA * ACC_COLS;                     // first operand column
@@ -163,6 +168,7 @@ template <int TOK> struct UmmaCfg {
   // the MMAs that read it have completed and signalled, a round trip of a couple of microseconds, so
   // the ring has to be deep for the transform warps to stay busy.
   static constexpr int S = (TMEM_COLS - A_COL0) / 32 > 12 ? 12 : (TMEM_COLS - A_COL0) / 32;
+  static_assert(RS >= RAW_ROUND && RS % RAW_ROUND == 0 && S % NG == 0, "ring depths in whole rounds of the transform groups");
 };
 
 template <int WK, bool BF16, int TOK, bool FAST>
