@@ -3,6 +3,7 @@
 #include "common.cuh"
 #include "smallm.cuh"
 #include "umma_gemm.cuh"
+#include "w4_stream.cuh"
 #include "peer_reduce.cuh"
 
 namespace b2q {
@@ -216,14 +217,12 @@ static int linear_int4_core(const void* x, int act_dtype, int64_t ldx, const voi
   if (peer) {
     const bool tiny_p = M <= 32 && N * K <= (int64_t)1 << 25;
     const bool umma_p = force >= 2 || (force == 0 && (kmajor || (M > 8 && !tiny_p)));
-    if (!umma_ok || !umma_p || M > 64 || (N % 128) != 0 || force == 5 || (force == 0 && umma_w4_i8_preferred(M, N, K) && M <= 16))
+    if (!umma_ok || !umma_p || M > 64 || (N % 128) != 0 || force == 5)
       return B2Q_ERR_UNSUPPORTED;
     ua.peer = peer;
   }
-  // the int8 tensor-core path (umma_w4_i8.cu): decode shapes, N-major nibbles, scratch available; on request, or
-  // where it measured fastest
-  if (!peer && (force == 5 || (force == 0 && umma_w4_i8_preferred(M, N, K))) && umma_ok && !kmajor && M <= 16 && workspace && aligned16(workspace) &&
-      workspace_bytes >= ws_i8_bytes(M, K)) {
+  // the int8 tensor-core path (umma_w4_i8.cu): decode shapes, N-major nibbles, scratch available; on request only
+  if (!peer && force == 5 && umma_ok && !kmajor && M <= 16 && workspace && aligned16(workspace) && workspace_bytes >= ws_i8_bytes(M, K)) {
     uint8_t* wsb = reinterpret_cast<uint8_t*>(workspace);
     float* inv = reinterpret_cast<float*>(wsb + align_up((size_t)umma_w4_i8_rows(M) * (size_t)K, 256));
     float* xsum = reinterpret_cast<float*>(reinterpret_cast<uint8_t*>(inv) + align_up((size_t)M * 4, 256));
@@ -238,8 +237,16 @@ static int linear_int4_core(const void* x, int act_dtype, int64_t ldx, const voi
     ia.partial_bytes = umma_w4_i8_partial_bytes();
     return umma_w4_i8_linear(ia, st);
   }
-  // measured on B200: the mma.sync streaming kernel wins only for a handful of tokens (its per-token cost is
-  // fragment traffic), the tcgen05 kernel is flat in M up to 64 and the only one for K-major layouts and prefill
+  // up to eight tokens, weights worth streaming: w4_stream.cu (w4_stream_preferred has the line and both sides of it)
+  if (!peer && !kmajor && (force == 7 ? M <= W4_STREAM_MAX_TOK : force == 0 && w4_stream_preferred(M, N, K))) {
+    W4StreamArgs sa{};
+    sa.x = x; sa.ldx = ldx; sa.bf16 = act_dtype == B2Q_BF16;
+    sa.w = w; sa.layout = w_layout; sa.scale = scale; sa.scale_dtype = scale_dtype; sa.s_stride_n = s_stride_n; sa.s_stride_g = s_stride_g;
+    sa.out = out; sa.ldo = ldo; sa.M = (int)M; sa.N = (int)N; sa.K = (int)K; sa.tile = (int)M;
+    sa.partials = workspace; sa.partial_bytes = workspace ? workspace_bytes : 0;
+    if (w4_stream_supported(sa)) return w4_stream_linear(sa, st);
+  }
+  // The tcgen05 kernel is flat in M up to 64 and the only one for K-major layouts and prefill.
   // small weights at small M: one launch of the streaming kernel beats pre-pass + GEMM (16 / 32 tokens: 1024 x 1024 3.5 / 5.4
   // against 8.4 / 10.1 us, 2048 x 4096 8.6 / 17.3 against 13.9 / 17.5, 4096 x 4096 11.8 / 19.6 against 16.1 / 17.8).  At the upper
   // end of the line umma_w4.cu is the faster one (8192 x 4096: 24.3 / 41.3 against 15.8 / 17.9 us), but it rounds
@@ -306,8 +313,8 @@ int b2q_linear_int4_allreduce(const void* x, int act_dtype, int64_t ldx, const v
 }
 
 size_t b2q_linear_workspace_bytes(int64_t M, int64_t N, int64_t K) {
-  const size_t a = ws_prep_bytes(M, K) + umma_w4_partial_bytes(M, N, K), b = ws_i8_bytes(M, K);
-  return a > b ? a : b;
+  const size_t a = ws_prep_bytes(M, K) + umma_w4_partial_bytes(M, N, K), b = ws_i8_bytes(M, K), c = w4_stream_partial_bytes(M, N, K);
+  return a > b ? (a > c ? a : c) : (b > c ? b : c);
 }
 size_t b2q_linear_fp8_workspace_bytes(int64_t M, int64_t N, int64_t K) {
   const size_t a = ws_prep_bytes(M, K) + umma_w8_strip_partial_bytes(M, N, K), b = ws_direct_bytes(M, K);

@@ -629,6 +629,7 @@ int umma_selftest_bounded_wait(int code, int* gave_up_dev, cudaStream_t st) {
 int w8a8_reset_state();
 int w8d_reset_state();
 int w4i_reset_state();
+int w4s_reset_state();
 
 // Clears, on the current device, the status word of every tcgen05 kernel family and the arrival counters of cut
 // strips.  A CTA that gave up on a wait never delivered its arrival, so its strip's counter is left non-zero and the
@@ -645,6 +646,7 @@ int umma_reset_status() {
   int rc = w8a8_reset_state();
   if (!rc) rc = w8d_reset_state();
   if (!rc) rc = w4i_reset_state();
+  if (!rc) rc = w4s_reset_state();
   return rc;
 }
 

@@ -1,0 +1,31 @@
+// Host-side interface of the INT4 decode streaming kernel (w4_stream.cu).
+#pragma once
+#include "common.cuh"
+
+namespace b2q {
+
+constexpr int W4_STREAM_MAX_TOK = 8;      // tokens per tile
+
+struct W4StreamArgs {
+  const void* x; int64_t ldx; bool bf16;
+  const void* w; int layout;                                     // N-major nibbles, offset or two's complement
+  const void* scale; int scale_dtype; int64_t s_stride_n, s_stride_g;
+  void* out; int64_t ldo;
+  int M, N, K;
+  int tile;                                                      // tokens per tile: M, or the height the tile list was built with
+  bool gated = false;                                            // rows are gate then up; out = silu(gate) * up, N / 2 wide
+  const int32_t* tiles = nullptr; int tile_cap = 0; int E = 1;   // grouped
+  const int32_t* expert_offsets = nullptr; const int32_t* row_map = nullptr; int row_div = 1; const int32_t* out_map = nullptr;
+  void* partials = nullptr; size_t partial_bytes = 0;            // dense: w4_stream_partial_bytes(M, N, K), or strips stay whole
+};
+
+bool w4_stream_supported(const W4StreamArgs& a);
+int w4_stream_linear(const W4StreamArgs& a, cudaStream_t st);
+size_t w4_stream_partial_bytes(int64_t M, int64_t N, int64_t K);
+
+// Dense launches that are better off here than in smallm.cuh, whose 16-row strips need no sum between CTAs and cost less to start:
+// 4096 x 4096, one token, 8.3 us there and 13.4 here, 5120 x 5120 10.7 and 16, but 28672 x 1024 12.8 and 11.9, 8192 x 4096 14.4 and
+// 11.4, 10240 x 8192 27.2 and 17.9 (eight tokens 30.5 and 18.6).
+inline bool w4_stream_preferred(int64_t M, int64_t N, int64_t K) { return M <= W4_STREAM_MAX_TOK && N * K >= (int64_t)7 << 22; }
+
+}  // namespace b2q

@@ -1,0 +1,101 @@
+"""The INT4 decode streaming kernel (csrc/w4_stream.cu) at the edges of its range: ragged strips, odd numbers of scale groups, stages beyond
+K, cut and whole strips, scale types and strides, both nibble encodings, infinities and NaN."""
+import pytest
+import torch
+
+from gpu_util import DEV
+
+pytestmark = pytest.mark.gpu
+TOL = {torch.bfloat16: 2.0 ** -8, torch.float16: 2.0 ** -11}      # one rounding of the result, over its largest value; fp32 sums add 1e-6
+
+
+@pytest.fixture()
+def e():
+    import custom_esimd_kernels_vllm as pkg
+    pkg.set_force_kernel(7)
+    yield pkg
+    pkg.set_force_kernel(0)
+    pkg.set_overlap_mode(1)
+
+
+def _inputs(M, N, K, dtype, sdtype, seed=0):
+    g = torch.Generator().manual_seed(seed)
+    q = torch.randint(0, 16, (N, K), generator=g, dtype=torch.uint8)
+    w = sum(q[:, j::8].to(torch.int64) << (4 * j) for j in range(8))
+    w = torch.where(w >= 2 ** 31, w - 2 ** 32, w).to(torch.int32)
+    s = ((0.5 + torch.rand(N, K // 128, generator=g)) / (4.6 * K ** 0.5)).to(sdtype)
+    x = torch.randn(M, K, generator=g).to(dtype)
+    return x, q, w, s
+
+
+def _exact(x, q, s):
+    return x.double() @ ((q.double() - 8) * s.double().repeat_interleave(128, 1)).t()
+
+
+def _close(out, ref, dtype):
+    err = (out.cpu().double() - ref).abs().max() / ref.abs().max()
+    assert err <= TOL[dtype] + 2e-6, float(err)
+
+
+@pytest.mark.parametrize("M", [1, 3, 8])
+@pytest.mark.parametrize("N,K", [(1, 128), (100, 256), (127, 384), (129, 1024), (4104, 1152), (300, 4096), (40000, 256)])
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16])
+def test_shapes(e, M, N, K, dtype):
+    """N below, at and above a strip of 128; K of one group, of odd groups (half a stage beyond K), of several scale slots; cut and whole."""
+    x, q, w, s = _inputs(M, N, K, dtype, dtype)
+    out = torch.empty(M, N, dtype=dtype, device=DEV)
+    e.esimd_gemm_int4_pgrp(x.to(DEV), w.to(DEV), s.to(DEV), out)
+    assert e.last_kernel() == "w4_stream"
+    _close(out, _exact(x, q, s), dtype)
+    assert e._lib.device_status() == 0
+
+
+@pytest.mark.parametrize("sdtype", [torch.bfloat16, torch.float16, torch.float32])
+@pytest.mark.parametrize("transposed", [False, True])
+@pytest.mark.parametrize("K", [128 * 3, 128 * 6, 128 * 16])       # element, 4-byte and 16-byte fetches of the scales
+def test_scales(e, sdtype, transposed, K):
+    x, q, w, s = _inputs(5, 260, K, torch.float16, sdtype)
+    sd = s.t().contiguous().to(DEV).t() if transposed else s.to(DEV)
+    out = torch.empty(5, 260, dtype=torch.float16, device=DEV)
+    e.esimd_gemm_int4_pgrp(x.to(DEV), w.to(DEV), sd, out)
+    assert e.last_kernel() == "w4_stream"
+    _close(out, _exact(x, q, s), torch.float16)
+
+
+@pytest.mark.parametrize("M,N,K", [(8, 2048, 2048), (1, 57344, 512)])
+def test_overlap_and_repeats_give_the_same_bits(e, M, N, K):
+    """Cut strips are summed in CTA order whoever comes last; no mode of overlap changes a bit."""
+    x, q, w, s = _inputs(M, N, K, torch.bfloat16, torch.bfloat16)
+    xd, wd, sd = x.to(DEV), w.to(DEV), s.to(DEV)
+    outs = []
+    for mode in (0, 1, 2):
+        e.set_overlap_mode(mode)
+        for _ in range(20):
+            out = torch.empty(M, N, dtype=torch.bfloat16, device=DEV)
+            e.esimd_gemm_int4_pgrp(xd, wd, sd, out)
+            outs.append(out)
+    torch.cuda.synchronize()
+    assert all(torch.equal(outs[0], o) for o in outs[1:])
+    _close(outs[0], _exact(x, q, s), torch.bfloat16)
+
+
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16])
+def test_infinities_and_nan_come_out_as_their_products(e, dtype):
+    x, q, w, s = _inputs(4, 256, 512, dtype, dtype)
+    x[0, 5], x[1, 300], x[2, 511] = float("inf"), float("nan"), float("-inf")
+    out = torch.empty(4, 256, dtype=dtype, device=DEV)
+    e.esimd_gemm_int4_pgrp(x.to(DEV), w.to(DEV), s.to(DEV), out)
+    o = out.cpu().double()
+    ref = _exact(x, q, s)
+    assert torch.equal(o.isnan(), ref.isnan())
+    assert torch.equal(torch.sign(o[:3].nan_to_num(0)), torch.sign(ref[:3].nan_to_num(0)))
+    _close(out[3:], ref[3:], dtype)
+
+
+def test_dispatch_takes_it_for_wide_layers_only(e):
+    e.set_force_kernel(0)
+    for M, N, K, name in ((8, 8192, 4096, "w4_stream"), (8, 4096, 4096, "smallm"), (9, 8192, 8192, "umma_w4")):
+        x, q, w, s = _inputs(M, N, K, torch.bfloat16, torch.bfloat16)
+        out = torch.empty(M, N, dtype=torch.bfloat16, device=DEV)
+        e.esimd_gemm_int4_pgrp(x.to(DEV), w.to(DEV), s.to(DEV), out)
+        assert e.last_kernel() == name
