@@ -7,6 +7,32 @@
 
 namespace b2q {
 
+// The small kernels of this file begin while the kernel before them on the stream drains and let the next one do the same:
+// launch latency is most of what they cost.  Each waits before it touches memory, and reads past L1 what a kernel before it wrote
+// (a line may have been fetched by the overlapping predecessor of that kernel).
+template <typename... KArgs, typename... Args>
+static inline void launch_small(void (*kern)(KArgs...), dim3 grid, dim3 block, size_t smem, cudaStream_t st, Args&&... args) {
+  launch_overlapped(kern, grid, block, smem, st, tls().overlap_mode > 0, args...);      // launch_status() reports
+}
+__device__ __forceinline__ void dep_enter() { grid_dep_release(); grid_dep_wait(); }
+// The same word read by many threads of a CTA: through L1, which the wait has made safe for an ordinary load, but never by the
+// read-only path, which a const __restrict__ pointer invites.
+__device__ __forceinline__ int32_t ld_shared_word(const int32_t* p) {
+  int32_t v;
+  asm volatile("ld.global.s32 %0, [%1];" : "=r"(v) : "l"(p) : "memory");
+  return v;
+}
+__device__ __forceinline__ float ld_shared_scalar(const void* p, int64_t i, int dt) {
+  if (dt == B2Q_F32) return __int_as_float(ld_shared_word(reinterpret_cast<const int32_t*>(p) + i));
+  unsigned short h;
+  asm volatile("ld.global.u16 %0, [%1];" : "=h"(h) : "l"(reinterpret_cast<const unsigned short*>(p) + i) : "memory");
+  return scalar_from_raw(h, dt);
+}
+__device__ __forceinline__ float load_scalar_cg(const void* p, int64_t i, int dt) {
+  if (dt == B2Q_F32) return __ldcg(reinterpret_cast<const float*>(p) + i);
+  return scalar_from_raw(__ldcg(reinterpret_cast<const unsigned short*>(p) + i), dt);
+}
+
 // ---------------------------------------------------------------------------
 // softmax -> top-k -> renormalise.  One warp per token; lane l owns experts
 // l, l+32, ... so loads are coalesced.  Selection order and tie rule follow
@@ -19,13 +45,14 @@ __global__ void moe_topk_kernel(const void* __restrict__ logits, int ldt, int64_
   const int warps_per_block = blockDim.x >> 5;
   const int64_t tok = (int64_t)blockIdx.x * warps_per_block + (threadIdx.x >> 5);
   const int lane = threadIdx.x & 31;
+  dep_enter();
   if (tok >= T) return;
   float v[PER_LANE];
   float mx = -INFINITY;
 #pragma unroll
   for (int j = 0; j < PER_LANE; ++j) {
     const int e = lane + 32 * j;
-    v[j] = e < E ? load_scalar(logits, tok * E + e, ldt) : -INFINITY;
+    v[j] = e < E ? load_scalar_cg(logits, tok * E + e, ldt) : -INFINITY;
     mx = fmaxf(mx, v[j]);
   }
 #pragma unroll
@@ -82,7 +109,7 @@ int moe_topk(const void* logits, int ldt, int64_t T, int E, int top_k, int renor
   const int wpb = 8;
   const int grid = (int)((T + wpb - 1) / wpb);
   if (grid == 0) return B2Q_OK;
-#define B2Q_TOPK(P) moe_topk_kernel<P><<<grid, wpb * 32, 0, st>>>(logits, ldt, T, E, top_k, renorm, weights, wdt, ids)
+#define B2Q_TOPK(P) launch_small(moe_topk_kernel<P>, dim3(grid), dim3(wpb * 32), 0, st, logits, ldt, T, E, top_k, renorm, weights, wdt, ids)
   if (E <= 64) B2Q_TOPK(2);
   else if (E <= 128) B2Q_TOPK(4);
   else if (E <= 256) B2Q_TOPK(8);
@@ -103,11 +130,12 @@ constexpr int ROUTE_CHUNK = 256;  // pairs per CTA (8 warps)
 
 __global__ void route_hist_kernel(const int32_t* __restrict__ ids, int64_t n_pairs, int E, int32_t* __restrict__ counts) {
   extern __shared__ int32_t sh[];
+  dep_enter();
   for (int i = threadIdx.x; i < E; i += blockDim.x) sh[i] = 0;
   __syncthreads();
   const int64_t i = (int64_t)blockIdx.x * ROUTE_CHUNK + threadIdx.x;
   if (i < n_pairs) {
-    const int e = ids[i];
+    const int e = __ldcg(ids + i);
     if (e >= 0 && e < E) atomicAdd(&sh[e], 1);
   }
   __syncthreads();
@@ -122,6 +150,7 @@ __global__ void route_prefix_kernel(int32_t* __restrict__ counts, int nchunks, i
   __shared__ int32_t part[1024];     // [segment][expert]
   __shared__ int32_t tot[1024];
   __shared__ int32_t scan[1024];
+  dep_enter();
   const int tid = threadIdx.x;
   const int segs = 1024 / E > 0 ? 1024 / E : 1;
   const int e = tid % E, seg = tid / E;
@@ -131,7 +160,7 @@ __global__ void route_prefix_kernel(int32_t* __restrict__ counts, int nchunks, i
   int sum = 0;
   if (active) {
 #pragma unroll 4
-    for (int b = b0; b < b1; ++b) sum += counts[(int64_t)b * E + e];
+    for (int b = b0; b < b1; ++b) sum += __ldcg(counts + (int64_t)b * E + e);
     part[seg * E + e] = sum;
   }
   __syncthreads();
@@ -173,11 +202,12 @@ __global__ void route_scatter_kernel(const int32_t* __restrict__ ids, int64_t n_
                                      int32_t* __restrict__ expert_tokens, int32_t* __restrict__ pair_to_perm) {
   extern __shared__ int32_t wc[];  // [8][E] per-warp counts
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  dep_enter();
   for (int i = threadIdx.x; i < 8 * E; i += blockDim.x) wc[i] = 0;
   __syncthreads();
   const int64_t i = (int64_t)blockIdx.x * ROUTE_CHUNK + threadIdx.x;
   int e = -1;
-  if (i < n_pairs) { e = ids[i]; if (e < 0 || e >= E) e = -1; }
+  if (i < n_pairs) { e = __ldcg(ids + i); if (e < 0 || e >= E) e = -1; }
   const unsigned peers = __match_any_sync(0xffffffffu, e);
   const int rank = __popc(peers & ((1u << lane) - 1u));
   if (e >= 0 && rank == 0) wc[warp * E + e] = __popc(peers);
@@ -186,7 +216,7 @@ __global__ void route_scatter_kernel(const int32_t* __restrict__ ids, int64_t n_
     if (e >= 0) {
       int before = 0;
       for (int w2 = 0; w2 < warp; ++w2) before += wc[w2 * E + e];
-      const int pos = expert_offsets[e] + base[(int64_t)blockIdx.x * E + e] + before + rank;
+      const int pos = __ldcg(expert_offsets + e) + __ldcg(base + (int64_t)blockIdx.x * E + e) + before + rank;
       expert_tokens[pos] = (int32_t)i;
       if (pair_to_perm) pair_to_perm[i] = pos;
     } else if (pair_to_perm) {
@@ -205,14 +235,14 @@ int moe_route(const int32_t* ids, int64_t n_pairs, int E, int32_t* expert_offset
   const int nchunks = (int)((n_pairs + ROUTE_CHUNK - 1) / ROUTE_CHUNK);
   int32_t* counts = reinterpret_cast<int32_t*>(workspace);
   if (nchunks > 0) {
-    route_hist_kernel<<<nchunks, ROUTE_CHUNK, E * sizeof(int32_t), st>>>(ids, n_pairs, E, counts);
+    launch_small(route_hist_kernel, dim3(nchunks), dim3(ROUTE_CHUNK), E * sizeof(int32_t), st, ids, n_pairs, E, counts);
     note_launch("route_hist");
   }
-  route_prefix_kernel<<<1, 1024, 0, st>>>(counts, nchunks, E, expert_offsets, rows_per_expert);
+  launch_small(route_prefix_kernel, dim3(1), dim3(1024), 0, st, counts, nchunks, E, expert_offsets, rows_per_expert);
   note_launch("route_prefix");
   if (nchunks > 0) {
-    route_scatter_kernel<<<nchunks, ROUTE_CHUNK, 8 * E * sizeof(int32_t), st>>>(ids, n_pairs, E, counts, expert_offsets,
-                                                                                 expert_tokens, pair_to_perm);
+    launch_small(route_scatter_kernel, dim3(nchunks), dim3(ROUTE_CHUNK), 8 * E * sizeof(int32_t), st, ids, n_pairs, E, counts, expert_offsets,
+                 expert_tokens, pair_to_perm);
     note_launch("route_scatter");
   }
   return launch_status();
@@ -225,8 +255,12 @@ int moe_route(const int32_t* ids, int64_t n_pairs, int E, int32_t* expert_offset
 // ---------------------------------------------------------------------------
 __global__ void moe_tiles_kernel(const int32_t* __restrict__ expert_offsets, int E, int tile, int32_t* __restrict__ ws) {
   __shared__ int32_t scan[1024];
+  // the GEMM that reads the list has large CTAs: in only when the pre-pass in front of this kernel no longer needs the SMs
+  // (INT4 pipeline at 4096 tokens: 569 us, 576 with the GEMM let in at once)
+  grid_dep_wait();
+  grid_dep_release();
   const int e = threadIdx.x;
-  const int rows = e < E ? expert_offsets[e + 1] - expert_offsets[e] : 0;
+  const int rows = e < E ? __ldcg(expert_offsets + e + 1) - __ldcg(expert_offsets + e) : 0;
   const int nt = (rows + tile - 1) / tile;
   int val = nt;
   scan[e] = val;
@@ -245,7 +279,7 @@ __global__ void moe_tiles_kernel(const int32_t* __restrict__ expert_offsets, int
 }
 
 int moe_build_tiles(const int32_t* expert_offsets, int E, int tile, int32_t* ws, cudaStream_t st) {
-  moe_tiles_kernel<<<1, 1024, 0, st>>>(expert_offsets, E, tile, ws);
+  launch_small(moe_tiles_kernel, dim3(1), dim3(1024), 0, st, expert_offsets, E, tile, ws);
   note_launch("moe_tiles");
   return launch_status();
 }
@@ -253,9 +287,10 @@ int moe_build_tiles(const int32_t* expert_offsets, int E, int tile, int32_t* ws,
 // ---------------------------------------------------------------------------
 __global__ void gather_rows_kernel(const uint4* __restrict__ src, const int32_t* __restrict__ idx, int div,
                                    uint4* __restrict__ dst, int64_t rows, int64_t vec_per_row) {
+  dep_enter();
   for (int64_t r = blockIdx.x; r < rows; r += gridDim.x) {
-    const int64_t s = idx ? (int64_t)(idx[r] / div) : r;
-    for (int64_t c = threadIdx.x; c < vec_per_row; c += blockDim.x) dst[r * vec_per_row + c] = src[s * vec_per_row + c];
+    const int64_t s = idx ? (int64_t)(__ldcg(idx + r) / div) : r;
+    for (int64_t c = threadIdx.x; c < vec_per_row; c += blockDim.x) dst[r * vec_per_row + c] = __ldcg(src + s * vec_per_row + c);
   }
 }
 
@@ -264,8 +299,7 @@ int gather_rows(const void* src, const int32_t* idx, int div, void* dst, int64_t
   if (rows == 0) return B2Q_OK;
   const int64_t vec = cols * elem_bytes / 16;
   const int grid = (int)(rows < 148 * 32 ? rows : 148 * 32);
-  gather_rows_kernel<<<grid, 128, 0, st>>>(reinterpret_cast<const uint4*>(src), idx, div, reinterpret_cast<uint4*>(dst),
-                                           rows, vec);
+  launch_small(gather_rows_kernel, dim3(grid), dim3(128), 0, st, reinterpret_cast<const uint4*>(src), idx, div, reinterpret_cast<uint4*>(dst), rows, vec);
   note_launch("gather_rows");
   return launch_status();
 }
@@ -278,12 +312,13 @@ __global__ void silu_mul_kernel(const uint4* __restrict__ in, uint4* __restrict_
                                 const int32_t* __restrict__ out_map, int64_t ld8) {
   using A = Act<BF16>;
   using T = typename A::T;
+  dep_enter();
   const int64_t total = rows * I8;
   for (int64_t idx = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; idx < total;
        idx += (int64_t)gridDim.x * blockDim.x) {
     const int64_t r = idx / I8, c = idx % I8;
-    const uint4 g = in[r * ld8 + c];
-    const uint4 u = in[r * ld8 + I8 + c];
+    const uint4 g = __ldcg(in + r * ld8 + c);
+    const uint4 u = __ldcg(in + r * ld8 + I8 + c);
     const T* gp = reinterpret_cast<const T*>(&g);
     const T* up = reinterpret_cast<const T*>(&u);
     uint4 o;
@@ -296,7 +331,7 @@ __global__ void silu_mul_kernel(const uint4* __restrict__ in, uint4* __restrict_
       else s = gv / (1.0f + expf(-gv));
       op[j] = A::from_f(s * A::to_f(up[j]));
     }
-    out[(out_map ? (int64_t)out_map[r] : r) * I8 + c] = o;
+    out[(out_map ? (int64_t)__ldcg(out_map + r) : r) * I8 + c] = o;
   }
 }
 
@@ -310,11 +345,11 @@ int silu_mul(const void* in, void* out, int dtype, int64_t rows, int64_t I, cons
   auto ci = reinterpret_cast<const uint4*>(in);
   auto co = reinterpret_cast<uint4*>(out);
   if (dtype == B2Q_BF16) {
-    if (gelu) silu_mul_kernel<true, true><<<(int)g, 256, 0, st>>>(ci, co, rows, I / 8, out_map, ld8);
-    else silu_mul_kernel<true, false><<<(int)g, 256, 0, st>>>(ci, co, rows, I / 8, out_map, ld8);
+    if (gelu) launch_small(silu_mul_kernel<true, true>, dim3((unsigned)g), dim3(256), 0, st, ci, co, rows, I / 8, out_map, ld8);
+    else launch_small(silu_mul_kernel<true, false>, dim3((unsigned)g), dim3(256), 0, st, ci, co, rows, I / 8, out_map, ld8);
   } else {
-    if (gelu) silu_mul_kernel<false, true><<<(int)g, 256, 0, st>>>(ci, co, rows, I / 8, out_map, ld8);
-    else silu_mul_kernel<false, false><<<(int)g, 256, 0, st>>>(ci, co, rows, I / 8, out_map, ld8);
+    if (gelu) launch_small(silu_mul_kernel<false, true>, dim3((unsigned)g), dim3(256), 0, st, ci, co, rows, I / 8, out_map, ld8);
+    else launch_small(silu_mul_kernel<false, false>, dim3((unsigned)g), dim3(256), 0, st, ci, co, rows, I / 8, out_map, ld8);
   }
   note_launch(gelu ? "gelu_tanh_mul" : "silu_mul");
   return launch_status();
@@ -330,10 +365,11 @@ __global__ void shared_gate_add_kernel(const uint4* __restrict__ x, const uint4*
   using T = typename A::T;
   __shared__ float red[32];
   __shared__ float gate_sh;
+  dep_enter();
   const int64_t t = blockIdx.x;
   float dot = 0.f;
   for (int c = threadIdx.x; c < H8; c += blockDim.x) {
-    const uint4 xv = x[t * H8 + c], gv = gate_w[c];
+    const uint4 xv = __ldcg(x + t * H8 + c), gv = __ldcg(gate_w + c);
     const T* xp = reinterpret_cast<const T*>(&xv);
     const T* gp = reinterpret_cast<const T*>(&gv);
 #pragma unroll
@@ -351,7 +387,7 @@ __global__ void shared_gate_add_kernel(const uint4* __restrict__ x, const uint4*
   __syncthreads();
   const float gate = gate_sh;
   for (int c = threadIdx.x; c < H8; c += blockDim.x) {
-    const uint4 sv = shared[t * H8 + c], rv = routed[t * H8 + c];
+    const uint4 sv = __ldcg(shared + t * H8 + c), rv = __ldcg(routed + t * H8 + c);
     const T* sp = reinterpret_cast<const T*>(&sv);
     const T* rp = reinterpret_cast<const T*>(&rv);
     uint4 o;
@@ -367,9 +403,9 @@ int shared_gate_add(const void* x, const void* gate_w, const void* shared, const
   if (T == 0) return B2Q_OK;
   auto u = [](const void* p) { return reinterpret_cast<const uint4*>(p); };
   if (dtype == B2Q_BF16)
-    shared_gate_add_kernel<true><<<(unsigned)T, 256, 0, st>>>(u(x), u(gate_w), u(shared), u(routed), reinterpret_cast<uint4*>(out), (int)(H / 8));
+    launch_small(shared_gate_add_kernel<true>, dim3((unsigned)T), dim3(256), 0, st, u(x), u(gate_w), u(shared), u(routed), reinterpret_cast<uint4*>(out), (int)(H / 8));
   else
-    shared_gate_add_kernel<false><<<(unsigned)T, 256, 0, st>>>(u(x), u(gate_w), u(shared), u(routed), reinterpret_cast<uint4*>(out), (int)(H / 8));
+    launch_small(shared_gate_add_kernel<false>, dim3((unsigned)T), dim3(256), 0, st, u(x), u(gate_w), u(shared), u(routed), reinterpret_cast<uint4*>(out), (int)(H / 8));
   note_launch("shared_gate_add");
   return launch_status();
 }
@@ -382,6 +418,7 @@ __global__ void moe_combine_kernel(const uint4* __restrict__ y, const void* __re
                                    int64_t H8, int w_by_row) {
   using A = Act<BF16>;
   using Ty = typename A::T;
+  dep_enter();
   const int64_t total = T * H8;
   for (int64_t idx = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; idx < total;
        idx += (int64_t)gridDim.x * blockDim.x) {
@@ -389,10 +426,10 @@ __global__ void moe_combine_kernel(const uint4* __restrict__ y, const void* __re
     float acc[8] = {0, 0, 0, 0, 0, 0, 0, 0};
     for (int s = 0; s < top_k; ++s) {
       const int64_t pair = t * top_k + s;
-      const int64_t row = perm ? (int64_t)perm[pair] : pair;
+      const int64_t row = perm ? (int64_t)ld_shared_word(perm + pair) : pair;
       if (row < 0) continue;
-      const float wt = w ? load_scalar(w, w_by_row ? row : pair, wdt) : 1.0f;
-      const uint4 v = y[row * H8 + c];
+      const float wt = w ? ld_shared_scalar(w, w_by_row ? row : pair, wdt) : 1.0f;
+      const uint4 v = __ldcg(y + row * H8 + c);
       const Ty* vp = reinterpret_cast<const Ty*>(&v);
 #pragma unroll
       for (int j = 0; j < 8; ++j) acc[j] += wt * A::to_f(vp[j]);
@@ -412,11 +449,11 @@ int moe_combine(const void* y, const void* w, int wdt, const int32_t* perm, void
   int64_t g = (total + 255) / 256;
   if (g > 148 * 16) g = 148 * 16;
   if (dtype == B2Q_BF16)
-    moe_combine_kernel<true><<<(int)g, 256, 0, st>>>(reinterpret_cast<const uint4*>(y), w, wdt, perm,
-                                                     reinterpret_cast<uint4*>(out), T, top_k, H / 8, w_by_row);
+    launch_small(moe_combine_kernel<true>, dim3((unsigned)g), dim3(256), 0, st, reinterpret_cast<const uint4*>(y), w, wdt, perm,
+                 reinterpret_cast<uint4*>(out), T, top_k, H / 8, w_by_row);
   else
-    moe_combine_kernel<false><<<(int)g, 256, 0, st>>>(reinterpret_cast<const uint4*>(y), w, wdt, perm,
-                                                      reinterpret_cast<uint4*>(out), T, top_k, H / 8, w_by_row);
+    launch_small(moe_combine_kernel<false>, dim3((unsigned)g), dim3(256), 0, st, reinterpret_cast<const uint4*>(y), w, wdt, perm,
+                 reinterpret_cast<uint4*>(out), T, top_k, H / 8, w_by_row);
   note_launch("moe_combine");
   return launch_status();
 }
@@ -430,12 +467,13 @@ __global__ void act_quant_1x128_kernel(const void* __restrict__ x, int64_t ldx, 
                                        float* __restrict__ xs, int64_t M, int64_t K) {
   using A = Act<BF16>;
   using T = typename A::T;
+  dep_enter();
   const int64_t kb_n = K >> 7;
   const int64_t wid = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
   const int lane = threadIdx.x & 31;
   if (wid >= M * kb_n) return;
   const int64_t m = wid / kb_n, kb = wid % kb_n;
-  const uint2 raw = *reinterpret_cast<const uint2*>(reinterpret_cast<const T*>(x) + m * ldx + kb * 128 + lane * 4);
+  const uint2 raw = __ldcg(reinterpret_cast<const uint2*>(reinterpret_cast<const T*>(x) + m * ldx + kb * 128 + lane * 4));
   const T* rp = reinterpret_cast<const T*>(&raw);
   float v[4];
   float amax = 0.f;
@@ -459,74 +497,10 @@ int act_quant_1x128(const void* x, int dtype, int64_t ldx, void* xq, float* xs, 
   if (warps == 0) return B2Q_OK;
   const int grid = (int)((warps + 7) / 8);
   if (dtype == B2Q_BF16)
-    act_quant_1x128_kernel<true><<<grid, 256, 0, st>>>(x, ldx, reinterpret_cast<uint8_t*>(xq), xs, M, K);
+    launch_small(act_quant_1x128_kernel<true>, dim3(grid), dim3(256), 0, st, x, ldx, reinterpret_cast<uint8_t*>(xq), xs, M, K);
   else
-    act_quant_1x128_kernel<false><<<grid, 256, 0, st>>>(x, ldx, reinterpret_cast<uint8_t*>(xq), xs, M, K);
+    launch_small(act_quant_1x128_kernel<false>, dim3(grid), dim3(256), 0, st, x, ldx, reinterpret_cast<uint8_t*>(xq), xs, M, K);
   note_launch("act_quant_1x128");
-  return launch_status();
-}
-
-}  // namespace b2q
-
-namespace b2q {
-
-// ---------------------------------------------------------------------------
-// Activation pre-pass for fp8-weight GEMMs with bf16 activations: rewrites every token row as
-// fp16 times a per-token power of two, x16[m, k] = fp16(x[m, k] * 2^e_m) with 2^e_m chosen so
-// that the row maximum lands in [2^14, 2^15).  A bf16 value has 8 significant bits, fp16 holds 11
-// and reaches down to 2^-24, so every element within 2^-31 of its row maximum converts exactly;
-// smaller ones keep an absolute error below rowmax * 2^-40.  inv_scale[m] = 2^-e_m (exact).
-// The point: e4m3 / e5m2 weights convert to fp16 with one instruction per pair, to bf16 with four.
-__global__ void act_to_scaled_f16_kernel(const __nv_bfloat16* __restrict__ x, int64_t ldx, __half* __restrict__ x16,
-                                         float* __restrict__ inv_scale, int K) {
-  __shared__ float red[32];
-  __shared__ float sc_sh;
-  const int64_t m = blockIdx.x;
-  const __nv_bfloat16* row = x + m * ldx;
-  float amax = 0.f;
-  for (int k = threadIdx.x * 8; k < K; k += blockDim.x * 8) {
-    const uint4 v = *reinterpret_cast<const uint4*>(row + k);
-    const __nv_bfloat16* e = reinterpret_cast<const __nv_bfloat16*>(&v);
-#pragma unroll
-    for (int j = 0; j < 8; ++j) amax = fmaxf(amax, fabsf(__bfloat162float(e[j])));
-  }
-#pragma unroll
-  for (int o = 16; o > 0; o >>= 1) amax = fmaxf(amax, __shfl_xor_sync(0xffffffffu, amax, o));
-  if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = amax;
-  __syncthreads();
-  if (threadIdx.x == 0) {
-    float a = 0.f;
-    for (int i = 0; i < (int)(blockDim.x >> 5); ++i) a = fmaxf(a, red[i]);
-    float sc = 1.f;
-    if (a > 0.f && a < INFINITY) {
-      const int ex = (int)((__float_as_uint(a) >> 23) & 0xFF) - 127;      // floor(log2 a) for normal a
-      int sh = 14 - ex;
-      sh = sh > 126 ? 126 : (sh < -126 ? -126 : sh);
-      sc = __uint_as_float((uint32_t)(sh + 127) << 23);
-    }
-    sc_sh = sc;
-    inv_scale[m] = 1.0f / sc;
-  }
-  __syncthreads();
-  const float sc = sc_sh;
-  for (int k = threadIdx.x * 8; k < K; k += blockDim.x * 8) {
-    const uint4 v = *reinterpret_cast<const uint4*>(row + k);
-    const __nv_bfloat16* e = reinterpret_cast<const __nv_bfloat16*>(&v);
-    uint4 o;
-    __half* oh = reinterpret_cast<__half*>(&o);
-#pragma unroll
-    for (int j = 0; j < 8; ++j) oh[j] = __float2half_rn(__bfloat162float(e[j]) * sc);
-    *reinterpret_cast<uint4*>(x16 + m * (int64_t)K + k) = o;
-  }
-}
-
-int act_to_scaled_f16(const void* x, int64_t ldx, void* x16, float* inv_scale, int64_t M, int K, cudaStream_t st) {
-  if (M == 0) return B2Q_OK;
-  int threads = (K / 8 + 31) / 32 * 32;
-  threads = threads > 512 ? 512 : (threads < 32 ? 32 : threads);
-  act_to_scaled_f16_kernel<<<(unsigned)M, threads, 0, st>>>(reinterpret_cast<const __nv_bfloat16*>(x), ldx,
-                                                            reinterpret_cast<__half*>(x16), inv_scale, K);
-  note_launch("act_to_scaled_f16");
   return launch_status();
 }
 
@@ -609,7 +583,8 @@ __device__ __forceinline__ float block_max(float v, float* red) {
 
 // ---------------------------------------------------------------------------
 // General activation pre-pass in front of the tcgen05 GEMM: optional row gather, per-token
-// power-of-two scaling into fp16 (see act_to_scaled_f16_kernel for why that is exact in practice)
+// power-of-two scaling into fp16 (a bf16 value has 8 significant bits, fp16 holds 11 and reaches down to 2^-24: every element within
+// 2^-31 of its row's largest converts exactly, smaller ones keep an absolute error below 2^-40 of that)
 // and an optional permutation inside every group of eight k so that the INT4 transform can emit
 // its nibble pairs in the order the bit tricks produce them instead of re-sorting them:
 //   perm 0: identity      perm 1: (0,4,1,5,2,6,3,7)  nibble i at bits 4i (GGML / N-major, plain K-major)
