@@ -416,6 +416,33 @@ B2Q_API int b2q_ep_dispatch(void* comm, const void* x, int dtype, int64_t ldx, c
 B2Q_API int b2q_ep_return(void* comm, const void* y, int dtype, int64_t ldy, void* stream);
 B2Q_API int b2q_ep_wait(void* comm, int phase, double wait_limit_ms, void* stream);
 
+/* Whole expert layers, from router logits to combined output: top-k with renormalised softmax weights, sort by expert, grouped
+ * GEMMs with the activation between them, weighted sum; for INT4 optionally plus sigmoid(x . gate_w) times an INT4 shared
+ * expert.  The pipelines of moe_prefill_full_int4 / moe_forward_full_int4 (csrc/moe_prefill/moe_prefill_int4.sycl:920-988,
+ * csrc/moe_batch/moe_int4.sycl:2933-3166) and moe_forward_full_gelu_tanh (csrc/moe_batch/moe.sycl:2249-2340).
+ * x [T, H], logits [T, E], out [T, H]; expert weights as for b2q_moe_gemm_int4 / _fp8 with N = 2 I (gate, then up), K = H and
+ * N = H, K = I.  fp8 scales: one fp32 per expert; activation GELU-tanh (INT4: SiLU).  workspace: 256-byte aligned,
+ * b2q_moe_forward_workspace_bytes(T, E, top_k, H, I, shared_I) bytes (shared_I = 0 without a shared expert). */
+typedef struct b2q_moe_int4 {
+  const void *x, *logits;
+  const void *w13, *s13, *w2, *s2;
+  const void *shared_w13, *shared_s13, *shared_w2, *shared_s2, *gate_w;      /* N-major nibbles; all NULL: no shared expert */
+  void* out;
+  int64_t T, E, top_k, H, I, shared_I;
+  int act_dtype, logits_dtype, layout, s13_dtype, s2_dtype;
+  int shared_layout, shared_s13_dtype, shared_s2_dtype, shared_scale_kmajor; /* scales [K/128, N] instead of [N, K/128] */
+} b2q_moe_int4;
+typedef struct b2q_moe_fp8 {
+  const void *x, *logits;
+  const void* w13; const float* s13; const void* w2; const float* s2;
+  void* out;
+  int64_t T, E, top_k, H, I;
+  int act_dtype, logits_dtype, fp8_format;
+} b2q_moe_fp8;
+B2Q_API size_t b2q_moe_forward_workspace_bytes(int64_t T, int E, int top_k, int64_t H, int64_t I, int64_t shared_I);
+B2Q_API int b2q_moe_forward_int4(const b2q_moe_int4* args, void* workspace, size_t workspace_bytes, void* stream);
+B2Q_API int b2q_moe_forward_fp8(const b2q_moe_fp8* args, void* workspace, size_t workspace_bytes, void* stream);
+
 /* Code of the first bounded device-side wait that expired since the library was loaded
  * (0 = none).  Synchronises the device; meant for tests and post-mortems.       */
 B2Q_API int b2q_device_status(int* out);

@@ -20,6 +20,8 @@ int moe_topk(const void*, int, int64_t, int, int, int, void*, int, int32_t*, cud
 size_t moe_route_workspace_bytes(int64_t, int);
 int moe_route(const int32_t*, int64_t, int, int32_t*, int32_t*, int32_t*, int32_t*, void*, cudaStream_t);
 int moe_build_tiles(const int32_t*, int, int, int32_t*, cudaStream_t);
+bool moe_route_fused_fits(int64_t, int, int);
+int moe_route_fused(const void*, int, int64_t, int, int, void*, int, int32_t*, int32_t*, int32_t*, int, int32_t*, int, cudaStream_t);
 int gather_rows(const void*, const int32_t*, int, void*, int64_t, int64_t, int, cudaStream_t);
 int silu_mul(const void*, void*, int, int64_t, int64_t, const int32_t*, cudaStream_t, int64_t ld_in = 0, bool gelu = false);
 int quantize_fp8(const void*, int, int64_t, void*, float*, int, int64_t, int64_t, cudaStream_t);
@@ -529,6 +531,14 @@ int b2q_selftest_bounded_wait(int code, int* gave_up, void* stream) {
   return umma_selftest_bounded_wait(code, gave_up, (cudaStream_t)stream);
 }
 
+// The tile list of the given height, unless the caller already has it there (tiles_built: its height, kept up to date; may be null).
+static int need_tiles(int* tiles_built, int tile, const int32_t* expert_offsets, int E, int32_t* tiles, cudaStream_t st) {
+  if (tiles_built && *tiles_built == tile) return B2Q_OK;
+  const int rc = moe_build_tiles(expert_offsets, E, tile, tiles, st);
+  if (!rc && tiles_built) *tiles_built = tile;
+  return rc;
+}
+
 // Shared tail of the grouped GEMMs once the kernel family is chosen: optional row gather in
 // front of the tcgen05 kernel, optional SiLU*mul behind either kernel.
 struct GroupedPlan {
@@ -543,10 +553,13 @@ static GroupedPlan plan_workspace(void* ws, int64_t rows, int E, int64_t K, bool
   return pl;
 }
 
-int b2q_moe_gemm_int4(const void* x, int act_dtype, int64_t ldx, const int32_t* row_map, int row_div, const void* w,
-                      int w_layout, const void* scale, int scale_dtype, const int32_t* expert_offsets, int E,
-                      void* out, int64_t ldo, const int32_t* out_map, int64_t rows, int64_t N, int64_t K, int group,
-                      int act, void* workspace, size_t workspace_bytes, void* stream) {
+}  // extern "C"
+
+// tiles: height of the tile list that the workspace already begins with, 0 = none; the list is built where it has another one.
+static int moe_gemm_int4_core(const void* x, int act_dtype, int64_t ldx, const int32_t* row_map, int row_div, const void* w,
+                              int w_layout, const void* scale, int scale_dtype, const int32_t* expert_offsets, int E,
+                              void* out, int64_t ldo, const int32_t* out_map, int64_t rows, int64_t N, int64_t K, int group,
+                              int act, void* workspace, size_t workspace_bytes, void* stream, int* tiles_built) {
   if (!x || !w || !scale || !expert_offsets || !out || !workspace) return B2Q_ERR_NULL;
   if (!is16(act_dtype) || scale_dtype < 0 || scale_dtype > 2) return B2Q_ERR_DTYPE;
   if (w_layout < 0 || w_layout > 3) return B2Q_ERR_LAYOUT;
@@ -596,7 +609,7 @@ int b2q_moe_gemm_int4(const void* x, int act_dtype, int64_t ldx, const int32_t* 
     if (rc) return rc;
     ua.x = pl.xg; ua.ldx = K; ua.bf16 = false; ua.tok_scale = pl.inv; ua.magic = true;
     const int tile = umma_w4_token_tile(ua);
-    rc = moe_build_tiles(expert_offsets, E, tile, tiles, st);
+    rc = need_tiles(tiles_built, tile, expert_offsets, E, tiles, st);
     if (rc) return rc;
     ua.tile_cap = (int)((rows + tile - 1) / tile + E);
     rc = umma_w4_linear(ua, st);
@@ -610,7 +623,7 @@ int b2q_moe_gemm_int4(const void* x, int act_dtype, int64_t ldx, const int32_t* 
       xin = pl.xg; ldin = K;
     }
     const int tile = grouped_tile(rows, E);
-    rc = moe_build_tiles(expert_offsets, E, tile, tiles, st);
+    rc = need_tiles(tiles_built, tile, expert_offsets, E, tiles, st);
     if (rc) return rc;
     SmallMParams p{};
     p.x = xin; p.ldx = ldin;
@@ -627,10 +640,10 @@ int b2q_moe_gemm_int4(const void* x, int act_dtype, int64_t ldx, const int32_t* 
   return silu_mul(pl.g, out, act_dtype, rows, N / 2, out_map, st);
 }
 
-int b2q_moe_gemm_fp8(const void* x, int act_dtype, int64_t ldx, const int32_t* row_map, int row_div, const void* w,
-                     int fp8_format, const float* scale, int scale_mode, const int32_t* expert_offsets, int E,
-                     void* out, int64_t ldo, const int32_t* out_map, int64_t rows, int64_t N, int64_t K, int act,
-                     void* workspace, size_t workspace_bytes, void* stream) {
+static int moe_gemm_fp8_core(const void* x, int act_dtype, int64_t ldx, const int32_t* row_map, int row_div, const void* w,
+                             int fp8_format, const float* scale, int scale_mode, const int32_t* expert_offsets, int E,
+                             void* out, int64_t ldo, const int32_t* out_map, int64_t rows, int64_t N, int64_t K, int act,
+                             void* workspace, size_t workspace_bytes, void* stream, int* tiles_built) {
   if (!x || !w || !scale || !expert_offsets || !out || !workspace) return B2Q_ERR_NULL;
   if (!is16(act_dtype)) return B2Q_ERR_DTYPE;
   if (fp8_format != B2Q_E4M3 && fp8_format != B2Q_E5M2) return B2Q_ERR_DTYPE;
@@ -672,13 +685,13 @@ int b2q_moe_gemm_fp8(const void* x, int act_dtype, int64_t ldx, const int32_t* r
       ua.x = pl.xg; ua.ldx = K;
     }
     const int tile = umma_w8_token_tile(ua);
-    rc = moe_build_tiles(expert_offsets, E, tile, tiles, st);
+    rc = need_tiles(tiles_built, tile, expert_offsets, E, tiles, st);
     if (rc) return rc;
     ua.tile_cap = (int)((rows + tile - 1) / tile + E);
     rc = umma_w8_linear(ua, st);
   } else {
     const int tile = grouped_tile(rows, E);
-    rc = moe_build_tiles(expert_offsets, E, tile, tiles, st);
+    rc = need_tiles(tiles_built, tile, expert_offsets, E, tiles, st);
     if (rc) return rc;
     SmallMParams p{};
     p.x = x; p.ldx = ldx;
@@ -694,6 +707,156 @@ int b2q_moe_gemm_fp8(const void* x, int act_dtype, int64_t ldx, const int32_t* r
   }
   if (rc || act == B2Q_ACT_NONE) return rc;
   return silu_mul(pl.g, out, act_dtype, rows, N / 2, out_map, st, 0, act == B2Q_ACT_GELU_TANH_MUL);
+}
+
+extern "C" {
+
+int b2q_moe_gemm_int4(const void* x, int act_dtype, int64_t ldx, const int32_t* row_map, int row_div, const void* w,
+                      int w_layout, const void* scale, int scale_dtype, const int32_t* expert_offsets, int E,
+                      void* out, int64_t ldo, const int32_t* out_map, int64_t rows, int64_t N, int64_t K, int group,
+                      int act, void* workspace, size_t workspace_bytes, void* stream) {
+  return moe_gemm_int4_core(x, act_dtype, ldx, row_map, row_div, w, w_layout, scale, scale_dtype, expert_offsets, E, out, ldo, out_map,
+                            rows, N, K, group, act, workspace, workspace_bytes, stream, nullptr);
+}
+
+int b2q_moe_gemm_fp8(const void* x, int act_dtype, int64_t ldx, const int32_t* row_map, int row_div, const void* w,
+                     int fp8_format, const float* scale, int scale_mode, const int32_t* expert_offsets, int E,
+                     void* out, int64_t ldo, const int32_t* out_map, int64_t rows, int64_t N, int64_t K, int act,
+                     void* workspace, size_t workspace_bytes, void* stream) {
+  return moe_gemm_fp8_core(x, act_dtype, ldx, row_map, row_div, w, fp8_format, scale, scale_mode, expert_offsets, E, out, ldo, out_map,
+                           rows, N, K, act, workspace, workspace_bytes, stream, nullptr);
+}
+
+}  // extern "C"
+
+// ------------------------------------------------------------------------------------------------
+// Whole expert layers: from router logits to combined output in one call, on one workspace.
+// ------------------------------------------------------------------------------------------------
+namespace {
+// The workspace's parts in order.  The grouped GEMMs' own scratch begins with the tile list, which both share.
+struct MoeParts {
+  uint8_t *weights, *ids, *offsets, *tokens, *perm, *route, *mid, *y, *shared_mid, *shared_act, *shared_y, *linear, *gemm;
+  size_t linear_bytes, gemm_bytes, total;
+};
+struct Carver {
+  uint8_t* base; size_t at = 0;
+  uint8_t* take(size_t bytes) { uint8_t* p = base + at; at += align_up(bytes, 256); return p; }
+};
+MoeParts moe_parts(void* ws, int64_t T, int E, int top_k, int64_t H, int64_t I, int64_t Is) {
+  MoeParts p{};
+  Carver c{reinterpret_cast<uint8_t*>(ws)};
+  const size_t rows = (size_t)T * top_k;
+  p.weights = c.take(rows * 4); p.ids = c.take(rows * 4); p.offsets = c.take((size_t)(E + 1) * 4);
+  p.tokens = c.take(rows * 4); p.perm = c.take(rows * 4);
+  p.route = c.take(moe_route_workspace_bytes((int64_t)rows, E));
+  p.mid = c.take(rows * 2 * I * 2); p.y = c.take(rows * H * 2);
+  if (Is > 0) {
+    p.shared_mid = c.take((size_t)T * 2 * Is * 2); p.shared_act = c.take((size_t)T * Is * 2); p.shared_y = c.take((size_t)T * H * 2);
+    const size_t a = b2q_linear_workspace_bytes(T, 2 * Is, H), b = b2q_linear_workspace_bytes(T, H, Is);
+    p.linear_bytes = a > b ? a : b;
+    p.linear = c.take(p.linear_bytes);
+  }
+  const size_t up = b2q_moe_gemm_workspace_bytes((int64_t)rows, E, 2 * I, H, B2Q_ACT_GELU_TANH_MUL, 1);
+  const size_t down = b2q_moe_gemm_workspace_bytes((int64_t)rows, E, H, I, B2Q_ACT_SILU_MUL_IN, 0);
+  p.gemm_bytes = up > down ? up : down;
+  p.gemm = c.take(p.gemm_bytes);
+  p.total = c.at;
+  return p;
+}
+
+// Top-k and the sort by expert; for a few pairs one launch, which also builds the tile list of the given height.
+int moe_front(const void* logits, int logits_dtype, int64_t T, int E, int top_k, int w_dtype, const MoeParts& p, int tile, int* tiles_built,
+              cudaStream_t st) {
+  int32_t *off = reinterpret_cast<int32_t*>(p.offsets), *tok = reinterpret_cast<int32_t*>(p.tokens), *perm = reinterpret_cast<int32_t*>(p.perm);
+  if (moe_route_fused_fits(T, E, top_k)) {
+    *tiles_built = tile;
+    return moe_route_fused(logits, logits_dtype, T, E, top_k, p.weights, w_dtype, off, tok, perm, tile, reinterpret_cast<int32_t*>(p.gemm), 0, st);
+  }
+  *tiles_built = 0;
+  int rc = moe_topk(logits, logits_dtype, T, E, top_k, 1, p.weights, w_dtype, reinterpret_cast<int32_t*>(p.ids), st);
+  if (rc) return rc;
+  return moe_route(reinterpret_cast<int32_t*>(p.ids), T * top_k, E, off, tok, perm, nullptr, p.route, st);
+}
+
+int moe_check(const void* x, const void* logits, int act_dtype, int logits_dtype, int64_t T, int64_t E, int64_t top_k, int64_t H, int64_t I,
+              const void* out, const void* ws, size_t ws_bytes, size_t need) {
+  if (!x || !logits || !out || (!ws && need)) return B2Q_ERR_NULL;
+  if (!is16(act_dtype) || logits_dtype < 0 || logits_dtype > 2) return B2Q_ERR_DTYPE;
+  if (T < 0 || E <= 0 || top_k <= 0 || top_k > E || H <= 0 || I <= 0 || (H % 8) != 0) return B2Q_ERR_SHAPE;
+  if (E > 1024 || top_k > 32 || T * top_k > INT32_MAX || 2 * I > INT32_MAX || H > INT32_MAX) return B2Q_ERR_LIMIT;
+  if (!aligned16(x) || !aligned16(out) || (reinterpret_cast<uintptr_t>(ws) & 255u)) return B2Q_ERR_ALIGN;
+  return ws_bytes < need ? B2Q_ERR_WORKSPACE : B2Q_OK;
+}
+}  // namespace
+
+extern "C" {
+
+size_t b2q_moe_forward_workspace_bytes(int64_t T, int E, int top_k, int64_t H, int64_t I, int64_t Is) {
+  if (T <= 0 || E <= 0 || top_k <= 0 || H <= 0 || I <= 0 || Is < 0) return 0;
+  return moe_parts(nullptr, T, E, top_k, H, I, Is).total;
+}
+
+int b2q_moe_forward_int4(const b2q_moe_int4* a, void* workspace, size_t workspace_bytes, void* stream) {
+  if (!a) return B2Q_ERR_NULL;
+  const bool shared = a->shared_w13 != nullptr;
+  const int64_t T = a->T, H = a->H, I = a->I, Is = shared ? a->shared_I : 0;
+  const int E = (int)a->E, k = (int)a->top_k;
+  const size_t need = b2q_moe_forward_workspace_bytes(T, E, k, H, I, Is);
+  int rc = moe_check(a->x, a->logits, a->act_dtype, a->logits_dtype, T, a->E, a->top_k, H, I, a->out, workspace, workspace_bytes, need);
+  if (rc) return rc;
+  if (!a->w13 || !a->s13 || !a->w2 || !a->s2) return B2Q_ERR_NULL;
+  if (shared && (!a->shared_s13 || !a->shared_w2 || !a->shared_s2 || !a->gate_w)) return B2Q_ERR_NULL;
+  if ((H % 128) != 0 || (I % 128) != 0 || (shared && (Is <= 0 || (Is % 128) != 0))) return B2Q_ERR_SHAPE;
+  if (T == 0) return B2Q_OK;
+  cudaStream_t st = (cudaStream_t)stream;
+  const MoeParts p = moe_parts(workspace, T, E, k, H, I, Is);
+  const int32_t *off = reinterpret_cast<int32_t*>(p.offsets), *tok = reinterpret_cast<int32_t*>(p.tokens), *perm = reinterpret_cast<int32_t*>(p.perm);
+  const int64_t rows = T * k;
+  int tiles = 0;
+  rc = moe_front(a->logits, a->logits_dtype, T, E, k, a->act_dtype, p, grouped_tok((int)rows, E), &tiles, st);
+  if (rc) return rc;
+  rc = moe_gemm_int4_core(a->x, a->act_dtype, H, tok, k, a->w13, a->layout, a->s13, a->s13_dtype, off, E, p.mid, 2 * I, nullptr, rows, 2 * I, H,
+                          128, B2Q_ACT_NONE, p.gemm, p.gemm_bytes, stream, &tiles);
+  if (rc) return rc;
+  rc = moe_gemm_int4_core(p.mid, a->act_dtype, 2 * I, nullptr, 1, a->w2, a->layout, a->s2, a->s2_dtype, off, E, p.y, H, nullptr, rows, H, I, 128,
+                          B2Q_ACT_SILU_MUL_IN, p.gemm, p.gemm_bytes, stream, &tiles);
+  if (rc) return rc;
+  rc = moe_combine(p.y, p.weights, a->act_dtype, perm, a->out, a->act_dtype, T, k, H, 0, st);
+  if (rc || !shared) return rc;
+  const int kmaj = a->shared_scale_kmajor;
+  rc = b2q_linear_int4(a->x, a->act_dtype, H, a->shared_w13, a->shared_layout, a->shared_s13, a->shared_s13_dtype, kmaj ? 1 : H / 128,
+                       kmaj ? 2 * Is : 1, p.shared_mid, 2 * Is, T, 2 * Is, H, 128, p.linear, p.linear_bytes, stream);
+  if (!rc) rc = silu_mul(p.shared_mid, p.shared_act, a->act_dtype, T, Is, nullptr, st);
+  if (!rc)
+    rc = b2q_linear_int4(p.shared_act, a->act_dtype, Is, a->shared_w2, a->shared_layout, a->shared_s2, a->shared_s2_dtype, kmaj ? 1 : Is / 128,
+                         kmaj ? H : 1, p.shared_y, H, T, H, Is, 128, p.linear, p.linear_bytes, stream);
+  if (!rc) rc = shared_gate_add(a->x, a->gate_w, p.shared_y, a->out, a->out, a->act_dtype, T, H, st);
+  return rc;
+}
+
+int b2q_moe_forward_fp8(const b2q_moe_fp8* a, void* workspace, size_t workspace_bytes, void* stream) {
+  if (!a) return B2Q_ERR_NULL;
+  const int64_t T = a->T, H = a->H, I = a->I;
+  const int E = (int)a->E, k = (int)a->top_k;
+  const size_t need = b2q_moe_forward_workspace_bytes(T, E, k, H, I, 0);
+  int rc = moe_check(a->x, a->logits, a->act_dtype, a->logits_dtype, T, a->E, a->top_k, H, I, a->out, workspace, workspace_bytes, need);
+  if (rc) return rc;
+  if (!a->w13 || !a->s13 || !a->w2 || !a->s2) return B2Q_ERR_NULL;
+  if (T == 0) return B2Q_OK;
+  cudaStream_t st = (cudaStream_t)stream;
+  const MoeParts p = moe_parts(workspace, T, E, k, H, I, 0);
+  const int32_t *off = reinterpret_cast<int32_t*>(p.offsets), *tok = reinterpret_cast<int32_t*>(p.tokens), *perm = reinterpret_cast<int32_t*>(p.perm);
+  const int64_t rows = T * k;
+  int tiles = 0;
+  rc = moe_front(a->logits, a->logits_dtype, T, E, k, a->act_dtype, p, (rows + E - 1) / E > 16 ? grouped_tok((int)rows, E) : grouped_tile(rows, E), &tiles, st);
+  if (rc) return rc;
+  rc = moe_gemm_fp8_core(a->x, a->act_dtype, H, tok, k, a->w13, a->fp8_format, a->s13, B2Q_SCALE_TENSOR, off, E, p.mid, I, nullptr, rows, 2 * I, H,
+                         B2Q_ACT_GELU_TANH_MUL, p.gemm, p.gemm_bytes, stream, &tiles);
+  if (rc) return rc;
+  rc = moe_gemm_fp8_core(p.mid, a->act_dtype, I, nullptr, 1, a->w2, a->fp8_format, a->s2, B2Q_SCALE_TENSOR, off, E, p.y, H, nullptr, rows, H, I,
+                         B2Q_ACT_NONE, p.gemm, p.gemm_bytes, stream, &tiles);
+  if (rc) return rc;
+  return moe_combine(p.y, p.weights, a->act_dtype, perm, a->out, a->act_dtype, T, k, H, 0, st);
 }
 
 }  // extern "C"

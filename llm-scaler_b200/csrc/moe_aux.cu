@@ -127,6 +127,7 @@ int moe_topk(const void* logits, int ldt, int64_t T, int E, int top_k, int renor
 // marks experts owned by another rank.
 // ---------------------------------------------------------------------------
 constexpr int ROUTE_CHUNK = 256;  // pairs per CTA (8 warps)
+constexpr int ROUTE_FUSED_PAIRS = 1024, ROUTE_FUSED_EXPERTS = 256;      // moe_route_fused
 
 __global__ void route_hist_kernel(const int32_t* __restrict__ ids, int64_t n_pairs, int E, int32_t* __restrict__ counts) {
   extern __shared__ int32_t sh[];
@@ -281,6 +282,138 @@ __global__ void moe_tiles_kernel(const int32_t* __restrict__ expert_offsets, int
 int moe_build_tiles(const int32_t* expert_offsets, int E, int tile, int32_t* ws, cudaStream_t st) {
   launch_small(moe_tiles_kernel, dim3(1), dim3(1024), 0, st, expert_offsets, E, tile, ws);
   note_launch("moe_tiles");
+  return launch_status();
+}
+
+// ---------------------------------------------------------------------------
+// The whole routing of a few tokens in one launch of one CTA: softmax -> top-k -> renormalise (the arithmetic and order of
+// moe_topk_kernel), the stable counting sort by expert, and the tile list.  Up to ROUTE_FUSED_PAIRS pairs, one thread each in the sort.
+// The five launches it stands for do next to nothing each and come one after the other.
+// shared != 0: a further "expert" E, which every token goes to, behind the routed rows: its rows are n_pairs + t, and expert_tokens
+// holds t * top_k there, so that a division by top_k gives the token everywhere.
+// ---------------------------------------------------------------------------
+template <int PER_LANE>
+__global__ void __launch_bounds__(1024) moe_route_fused_kernel(const void* __restrict__ logits, int ldt, int T, int E, int top_k,
+                                                               void* __restrict__ weights, int wdt, int32_t* __restrict__ expert_offsets,
+                                                               int32_t* __restrict__ expert_tokens, int32_t* __restrict__ pair_to_perm,
+                                                               int tile, int32_t* __restrict__ tiles, int shared) {
+  __shared__ int16_t ids[ROUTE_FUSED_PAIRS];
+  __shared__ int16_t wc[32][ROUTE_FUSED_EXPERTS];      // pairs of an expert in each warp's run of pairs, then before it
+  __shared__ int32_t off[ROUTE_FUSED_EXPERTS + 2], tile0[ROUTE_FUSED_EXPERTS + 2], wsum[2][32];
+  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, n_pairs = T * top_k;
+  for (int i = tid; i < 32 * E; i += 1024) wc[i / E][i % E] = 0;
+  dep_enter();
+  for (int tok = warp; tok < T; tok += 32) {
+    float v[PER_LANE];
+    float mx = -INFINITY;
+#pragma unroll
+    for (int j = 0; j < PER_LANE; ++j) {
+      const int e = lane + 32 * j;
+      v[j] = e < E ? load_scalar_cg(logits, (int64_t)tok * E + e, ldt) : -INFINITY;
+      mx = fmaxf(mx, v[j]);
+    }
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, o));
+    float sum = 0.f;
+#pragma unroll
+    for (int j = 0; j < PER_LANE; ++j) {
+      const int e = lane + 32 * j;
+      v[j] = e < E ? expf(v[j] - mx) : 0.f;
+      sum += v[j];
+    }
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) sum += __shfl_xor_sync(0xffffffffu, sum, o);
+    const float inv = 1.0f / sum;
+#pragma unroll
+    for (int j = 0; j < PER_LANE; ++j) {
+      const int e = lane + 32 * j;
+      v[j] = e < E ? v[j] * inv : -2.f;
+    }
+    float tv = 0.f, tsum = 0.f;
+    int ti = 0;
+    for (int r = 0; r < top_k; ++r) {
+      float bv = -3.f;
+      int bi = 0x7fffffff;
+#pragma unroll
+      for (int j = 0; j < PER_LANE; ++j)
+        if (v[j] > bv) { bv = v[j]; bi = lane + 32 * j; }
+#pragma unroll
+      for (int o = 16; o > 0; o >>= 1) {
+        const float ov = __shfl_xor_sync(0xffffffffu, bv, o);
+        const int oi = __shfl_xor_sync(0xffffffffu, bi, o);
+        if (ov > bv || (ov == bv && oi < bi)) { bv = ov; bi = oi; }
+      }
+#pragma unroll
+      for (int j = 0; j < PER_LANE; ++j)
+        if (lane + 32 * j == bi) v[j] = -1.f;
+      if (lane == r) { tv = bv; ti = bi; }
+      tsum += bv;
+    }
+    if (lane < top_k) {
+      store_scalar(weights, (int64_t)tok * top_k + lane, wdt, tv * (1.0f / tsum));
+      // NaN logits leave no maximum: such a pair belongs to no expert, as in the separate kernels, whose sort drops it
+      ids[tok * top_k + lane] = (int16_t)(ti < E ? ti : -1);
+    }
+  }
+  __syncthreads();
+  // rank of a pair among its expert's: within the warp, then the warps before
+  const int e = tid < n_pairs ? ids[tid] : -1;
+  const unsigned peers = __match_any_sync(0xffffffffu, e);
+  const int rank = __popc(peers & ((1u << lane) - 1u));
+  if (e >= 0 && rank == 0) wc[warp][e] = (int16_t)__popc(peers);
+  __syncthreads();
+  int rows = 0;
+  if (tid < E)
+    for (int w2 = 0; w2 < 32; ++w2) { const int c = wc[w2][tid]; wc[w2][tid] = (int16_t)rows; rows += c; }
+  if (tid == E && shared) rows = T;
+  const int nt = (rows + tile - 1) / tile;
+  int a = rows, b = nt;                                  // inclusive sums over the experts
+#pragma unroll
+  for (int o = 1; o < 32; o <<= 1) {
+    const int x = __shfl_up_sync(0xffffffffu, a, o), y = __shfl_up_sync(0xffffffffu, b, o);
+    if (lane >= o) { a += x; b += y; }
+  }
+  if (lane == 31) { wsum[0][warp] = a; wsum[1][warp] = b; }
+  __syncthreads();
+  if (warp == 0) {
+    int x = wsum[0][lane], y = wsum[1][lane];
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+      const int p = __shfl_up_sync(0xffffffffu, x, o), q = __shfl_up_sync(0xffffffffu, y, o);
+      if (lane >= o) { x += p; y += q; }
+    }
+    wsum[0][lane] = x; wsum[1][lane] = y;
+  }
+  __syncthreads();
+  if (warp > 0) { a += wsum[0][warp - 1]; b += wsum[1][warp - 1]; }
+  const int last = shared ? E : E - 1;
+  if (tid <= last) {
+    off[tid] = a - rows; tile0[tid] = b - nt;
+    expert_offsets[tid] = a - rows;
+    if (tid == last) { expert_offsets[last + 1] = a; tiles[0] = b; }
+    int2* list = reinterpret_cast<int2*>(tiles + 4);
+    for (int i = 0; i < nt; ++i) list[b - nt + i] = make_int2(tid, i * tile);
+  }
+  __syncthreads();
+  if (tid < n_pairs) {
+    int pos = -1;
+    if (e >= 0) { pos = off[e] + wc[warp][e] + rank; expert_tokens[pos] = tid; }
+    pair_to_perm[tid] = pos;
+  }
+  if (shared && tid < T) expert_tokens[off[E] + tid] = tid * top_k;
+}
+
+bool moe_route_fused_fits(int64_t T, int E, int top_k) { return T * top_k <= ROUTE_FUSED_PAIRS && E < ROUTE_FUSED_EXPERTS && top_k <= 32; }
+
+int moe_route_fused(const void* logits, int ldt, int64_t T, int E, int top_k, void* weights, int wdt, int32_t* expert_offsets,
+                    int32_t* expert_tokens, int32_t* pair_to_perm, int tile, int32_t* tiles, int shared, cudaStream_t st) {
+#define B2Q_ROUTE(P) launch_small(moe_route_fused_kernel<P>, dim3(1), dim3(1024), 0, st, logits, ldt, (int)T, E, top_k, weights, wdt, \
+                                  expert_offsets, expert_tokens, pair_to_perm, tile, tiles, shared)
+  if (E <= 64) B2Q_ROUTE(2);
+  else if (E <= 128) B2Q_ROUTE(4);
+  else B2Q_ROUTE(8);
+#undef B2Q_ROUTE
+  note_launch("moe_route_fused");
   return launch_status();
 }
 

@@ -146,6 +146,46 @@ at::Tensor fp8_blockscale(const at::Tensor& input, const at::Tensor& weight, con
   return linear_fp8(input, weight, weight_scale, output, B2Q_SCALE_BLOCK128, -1, -1);
 }
 
+// out[:rows] = silu(gate) * up of input[:rows] (custom_esimd_kernels_vllm/_register.py: _moe_silu_mul over _impl.silu_mul)
+at::Tensor moe_silu_mul(const at::Tensor& input, at::Tensor output, int64_t N_gate_up, int64_t N_half, int64_t total_rows) {
+  TORCH_CHECK(N_gate_up == 2 * N_half, "N_gate_up must be 2 * N_half");
+  require_cuda({&input});
+  const at::Tensor in = input.slice(0, 0, total_rows), out = output.slice(0, 0, total_rows);
+  TORCH_CHECK(in.dim() == 2 && in.is_contiguous(), "gate_up must be contiguous [rows, 2I]");
+  const c10::cuda::CUDAGuard guard(in.device());
+  check(b2q_silu_mul(in.data_ptr(), out.data_ptr(), act_dtype(in), in.size(0), in.size(1) / 2,
+                     c10::cuda::getCurrentCUDAStream(in.device().index()).stream()));
+  return output;
+}
+
+// residual += hidden; normed_out = rmsnorm(residual) * norm_weight; output = normed_out @ W^T (_impl.resadd_norm_linear_fp8)
+at::Tensor resadd_norm_gemv_fp8_pert(const at::Tensor& hidden, at::Tensor residual, const at::Tensor& norm_weight, const at::Tensor& weight,
+                                     const at::Tensor& weight_scale, at::Tensor output, at::Tensor normed_out, double eps) {
+  TORCH_CHECK(weight_scale.numel() == 1 && weight_scale.scalar_type() == at::kFloat, "per-tensor scale must be one fp32");
+  require_cuda({&hidden, &residual, &norm_weight, &normed_out, &weight, &weight_scale, &output});
+  TORCH_CHECK(hidden.dim() == 2 && (hidden.scalar_type() == at::kBFloat16 || hidden.scalar_type() == at::kHalf), "hidden_states must be 2-D bf16 / fp16");
+  const int64_t M = hidden.size(0), K = hidden.size(1);
+  const at::Tensor* const same[] = {&hidden, &residual, &normed_out};
+  const char* const names[] = {"hidden_states", "residual", "normed_out"};
+  for (int i = 0; i < 3; ++i)
+    TORCH_CHECK(same[i]->scalar_type() == hidden.scalar_type() && same[i]->dim() == 2 && same[i]->size(0) == M && same[i]->size(1) == K &&
+                    same[i]->is_contiguous(), names[i], " must be a contiguous [M, K] tensor of the activation type");
+  TORCH_CHECK(norm_weight.scalar_type() == hidden.scalar_type() && norm_weight.numel() == K && norm_weight.is_contiguous(),
+              "norm_weight must be a contiguous [K] tensor of the activation type");
+  TORCH_CHECK(weight.dim() == 2 && weight.is_contiguous() && weight.size(1) == K, "fp8 weight must be a contiguous [N, K] tensor");
+  const int64_t N = weight.size(0);
+  TORCH_CHECK(output.dim() == 2 && output.size(0) == M && output.size(1) == N && output.scalar_type() == hidden.scalar_type() && output.stride(1) == 1,
+              "output must be [M, N] of the activation type");
+  const c10::cuda::CUDAGuard guard(hidden.device());
+  const size_t wsb = b2q_linear_fp8_workspace_bytes(M, N, K);
+  const at::Tensor ws = scratch(wsb, hidden);
+  check(b2q_resadd_norm_linear_fp8(hidden.data_ptr(), residual.data_ptr(), norm_weight.data_ptr(), normed_out.data_ptr(), (float)eps, 1.0f,
+                                   act_dtype(hidden), weight.data_ptr(), fp8_format(weight), weight_scale.data_ptr(), act_dtype(weight_scale),
+                                   B2Q_SCALE_TENSOR, output.data_ptr(), M > 1 ? output.stride(0) : N, M, N, K, wsb ? ws.data_ptr() : nullptr, wsb,
+                                   c10::cuda::getCurrentCUDAStream(hidden.device().index()).stream()));
+  return output;
+}
+
 const char* const kOps =
     "esimd_gemv_int4,esimd_gemm_int4_pgrp,esimd_gemv_fp8_pern,esimd_gemv_fp8_pert,esimd_gemv_fp8_pert_bmg,"
     "esimd_gemm_fp8_pert,esimd_gemm_fp8_blockscale";
@@ -155,7 +195,12 @@ const char* const kOps =
 // Names (comma separated, namespace custom_esimd_kernels_vllm) this library implements for the CUDA key.
 extern "C" __attribute__((visibility("default"))) const char* b2q_torch_ops() { return kOps; }
 
+// The same for the ops between the linears of a layer.
+extern "C" __attribute__((visibility("default"))) const char* b2q_torch_layer_ops() { return "esimd_moe_silu_mul,esimd_resadd_norm_gemv_fp8_pert"; }
+
 TORCH_LIBRARY_IMPL(custom_esimd_kernels_vllm, CUDA, m) {
+  m.impl("esimd_moe_silu_mul", &moe_silu_mul);
+  m.impl("esimd_resadd_norm_gemv_fp8_pert", &resadd_norm_gemv_fp8_pert);
   m.impl("esimd_gemv_int4", &gemv_int4);
   m.impl("esimd_gemm_int4_pgrp", &gemv_int4);
   m.impl("esimd_gemv_fp8_pern", &gemv_fp8_pern);

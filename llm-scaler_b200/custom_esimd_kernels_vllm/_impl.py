@@ -448,15 +448,84 @@ def moe_forward_int4(x, logits, w13, s13, w2, s2, top_k, num_experts, layout=Non
 
     The pipeline of moe_prefill_full_int4 (csrc/moe_prefill/moe_prefill_int4.sycl:920-988).  The
     activations are never materialised in expert order: the up GEMM gathers token rows through
-    expert_tokens and the combine reads the down result through pair_to_perm.
+    expert_tokens and the combine reads the down result through pair_to_perm.  One native call where the
+    operands are the usual ones, the same steps one by one otherwise.
     """
     T = x.shape[0]
+    out = _moe_forward_int4_native(x, logits, w13, s13, w2, s2, top_k, num_experts, layout)
+    if out is not None:
+        return out
     wts, ids = moe_topk(logits, top_k, True, weight_dtype=x.dtype)
     offsets, tokens, p2p, _ = moe_route(ids, num_experts)
     rows = T * top_k
     gate_up = moe_gemm_int4(x, w13, s13, offsets, rows, row_map=tokens, row_div=top_k, layout=layout)
     y = moe_gemm_int4(gate_up, w2, s2, offsets, rows, act=L.ACT_SILU_MUL_IN, layout=layout)
     return moe_combine(y, wts, p2p, T, top_k)
+
+
+def _plain_experts(x, logits, num_experts, top_k, *weights):
+    """Whether a native expert pipeline takes these operands: contiguous rows and weights, one logit per expert."""
+    return (x.is_cuda and logits.is_cuda and x.dim() == 2 and logits.dim() == 2 and x.shape[0] > 0 and x.is_contiguous() and logits.is_contiguous()
+            and logits.shape == (x.shape[0], num_experts) and 0 < top_k <= min(32, num_experts) and num_experts <= 1024
+            and x.dtype in (torch.bfloat16, torch.float16) and logits.dtype in L._DT
+            and all(w.is_cuda and w.dim() >= 1 and w.shape[0] == num_experts and w.is_contiguous() for w in weights))
+
+
+def _moe_forward_int4_native(x, logits, w13, s13, w2, s2, top_k, num_experts, layout, shared=None):
+    """b2q_moe_forward_int4, or None where the operands are not its.  shared: (w13, s13, w2, s2, gate_w) of the shared expert,
+    column-major repacked nibbles with scales [K/128, N]."""
+    if not _plain_experts(x, logits, num_experts, top_k, w13, s13, w2, s2) or not all(t.dim() == 3 for t in (w13, s13, w2, s2)):
+        return None
+    T, H = x.shape
+    N, kmajor = _moe_int4_layout(w13, s13, H)
+    if N % 256 or H % 128 or s13.dtype not in L._DT or s2.dtype not in L._DT:
+        return None
+    if _moe_int4_layout(w2, s2, N // 2) != (H, kmajor):
+        return None
+    if layout is None:
+        layout = L.W4_NMAJOR if not kmajor else L.W4_KMAJOR_MARLIN
+    out = torch.empty(T, H, dtype=x.dtype, device=x.device)
+    a = L.MoeInt4(x=x.data_ptr(), logits=logits.data_ptr(), w13=w13.data_ptr(), s13=s13.data_ptr(), w2=w2.data_ptr(), s2=s2.data_ptr(),
+                  out=out.data_ptr(), T=T, E=num_experts, top_k=top_k, H=H, I=N // 2, act_dtype=L.dt(x), logits_dtype=L.dt(logits),
+                  layout=layout, s13_dtype=L.dt(s13), s2_dtype=L.dt(s2))
+    if shared is not None:
+        gu, gus, dn, dns, gate = shared
+        Is = gu.numel() * gu.element_size() // H
+        if Is % 128 or gate.dtype != x.dtype or any(not t.is_cuda or not t.is_contiguous() for t in shared) or gus.dtype not in L._DT \
+                or dns.dtype not in L._DT or dn.numel() * dn.element_size() * 2 != H * Is or gus.numel() * GROUP != 2 * Is * H \
+                or dns.numel() * GROUP != H * Is or gate.numel() != H:
+            return None
+        a.shared_w13, a.shared_s13, a.shared_w2, a.shared_s2, a.gate_w = (t.data_ptr() for t in shared)
+        a.shared_I, a.shared_layout, a.shared_scale_kmajor = Is, L.W4_NMAJOR, 1
+        a.shared_s13_dtype, a.shared_s2_dtype = L.dt(gus), L.dt(dns)
+    with L.on_device(x):
+        wsb = L.lib.b2q_moe_forward_workspace_bytes(T, num_experts, top_k, H, N // 2, a.shared_I)
+        ws = torch.empty(wsb, dtype=torch.uint8, device=x.device)
+        L.check(L.lib.b2q_moe_forward_int4(a, ws.data_ptr(), wsb, L.stream(x)))
+    return out
+
+
+def moe_forward_fp8(x, logits, w13, s13, w2, s2, top_k, num_experts):
+    """Router logits -> FP8 experts with GELU-tanh -> combined output in one native call (b2q_moe_forward_fp8), or None where the operands
+    are not its."""
+    if not _plain_experts(x, logits, num_experts, top_k, w13, w2) or w13.dim() != 3 or w2.dim() != 3:
+        return None
+    T, H = x.shape
+    w13, w2 = _fp8_experts(w13), _fp8_experts(w2)
+    I = w2.shape[2]
+    if w13.shape[1:] != (2 * I, H) or w2.shape[1] != H or w13.dtype != w2.dtype or H % 16 or I % 16 \
+            or s13.numel() != num_experts or s2.numel() != num_experts or not s13.is_cuda or not s2.is_cuda:
+        return None
+    s13, s2 = s13.float().contiguous(), s2.float().contiguous()
+    out = torch.empty(T, H, dtype=x.dtype, device=x.device)
+    a = L.MoeFp8(x=x.data_ptr(), logits=logits.data_ptr(), w13=w13.data_ptr(), s13=s13.data_ptr(), w2=w2.data_ptr(), s2=s2.data_ptr(),
+                 out=out.data_ptr(), T=T, E=num_experts, top_k=top_k, H=H, I=I, act_dtype=L.dt(x), logits_dtype=L.dt(logits),
+                 fp8_format=L.fp8_fmt(w13))
+    with L.on_device(x):
+        wsb = L.lib.b2q_moe_forward_workspace_bytes(T, num_experts, top_k, H, I, 0)
+        ws = torch.empty(wsb, dtype=torch.uint8, device=x.device)
+        L.check(L.lib.b2q_moe_forward_fp8(a, ws.data_ptr(), wsb, L.stream(x)))
+    return out
 
 
 def moe_shared_gate_add(x, gate_w, shared, routed, out=None):
@@ -528,6 +597,12 @@ def moe_forward_full_int4(x, logits, gate_up_qweight, gate_up_scales, shared_gat
     _chk(num_shared_experts in (0, 1), "0 or 1 shared experts are supported")
     x = x.contiguous()
     layout = L.W4_NMAJOR if use_ggml_layout else L.W4_KMAJOR_MARLIN
+    if num_shared_experts == 1 and shared_gate_up_weight.numel() > 0 and shared_gate_up_weight.dtype in (torch.int32, torch.uint8):
+        out = _moe_forward_int4_native(x, logits.contiguous(), gate_up_qweight, gate_up_scales, down_qweight, down_scales, top_k,
+                                       n_routed_experts, layout, (shared_gate_up_weight, shared_gate_up_scale, shared_down_weight,
+                                                                  shared_down_scale, shared_expert_gate_weight))
+        if out is not None:
+            return out
     routed = moe_forward_int4(x, logits.contiguous(), gate_up_qweight, gate_up_scales, down_qweight, down_scales,
                               top_k, n_routed_experts, layout=layout)
     if num_shared_experts == 0 or shared_gate_up_weight.numel() == 0:

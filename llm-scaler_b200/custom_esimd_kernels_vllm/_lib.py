@@ -21,6 +21,21 @@ lib = C.CDLL(LIB_PATH)
 
 vp, i32, i64, sz = C.c_void_p, C.c_int, C.c_int64, C.c_size_t
 
+class MoeInt4(C.Structure):
+    """struct b2q_moe_int4"""
+    _fields_ = [(n, vp) for n in ("x", "logits", "w13", "s13", "w2", "s2", "shared_w13", "shared_s13", "shared_w2", "shared_s2",
+                                  "gate_w", "out")] \
+        + [(n, i64) for n in ("T", "E", "top_k", "H", "I", "shared_I")] \
+        + [(n, i32) for n in ("act_dtype", "logits_dtype", "layout", "s13_dtype", "s2_dtype", "shared_layout", "shared_s13_dtype",
+                              "shared_s2_dtype", "shared_scale_kmajor")]
+
+
+class MoeFp8(C.Structure):
+    """struct b2q_moe_fp8"""
+    _fields_ = [(n, vp) for n in ("x", "logits", "w13", "s13", "w2", "s2", "out")] \
+        + [(n, i64) for n in ("T", "E", "top_k", "H", "I")] + [(n, i32) for n in ("act_dtype", "logits_dtype", "fp8_format")]
+
+
 _SIGS = {
     "b2q_strerror": (C.c_char_p, [i32]),
     "b2q_version": (i32, []),
@@ -57,6 +72,9 @@ _SIGS = {
                                 i64, i64, i64, i32, i32, vp, sz, vp]),
     "b2q_moe_gemm_fp8": (i32, [vp, i32, i64, vp, i32, vp, i32, vp, i32, vp, i32, vp, i64, vp,
                                i64, i64, i64, i32, vp, sz, vp]),
+    "b2q_moe_forward_workspace_bytes": (sz, [i64, i32, i32, i64, i64, i64]),
+    "b2q_moe_forward_int4": (i32, [C.POINTER(MoeInt4), vp, sz, vp]),
+    "b2q_moe_forward_fp8": (i32, [C.POINTER(MoeFp8), vp, sz, vp]),
     "b2q_comm_create": (i32, [i32, i32, i64, i64, vp, vp]),
     "b2q_comm_create_mode": (i32, [i32, i32, i64, i64, i32, vp, vp]),
     "b2q_comm_connect": (i32, [vp, vp]),

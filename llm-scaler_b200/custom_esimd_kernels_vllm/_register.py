@@ -23,7 +23,8 @@ IMPLEMENTED = {}      # namespace -> names of the ops registered with an impleme
 # The dense linears are implemented for the CUDA key in C++ (csrc/torch_ops.cpp -> libb2q_torch.so, straight over the
 # C ABI): loading that library registers them, and the Python implementations below are then not attached to those
 # names.  B2Q_PYTHON_DISPATCH=1 keeps every op on its Python implementation (the two must agree; a test runs both).
-CPP_OPS = frozenset()
+CPP_OPS = frozenset()            # the dense linears
+CPP_LAYER_OPS = frozenset()      # and what runs between them in a layer
 _CPP_PATH = os.path.join(os.path.dirname(os.path.abspath(__file__)), "libb2q_torch.so")
 # B2Q_CHECK_STATUS=1 (debugging, tests): every op synchronises after its launches and raises if a bounded device-side
 # wait has expired, instead of leaving that to a caller who polls b2q_device_status.  It implies Python dispatch.
@@ -35,6 +36,8 @@ if os.environ.get("B2Q_PYTHON_DISPATCH") != "1" and not CHECK_STATUS:
     _h = ctypes.CDLL(_CPP_PATH)
     _h.b2q_torch_ops.restype = ctypes.c_char_p
     CPP_OPS = frozenset(_h.b2q_torch_ops().decode().split(","))
+    _h.b2q_torch_layer_ops.restype = ctypes.c_char_p
+    CPP_LAYER_OPS = frozenset(_h.b2q_torch_layer_ops().decode().split(","))
 
 
 def _lib(ns):
@@ -60,7 +63,7 @@ def _op(ns, schema, fn, meta=None):
     IMPLEMENTED.setdefault(ns, []).append(name)
     if CHECK_STATUS:
         fn = _checked(fn, ns + "::" + name)
-    if not (ns == "custom_esimd_kernels_vllm" and name in CPP_OPS):
+    if not (ns == "custom_esimd_kernels_vllm" and name in CPP_OPS | CPP_LAYER_OPS):
         lib.impl(name, fn, "CUDA")
     if meta is not None:
         lib.impl(name, meta, "Meta")
@@ -501,6 +504,9 @@ def _routed_fp8(x, topk_weights, topk_indices, gu_w, gu_s, dn_w, dn_s, top_k, ac
 
 
 def _full_gelu_tanh(x, logits, gu_w, gu_s, dn_w, dn_s, top_k, n_routed_experts):
+    out = I.moe_forward_fp8(x, logits, gu_w, gu_s, dn_w, dn_s, top_k, n_routed_experts)
+    if out is not None:
+        return out
     w, ids = I.moe_topk(logits.contiguous(), top_k, True, weight_dtype=x.dtype)
     return _routed_fp8(x, w, ids, gu_w, gu_s, dn_w, dn_s, top_k)
 
