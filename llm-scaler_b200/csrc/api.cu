@@ -21,6 +21,7 @@ size_t moe_route_workspace_bytes(int64_t, int);
 int moe_route(const int32_t*, int64_t, int, int32_t*, int32_t*, int32_t*, int32_t*, void*, cudaStream_t);
 int moe_build_tiles(const int32_t*, int, int, int32_t*, cudaStream_t);
 bool moe_route_fused_fits(int64_t, int, int);
+int moe_combine_shared(const void*, const void*, const int32_t*, const void*, const void*, const int32_t*, void*, int, int64_t, int, int64_t, cudaStream_t);
 int moe_route_fused(const void*, int, int64_t, int, int, void*, int, int32_t*, int32_t*, int32_t*, int, int32_t*, int, cudaStream_t);
 int gather_rows(const void*, const int32_t*, int, void*, int64_t, int64_t, int, cudaStream_t);
 int silu_mul(const void*, void*, int, int64_t, int64_t, const int32_t*, cudaStream_t, int64_t ld_in = 0, bool gelu = false);
@@ -746,10 +747,10 @@ MoeParts moe_parts(void* ws, int64_t T, int E, int top_k, int64_t H, int64_t I, 
   MoeParts p{};
   Carver c{reinterpret_cast<uint8_t*>(ws)};
   const size_t rows = (size_t)T * top_k;
-  p.weights = c.take(rows * 4); p.ids = c.take(rows * 4); p.offsets = c.take((size_t)(E + 1) * 4);
-  p.tokens = c.take(rows * 4); p.perm = c.take(rows * 4);
+  p.weights = c.take(rows * 4); p.ids = c.take(rows * 4); p.offsets = c.take((size_t)(E + 2) * 4);
+  p.tokens = c.take((rows + T) * 4); p.perm = c.take(rows * 4);
   p.route = c.take(moe_route_workspace_bytes((int64_t)rows, E));
-  p.mid = c.take(rows * 2 * I * 2); p.y = c.take(rows * H * 2);
+  p.mid = c.take((rows * 2 + T) * I * 2); p.y = c.take((rows + T) * H * 2);       // rows of the shared expert behind the routed ones
   if (Is > 0) {
     p.shared_mid = c.take((size_t)T * 2 * Is * 2); p.shared_act = c.take((size_t)T * Is * 2); p.shared_y = c.take((size_t)T * H * 2);
     const size_t a = b2q_linear_workspace_bytes(T, 2 * Is, H), b = b2q_linear_workspace_bytes(T, H, Is);
@@ -757,8 +758,9 @@ MoeParts moe_parts(void* ws, int64_t T, int E, int top_k, int64_t H, int64_t I, 
     p.linear = c.take(p.linear_bytes);
   }
   const size_t up = b2q_moe_gemm_workspace_bytes((int64_t)rows, E, 2 * I, H, B2Q_ACT_GELU_TANH_MUL, 1);
-  const size_t down = b2q_moe_gemm_workspace_bytes((int64_t)rows, E, H, I, B2Q_ACT_SILU_MUL_IN, 0);
+  const size_t down = b2q_moe_gemm_workspace_bytes((int64_t)rows, E, H, I, B2Q_ACT_SILU_MUL_IN, 0), list = tile_list_bytes(rows + T, E + 1, 8);
   p.gemm_bytes = up > down ? up : down;
+  if (p.gemm_bytes < list) p.gemm_bytes = list;
   p.gemm = c.take(p.gemm_bytes);
   p.total = c.at;
   return p;
@@ -813,17 +815,48 @@ int b2q_moe_forward_int4(const b2q_moe_int4* a, void* workspace, size_t workspac
   const int32_t *off = reinterpret_cast<int32_t*>(p.offsets), *tok = reinterpret_cast<int32_t*>(p.tokens), *perm = reinterpret_cast<int32_t*>(p.perm);
   const int64_t rows = T * k;
   int tiles = 0;
-  rc = moe_front(a->logits, a->logits_dtype, T, E, k, a->act_dtype, p, grouped_tok((int)rows, E), &tiles, st);
-  if (rc) return rc;
-  rc = moe_gemm_int4_core(a->x, a->act_dtype, H, tok, k, a->w13, a->layout, a->s13, a->s13_dtype, off, E, p.mid, 2 * I, nullptr, rows, 2 * I, H,
-                          128, B2Q_ACT_NONE, p.gemm, p.gemm_bytes, stream, &tiles);
-  if (rc) return rc;
-  rc = moe_gemm_int4_core(p.mid, a->act_dtype, 2 * I, nullptr, 1, a->w2, a->layout, a->s2, a->s2_dtype, off, E, p.y, H, nullptr, rows, H, I, 128,
-                          B2Q_ACT_SILU_MUL_IN, p.gemm, p.gemm_bytes, stream, &tiles);
-  if (rc) return rc;
-  rc = moe_combine(p.y, p.weights, a->act_dtype, perm, a->out, a->act_dtype, T, k, H, 0, st);
+  // Few rows per expert: the streaming kernel gathers and activates by itself, and takes the shared expert along where that has the
+  // routed experts' shape: four launches in all.
+  W4StreamArgs up{};
+  const bool kmaj_shared = a->shared_scale_kmajor != 0;
+  const bool merge = shared && Is == I && a->shared_layout == a->layout && a->shared_s13_dtype == a->s13_dtype && a->shared_s2_dtype == a->s2_dtype;
+  up.x = a->x; up.ldx = H; up.bf16 = a->act_dtype == B2Q_BF16;
+  up.w = a->w13; up.layout = a->layout; up.scale = a->s13; up.scale_dtype = a->s13_dtype; up.s_stride_n = H / 128; up.s_stride_g = 1;
+  up.out = p.mid; up.ldo = I; up.M = (int)rows; up.N = (int)(2 * I); up.K = (int)H; up.tile = W4_STREAM_MAX_TOK; up.gated = true;
+  up.tiles = reinterpret_cast<int32_t*>(p.gemm); up.E = E; up.expert_offsets = off; up.row_map = tok; up.row_div = k;
+  up.tile_cap = (int)((rows + 7) / 8 + E);
+  W4StreamArgs down = up;
+  down.x = p.mid; down.ldx = I; down.w = a->w2; down.scale = a->s2; down.scale_dtype = a->s2_dtype; down.s_stride_n = I / 128;
+  down.out = p.y; down.ldo = H; down.N = (int)H; down.K = (int)I; down.gated = false; down.row_map = nullptr;
+  if (merge) {
+    up.shared_w = a->shared_w13; up.shared_scale = a->shared_s13; up.shared_stride_n = kmaj_shared ? 1 : H / 128; up.shared_stride_g = kmaj_shared ? 2 * I : 1;
+    down.shared_w = a->shared_w2; down.shared_scale = a->shared_s2; down.shared_stride_n = kmaj_shared ? 1 : I / 128; down.shared_stride_g = kmaj_shared ? H : 1;
+    up.tile_cap = down.tile_cap = (int)((rows + 7) / 8 + E + (T + 7) / 8);
+  }
+  const int force = tls().force_kernel;
+  const bool use_stream = moe_route_fused_fits(T, E, k) && (force == 7 || (force == 0 && w4_stream_grouped_preferred(rows, E))) && w4_stream_supported(up) &&
+                      w4_stream_supported(down);
+  if (use_stream) {
+    rc = moe_route_fused(a->logits, a->logits_dtype, T, E, k, p.weights, a->act_dtype, reinterpret_cast<int32_t*>(p.offsets), reinterpret_cast<int32_t*>(p.tokens),
+                         reinterpret_cast<int32_t*>(p.perm), W4_STREAM_MAX_TOK, reinterpret_cast<int32_t*>(p.gemm), merge ? 1 : 0, st);
+    if (!rc) rc = w4_stream_linear(up, st);
+    if (!rc) rc = w4_stream_linear(down, st);
+    if (rc) return rc;
+    if (merge) return moe_combine_shared(p.y, p.weights, perm, a->x, a->gate_w, off + E, a->out, a->act_dtype, T, k, H, st);
+    rc = moe_combine(p.y, p.weights, a->act_dtype, perm, a->out, a->act_dtype, T, k, H, 0, st);
+  } else {
+    rc = moe_front(a->logits, a->logits_dtype, T, E, k, a->act_dtype, p, grouped_tok((int)rows, E), &tiles, st);
+    if (rc) return rc;
+    rc = moe_gemm_int4_core(a->x, a->act_dtype, H, tok, k, a->w13, a->layout, a->s13, a->s13_dtype, off, E, p.mid, 2 * I, nullptr, rows, 2 * I, H,
+                            128, B2Q_ACT_NONE, p.gemm, p.gemm_bytes, stream, &tiles);
+    if (rc) return rc;
+    rc = moe_gemm_int4_core(p.mid, a->act_dtype, 2 * I, nullptr, 1, a->w2, a->layout, a->s2, a->s2_dtype, off, E, p.y, H, nullptr, rows, H, I, 128,
+                            B2Q_ACT_SILU_MUL_IN, p.gemm, p.gemm_bytes, stream, &tiles);
+    if (rc) return rc;
+    rc = moe_combine(p.y, p.weights, a->act_dtype, perm, a->out, a->act_dtype, T, k, H, 0, st);
+  }
   if (rc || !shared) return rc;
-  const int kmaj = a->shared_scale_kmajor;
+  const bool kmaj = kmaj_shared;
   rc = b2q_linear_int4(a->x, a->act_dtype, H, a->shared_w13, a->shared_layout, a->shared_s13, a->shared_s13_dtype, kmaj ? 1 : H / 128,
                        kmaj ? 2 * Is : 1, p.shared_mid, 2 * Is, T, 2 * Is, H, 128, p.linear, p.linear_bytes, stream);
   if (!rc) rc = silu_mul(p.shared_mid, p.shared_act, a->act_dtype, T, Is, nullptr, st);

@@ -592,6 +592,71 @@ int moe_combine(const void* y, const void* w, int wdt, const int32_t* perm, void
 }
 
 // ---------------------------------------------------------------------------
+// The end of a decode pass with a shared expert in one launch: out[t, :] = sum_s w[t, s] * y[perm[t, s], :] + sigmoid(x[t, :] . gate_w) *
+// y[*shared_row0 + t, :], in fp32 with one rounding.  One CTA per token.
+template <bool BF16>
+__global__ void __launch_bounds__(256) moe_combine_shared_kernel(const uint4* __restrict__ y, const void* __restrict__ w, const int32_t* __restrict__ perm,
+                                                                 const uint4* __restrict__ x, const uint4* __restrict__ gate_w,
+                                                                 const int32_t* __restrict__ shared_row0, uint4* __restrict__ out, int top_k, int H8) {
+  using A = Act<BF16>;
+  using Ty = typename A::T;
+  __shared__ float red[8];
+  __shared__ int32_t rows[32];
+  __shared__ float wts[32];
+  dep_enter();
+  const int64_t t = blockIdx.x;
+  float dot = 0.f;
+  for (int c = threadIdx.x; c < H8; c += 256) {
+    const uint4 xv = __ldcg(x + t * H8 + c), gv = __ldcg(gate_w + c);
+    const Ty* xp = reinterpret_cast<const Ty*>(&xv);
+    const Ty* gp = reinterpret_cast<const Ty*>(&gv);
+#pragma unroll
+    for (int j = 0; j < 8; ++j) dot += A::to_f(xp[j]) * A::to_f(gp[j]);
+  }
+  if (threadIdx.x < top_k) {
+    rows[threadIdx.x] = __ldcg(perm + t * top_k + threadIdx.x);
+    wts[threadIdx.x] = load_scalar_cg(w, t * top_k + threadIdx.x, BF16 ? B2Q_BF16 : B2Q_F16);
+  }
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) dot += __shfl_xor_sync(0xffffffffu, dot, o);
+  if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = dot;
+  __syncthreads();
+  float a = 0.f;
+#pragma unroll
+  for (int i = 0; i < 8; ++i) a += red[i];
+  const float gate = 1.0f / (1.0f + expf(-a));
+  const int64_t srow = __ldcg(shared_row0) + t;
+  for (int c = threadIdx.x; c < H8; c += 256) {
+    float acc[8] = {0, 0, 0, 0, 0, 0, 0, 0};
+    auto add = [&](int64_t row, float wt) {
+      const uint4 v = __ldcg(y + row * H8 + c);
+      const Ty* vp = reinterpret_cast<const Ty*>(&v);
+#pragma unroll
+      for (int j = 0; j < 8; ++j) acc[j] += wt * A::to_f(vp[j]);
+    };
+#pragma unroll 4
+    for (int s = 0; s < top_k; ++s)
+      if (rows[s] >= 0) add(rows[s], wts[s]);
+    add(srow, gate);
+    uint4 o;
+    Ty* op = reinterpret_cast<Ty*>(&o);
+#pragma unroll
+    for (int j = 0; j < 8; ++j) op[j] = A::from_f(acc[j]);
+    out[t * H8 + c] = o;
+  }
+}
+
+int moe_combine_shared(const void* y, const void* w, const int32_t* perm, const void* x, const void* gate_w, const int32_t* shared_row0, void* out,
+                       int dtype, int64_t T, int top_k, int64_t H, cudaStream_t st) {
+  auto u = [](const void* p) { return reinterpret_cast<const uint4*>(p); };
+  auto go = [&](auto kern) { launch_small(kern, dim3((unsigned)T), dim3(256), 0, st, u(y), w, perm, u(x), u(gate_w), shared_row0, reinterpret_cast<uint4*>(out), top_k, (int)(H / 8)); };
+  if (dtype == B2Q_BF16) go(moe_combine_shared_kernel<true>);
+  else go(moe_combine_shared_kernel<false>);
+  note_launch("moe_combine_shared");
+  return launch_status();
+}
+
+// ---------------------------------------------------------------------------
 // Dynamic e4m3 quantisation of activations, one warp per (row, 128 columns).
 // scale = max(amax, 1e-12) / 448 ; q = e4m3_rn(x / scale) with true division,
 // the recipe of tests/test_fp8_blockscale_gemm.py:13-28 applied to a 1x128 tile.

@@ -62,8 +62,10 @@ static_assert(RS % XW == 0 && RS % (EW / BLOCKS) == 0 && SMEM <= 115712, "ring d
 
 struct W4SParams {
   const void* x; int64_t ldx;
-  const void* scale; int64_t s_stride_n, s_stride_g, s_expert_elems;
-  int scale_vec;               // bytes of a row's scales per asynchronous copy: 16 or 4, 0 = element by element
+  // scales of the experts and of the shared expert; vec: bytes of a row's scales per asynchronous copy, 16 or 4, 0 = element by element
+  struct Scales { const void* p; int64_t stride_n, stride_g; int vec; } sc, sc2;
+  int64_t s_expert_elems;
+  int shared_e;                // grouped: the "expert" whose weights are those of the second tensor map, or -1
   void* out; int64_t ldo;
   int M, N, K;                 // rows of W (gate and up together), k
   int half;                    // GATED: rows of the gate half, the up half follows
@@ -160,7 +162,7 @@ struct Cursor {
 
 template <bool BF16, int SD, bool GATED>      // SD: type of the group scales
 __global__ void __launch_bounds__(w4s::THREADS, 2)
-w4_stream_kernel(const __grid_constant__ CUtensorMap tm_w, const W4SParams p) {
+w4_stream_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constant__ CUtensorMap tm_w2, const W4SParams p) {
   using namespace w4s;
   constexpr int ESZ = SD == B2Q_F32 ? 4 : 2, GPS = 16 / ESZ;       // bytes of a scale, groups per scale slot
   extern __shared__ uint8_t smem_raw[];
@@ -199,14 +201,16 @@ w4_stream_kernel(const __grid_constant__ CUtensorMap tm_w, const W4SParams p) {
       uint32_t par = 1u;
       bool ok = true;
       while (ok && cur.next(p, sg)) {
-        const int r0 = sg.expert * p.N + sg.strip * (GATED ? ROWS / 2 : ROWS), r1 = r0 + (GATED ? p.half : ROWS / 2);
+        const bool sh = sg.expert == p.shared_e;
+        const CUtensorMap* tm = sh ? &tm_w2 : &tm_w;
+        const int r0 = (sh ? 0 : sg.expert * p.N) + sg.strip * (GATED ? ROWS / 2 : ROWS), r1 = r0 + (GATED ? p.half : ROWS / 2);
         for (int i = 0; i < sg.nst; ++i) {
           ok = mbar_wait(empty + 8 * s, par, abort_flag, p.status, ST_EMPTY);
           if (!ok) break;
           ++issued;
           mbar_expect_tx(full + 8 * s, RAW_BYTES);
-          tma_load_2d(base + s * RAW_BYTES, &tm_w, (sg.st0 + i) * 128, r0, full + 8 * s);
-          tma_load_2d(base + s * RAW_BYTES + RAW_BYTES / 2, &tm_w, (sg.st0 + i) * 128, r1, full + 8 * s);
+          tma_load_2d(base + s * RAW_BYTES, tm, (sg.st0 + i) * 128, r0, full + 8 * s);
+          tma_load_2d(base + s * RAW_BYTES + RAW_BYTES / 2, tm, (sg.st0 + i) * 128, r1, full + 8 * s);
           if (++s == RS) { s = 0; par ^= 1u; }
         }
       }
@@ -222,23 +226,25 @@ w4_stream_kernel(const __grid_constant__ CUtensorMap tm_w, const W4SParams p) {
     bool ok = true;
     while (ok && cur.next(p, sg)) {
       const int g0 = 2 * sg.st0 / GPS * GPS, g1 = 2 * (sg.st0 + sg.nst);
+      const bool sh = sg.expert == p.shared_e;
+      const W4SParams::Scales& sc = sh ? p.sc2 : p.sc;
       const uint8_t* rp[ROWS / 32];
 #pragma unroll
       for (int i = 0; i < ROWS / 32; ++i) {
         const int r = lane + 32 * i;
         const int n = !GATED ? min(sg.strip * ROWS + r, p.N - 1)
                              : (r < ROWS / 2 ? min(sg.strip * (ROWS / 2) + r, p.half - 1) : min(p.half + sg.strip * (ROWS / 2) + r - ROWS / 2, p.N - 1));
-        rp[i] = reinterpret_cast<const uint8_t*>(p.scale) + (sg.expert * p.s_expert_elems + n * p.s_stride_n) * ESZ;
+        rp[i] = reinterpret_cast<const uint8_t*>(sc.p) + ((sh ? 0 : sg.expert * p.s_expert_elems) + n * sc.stride_n) * ESZ;
       }
       for (int g = g0; g < g1; g += GPS) {
         ok = mbar_wait_warp(sc_empty + 8 * ss, par, abort_flag, p.status, ST_SCEMPTY);
         if (!ok) break;
         const uint32_t dst = sc_smem + ss * SC_BYTES + lane * 16;
-        if (p.scale_vec) {
+        if (sc.vec) {
 #pragma unroll
           for (int i = 0; i < ROWS / 32; ++i) {
             const uint8_t* src = rp[i] + (int64_t)g * ESZ;
-            if (p.scale_vec == 16) {
+            if (sc.vec == 16) {
               cp_async16(dst + 512 * i, src, 16);
             } else {
 #pragma unroll
@@ -257,7 +263,7 @@ w4_stream_kernel(const __grid_constant__ CUtensorMap tm_w, const W4SParams p) {
             for (int j = 0; j < 8; ++j) {
               e[j] = 0u;
               if (j < GPS && g + j < groups) {
-                const uint8_t* src = rp[i] + (int64_t)(g + j) * p.s_stride_g * ESZ;
+                const uint8_t* src = rp[i] + (int64_t)(g + j) * sc.stride_g * ESZ;
                 e[j] = ESZ == 4 ? __ldg(reinterpret_cast<const uint32_t*>(src)) : (uint32_t)__ldg(reinterpret_cast<const unsigned short*>(src));
               }
             }
@@ -553,7 +559,7 @@ size_t w4_stream_partial_bytes(int64_t M, int64_t N, int64_t K) {
 }
 
 template <bool BF16, int SD, bool GATED>
-static int launch(const CUtensorMap& tw, const W4SParams& p, int grid, bool overlap, cudaStream_t st) {
+static int launch(const CUtensorMap& tw, const CUtensorMap& tw2, const W4SParams& p, int grid, bool overlap, cudaStream_t st) {
   auto kern = w4_stream_kernel<BF16, SD, GATED>;
   static thread_local bool configured[16] = {false};
   int dev = 0;
@@ -562,25 +568,25 @@ static int launch(const CUtensorMap& tw, const W4SParams& p, int grid, bool over
     if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, w4s::SMEM) != cudaSuccess) return B2Q_ERR_CUDA;
     if (dev < 16) configured[dev] = true;
   }
-  if (launch_overlapped(kern, dim3(grid), dim3(w4s::THREADS), w4s::SMEM, st, overlap, tw, p) != cudaSuccess) return B2Q_ERR_CUDA;
+  if (launch_overlapped(kern, dim3(grid), dim3(w4s::THREADS), w4s::SMEM, st, overlap, tw, tw2, p) != cudaSuccess) return B2Q_ERR_CUDA;
   note_launch("w4_stream");
   return launch_status();
 }
 
 template <bool BF16, int SD>
-static int launch_gated(bool gated, const CUtensorMap& tw, const W4SParams& p, int grid, bool overlap, cudaStream_t st) {
-  return gated ? launch<BF16, SD, true>(tw, p, grid, overlap, st) : launch<BF16, SD, false>(tw, p, grid, overlap, st);
+static int launch_gated(bool gated, const CUtensorMap& tw, const CUtensorMap& tw2, const W4SParams& p, int grid, bool overlap, cudaStream_t st) {
+  return gated ? launch<BF16, SD, true>(tw, tw2, p, grid, overlap, st) : launch<BF16, SD, false>(tw, tw2, p, grid, overlap, st);
 }
 template <bool BF16>
-static int launch_scale(int sd, bool gated, const CUtensorMap& tw, const W4SParams& p, int grid, bool overlap, cudaStream_t st) {
-  if (sd == B2Q_F32) return launch_gated<BF16, B2Q_F32>(gated, tw, p, grid, overlap, st);
-  return sd == B2Q_BF16 ? launch_gated<BF16, B2Q_BF16>(gated, tw, p, grid, overlap, st) : launch_gated<BF16, B2Q_F16>(gated, tw, p, grid, overlap, st);
+static int launch_scale(int sd, bool gated, const CUtensorMap& tw, const CUtensorMap& tw2, const W4SParams& p, int grid, bool overlap, cudaStream_t st) {
+  if (sd == B2Q_F32) return launch_gated<BF16, B2Q_F32>(gated, tw, tw2, p, grid, overlap, st);
+  return sd == B2Q_BF16 ? launch_gated<BF16, B2Q_BF16>(gated, tw, tw2, p, grid, overlap, st) : launch_gated<BF16, B2Q_F16>(gated, tw, tw2, p, grid, overlap, st);
 }
 
 bool w4_stream_supported(const W4StreamArgs& a) {
   if (a.K <= 0 || (a.K % 128) != 0 || !aligned16(a.x) || !aligned16(a.w) || ((a.ldx * 2) & 15)) return false;
   if (a.layout != B2Q_W4_NMAJOR && a.layout != B2Q_W4_NMAJOR_S4) return false;
-  if (a.tile > W4_STREAM_MAX_TOK || (a.gated && (a.N % 2) != 0)) return false;
+  if (a.tile > W4_STREAM_MAX_TOK || (a.gated && (a.N % 2) != 0) || (a.shared_w && !aligned16(a.shared_w))) return false;
   return (int64_t)a.E * a.N <= INT32_MAX && tensor_map_encoder() != nullptr && umma_status_ptr() != nullptr;
 }
 
@@ -593,13 +599,25 @@ int w4_stream_linear(const W4StreamArgs& a, cudaStream_t st) {
   if (rc) return rc;
   W4SParams p{};
   p.x = a.x; p.ldx = a.ldx;
-  p.scale = a.scale; p.s_stride_n = a.s_stride_n; p.s_stride_g = a.s_stride_g;
-  p.s_expert_elems = (int64_t)a.N * (a.K / 128);
   const int esz = dtype_bytes(a.scale_dtype), G = a.K / 128;
-  const uintptr_t sp = reinterpret_cast<uintptr_t>(a.scale);
-  if (a.s_stride_g == 1) {
-    if ((G * esz) % 16 == 0 && (a.s_stride_n * esz) % 16 == 0 && (sp & 15u) == 0) p.scale_vec = 16;
-    else if ((G * esz) % 4 == 0 && (a.s_stride_n * esz) % 4 == 0 && (sp & 3u) == 0) p.scale_vec = 4;
+  auto scales = [&](const void* sp, int64_t sn, int64_t sg) {
+    W4SParams::Scales sc{sp, sn, sg, 0};
+    const uintptr_t at = reinterpret_cast<uintptr_t>(sp);
+    if (sg == 1) {
+      if ((G * esz) % 16 == 0 && (sn * esz) % 16 == 0 && (at & 15u) == 0) sc.vec = 16;
+      else if ((G * esz) % 4 == 0 && (sn * esz) % 4 == 0 && (at & 3u) == 0) sc.vec = 4;
+    }
+    return sc;
+  };
+  p.sc = scales(a.scale, a.s_stride_n, a.s_stride_g);
+  p.s_expert_elems = (int64_t)a.N * G;
+  p.shared_e = -1;
+  CUtensorMap tw2 = tw;
+  if (a.shared_w) {
+    rc = make_tmap_2d(&tw2, CU_TENSOR_MAP_DATA_TYPE_UINT8, 1, a.shared_w, a.N, a.K / 2, (uint64_t)a.K / 2, w4s::ROWS / 2, 128, CU_TENSOR_MAP_SWIZZLE_128B);
+    if (rc) return rc;
+    p.sc2 = scales(a.shared_scale, a.shared_stride_n, a.shared_stride_g);
+    p.shared_e = a.E;
   }
   p.out = a.out; p.ldo = a.ldo; p.M = a.M; p.N = a.N; p.K = a.K;
   p.half = a.N / 2;
@@ -625,7 +643,7 @@ int w4_stream_linear(const W4StreamArgs& a, cudaStream_t st) {
   // which needs the caller's word that no kernel in front writes them.
   const int mode = tls().overlap_mode;
   const bool overlap = grouped ? mode > 0 : mode == 2;
-  return a.bf16 ? launch_scale<true>(a.scale_dtype, a.gated, tw, p, grid, overlap, st) : launch_scale<false>(a.scale_dtype, a.gated, tw, p, grid, overlap, st);
+  return a.bf16 ? launch_scale<true>(a.scale_dtype, a.gated, tw, tw2, p, grid, overlap, st) : launch_scale<false>(a.scale_dtype, a.gated, tw, tw2, p, grid, overlap, st);
 }
 
 }  // namespace b2q

@@ -16,6 +16,8 @@ struct W4StreamArgs {
   bool gated = false;                                            // rows are gate then up; out = silu(gate) * up, N / 2 wide
   const int32_t* tiles = nullptr; int tile_cap = 0; int E = 1;   // grouped
   const int32_t* expert_offsets = nullptr; const int32_t* row_map = nullptr; int row_div = 1; const int32_t* out_map = nullptr;
+  // grouped: "expert" E of the tile list, a weight of its own of the same shape, scale type and nibbles
+  const void* shared_w = nullptr; const void* shared_scale = nullptr; int64_t shared_stride_n = 0, shared_stride_g = 0;
   void* partials = nullptr; size_t partial_bytes = 0;            // dense: w4_stream_partial_bytes(M, N, K), or strips stay whole
 };
 
@@ -27,5 +29,10 @@ size_t w4_stream_partial_bytes(int64_t M, int64_t N, int64_t K);
 // 4096 x 4096, one token, 8.3 us there and 13.4 here, 5120 x 5120 10.7 and 16, but 28672 x 1024 12.8 and 11.9, 8192 x 4096 14.4 and
 // 11.4, 10240 x 8192 27.2 and 17.9 (eight tokens 30.5 and 18.6).
 inline bool w4_stream_preferred(int64_t M, int64_t N, int64_t K) { return M <= W4_STREAM_MAX_TOK && N * K >= (int64_t)7 << 22; }
+
+// Grouped launches of the expert pipeline: up to four rows per expert on average; from about six on tiles of eight tokens repeat too
+// much of the decoding.  Whole pass in us against the tcgen05 kernel behind its pre-passes, 128 experts of 2048 x 768, top-8, at 1 / 16 /
+// 64 / 128 tokens: 28 / 82 / 119 / 163 against 31 / 89 / 127 / 145; 32 of 2048 x 1024, top-4, at 4 / 32 / 64: 32 / 51 / 69 against 39 / 60 / 66.
+inline bool w4_stream_grouped_preferred(int64_t rows, int E) { return rows <= 4 * (int64_t)E; }
 
 }  // namespace b2q
