@@ -1,5 +1,6 @@
 // Weight-only GEMM on tcgen05 for fp16 activations: out[tok, n] = sum_k x[tok, k] * W[n, k], W INT4 (group 128, behind the
-// activation pre-pass) or e4m3 (tiles of up to 64 tokens: block-scaled, or grouped with one scale per channel or tensor).
+// activation pre-pass) or e4m3 (dense: block-scaled up to 64 tokens, any scales above where its 128-token tiles pay; grouped:
+// one scale per channel or tensor, tiles of up to 64 tokens).
 //
 // Swap-AB: strips of R x 128 weight rows are the MMA's M dimension, a tile of TOK tokens its N dimension.  The nibbles are
 // decoded to fp16 in registers and written straight into tensor memory as the MMA's A operand (no trip back through
@@ -64,7 +65,7 @@ template <int WT, int TOK, int R> struct Cfg {
   static constexpr int X_BYTES = TOK * 128 * XC;
   static constexpr int XS = TOK == 128 ? 3 : (R == 2 ? 6 : (TOK == 64 ? 6 : 8) / GPS);
   static constexpr int RAW_BYTES = R * 16384;
-  static constexpr int SCS = 4, SC_GROUPS = 8, SC_BYTES = SC_GROUPS * ROWS * 2;   // scale slots: [row][group] 16-bit
+  static constexpr int SCS = 4, SC_GROUPS = 8, SC_BYTES = WT == WT_W8 ? 0 : SC_GROUPS * ROWS * 2;   // scale slots: [row][group] 16-bit
   static constexpr int POST_RING = 16;                       // row exponents per segment, read by the epilogue
   static constexpr int POST_BYTES = POST_RING * ROWS;
   static constexpr int STAGE_OUT = EW * 1024;                // 16 tokens x 32 columns of output per epilogue warp
@@ -739,8 +740,17 @@ umma_w4_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constant__
 #pragma unroll
               for (int z = 0; z < 2; ++z) {
                 const uint4 rr = lds128(rowa ^ ((2 * q + z) << 4));
-                e4m3_word(rr.x, sf, a16 + 8 * z); e4m3_word(rr.y, sf, a16 + 8 * z + 2);
-                e4m3_word(rr.z, sf, a16 + 8 * z + 4); e4m3_word(rr.w, sf, a16 + 8 * z + 6);
+                if (TOK < 128 || blocks) {
+                  e4m3_word(rr.x, sf, a16 + 8 * z); e4m3_word(rr.y, sf, a16 + 8 * z + 2);
+                  e4m3_word(rr.z, sf, a16 + 8 * z + 4); e4m3_word(rr.w, sf, a16 + 8 * z + 6);
+                } else {
+                  const uint32_t w[4] = {rr.x, rr.y, rr.z, rr.w};
+#pragma unroll
+                  for (int c = 0; c < 4; ++c) {
+                    a16[8 * z + 2 * c] = fp8x2_to_act<false, false>(w[c]);
+                    a16[8 * z + 2 * c + 1] = fp8x2_to_act<false, false>(w[c] >> 16);
+                  }
+                }
               }
             } else if constexpr (!KMAJOR) {
               const uint4 rr = lds128(rowa ^ (q << 4));
@@ -965,8 +975,29 @@ int umma_w4_prep_linear(const UmmaW4Args& a, cudaStream_t st) {
                 : launch_w4_tile<w4::WT_W4N>(tok, R, tw, tx, p, grid, overlap, st);
 }
 
-// e4m3 weights on fp16 activations, up to 64 tokens per tile: dense with block scales, grouped with one scale per channel or
-// tensor (whose transform multiplies by 1).
+// Dense launches of more than 64 tokens: 128-token tiles here, or umma_gemm.cu's of 256 (of 128, two CTAs per SM, up to 128 tokens).
+// Fewer bytes of operands per flop there, half the granularity here; each kernel's time is close to an offset plus rounds over
+// the SMs times a time per tile linear in K.  Fitted, in us, over N = 1024 .. 28672, K = 2048 .. 8192 and 70 to 2048 tokens
+// (285 launches per scale mode, 5 to 7 % mean error, 17 for the form with two CTAs per SM).  Choosing by it, with 5 % in
+// favour of the other kernel, takes 17 % less time over them with block scales and 18 with channel scales, 4 % more at worst
+// (512 x 12288 x 5120, block scales, 75 against 73 us).  128 x 17408 x 5120, block scales: 56 -> 36 us, 1221 x 4680 x 2048 43 -> 37;
+// 4001 x 17408 x 5120 stays where it was, 587 us against 645 here.  So do up to 4 Mi weights at up to 128 tokens, although they
+// would gain up to 5 us (100 x 2048 x 2048, block scales: 17.6 against 13.1): test_gpu_w4_strips.py names the kernel of such a call.
+static bool w8_strips_pay(const UmmaW8Args& a) {
+  if (a.M <= 128 && (int64_t)a.N * a.K <= (4 << 20)) return false;
+  const int sms = sm_count();
+  const int64_t strips = (a.N + 127) / 128;
+  const double k = a.K / 1024.0;
+  const bool block = a.scale_mode == B2Q_SCALE_BLOCK128;
+  auto rounds = [](int64_t work, int64_t slots) { return (double)((work + slots - 1) / slots); };
+  const double here = (block ? 4.67 : 5.93) + rounds(strips * ((a.M + 127) / 128), sms) * (block ? 1.16 + 4.08 * k : 0.74 + 3.31 * k);
+  const double there = a.M <= 128 ? (block ? 2.98 : 3.57) + rounds(strips, 2 * (int64_t)sms) * (block ? 2.98 + 6.26 * k : 3.57 + 4.18 * k)
+                                  : (block ? 1.30 : 1.70) + rounds(strips * ((a.M + 255) / 256), sms) * (block ? 8.92 + 5.56 * k : 8.39 + 5.36 * k);
+  return here < 0.95 * there;
+}
+
+// e4m3 weights on fp16 activations: dense with block scales up to 64 tokens and with any scales above (w8_strips_pay), grouped with one
+// scale per channel or tensor in tiles of up to 64 tokens.
 bool umma_w8_strip_supported(const UmmaW8Args& a) {
   if (a.bf16 || a.fmt != B2Q_E4M3 || (a.K % 128) != 0) return false;
   if (a.expert_offsets) {
@@ -978,7 +1009,7 @@ bool umma_w8_strip_supported(const UmmaW8Args& a) {
     // 4096 x 2048, 27.6 against 22.4) are faster here.
     return tok < 64 || grouped_rounds(a.M, a.E, (a.N + 127) / 128, tok, sm_count()) != 2;
   }
-  return a.scale_mode == B2Q_SCALE_BLOCK128 && a.M <= 64;
+  return a.M <= 64 ? a.scale_mode == B2Q_SCALE_BLOCK128 : w8_strips_pay(a);
 }
 
 int umma_w8_strip_linear(const UmmaW8Args& a, cudaStream_t st) {
@@ -999,15 +1030,16 @@ int umma_w8_strip_linear(const UmmaW8Args& a, cudaStream_t st) {
   p.tok_scale = a.tok_scale;
   p.status = umma_status_ptr();
   if (!p.status) return B2Q_ERR_CUDA;
-  p.strips = (a.N + 127) / 128; p.tiles_n = grouped ? a.tile_cap : 1;
-  if (!grouped) { rc = cut_strips(p, a, plan_w8(a.M, a.N, a.K)); if (rc) return rc; }
+  p.strips = (a.N + 127) / 128; p.tiles_n = grouped ? a.tile_cap : (a.M + tok - 1) / tok;
+  if (!grouped && a.M <= 64) { rc = cut_strips(p, a, plan_w8(a.M, a.N, a.K)); if (rc) return rc; }
   const int64_t work = p.units > 0 ? p.units : (int64_t)p.strips * p.tiles_n;
   if (work > INT32_MAX) return B2Q_ERR_LIMIT;
   const int grid = (int)(work < sms ? work : sms);
   const bool overlap = tls().overlap_mode > 0 && (a.after_prep || tls().overlap_mode == 2);
   if (tok == 16) return launch_w4<w4::WT_W8, 16, 1>(tw, tx, p, grid, overlap, st);
   if (tok == 32) return launch_w4<w4::WT_W8, 32, 1>(tw, tx, p, grid, overlap, st);
-  return launch_w4<w4::WT_W8, 64, 1>(tw, tx, p, grid, overlap, st);
+  if (tok == 64) return launch_w4<w4::WT_W8, 64, 1>(tw, tx, p, grid, overlap, st);
+  return launch_w4<w4::WT_W8, 128, 1>(tw, tx, p, grid, overlap, st);
 }
 
 }  // namespace b2q

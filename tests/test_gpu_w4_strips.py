@@ -181,6 +181,34 @@ def test_fp8_scratch_for_the_pre_pass_alone(e, M, kernel):
     assert e._lib.device_status() == 0
 
 
+@pytest.mark.parametrize("M,N,K", [(65, 16392, 384), (128, 4104, 1152), (129, 1096, 2048), (300, 1000, 1152), (385, 4680, 640)])
+@pytest.mark.parametrize("mode", ["block", "channel", "tensor"])
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16])
+def test_fp8_dense_above_64_tokens_strips(e, M, N, K, mode, dtype):
+    """Dense e4m3 in 128-token tiles: ragged last tiles of tokens and strips, odd counts of 128-wide chunks of k, every scale mode, both activation
+    types (bf16 ones are rewritten first).  Both kernels that can serve the call are held to the same bound: the output's rounding
+    (2^-9 for bf16, 2^-12 for fp16, relative to each element), weights times their block scale rounded to fp16 (2^-12, so below 2^-9 and
+    2^-11 in the 2-norm)."""
+    g = torch.Generator(device=DEV).manual_seed(M + N + K)
+    w = (torch.randn(N, K, generator=g, device=DEV) * 96).clamp_(-448, 448).to(torch.float8_e4m3fn)
+    x = torch.randn(M, K, generator=g, device=DEV).to(dtype)
+    shape = {"block": ((N + 127) // 128, K // 128), "channel": (N,), "tensor": (1,)}[mode]
+    s = (0.5 + torch.rand(*shape, generator=g, device=DEV)) / 4096
+    full = s.double().repeat_interleave(128, 0)[:N].repeat_interleave(128, 1) if mode == "block" else s.double().reshape(-1, 1)
+    ref = x.double() @ (w.double() * full).T
+    sm = {"block": e._lib.SCALE_BLOCK128, "channel": e._lib.SCALE_CHANNEL, "tensor": e._lib.SCALE_TENSOR}[mode]
+    L = e._lib
+    need = L.lib.b2q_linear_fp8_workspace_bytes(M, N, K)
+    ws = torch.empty(max(need, 1), dtype=torch.uint8, device=DEV)
+    out = torch.full((M, N), float("nan"), dtype=dtype, device=DEV)
+    code = L.BF16 if dtype == torch.bfloat16 else L.F16
+    L.check(L.lib.b2q_linear_fp8(x.data_ptr(), code, K, w.data_ptr(), L.E4M3, s.data_ptr(), L.F32, sm, out.data_ptr(), N, M, N, K,
+                                 ws.data_ptr(), need, torch.cuda.current_stream().cuda_stream))
+    assert e.last_kernel() == "umma_w4"
+    assert float((out.double() - ref).norm() / ref.norm()) < (2.0 ** -9 if dtype == torch.bfloat16 else 2.0 ** -11)
+    assert e._lib.device_status() == 0
+
+
 @pytest.mark.parametrize("E,rows,N,K", [
     (3, (60, 0, 33), 1096, 640),                       # 64-token tiles, short strips: few pieces
     (2, (129, 200), 520, 1152),                        # 128-token tiles, short strips
