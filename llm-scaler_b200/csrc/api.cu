@@ -4,6 +4,7 @@
 #include "smallm.cuh"
 #include "umma_gemm.cuh"
 #include "w4_stream.cuh"
+#include "w8_stream.cuh"
 #include "peer_reduce.cuh"
 
 namespace b2q {
@@ -346,6 +347,18 @@ static int linear_fp8_core(const void* x, int act_dtype, int64_t ldx, const void
   cudaStream_t st = (cudaStream_t)stream;
   const int force = tls().force_kernel;
 
+  // up to sixteen tokens: w8_stream.cu (w8_stream_preferred has the line and both sides of it)
+  if (M <= W8_STREAM_MAX_TOK && (force == 8 || force == 0)) {
+    W8StreamArgs sa{x, ldx, act_dtype == B2Q_BF16, w, fp8_format, scale, scale_dtype, scale_mode, out, ldo, (int)M, (int)N, (int)K};
+    if (w8_stream_supported(sa) && (force == 8 || w8_stream_preferred(sa))) {
+      if (nf) {
+        int rc = resadd_rmsnorm(nf->hidden, nf->residual, nf->norm_weight, const_cast<void*>(x), nullptr, nullptr,
+                                act_dtype == B2Q_BF16, M, (int)K, nf->eps, nf->scalar, st);
+        if (rc) return rc;
+      }
+      return w8_stream_linear(sa, st);
+    }
+  }
   UmmaW8Args ua{};
   ua.x = x; ua.ldx = ldx; ua.bf16 = (act_dtype == B2Q_BF16); ua.out_bf16 = ua.bf16; ua.tok_scale = nullptr;
   ua.w = w; ua.fmt = fp8_format; ua.scale = scale; ua.scale_dtype = scale_dtype; ua.scale_mode = scale_mode;

@@ -186,9 +186,8 @@ def test_fp8_scratch_for_the_pre_pass_alone(e, M, kernel):
 @pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16])
 def test_fp8_dense_above_64_tokens_strips(e, M, N, K, mode, dtype):
     """Dense e4m3 in 128-token tiles: ragged last tiles of tokens and strips, odd counts of 128-wide chunks of k, every scale mode, both activation
-    types (bf16 ones are rewritten first).  Both kernels that can serve the call are held to the same bound: the output's rounding
-    (2^-9 for bf16, 2^-12 for fp16, relative to each element), weights times their block scale rounded to fp16 (2^-12, so below 2^-9 and
-    2^-11 in the 2-norm)."""
+    types (bf16 ones are rewritten first).  The output is rounded once, at most 2^-8 (bf16) or 2^-11 (fp16) of each element, and
+    spread evenly below 0.58 of that in the 2-norm; so are weights times their block scale, at most 2^-11: together below 2^-8 and 2^-10."""
     g = torch.Generator(device=DEV).manual_seed(M + N + K)
     w = (torch.randn(N, K, generator=g, device=DEV) * 96).clamp_(-448, 448).to(torch.float8_e4m3fn)
     x = torch.randn(M, K, generator=g, device=DEV).to(dtype)
@@ -205,7 +204,7 @@ def test_fp8_dense_above_64_tokens_strips(e, M, N, K, mode, dtype):
     L.check(L.lib.b2q_linear_fp8(x.data_ptr(), code, K, w.data_ptr(), L.E4M3, s.data_ptr(), L.F32, sm, out.data_ptr(), N, M, N, K,
                                  ws.data_ptr(), need, torch.cuda.current_stream().cuda_stream))
     assert e.last_kernel() == "umma_w4"
-    assert float((out.double() - ref).norm() / ref.norm()) < (2.0 ** -9 if dtype == torch.bfloat16 else 2.0 ** -11)
+    assert float((out.double() - ref).norm() / ref.norm()) < (2.0 ** -8 if dtype == torch.bfloat16 else 2.0 ** -10)
     assert e._lib.device_status() == 0
 
 
