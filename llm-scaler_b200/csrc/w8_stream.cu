@@ -13,8 +13,8 @@
 //
 // What it replaces, umma_w8_direct.cu behind a pre-pass that splits the activations into e4m3 terms (umma_w4.cu behind act_prep for
 // block scales), pays for a second launch and its latency, and for the sums of cut strips.  One scale per tensor, three tokens, fp16,
-// there -> here: 2048 x 2048 14.6 -> 3.8 us, 5120 x 5120 16.2 -> 7.8, 7168 x 5120 17.3 -> 8.8, 5120 x 13824 25.2 -> 15.3, 17408 x 5120
-// 19.1 -> 16.4 (5.4 TB/s); eight tokens, bf16: 13.9 -> 4.2, 15.7 -> 10.0, 16.7 -> 11.7, 25.0 -> 21.
+// there -> here: 2048 x 2048 14.6 -> 3.4 us, 5120 x 5120 16.2 -> 8.0, 7168 x 5120 17.3 -> 8.7, 5120 x 13824 25.2 -> 14.6, 17408 x 5120
+// 19.1 -> 15.7 (5.7 TB/s), 27648 x 5120 26.4 -> 24.7; eight tokens, bf16: 13.9 -> 4.2, 15.7 -> 9.5, 16.7 -> 10.6, 25.0 -> 21.3, 18.7 -> 17.4.
 // What was found on the way:
 // * A bulk copy per row instead of TMA boxes costs some 55 cycles per copy and SM whatever its length: 1.1 to 2.7 TB/s.
 // * bf16 activations brought to fp16 by the staging warps, a power of two per stage, to save the weights' second conversion: 5120 x
@@ -22,6 +22,7 @@
 // * Tokens as the MMA's M and weight rows as its N, in eights: the same for few tokens, slower with block scales.
 // * Converting the empty half of a last tile: 10240 x 5120, bf16, one token 15.2 us, 13.8 without.
 // * One CTA per SM: 27648 x 5120 27.8 us against 25.6, 5120 x 13824 behind a norm 28.8 against 20.4; better below 16 rows per CTA only.
+// * INT4 in the same way: better than w4_stream.cu for one or two tokens of some shapes (8192 x 4096 14 -> 10 us), 0.3 to 0.8 of its speed otherwise.
 //
 // Every mbarrier wait is bounded; on expiry the CTA records a code in the status word and ends.
 //
@@ -91,6 +92,10 @@ __global__ void __launch_bounds__(w8s::THREADS, 2) w8_stream_kernel(const __grid
   const int box = (p.cap + 7) / 8 * 1024, w_slot = box * (C::KS / 128), x_slot = p.M * C::X_PITCH, nst = (p.K + C::KS - 1) / C::KS;
   const uint32_t x_smem = base + p.ns * w_slot;
   const int r0 = (int)((int64_t)blockIdx.x * p.N / gridDim.x), rows = (int)((int64_t)(blockIdx.x + 1) * p.N / gridDim.x) - r0;
+  // Every CTA begins its passes at another stage: all of them read the same activations, and in step they would ask the same L2 lines
+  // for them at the same moment.  17408 x 5120, fp16, 16 tokens 21.5 -> 17.3 us; 27648 x 5120, eight tokens 26.8 -> 24.7.
+  const int rot = (int)((blockIdx.x * 5u) % (unsigned)nst);
+  auto turn = [&](int i) { return i + rot < nst ? i + rot : i + rot - nst; };
   auto pass_row = [&](int i) { return r0 + (int)((int64_t)i * rows / p.passes); };
 
   // The next kernel may start at once.  This one waits for the kernels before it where it reads activations (warp 1); the outputs
@@ -112,7 +117,8 @@ __global__ void __launch_bounds__(w8s::THREADS, 2) w8_stream_kernel(const __grid
       bool ok = true;
       for (int i = 0; ok && i < p.passes; ++i) {
         const int n0 = pass_row(i);
-        for (int st = 0; st < nst; ++st) {
+        for (int j = 0; j < nst; ++j) {
+          const int st = turn(j);
           ok = mbar_wait(empty + 8 * s, par, abort_flag, p.status, ST_EMPTY);
           if (!ok) break;
           ++issued;
@@ -133,7 +139,8 @@ __global__ void __launch_bounds__(w8s::THREADS, 2) w8_stream_kernel(const __grid
     uint32_t par = 1u;
     bool ok = true;
     for (int i = 0; ok && i < p.passes; ++i) {
-      for (int st = 0; st < nst; ++st) {
+      for (int j = 0; j < nst; ++j) {
+        const int st = turn(j);
         ok = mbar_wait_warp(empty + 8 * s, par, abort_flag, p.status, ST_XEMPTY);
         if (!ok) break;
         const uint32_t dst = x_smem + s * x_slot + 16 * lane;
@@ -192,8 +199,8 @@ __global__ void __launch_bounds__(w8s::THREADS, 2) w8_stream_kernel(const __grid
       }
     }
 #pragma unroll 1
-    for (int st = 0; st < nst; ++st) {
-      const int k0 = st * C::KS + 64 * kg;
+    for (int j = 0; j < nst; ++j) {
+      const int st = turn(j), k0 = st * C::KS + 64 * kg;
       float fa[TW], fb[TW];
       if constexpr (BLOCK) {
         const int kb = min(k0 >> 7, nkb - 1);
@@ -364,29 +371,31 @@ static W8SPlan plan(int N) {
   return pl;
 }
 
-// Launches that are better off here than on umma_w8_direct.cu / umma_w4.cu.  Both sides were timed over 708 launches per scale mode (N =
-// 2048 .. 28672, K = 2048 .. 13824, 1 to 16 tokens); with this line they take 0.78 (bf16) and 0.70 (fp16) of the time there with one
-// scale per tensor or channel, 0.83 and 0.84 with block scales.
-// * More than one pass (N above some 19000): not faster than there on the whole, 0.6 to 1.4 of the speed, by how the rows fall.
-// * One scale per tensor or channel, fp16: 1.04 to 4.8 times as fast.  bf16: 1.06 to 4.6 where the strips there are cut along k (umma_w8_direct_linear),
-//   with more than eight tokens up to 48 Mi weights (5120 x 13824, 16 tokens: 31.4 us against 30.2); beyond, conversions weigh as much as
-//   the launch that is saved, 0.8 to 1.12.  Below 4 Mi weights the call stays there although it would gain 10 us: test_gpu_dense.py names
-//   the kernel of such calls.
-// * Block scales: by a fitted cost of both kernels in us.  The sums of every 64 k are scaled and added up here, per eight rows and per token.
+// Launches that are better off here than on umma_w8_direct.cu / umma_w4.cu.  Both sides were timed over 680 launches per scale mode and
+// activation type (N = 2048 .. 28672, K = 2048 .. 13824, 1 to 16 tokens); with this line they take 0.77 (bf16) and 0.65 (fp16) of the
+// time there with one scale per tensor or channel, 0.81 with block scales.
+// * One scale per tensor or channel, fp16, one pass (N up to some 19000): 1.2 to 5.5 times as fast.  More passes: up to eight tokens
+//   from 64 Mi weights 0.97 to 1.75; shorter or with more tokens 0.8 to 1.9, by how the strips there fall.
+// * bf16, which costs a second conversion: 1.1 to 5.4 where the strips there are cut along k (umma_w8_direct_linear); beyond, in one
+//   pass, 0.98 to 1.17 up to eight tokens and k of 6144, down to 0.83 otherwise; in more 0.6 to 1.4.
+// * Below 4 Mi weights such calls stay there although they would gain 10 us: test_gpu_dense.py names their kernel.
+// * Block scales: by a fitted cost of both kernels in us, 5 to 8 % mean error.  The sums of every 64 k are scaled and added up here, per
+//   eights of rows and per token; two unequal groups of MMA warps (33 to 48 rows) cost a fifth more.
 bool w8_stream_preferred(const W8StreamArgs& a) {
   const W8SPlan pl = plan(a.N);
   const int64_t weights = (int64_t)a.N * a.K;
-  if (pl.passes > 1) return false;
+  const bool few = a.M <= 8;
   if (a.scale_mode != B2Q_SCALE_BLOCK128) {
     if (weights < (4 << 20)) return false;
-    return !a.bf16 || ((a.N + 127) / 128 * 2 <= sm_count() && (a.M <= 8 || weights <= (48 << 20)));
+    if (!a.bf16) return pl.passes == 1 || (few && weights >= (64 << 20));
+    return (a.N + 127) / 128 * 2 <= sm_count() || (pl.passes == 1 && few && a.K <= 6144);
   }
-  int eights = (pl.cap + 7) / 8;
-  eights = eights < 2 ? 2 : (eights == 7 ? 8 : eights);
+  if (pl.passes > 1) return false;
+  const int eights = pl.cap <= 16 ? 2 : (pl.cap > 48 ? 8 : (pl.cap + 7) / 8);
   const double k = a.K / 1024.0, ctas = pl.grid > sm_count() ? 2.0 : 1.0;
-  const double here = 2.9 + k * ctas * ((a.bf16 ? 0.205 : 0.165) * eights + (a.M > 8 ? 0.04 : 0.029) * a.M);
-  const double there = (a.bf16 ? 10.5 : 9.3) + 0.135e-6 * (double)weights + 0.1 * k;
-  return here < 0.85 * there;
+  const double here = 2.65 + k * ctas * ((a.bf16 ? 0.218 : (few ? 0.170 : 0.196)) * eights * (eights == 5 || eights == 6 ? 1.2 : 1.0) + (few ? 0.020 : 0.026) * a.M);
+  const double there = (a.bf16 ? 10.1 : 8.6) + 0.116e-6 * (double)weights + (a.bf16 ? 0.44 : 0.28) * k;
+  return here < 0.92 * there;
 }
 
 bool w8_stream_supported(const W8StreamArgs& a) {
