@@ -583,6 +583,15 @@ static int launch_scale(int sd, bool gated, const CUtensorMap& tw, const CUtenso
   return sd == B2Q_BF16 ? launch_gated<BF16, B2Q_BF16>(gated, tw, tw2, p, grid, overlap, st) : launch_gated<BF16, B2Q_F16>(gated, tw, tw2, p, grid, overlap, st);
 }
 
+bool w4_stream_preferred(int64_t M, int64_t N, int64_t K) {
+  if (M > W4_STREAM_MAX_TOK) return false;
+  const double k = (double)K / 1024.0;
+  const int64_t slots = 3 * (int64_t)sm_count(), rounds = ((N + 15) / 16 + slots - 1) / slots;
+  const double there = 1.0 + (double)rounds * (0.9 + 1.38 * k) * (1.0 + 0.02 * (double)(M - 1));
+  const double here = 9.5 + 0.1e-6 * (double)N * (double)K + 0.2 * k;
+  return here < 0.97 * there;
+}
+
 bool w4_stream_supported(const W4StreamArgs& a) {
   if (a.K <= 0 || (a.K % 128) != 0 || !aligned16(a.x) || !aligned16(a.w) || ((a.ldx * 2) & 15)) return false;
   if (a.layout != B2Q_W4_NMAJOR && a.layout != B2Q_W4_NMAJOR_S4) return false;

@@ -25,10 +25,11 @@ bool w4_stream_supported(const W4StreamArgs& a);
 int w4_stream_linear(const W4StreamArgs& a, cudaStream_t st);
 size_t w4_stream_partial_bytes(int64_t M, int64_t N, int64_t K);
 
-// Dense launches that are better off here than in smallm.cuh, whose 16-row strips need no sum between CTAs and cost less to start:
-// 4096 x 4096, one token, 8.3 us there and 13.4 here, 5120 x 5120 10.7 and 16, but 28672 x 1024 12.8 and 11.9, 8192 x 4096 14.4 and
-// 11.4, 10240 x 8192 27.2 and 17.9 (eight tokens 30.5 and 18.6).
-inline bool w4_stream_preferred(int64_t M, int64_t N, int64_t K) { return M <= W4_STREAM_MAX_TOK && N * K >= (int64_t)7 << 22; }
+// Dense launches that are better off here than in smallm.cuh, whose 16-row strips need no sum between CTAs and cost less to start, but
+// come in rounds of three CTAs per SM that take their time for all of k.  By a fitted cost of both in us; one / eight tokens, there and
+// here: 4096 x 4096 8.3 / 8.8 and 13.4, 5888 x 5888 10.0 / 11.3 and 13.9, 10240 x 4096 14.2 / 15.5 and 15.1, but 7168 x 4224 14.3 / 17.3
+// and 13.4, 28672 x 1024 13.0 / 13.9 and 11.5, 2048 x 16384 26.8 / 30.7 and 17.4, 10240 x 8192 27.2 / 30.5 and 17.9.
+bool w4_stream_preferred(int64_t M, int64_t N, int64_t K);
 
 // Grouped launches of the expert pipeline: up to four rows per expert on average; from about six on tiles of eight tokens repeat too
 // much of the decoding.  Whole pass in us against the tcgen05 kernel behind its pre-passes, 128 experts of 2048 x 768, top-8, at 1 / 16 /

@@ -92,9 +92,10 @@ def test_infinities_and_nan_come_out_as_their_products(e, dtype):
     _close(out[3:], ref[3:], dtype)
 
 
-def test_dispatch_takes_it_for_wide_layers_only(e):
+def test_dispatch_takes_it_where_the_other_kernel_needs_more_rounds(e):
     e.set_force_kernel(0)
-    for M, N, K, name in ((8, 8192, 4096, "w4_stream"), (8, 4096, 4096, "smallm"), (9, 8192, 8192, "umma_w4")):
+    for M, N, K, name in ((8, 8192, 4096, "w4_stream"), (8, 4096, 4096, "smallm"), (1, 5888, 5888, "smallm"), (1, 7168, 5888, "w4_stream"), (1, 2048, 12288, "w4_stream"),
+                          (9, 8192, 8192, "umma_w4")):
         x, q, w, s = _inputs(M, N, K, torch.bfloat16, torch.bfloat16)
         out = torch.empty(M, N, dtype=torch.bfloat16, device=DEV)
         e.esimd_gemm_int4_pgrp(x.to(DEV), w.to(DEV), s.to(DEV), out)
