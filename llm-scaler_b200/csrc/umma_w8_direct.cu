@@ -34,15 +34,16 @@ __device__ int g_w8d_counters[W8D_BANKS * W8D_MAX_STRIPS];
 namespace w8d {
 enum { ST_FULL = 301, ST_EMPTY = 302, ST_ACCUM = 303, ST_ACCEMPTY = 304, ST_FIXUP = 305 };
 
-template <int NTOK> struct Cfg {
+template <int NTOK, bool DEEP = false> struct Cfg {
   static constexpr int W_BYTES = 16384;                                 // up to 128 rows x 128 k
   static constexpr int X_BYTES = NTOK * 128;
   static constexpr int STAGE = W_BYTES + X_BYTES;
   // measured: two CTAs per SM with about 100 KB of ring each stream fastest and leave room for the CTAs of the
-  // next launch to start (programmatic dependent launch) while this one drains
-  static constexpr int NS = NTOK <= 16 ? 6 : (NTOK == 32 ? 5 : (NTOK == 64 ? 4 : (NTOK == 128 ? 3 : 4)));
+  // next launch to start (programmatic dependent launch) while this one drains.  DEEP: launches of one CTA per SM at most
+  // have twice the ring; a stage takes 0.2 us there instead of 0.4, as its latency is spread over twice as many.
+  static constexpr int NS = (NTOK <= 16 ? 6 : (NTOK == 32 ? 5 : (NTOK == 64 ? 4 : (NTOK == 128 ? 3 : 4)))) * (DEEP ? 2 : 1);
   static constexpr int SMEM = NS * STAGE + 1024 + 256;
-  static constexpr int CTAS = NTOK <= 128 ? 2 : 1;
+  static constexpr int CTAS = NTOK <= 128 && !DEEP ? 2 : 1;
   static constexpr int ACC_COLS = NTOK < 32 ? 32 : NTOK;                // two accumulators: the epilogue of one segment
   static constexpr int TMEM_COLS = 2 * ACC_COLS;                        // runs under the MMAs of the next
   static constexpr int THREADS = 7 * 32;                                // W TMA, MMA, X TMA, four epilogue warps
@@ -65,15 +66,13 @@ struct W8DParams {
   int* status;
 };
 
-// A persistent grid of one CTA per SM.  The work, (strips) x (stages of 128 k), is cut into equal contiguous
-// runs, so a CTA streams up to two partial strips around any number of whole ones and every SM moves the same
-// number of bytes with all of its shared memory as the ring.  A strip that is cut is completed by whichever of
-// its CTAs delivers last: it adds the partial sums up in CTA order (so the result does not depend on who that
-// is) and writes the output.  Nobody waits for another CTA.
-template <int NTOK>
-__global__ void __launch_bounds__(w8d::Cfg<NTOK>::THREADS, w8d::Cfg<NTOK>::CTAS)
+// A CTA has one strip, or one of the equal pieces along k that a strip is cut into (umma_w8_direct_linear).  A cut strip is
+// completed by whichever of its CTAs delivers last: it adds the partial sums up in CTA order (so the result does not depend on who
+// that is) and writes the output.  Nobody waits for another CTA.
+template <int NTOK, bool DEEP>
+__global__ void __launch_bounds__(w8d::Cfg<NTOK, DEEP>::THREADS, w8d::Cfg<NTOK, DEEP>::CTAS)
 umma_w8_direct_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constant__ CUtensorMap tm_x, const W8DParams p) {
-  using C = w8d::Cfg<NTOK>;
+  using C = w8d::Cfg<NTOK, DEEP>;
   using namespace w8d;
   constexpr int NS = C::NS;
   extern __shared__ uint8_t smem_raw[];
@@ -266,11 +265,23 @@ umma_w8_direct_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_con
             float v[8];
 #pragma unroll
             for (int i = 0; i < 8; ++i) v[i] = 0.f;
-            for (int b = b_lo; b <= b_hi; ++b) {
-              const int64_t bu0 = (int64_t)b * U / G;
-              const float* src = p.partials + ((size_t)(b * 2 + (bu0 >= us ? 0 : 1)) * p.Mp) * 128 + rowi;
+            // all contributors' loads in flight at once: a trip through L2 per eight tokens, not one per contributor
+#pragma unroll 1
+            for (int b0 = b_lo; b0 <= b_hi; b0 += 4) {
+              float t[4][8];
 #pragma unroll
-              for (int i = 0; i < 8; ++i) v[i] += __ldcg(src + (m0 + i) * 128);
+              for (int q = 0; q < 4; ++q) {
+                const int b = min(b0 + q, b_hi);
+                const int64_t bu0 = (int64_t)b * U / G;
+                const float* src = p.partials + ((size_t)(b * 2 + (bu0 >= us ? 0 : 1)) * p.Mp) * 128 + rowi;
+#pragma unroll
+                for (int i = 0; i < 8; ++i) t[q][i] = __ldcg(src + (m0 + i) * 128);
+              }
+#pragma unroll
+              for (int q = 0; q < 4; ++q)
+                if (b0 + q <= b_hi)
+#pragma unroll
+                  for (int i = 0; i < 8; ++i) v[i] += t[q][i];
             }
             write_out(v, m0);
           }
@@ -334,10 +345,10 @@ static int pick_strip_rows(int N, int sms) {
   return best;
 }
 
-template <int NTOK>
+template <int NTOK, bool DEEP>
 static int launch_direct(const CUtensorMap& tw, const CUtensorMap& tx, const W8DParams& p, int grid, bool overlap, cudaStream_t st) {
-  using C = w8d::Cfg<NTOK>;
-  auto kern = umma_w8_direct_kernel<NTOK>;
+  using C = w8d::Cfg<NTOK, DEEP>;
+  auto kern = umma_w8_direct_kernel<NTOK, DEEP>;
   static thread_local bool configured[16] = {false};
   int dev = 0;
   cudaGetDevice(&dev);
@@ -364,27 +375,39 @@ int umma_w8_direct_linear(const UmmaW8DirectArgs& a, cudaStream_t st) {
   void* sym = nullptr;
   if (cudaGetSymbolAddress(&sym, g_w8d_status) != cudaSuccess) return B2Q_ERR_CUDA;
   p.status = reinterpret_cast<int*>(sym);
-  const int sms = sm_count(), slots = sms * (ntok <= 128 ? 2 : 1), nst = (a.K + 127) / 128;
-  // Few rows (less than one strip for every other SM): strips of 128 rows are cut along k into equal runs, which
-  // needs the scratch for partial sums.  Otherwise one CTA per strip, and the strip height is chosen so that the
-  // SMs end up with equal numbers of rows: the MMA always works on 128 rows, a lower strip just loads fewer.
-  const bool cut = ((a.N + 127) / 128) * 2 <= sms && a.partials && a.partial_bytes >= umma_w8_direct_partial_bytes(a.M);
+  const int sms = sm_count(), nst = (a.K + 127) / 128;
+  // One CTA per strip, and the strip height is chosen so that the SMs end up with equal numbers of rows: the MMA always works on 128
+  // rows, a lower strip just loads fewer.  Few rows (less than one strip for every other SM) with long k: strips of 128 rows, cut along k
+  // into up to four pieces, no more than there are SMs, which needs the scratch for partial sums.  The sums cost some 6 us, a stage of
+  // a whole strip 0.25 us: 20 tokens, fp16, 5120 rows, whole / three pieces 17.4 / 16.7 us for K = 6144, 21.3 / 18.9 for 8192, 26.1 / 22.1
+  // for 10240; 48 tokens, bf16, 19.6 / 21.5, 23.7 / 23.8, 28.0 / 26.5.  Equal runs over two CTAs per SM, a dozen pieces for short strips,
+  // whose sums were fetched one after the other: 31 tokens x 2752 x 2688 36.6 us, 10.0 now, 64 x 2048 x 2048 71 -> 12.5, 48 x 5120 x 13824
+  // 51 -> 30.
+  const int tall = (a.N + 127) / 128, pieces = sms / tall < 4 ? sms / tall : 4;
+  const bool cut = pieces >= 2 && nst >= 60 && a.partials && a.partial_bytes >= umma_w8_direct_partial_bytes(a.M);
   p.h = cut ? 128 : pick_strip_rows(a.N, sms);
   const int strips = (a.N + p.h - 1) / p.h;
   rc = make_tmap_2d(&tw, CU_TENSOR_MAP_DATA_TYPE_UINT8, 1, a.w, a.N, a.K, (uint64_t)a.K, p.h, 128, CU_TENSOR_MAP_SWIZZLE_128B);
   if (rc) return rc;
-  p.ust = cut ? 1 : nst; p.sps = cut ? nst : 1; p.units = strips * p.sps;
+  p.ust = cut ? (nst + pieces - 1) / pieces : nst; p.sps = (nst + p.ust - 1) / p.ust; p.units = strips * p.sps;
   p.partials = reinterpret_cast<float*>(a.partials);
   p.counters = cut ? w8d_counter_bank() : nullptr;
   if (cut && !p.counters) return B2Q_ERR_CUDA;
-  const int grid = cut ? (p.units < slots ? p.units : slots) : strips;
+  const int grid = p.units;
   const bool overlap = tls().overlap_mode > 0;     // always directly behind its own pre-pass
+  const bool deep = grid <= sms && ntok <= 128;
+  if (deep) switch (ntok) {
+    case 16: return launch_direct<16, true>(tw, tx, p, grid, overlap, st);
+    case 32: return launch_direct<32, true>(tw, tx, p, grid, overlap, st);
+    case 64: return launch_direct<64, true>(tw, tx, p, grid, overlap, st);
+    default: return launch_direct<128, true>(tw, tx, p, grid, overlap, st);
+  }
   switch (ntok) {
-    case 16: return launch_direct<16>(tw, tx, p, grid, overlap, st);
-    case 32: return launch_direct<32>(tw, tx, p, grid, overlap, st);
-    case 64: return launch_direct<64>(tw, tx, p, grid, overlap, st);
-    case 128: return launch_direct<128>(tw, tx, p, grid, overlap, st);
-    default: return launch_direct<256>(tw, tx, p, grid, overlap, st);
+    case 16: return launch_direct<16, false>(tw, tx, p, grid, overlap, st);
+    case 32: return launch_direct<32, false>(tw, tx, p, grid, overlap, st);
+    case 64: return launch_direct<64, false>(tw, tx, p, grid, overlap, st);
+    case 128: return launch_direct<128, false>(tw, tx, p, grid, overlap, st);
+    default: return launch_direct<256, false>(tw, tx, p, grid, overlap, st);
   }
 }
 

@@ -12,9 +12,9 @@
 //   next 8     conversion and MMA, a share of every stage's k each; they add up through shared memory at the end of a pass
 //
 // What it replaces, umma_w8_direct.cu behind a pre-pass that splits the activations into e4m3 terms (umma_w4.cu behind act_prep for
-// block scales), pays for a second launch and its latency, and for the sums of cut strips.  One scale per tensor, three tokens, fp16,
-// there -> here: 2048 x 2048 14.6 -> 3.4 us, 5120 x 5120 16.2 -> 8.0, 7168 x 5120 17.3 -> 8.7, 5120 x 13824 25.2 -> 14.6, 17408 x 5120
-// 19.1 -> 15.7 (5.7 TB/s), 27648 x 5120 26.4 -> 24.7; eight tokens, bf16: 13.9 -> 4.2, 15.7 -> 9.5, 16.7 -> 10.6, 25.0 -> 21.3, 18.7 -> 17.4.
+// block scales), pays for a second launch and its latency, and for a whole MMA of 128 rows wherever a CTA has fewer.  One scale per
+// tensor, four tokens, fp16, there -> here: 2048 x 2048 7.4 -> 3.3 us, 5120 x 5120 11.5 -> 8.3, 7168 x 5120 11.8 -> 8.6, 5120 x 13824 20.8 ->
+// 14.8, 17408 x 5120 19.1 -> 15.7 (5.7 TB/s), 27648 x 5120 26.4 -> 24.7; eight tokens, bf16: 7.0 -> 4.1, 10.9 -> 9.6, 11.0 -> 10.4, 18.7 -> 17.4.
 // What was found on the way:
 // * A bulk copy per row instead of TMA boxes costs some 55 cycles per copy and SM whatever its length: 1.1 to 2.7 TB/s.
 // * bf16 activations brought to fp16 by the staging warps, a power of two per stage, to save the weights' second conversion: 5120 x
@@ -371,14 +371,15 @@ static W8SPlan plan(int N) {
   return pl;
 }
 
-// Launches that are better off here than on umma_w8_direct.cu / umma_w4.cu.  Both sides were timed over 680 launches per scale mode and
-// activation type (N = 2048 .. 28672, K = 2048 .. 13824, 1 to 16 tokens); with this line they take 0.77 (bf16) and 0.65 (fp16) of the
-// time there with one scale per tensor or channel, 0.81 with block scales.
-// * One scale per tensor or channel, fp16, one pass (N up to some 19000): 1.2 to 5.5 times as fast.  More passes: up to eight tokens
-//   from 64 Mi weights 0.97 to 1.75; shorter or with more tokens 0.8 to 1.9, by how the strips there fall.
-// * bf16, which costs a second conversion: 1.1 to 5.4 where the strips there are cut along k (umma_w8_direct_linear); beyond, in one
-//   pass, 0.98 to 1.17 up to eight tokens and k of 6144, down to 0.83 otherwise; in more 0.6 to 1.4.
-// * Below 4 Mi weights such calls stay there although they would gain 10 us: test_gpu_dense.py names their kernel.
+// Launches that are better off here than on umma_w8_direct.cu / umma_w4.cu.  Both sides were timed over some 700 launches per scale mode
+// and activation type (N = 1024 .. 28672, K = 1024 .. 13824, 1 to 16 tokens).
+// * One scale per tensor or channel, fp16: 1.0 to 2.5 times as fast up to 9472 rows, 1.2 to 1.5 in one pass (N up to some 19000), but 0.88 for
+//   1024 x 13824 with 16 tokens, hardly more than one MMA tile's rows for long.  More passes: up to eight tokens from 64 Mi weights 0.97
+//   to 1.75; shorter or with more tokens 0.8 to 1.9, by how the strips there fall.
+// * bf16, which costs a second conversion.  Up to eight tokens and k of 8192 1.0 to 2.1 up to 9472 rows; longer k 1.02 to 1.3 for four
+//   tokens, 0.94 for eight (5120 x 13824).  More rows in one pass 0.98 to 1.17 up to k of 6144, down to 0.93 otherwise; in more 0.6 to 1.4.  More
+//   than eight tokens: 1.04 to 1.8 with one CTA per SM and k of 8192, or with k of 2048; 0.87 to 1.07 with two CTAs' fetches of activations.
+// * Below 4 Mi weights such calls stay there although they would gain up to 4 us: test_gpu_dense.py names their kernel.
 // * Block scales: by a fitted cost of both kernels in us, 5 to 8 % mean error.  The sums of every 64 k are scaled and added up here, per
 //   eights of rows and per token; two unequal groups of MMA warps (33 to 48 rows) cost a fifth more.
 bool w8_stream_preferred(const W8StreamArgs& a) {
@@ -387,8 +388,10 @@ bool w8_stream_preferred(const W8StreamArgs& a) {
   const bool few = a.M <= 8;
   if (a.scale_mode != B2Q_SCALE_BLOCK128) {
     if (weights < (4 << 20)) return false;
+    if (a.N < 2048 && a.K > 8192) return false;
     if (!a.bf16) return pl.passes == 1 || (few && weights >= (64 << 20));
-    return (a.N + 127) / 128 * 2 <= sm_count() || (pl.passes == 1 && few && a.K <= 6144);
+    if (!few) return (a.N + 127) / 128 * 2 <= sm_count() && (a.K <= 2048 || (a.K <= 8192 && pl.grid <= sm_count()));
+    return (a.N + 127) / 128 * 2 <= sm_count() ? a.K <= 8192 || a.M <= 4 : pl.passes == 1 && a.K <= 6144;
   }
   if (pl.passes > 1) return false;
   const int eights = pl.cap <= 16 ? 2 : (pl.cap > 48 ? 8 : (pl.cap + 7) / 8);

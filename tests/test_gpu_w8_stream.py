@@ -103,7 +103,8 @@ def test_overlap_and_repeats_give_the_same_bits(e, mode):
 
 @pytest.mark.parametrize("M,N,K,dtype,mode,stream", [
     (1, 4096, 1024, torch.bfloat16, "tensor", True), (1, 4096, 1008, torch.bfloat16, "tensor", False),
-    (16, 9472, 512, torch.bfloat16, "channel", True), (16, 9473, 512, torch.bfloat16, "channel", False), (8, 9473, 512, torch.bfloat16, "channel", True),
+    (16, 9472, 512, torch.bfloat16, "channel", True), (16, 9473, 512, torch.bfloat16, "channel", False), (9, 4735, 2064, torch.bfloat16, "tensor", True), (9, 4736, 2064, torch.bfloat16, "tensor", False),
+    (8, 3072, 8208, torch.bfloat16, "tensor", False), (4, 3072, 8208, torch.bfloat16, "tensor", True), (8, 9473, 512, torch.bfloat16, "channel", True),
     (8, 18945, 512, torch.bfloat16, "channel", False), (8, 9473, 6160, torch.bfloat16, "channel", False), (16, 9473, 512, torch.float16, "channel", True),
     (8, 18945, 3552, torch.float16, "tensor", True), (8, 18945, 3536, torch.float16, "tensor", False),
     (16, 18944, 512, torch.float16, "tensor", True), (16, 18945, 512, torch.float16, "tensor", False), (17, 4096, 1024, torch.float16, "tensor", False),
