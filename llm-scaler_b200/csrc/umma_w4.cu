@@ -812,26 +812,30 @@ static int sm_count() {
 
 static int dense_tok(int64_t M) { return M <= 16 ? 16 : (M <= 32 ? 32 : (M <= 64 ? 64 : 128)); }
 
-// CTAs among which strips of n raw stages are best cut for a 128-token tile; 0 = whole strips.  Every contributor to a strip adds
-// 64 KB of partial sums that one CTA reads back, so here a cut has to be weighed, and into few and equal pieces where
-// possible.  Fitted over N = 512 .. 12288 x K = 1024 .. 28672 at 65, 96 and 128 tokens (0.3 % above the best of seven divisions
-// on average, 6 % at most): 0.8 us per stage of a strip, and for cut strips 4 us, 2 us per contributor, and 1.2 us more where
-// the pieces do not line up with the strips, which then have one contributor more; 256-row strips take twice of each.  In
-// half stages below.  Against cutting over the whole grid: 128 x 2048 x 2048 25.9 -> 11.7 us, 128 x 4096 x 4096 35.0 -> 18.1,
-// 128 x 4096 x 14336 37.8 -> 32.1, 128 x 24576 x 4096 34.2 -> 31.3; unchanged 128 x 8192 x 28672, 64 us (97 with whole strips).
-static int cut_grid_128(int64_t strips, int64_t n, int sms) {
-  int64_t best = 2 * ((strips + sms - 1) / sms) * n, grid = 0;
+// CTAs among which strips of n raw stages are best cut; 0 = whole strips.  A cut has to be weighed, and into few and equal pieces
+// where possible: the last contributor to a strip adds up everybody's partial sums, and pieces that do not line up with the strips
+// have one contributor more.  cost, in us: per stage of a strip, per cut strip, per contributor to it.
+// 128-token tiles: fitted over N = 512 .. 12288 x K = 1024 .. 28672 at 65, 96 and 128 tokens (0.3 % above the best of seven divisions on
+// average, 6 % at most); 256-row strips take twice of each.  Against cutting over the whole grid: 128 x 2048 x 2048 25.9 -> 11.7 us, 128 x
+// 4096 x 4096 35.0 -> 18.1, 128 x 4096 x 14336 37.8 -> 32.1; unchanged 128 x 8192 x 28672, 64 us (97 with whole strips).
+// Lower tiles: over N = 1024 .. 14336 x K = 2048 .. 14336, whole, 2, 3, 4, 6, 8 pieces and the whole grid (before).  INT4, 64 tokens, 2048 x
+// 2048 8.9, 10.9, 11.3, 11.8, 13.6, 14.9 and 15.0 us, 2048 x 8192 21.9, 18.3, 16.3, 15.6, 16.6, 18.6 and 22.0, 14336 x 5120 16.8 whole, 23.6 over
+// the grid; e4m3 with block scales, 32 tokens, 1024 x 5120 17.8 whole, 30.2 over the grid, 14336 x 5120 19.8 and 24.6, 8192 x 14336 45.1 and 33.8.
+struct CutCost { double stage, strip, contributor; };
+static int cut_grid(int64_t strips, int64_t n, int sms, const CutCost& c) {
+  double best = c.stage * (double)((strips + sms - 1) / sms * n);
+  int64_t grid = 0;
   for (int64_t p = 2; p <= n && p * strips <= sms; ++p) {
-    const int64_t t = 2 * ((n + p - 1) / p) + 10 + 5 * p;
+    const double t = c.stage * (double)((n + p - 1) / p) + c.strip + c.contributor * (double)p;
     if (t < best) { best = t; grid = p * strips; }
   }
   const int64_t g = strips * n < sms ? strips * n : sms, pieces = (g + strips - 1) / strips;
-  if (g % strips != 0 && 2 * ((strips * n + g - 1) / g) + 13 + 5 * (pieces + 1) < best) grid = g;
+  if (g % strips != 0 && c.stage * (double)((strips * n + g - 1) / g) + 1.3 * c.strip + c.contributor * (double)(pieces + 1) < best) grid = g;
   return (int)grid;
 }
 
 // How one token tile of a dense launch is shared out: strips of R x 128 rows, cut along k, raw stage by raw stage, when whole
-// ones would leave more than a twentieth of the machine idle in the last round (128-token tiles: cut_grid_128).
+// ones would leave more than a twentieth of the machine idle in the last round and cut_grid finds a cut that pays.
 struct StripPlan { int R, strips, sps, units, grid; size_t partial_bytes; };      // sps, units: raw stages per strip and in total, 0 = whole strips
 static StripPlan plan_strips(int64_t M, int64_t N, int64_t K, int k_per_stage, bool tall) {
   StripPlan pl{};
@@ -843,7 +847,9 @@ static StripPlan plan_strips(int64_t M, int64_t N, int64_t K, int k_per_stage, b
   pl.grid = (int)(strips < sms ? strips : sms);
   if (M > tok || (K % k_per_stage) != 0 || strips > UMMA_MAX_CUT_STRIPS || units > INT32_MAX) return pl;
   if ((double)strips / ((double)((strips + sms - 1) / sms) * sms) > 0.95) return pl;
-  const int grid = tok == 128 ? cut_grid_128(strips, K / k_per_stage, sms) : (int)(units < sms ? units : sms);
+  const bool w8 = k_per_stage == 128;
+  const CutCost cost = tok == 128 ? CutCost{0.8, 4.0, 2.0} : (tok == 64 ? CutCost{w8 ? 0.46 : 0.54, 3.0, 1.0} : CutCost{w8 ? 0.35 : 0.5, 2.0, 0.75});
+  const int grid = cut_grid(strips, K / k_per_stage, sms, cost);
   if (!grid) return pl;
   pl.sps = (int)(K / k_per_stage); pl.units = (int)units; pl.grid = grid;
   pl.partial_bytes = (size_t)2 * pl.grid * pl.R * 128 * tok * sizeof(float);       // two slots per CTA
@@ -1031,8 +1037,13 @@ int umma_w8_strip_linear(const UmmaW8Args& a, cudaStream_t st) {
   p.status = umma_status_ptr();
   if (!p.status) return B2Q_ERR_CUDA;
   p.strips = (a.N + 127) / 128; p.tiles_n = grouped ? a.tile_cap : (a.M + tok - 1) / tok;
-  if (!grouped && a.M <= 64) { rc = cut_strips(p, a, plan_w8(a.M, a.N, a.K)); if (rc) return rc; }
-  const int64_t work = p.units > 0 ? p.units : (int64_t)p.strips * p.tiles_n;
+  int64_t work = (int64_t)p.strips * p.tiles_n;
+  if (!grouped && a.M <= 64) {
+    const StripPlan pl = plan_w8(a.M, a.N, a.K);
+    rc = cut_strips(p, a, pl);
+    if (rc) return rc;
+    if (p.units > 0) work = pl.grid;
+  }
   if (work > INT32_MAX) return B2Q_ERR_LIMIT;
   const int grid = (int)(work < sms ? work : sms);
   const bool overlap = tls().overlap_mode > 0 && (a.after_prep || tls().overlap_mode == 2);

@@ -380,8 +380,9 @@ static W8SPlan plan(int N) {
 //   tokens, 0.94 for eight (5120 x 13824).  More rows in one pass 0.98 to 1.17 up to k of 6144, down to 0.93 otherwise; in more 0.6 to 1.4.  More
 //   than eight tokens: 1.04 to 1.8 with one CTA per SM and k of 8192, or with k of 2048; 0.87 to 1.07 with two CTAs' fetches of activations.
 // * Below 4 Mi weights such calls stay there although they would gain up to 4 us: test_gpu_dense.py names their kernel.
-// * Block scales: by a fitted cost of both kernels in us, 5 to 8 % mean error.  The sums of every 64 k are scaled and added up here, per
-//   eights of rows and per token; two unequal groups of MMA warps (33 to 48 rows) cost a fifth more.
+// * Block scales, whose sums of every 64 k are scaled and added up here: up to eight tokens 0.99 to 3.1 up to 9472 rows and k of 8192, 0.81 to
+//   1.4 beyond; more rows in one pass 0.97 to 1.3 (bf16, k of 4096) and 1.0 to 1.27 (fp16, k of 5120), down to 0.76 beyond.  More than eight
+//   tokens, k of 4096: 1.02 to 2.6 (bf16, up to 9472 rows) and 1.08 to 2.0 (fp16, one CTA per SM; 0.73 to 1.28 with two).
 bool w8_stream_preferred(const W8StreamArgs& a) {
   const W8SPlan pl = plan(a.N);
   const int64_t weights = (int64_t)a.N * a.K;
@@ -394,11 +395,8 @@ bool w8_stream_preferred(const W8StreamArgs& a) {
     return (a.N + 127) / 128 * 2 <= sm_count() ? a.K <= 8192 || a.M <= 4 : pl.passes == 1 && a.K <= 6144;
   }
   if (pl.passes > 1) return false;
-  const int eights = pl.cap <= 16 ? 2 : (pl.cap > 48 ? 8 : (pl.cap + 7) / 8);
-  const double k = a.K / 1024.0, ctas = pl.grid > sm_count() ? 2.0 : 1.0;
-  const double here = 2.65 + k * ctas * ((a.bf16 ? 0.218 : (few ? 0.170 : 0.196)) * eights * (eights == 5 || eights == 6 ? 1.2 : 1.0) + (few ? 0.020 : 0.026) * a.M);
-  const double there = (a.bf16 ? 10.1 : 8.6) + 0.116e-6 * (double)weights + (a.bf16 ? 0.44 : 0.28) * k;
-  return here < 0.92 * there;
+  if (few) return a.K <= (pl.cap <= 32 ? 8192 : (a.bf16 ? 4096 : 6144));
+  return pl.cap <= 32 && a.K <= 4096 && (a.bf16 || pl.grid <= sm_count());
 }
 
 bool w8_stream_supported(const W8StreamArgs& a) {

@@ -108,7 +108,9 @@ def test_overlap_and_repeats_give_the_same_bits(e, mode):
     (8, 18945, 512, torch.bfloat16, "channel", False), (8, 9473, 6160, torch.bfloat16, "channel", False), (16, 9473, 512, torch.float16, "channel", True),
     (8, 18945, 3552, torch.float16, "tensor", True), (8, 18945, 3536, torch.float16, "tensor", False),
     (16, 18944, 512, torch.float16, "tensor", True), (16, 18945, 512, torch.float16, "tensor", False), (17, 4096, 1024, torch.float16, "tensor", False),
-    (1, 5120, 5120, torch.bfloat16, "block", True), (16, 22528, 512, torch.bfloat16, "block", False)])
+    (1, 5120, 8192, torch.bfloat16, "block", True), (1, 5120, 8320, torch.bfloat16, "block", False), (8, 9473, 4096, torch.bfloat16, "block", True),
+    (8, 9473, 4224, torch.bfloat16, "block", False), (8, 9473, 6144, torch.float16, "block", True), (9, 9472, 4096, torch.bfloat16, "block", True),
+    (9, 4736, 1024, torch.float16, "block", False), (9, 4735, 1024, torch.float16, "block", True), (16, 22528, 512, torch.bfloat16, "block", False)])
 def test_both_sides_of_the_dispatch_agree(e, M, N, K, dtype, mode, stream):
     """Which calls it takes by itself; those and their neighbours give the product on either kernel, with scratch or without."""
     e.set_force_kernel(0)
