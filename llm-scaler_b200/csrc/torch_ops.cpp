@@ -8,7 +8,8 @@
 // Built by build.py into custom_esimd_kernels_vllm/libb2q_torch.so, which links libb2q.so and libtorch.  Only
 // TORCH_LIBRARY_IMPL blocks live here: the schemas are defined once, by the Python registration module, which skips
 // its own implementation for the names this library reports through b2q_torch_ops().  The checks and their messages
-// are those of the Python implementation (custom_esimd_kernels_vllm/_impl.py: linear_int4, linear_fp8).
+// are those of the Python implementation (custom_esimd_kernels_vllm/_impl.py: linear_int4, linear_fp8).  Two ops that a decode layer has
+// between its linears are here as well, reported by b2q_torch_layer_ops().
 #include <ATen/ATen.h>
 #include <c10/cuda/CUDAGuard.h>
 #include <c10/cuda/CUDAStream.h>
