@@ -25,12 +25,14 @@
 #include "sm100.cuh"
 #include "smallm.cuh"   // nib2_to_act / fp8x2_to_act / lds128
 #include "peer_reduce.cuh"
+#include "arrivals.cuh"
 
 namespace b2q {
 
 using namespace sm100;
 
 __device__ int g_umma_status = 0;
+__device__ Arrivals g_arrivals_epoch = 0;
 constexpr int SK_BANKS = 64, SK_MAX_STRIPS = UMMA_MAX_CUT_STRIPS;
 __device__ int g_sk_counters[SK_BANKS * SK_MAX_STRIPS];     // arrival counters of cut strips (see umma_strip_counters)
 
@@ -602,6 +604,19 @@ static int* status_ptr() {
 
 int* umma_status_ptr() { return status_ptr(); }
 
+const Arrivals* arrivals_epoch() {
+  static thread_local const Arrivals* ptr[16] = {nullptr};
+  int dev = 0;
+  cudaGetDevice(&dev);
+  if (dev < 0 || dev >= 16) return nullptr;
+  if (!ptr[dev]) {
+    void* p = nullptr;
+    if (cudaGetSymbolAddress(&p, g_arrivals_epoch) != cudaSuccess) return nullptr;
+    ptr[dev] = reinterpret_cast<const Arrivals*>(p);
+  }
+  return ptr[dev];
+}
+
 // Self-test of the bounded-wait machinery: one CTA waits on an mbarrier that nobody ever arrives on, with a limit of
 // about a millisecond instead of two seconds.  The wait must give up, record `code` in the status word and return;
 // the context stays usable.  Nothing here faults or spins without bound.
@@ -629,7 +644,6 @@ int umma_selftest_bounded_wait(int code, int* gave_up_dev, cudaStream_t st) {
 int w8a8_reset_state();
 int w8d_reset_state();
 int w4i_reset_state();
-int w4s_reset_state();
 
 // Clears, on the current device, the status word of every tcgen05 kernel family and the arrival counters of cut
 // strips.  A CTA that gave up on a wait never delivered its arrival, so its strip's counter is left non-zero and the
@@ -643,10 +657,12 @@ int umma_reset_status() {
   void* c = nullptr;
   if (cudaGetSymbolAddress(&c, g_sk_counters) != cudaSuccess) return B2Q_ERR_CUDA;
   if (cudaMemset(c, 0, sizeof(int) * SK_BANKS * SK_MAX_STRIPS) != cudaSuccess) return B2Q_ERR_CUDA;
+  static std::atomic<Arrivals> resets{0};
+  const Arrivals epoch = resets.fetch_add(1, std::memory_order_relaxed) + 1;
+  if (cudaMemcpyToSymbol(g_arrivals_epoch, &epoch, sizeof(epoch)) != cudaSuccess) return B2Q_ERR_CUDA;
   int rc = w8a8_reset_state();
   if (!rc) rc = w8d_reset_state();
   if (!rc) rc = w4i_reset_state();
-  if (!rc) rc = w4s_reset_state();
   return rc;
 }
 

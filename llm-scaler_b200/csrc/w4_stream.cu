@@ -29,18 +29,15 @@
 //
 // Reference counterparts: esimd_gemv_int4 (csrc/xpu/esimd_kernels/int4_GEMV.h:165-251), GEMM_int4_pgrp_kernel
 // (int4_GEMM.h:81-270), the tiny-M expert kernels of csrc/moe_batch/moe_int4.sycl.
-#include <atomic>
 #include "umma_gemm.cuh"
 #include "sm100.cuh"
+#include "arrivals.cuh"
 #include "smallm.cuh"   // lds128, mma16816, cp_async16
 #include "w4_stream.cuh"
 
 namespace b2q {
 
 using namespace sm100;
-
-constexpr int W4S_BANKS = 64, W4S_MAX_STRIPS = 1024;
-__device__ int g_w4s_counters[W4S_BANKS * W4S_MAX_STRIPS * 4];     // arrivals per strip and block, zero between launches
 
 namespace w4s {
 enum { ST_EMPTY = 601, ST_XEMPTY = 602, ST_SCEMPTY = 603, ST_FULL = 604, ST_SCFULL = 605 };
@@ -70,7 +67,8 @@ struct W4SParams {
   int M, N, K;                 // rows of W (gate and up together), k
   int half;                    // GATED: rows of the gate half, the up half follows
   int strips, sps, units;      // strips, stages per strip, stages in total (cut launches; 0 = whole strips)
-  float4* partials; int* counters;
+  float4* partials;            // [2 * grid][BLOCKS][2][32] sums of cut strips
+  Arrivals* arrivals; Arrivals tag; const Arrivals* epoch;      // [strips][BLOCKS] counts behind the partial sums
   uint32_t flip;               // 0x00080008 for two's-complement nibbles
   const int32_t* tiles; const int32_t* expert_offsets; const int32_t* row_map; int row_div; const int32_t* out_map;
   int* status;
@@ -286,7 +284,7 @@ w4_stream_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constant
     const uint32_t dst0 = x_smem + ((lane >> 4) * 4 + (lane & 3)) * 512 + ((lane >> 2) & 3) * 16;
     int i = 0, s = 0;                                    // stages handed out so far; ring position
     uint32_t par = 1u;
-    bool ok = true;
+    bool ok = true, open = !GATED && p.units > 0 && me == 0;      // gated launches are grouped: whole strips
     while (ok && cur.next(p, sg)) {
       const int m_left = min(sg.M - sg.tok0, 8);
       int64_t row_off = 0;                               // lane m: where token m's row begins
@@ -311,6 +309,13 @@ w4_stream_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constant
         if (i % XW == me) {
           ok = mbar_wait_warp(empty + 8 * s, par, abort_flag, p.status, ST_XEMPTY);
           if (!ok) break;
+          // The counts of the CTA's cut strips, which only a run's ends can be, are opened before the first segment's last stage is
+          // handed to the warps that will add to them; behind the first stages, as the trip to DRAM would hold these up (decoder layer
+          // of one token 126.4 us that way, 126.0 here, 125.2 with counts that nobody has to open).
+          if (open && (i == RS || st + XW >= sg.nst)) {
+            if (lane < 2 * BLOCKS) arrivals_open(p.arrivals + ((lane & 1) ? cur.u1 - 1 : cur.u0) / p.sps * BLOCKS + (lane >> 1), p.tag, p.epoch);
+            open = false;
+          }
 #pragma unroll
           for (int j = 0; j < 8; ++j)
             if (j < m_left)
@@ -443,8 +448,8 @@ w4_stream_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constant
       if (!ok) break;
       if (turn == 1) continue;
       bool deliver = true;
-      if (sg.part) {
-        // CTAs b_lo .. b_hi share the strip; this warp's rows are finished by the last of their warps w to get here
+      if (!GATED && sg.part) {
+        // this warp's rows are finished by the last of the sharers' warps w to get here
         const int64_t U = p.units, G = gridDim.x, us = (int64_t)sg.strip * p.sps, ue = us + p.sps - 1;
         const int b_lo = (int)(((us + 1) * G + U - 1) / U) - 1, b_hi = (int)(((ue + 1) * G + U - 1) / U) - 1;
 #pragma unroll
@@ -453,11 +458,7 @@ w4_stream_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constant
         __threadfence();
         __syncwarp();
         int last = 0;
-        if (lane == 0) {
-          int* c = p.counters + sg.strip * BLOCKS + w;
-          last = atomicAdd(c, 1) == b_hi - b_lo;
-          if (last) *c = 0;                              // every contributor has arrived: ready for the next launch
-        }
+        if (lane == 0) last = arrivals_last(p.arrivals + sg.strip * BLOCKS + w, b_hi - b_lo);
         deliver = __shfl_sync(0xffffffffu, last, 0) != 0;
         if (deliver) {
           __threadfence();
@@ -518,44 +519,24 @@ static int sm_count() {
   return sms[dev];
 }
 
-// Launches take one of the banks in turn, so that launches that overlap in time do not share counters.
-static int* w4s_counter_bank() {
-  static thread_local int* basep[16] = {nullptr};
-  static std::atomic<unsigned> next_bank{0};
-  int dev = 0;
-  cudaGetDevice(&dev);
-  if (dev < 0 || dev >= 16) return nullptr;
-  if (!basep[dev]) {
-    void* p = nullptr;
-    if (cudaGetSymbolAddress(&p, g_w4s_counters) != cudaSuccess) return nullptr;
-    basep[dev] = reinterpret_cast<int*>(p);
-  }
-  return basep[dev] + (size_t)(next_bank.fetch_add(1, std::memory_order_relaxed) % W4S_BANKS) * W4S_MAX_STRIPS * 4;
-}
-
-int w4s_reset_state() {
-  void* p = nullptr;
-  if (cudaGetSymbolAddress(&p, g_w4s_counters) != cudaSuccess) return B2Q_ERR_CUDA;
-  return cuda_status(cudaMemset(p, 0, sizeof(int) * W4S_BANKS * W4S_MAX_STRIPS * 4));
-}
-
 // Stages are shared out evenly among all CTAs (two per SM) unless whole strips already keep 97 of 100 busy.
-struct W4SPlan { int strips, sps, grid; bool cut; size_t partial_bytes; };
-static W4SPlan plan(int64_t M, int64_t N, int64_t K) {
+struct W4SPlan { int strips, sps, grid; bool cut; size_t partial_bytes; };      // partial_bytes: sums, then arrival counts
+static size_t sum_bytes(int grid) { return (size_t)2 * grid * w4s::ROWS * 8 * sizeof(float); }      // two slots per CTA
+static W4SPlan plan(int64_t N, int64_t K) {
   W4SPlan pl{};
   const int slots = 2 * sm_count();
   const int64_t strips = (N + w4s::ROWS - 1) / w4s::ROWS, sps = (K + 255) / 256, units = strips * sps;
   pl.strips = (int)strips; pl.sps = (int)sps;
   pl.grid = (int)(strips < slots ? strips : slots);
-  if (strips > W4S_MAX_STRIPS || units > INT32_MAX / 4) return pl;
+  if (strips > UMMA_MAX_CUT_STRIPS || slots > ARRIVALS_MAX || units > INT32_MAX / 4) return pl;
   if ((double)strips / ((double)((strips + slots - 1) / slots) * slots) > 0.97 || units <= strips) return pl;
   pl.cut = true;
   pl.grid = (int)(units < slots ? units : slots);
-  pl.partial_bytes = (size_t)2 * pl.grid * w4s::ROWS * 8 * sizeof(float);        // two slots per CTA
+  pl.partial_bytes = sum_bytes(pl.grid) + (size_t)strips * w4s::BLOCKS * sizeof(Arrivals);
   return pl;
 }
 size_t w4_stream_partial_bytes(int64_t M, int64_t N, int64_t K) {
-  return M > 0 && M <= W4_STREAM_MAX_TOK && N > 0 && K > 0 ? plan(M, N, K).partial_bytes : 0;
+  return M > 0 && M <= W4_STREAM_MAX_TOK && N > 0 && K > 0 ? plan(N, K).partial_bytes : 0;
 }
 
 template <bool BF16, int SD, bool GATED>
@@ -595,7 +576,7 @@ bool w4_stream_preferred(int64_t M, int64_t N, int64_t K) {
 bool w4_stream_supported(const W4StreamArgs& a) {
   if (a.K <= 0 || (a.K % 128) != 0 || !aligned16(a.x) || !aligned16(a.w) || ((a.ldx * 2) & 15)) return false;
   if (a.layout != B2Q_W4_NMAJOR && a.layout != B2Q_W4_NMAJOR_S4) return false;
-  if (a.tile > W4_STREAM_MAX_TOK || (a.gated && (a.N % 2) != 0) || (a.shared_w && !aligned16(a.shared_w))) return false;
+  if (a.tile > W4_STREAM_MAX_TOK || (a.gated && ((a.N % 2) != 0 || !a.tiles)) || (a.shared_w && !aligned16(a.shared_w))) return false;
   return (int64_t)a.E * a.N <= INT32_MAX && tensor_map_encoder() != nullptr && umma_status_ptr() != nullptr;
 }
 
@@ -638,11 +619,11 @@ int w4_stream_linear(const W4StreamArgs& a, cudaStream_t st) {
   p.strips = a.gated ? (p.half + w4s::ROWS / 2 - 1) / (w4s::ROWS / 2) : (a.N + w4s::ROWS - 1) / w4s::ROWS;
   int64_t work = (int64_t)p.strips * (grouped ? a.tile_cap : 1);
   if (!grouped) {
-    const W4SPlan pl = plan(a.M, a.gated ? p.strips * w4s::ROWS : a.N, a.K);
+    const W4SPlan pl = plan(a.N, a.K);
     if (pl.cut && a.partials && aligned16(a.partials) && a.partial_bytes >= pl.partial_bytes) {
-      p.counters = w4s_counter_bank();
-      if (!p.counters) return B2Q_ERR_CUDA;
       p.units = pl.strips * pl.sps; p.partials = reinterpret_cast<float4*>(a.partials);
+      p.arrivals = reinterpret_cast<Arrivals*>(reinterpret_cast<uint8_t*>(a.partials) + sum_bytes(pl.grid)); p.tag = arrivals_tag(); p.epoch = arrivals_epoch();
+      if (!p.epoch) return B2Q_ERR_CUDA;
       work = pl.grid;
     }
   }
