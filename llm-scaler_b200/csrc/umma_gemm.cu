@@ -33,8 +33,6 @@ using namespace sm100;
 
 __device__ int g_umma_status = 0;
 __device__ Arrivals g_arrivals_epoch = 0;
-constexpr int SK_BANKS = 64, SK_MAX_STRIPS = UMMA_MAX_CUT_STRIPS;
-__device__ int g_sk_counters[SK_BANKS * SK_MAX_STRIPS];     // arrival counters of cut strips (see umma_strip_counters)
 
 enum { WK_W4N = 0, WK_W4K = 1, WK_W8 = 2 };
 enum { ST_XFULL = 101, ST_AFULL = 102, ST_EMPTY = 103, ST_RAWFULL = 104, ST_RAWEMPTY = 105, ST_ACCUM = 106, ST_FIXUP = 108 };
@@ -654,9 +652,6 @@ int umma_reset_status() {
   if (!p) return B2Q_ERR_CUDA;
   if (cudaDeviceSynchronize() != cudaSuccess) return B2Q_ERR_CUDA;
   if (cudaMemset(p, 0, sizeof(int)) != cudaSuccess) return B2Q_ERR_CUDA;
-  void* c = nullptr;
-  if (cudaGetSymbolAddress(&c, g_sk_counters) != cudaSuccess) return B2Q_ERR_CUDA;
-  if (cudaMemset(c, 0, sizeof(int) * SK_BANKS * SK_MAX_STRIPS) != cudaSuccess) return B2Q_ERR_CUDA;
   static std::atomic<Arrivals> resets{0};
   const Arrivals epoch = resets.fetch_add(1, std::memory_order_relaxed) + 1;
   if (cudaMemcpyToSymbol(g_arrivals_epoch, &epoch, sizeof(epoch)) != cudaSuccess) return B2Q_ERR_CUDA;
@@ -678,23 +673,6 @@ int umma_read_status(int* out) {
   return w4i_read_status(out);
 }
 
-
-// Arrival counters of cut strips.  They are zero whenever no launch is in flight (the last arriver of a
-// strip resets its counter), so nothing has to be cleared per launch; launches take one of 64 banks in turn
-// so that launches overlapping in time (other streams, programmatic dependent launch) do not share counters.
-int* umma_strip_counters() {
-  static thread_local int* basep[16] = {nullptr};
-  static std::atomic<unsigned> next_bank{0};
-  int dev = 0;
-  cudaGetDevice(&dev);
-  if (dev < 0 || dev >= 16) return nullptr;
-  if (!basep[dev]) {
-    void* p = nullptr;
-    if (cudaGetSymbolAddress(&p, g_sk_counters) != cudaSuccess) return nullptr;
-    basep[dev] = reinterpret_cast<int*>(p);
-  }
-  return basep[dev] + (size_t)(next_bank.fetch_add(1, std::memory_order_relaxed) % SK_BANKS) * SK_MAX_STRIPS;
-}
 
 static int pick_tok(int m) { return m <= 16 ? 16 : (m <= 32 ? 32 : (m <= 64 ? 64 : (m <= 128 ? 128 : 256))); }
 

@@ -109,10 +109,9 @@ bool umma_w8_strip_supported(const UmmaW8Args& a);
 int umma_w8_strip_linear(const UmmaW8Args& a, cudaStream_t st);
 size_t umma_w8_strip_partial_bytes(int64_t M, int64_t N, int64_t K);
 
-// shared by the weight-only kernels: the device's status word, and a bank of zeroed arrival counters for cut strips
+// shared by the weight-only kernels: the device's status word, and how many strips a launch may cut
 constexpr int UMMA_MAX_CUT_STRIPS = 1024;
 int* umma_status_ptr();
-int* umma_strip_counters();
 
 bool umma_w8_supported(const UmmaW8Args& a);
 int umma_w8_token_tile(const UmmaW8Args& a);

@@ -28,6 +28,7 @@
 // moe_prefill_up/down_forward_kernel (csrc/moe_prefill/moe_prefill_int4.sycl:121-395).
 #include "umma_gemm.cuh"
 #include "sm100.cuh"
+#include "arrivals.cuh"
 #include "smallm.cuh"   // lds128
 #include "peer_reduce.cuh"
 
@@ -98,7 +99,7 @@ struct W4Params {
   int strips, tiles_n;       // strips of R * 128 rows; token tiles of a dense launch
   int sps, units;            // cut strips: raw stages per strip and in total (0 = whole strips)
   float* partials;           // [2 * grid][R][TOK / 4][128][4] fp32 partial sums of cut strips
-  int* counters;             // arrivals per strip, zero between launches
+  Arrivals* arrivals; Arrivals tag; const Arrivals* epoch;      // [strips], in the partial sums' last slot (see cut_strips)
   const int32_t* tiles; const int32_t* expert_offsets; const int32_t* out_map;
   int w_rows_per_expert;     // tensor-map rows per expert: N (N-major) or K/8 (K-major)
   const float* tok_scale;    // per-token output multiplier (undoes the activation pre-scale)
@@ -488,6 +489,11 @@ umma_w4_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constant__
     bool ok = true;
     int segno = 0, fixn = 0, b = 0;
     uint32_t bpar = 0u;
+    if (p.units > 0 && warp == C::CW) {
+      grid_dep_wait();                             // the scratch may be an earlier launch's until then; activations come no sooner
+      if (lane < 2) arrivals_open(p.arrivals + (lane ? cur.u1 - 1 : cur.u0) / p.sps, p.tag, p.epoch);      // only a run's ends can be cut strips
+      __syncwarp();
+    }
     while (ok && cur.next(p, sg)) {
       ok = mbar_wait_warp(acc_full + 8 * b, bpar, abort_flag, p.status, ST_ACCUM);
       if (!ok) break;
@@ -622,10 +628,7 @@ umma_w4_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constant__
         if (!ok) break;
         if (leader) {
           __threadfence();
-          const int old = atomicAdd(p.counters + sg.strip, 1);
-          const int last = old == b_hi - b_lo;
-          if (last) p.counters[sg.strip] = 0;          // every contributor has arrived: ready for the next launch
-          *last_flag = last;
+          *last_flag = arrivals_last(p.arrivals + sg.strip, b_hi - b_lo);
           __threadfence();
         }
         ok = all_epilogue_warps();
@@ -845,13 +848,14 @@ static StripPlan plan_strips(int64_t M, int64_t N, int64_t K, int k_per_stage, b
   const int64_t strips = pl.R == 2 ? strips2 : (N + 127) / 128, units = strips * (K / k_per_stage);
   pl.strips = (int)strips;
   pl.grid = (int)(strips < sms ? strips : sms);
-  if (M > tok || (K % k_per_stage) != 0 || strips > UMMA_MAX_CUT_STRIPS || units > INT32_MAX) return pl;
+  if (M > tok || (K % k_per_stage) != 0 || strips > UMMA_MAX_CUT_STRIPS || sms > ARRIVALS_MAX || units > INT32_MAX) return pl;
   if ((double)strips / ((double)((strips + sms - 1) / sms) * sms) > 0.95) return pl;
   const bool w8 = k_per_stage == 128;
   const CutCost cost = tok == 128 ? CutCost{0.8, 4.0, 2.0} : (tok == 64 ? CutCost{w8 ? 0.46 : 0.54, 3.0, 1.0} : CutCost{w8 ? 0.35 : 0.5, 2.0, 0.75});
   const int grid = cut_grid(strips, K / k_per_stage, sms, cost);
   if (!grid) return pl;
   pl.sps = (int)(K / k_per_stage); pl.units = (int)units; pl.grid = grid;
+  static_assert(128 * 16 * sizeof(float) >= UMMA_MAX_CUT_STRIPS * sizeof(Arrivals), "a slot holds the arrival counts");
   pl.partial_bytes = (size_t)2 * pl.grid * pl.R * 128 * tok * sizeof(float);       // two slots per CTA
   return pl;
 }
@@ -886,13 +890,16 @@ static int launch_w4_tile(int tok, int R, const CUtensorMap& tw, const CUtensorM
   return R == 2 ? launch_w4<WT, 128, 2>(tw, tx, p, grid, overlap, st) : launch_w4<WT, 128, 1>(tw, tx, p, grid, overlap, st);
 }
 
-// Takes the plan's cut over where the caller's scratch holds its partial sums; without it every strip stays whole.
+// Takes the plan's cut over where the caller's scratch holds its partial sums; without it every strip stays whole.  The arrival counts
+// lie in the second slot of the last CTA, whose run ends with the last strip: what it has behind its first segment are whole strips.
 template <class Args>
 static int cut_strips(W4Params& p, const Args& a, const StripPlan& pl) {
   if (!pl.units || !a.sk_ws || !aligned16(a.sk_ws) || a.sk_ws_bytes < pl.partial_bytes || tls().force_kernel == 4) return B2Q_OK;
-  p.counters = umma_strip_counters();
-  if (!p.counters) return B2Q_ERR_CUDA;
+  p.epoch = arrivals_epoch();
+  if (!p.epoch) return B2Q_ERR_CUDA;
   p.sps = pl.sps; p.units = pl.units; p.partials = reinterpret_cast<float*>(a.sk_ws);
+  p.arrivals = reinterpret_cast<Arrivals*>(reinterpret_cast<uint8_t*>(a.sk_ws) + pl.partial_bytes / (2 * pl.grid) * (2 * pl.grid - 1));
+  p.tag = arrivals_tag();
   return B2Q_OK;
 }
 
