@@ -15,9 +15,9 @@
 // Reference counterpart: the per-channel / per-tensor FP8 GEMV and GEMM of
 // vllm/custom-esimd-kernels-vllm/csrc/xpu/esimd_kernels.sycl (esimd_gemv_fp8_pern, esimd_gemv_fp8_pert,
 // esimd_gemm_fp8_pern), which dequantise in registers and keep the activation in 16 bit.
-#include <atomic>
 #include "umma_gemm.cuh"
 #include "sm100.cuh"
+#include "arrivals.cuh"
 
 namespace b2q {
 
@@ -25,14 +25,8 @@ using namespace sm100;
 
 __device__ int g_w8d_status = 0;
 
-// Arrival counters of strips that are cut between CTAs: zero whenever no launch is in flight (the last
-// arriver of a strip resets its counter); launches take one of 64 banks in turn so that launches that
-// overlap in time (other streams, programmatic dependent launch) never share counters.
-constexpr int W8D_BANKS = 64, W8D_MAX_STRIPS = 2048;
-__device__ int g_w8d_counters[W8D_BANKS * W8D_MAX_STRIPS];
-
 namespace w8d {
-enum { ST_FULL = 301, ST_EMPTY = 302, ST_ACCUM = 303, ST_ACCEMPTY = 304, ST_FIXUP = 305 };
+enum { ST_FULL = 301, ST_EMPTY = 302, ST_ACCUM = 303, ST_FIXUP = 305 };
 
 template <int NTOK, bool DEEP = false> struct Cfg {
   static constexpr int W_BYTES = 16384;                                 // up to 128 rows x 128 k
@@ -44,13 +38,9 @@ template <int NTOK, bool DEEP = false> struct Cfg {
   static constexpr int NS = (NTOK <= 16 ? 6 : (NTOK == 32 ? 5 : (NTOK == 64 ? 4 : (NTOK == 128 ? 3 : 4)))) * (DEEP ? 2 : 1);
   static constexpr int SMEM = NS * STAGE + 1024 + 256;
   static constexpr int CTAS = NTOK <= 128 && !DEEP ? 2 : 1;
-  static constexpr int ACC_COLS = NTOK < 32 ? 32 : NTOK;                // two accumulators: the epilogue of one segment
-  static constexpr int TMEM_COLS = 2 * ACC_COLS;                        // runs under the MMAs of the next
+  static constexpr int TMEM_COLS = NTOK < 32 ? 32 : NTOK;
   static constexpr int THREADS = 7 * 32;                                // W TMA, MMA, X TMA, four epilogue warps
 };
-
-// One piece of a CTA's work: stages [st_begin, st_end) of 128 k of the strip of 128 weight rows at n0.
-struct Segment { int n0, strip, st_begin, st_end, part, slot, rot; };   // stage order: st_begin + (i + rot) % count
 }  // namespace w8d
 
 struct W8DParams {
@@ -59,9 +49,9 @@ struct W8DParams {
   void* out; int64_t ldo; int out_bf16;
   int M, Mp, NT, N, K;
   int e5m2;
-  int sps, ust, units;               // work units: units per strip, stages per unit, units in total
-  float* partials;                   // [grid][2 slots][Mp][128] fp32 sums of cut strips (terms already combined)
-  int* counters;                     // [strips]
+  int sps, ust;                      // pieces per strip (CTAs), stages of 128 k per piece
+  float* partials;                   // [grid][Mp][128] fp32 sums of cut strips (terms already combined)
+  Arrivals* arrivals; Arrivals tag; const Arrivals* epoch;      // [strips]
   int h;                             // weight rows per strip (a multiple of 8, at most 128)
   int* status;
 };
@@ -79,8 +69,8 @@ umma_w8_direct_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_con
   const uint32_t base = (smem_u32(smem_raw) + 1023u) & ~1023u;
   uint8_t* gen = smem_raw + (base - smem_u32(smem_raw));
   const uint32_t bar = base + NS * C::STAGE;
-  const uint32_t full = bar, empty = bar + 8 * NS, accum_full = bar + 16 * NS, accum_empty = accum_full + 16;
-  const uint32_t fix_bar = accum_empty + 16;
+  const uint32_t full = bar, empty = bar + 8 * NS, accum_full = bar + 16 * NS;
+  const uint32_t fix_bar = accum_full + 8;
   volatile uint32_t* tmem_slot = reinterpret_cast<volatile uint32_t*>(gen + (fix_bar + 8 - base));
   volatile int* abort_flag = reinterpret_cast<volatile int*>(gen + (fix_bar + 16 - base));
   volatile int* last_flag = reinterpret_cast<volatile int*>(gen + (fix_bar + 20 - base));
@@ -91,26 +81,15 @@ umma_w8_direct_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_con
   // the next kernel of the stream may start; this one waits for its predecessors only before it reads activations
   grid_dep_release();
 
-  // every role walks the same list of segments with its own copy of this cursor
-  const int u0 = (int)((int64_t)blockIdx.x * p.units / gridDim.x), u1 = (int)((int64_t)(blockIdx.x + 1) * p.units / gridDim.x);
-  int u = u0;
-  auto next_segment = [&](Segment& sg) -> bool {
-    if (u >= u1) return false;
-    const int strip = u / p.sps, r0 = u - strip * p.sps;
-    const int take = min(p.sps - r0, u1 - u);
-    sg.strip = strip; sg.n0 = strip * p.h;
-    sg.st_begin = r0 * p.ust; sg.st_end = min(nst, (r0 + take) * p.ust);
-    sg.part = take != p.sps; sg.slot = (u == u0) ? 0 : 1;
-    // Every CTA starts at a different stage: all CTAs read the same small activation array, and in step they would
-    // all ask the same L2 lines for it at the same moment.
-    sg.rot = (int)((blockIdx.x * 5u + (unsigned)strip) % (unsigned)(sg.st_end - sg.st_begin));
-    u += take;
-    return true;
-  };
+  const int strip = blockIdx.x / p.sps, n0 = strip * p.h, st_begin = (blockIdx.x - strip * p.sps) * p.ust, cnt = min(nst, st_begin + p.ust) - st_begin;
+  const bool part = p.sps > 1;
+  // Every CTA starts at a different stage: all CTAs read the same small activation array, and in step they would
+  // all ask the same L2 lines for it at the same moment.
+  const int rot = (int)((blockIdx.x * 5u + (unsigned)strip) % (unsigned)cnt);
 
   if (threadIdx.x == 0) {
     for (int i = 0; i < NS; ++i) { mbar_init(full + 8 * i, 2); mbar_init(empty + 8 * i, 1); }
-    for (int i = 0; i < 2; ++i) { mbar_init(accum_full + 8 * i, 1); mbar_init(accum_empty + 8 * i, 128); }
+    mbar_init(accum_full, 1);
     mbar_init(fix_bar, 128);
     *abort_flag = 0;
     fence_barrier_init();
@@ -120,89 +99,70 @@ umma_w8_direct_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_con
   __syncthreads();
   tc_fence_after();
   const uint32_t tmem = *tmem_slot;
-  Segment sg;
 
   if (warp == 0) {
     // ---- weight producer: one 128 x 128 box per stage ----
     if (elect_one()) {
       tma_prefetch_desc(&tm_w);
-      int g = 0;
-      bool ok = true;
-      while (ok && next_segment(sg)) {
-        const int cnt = sg.st_end - sg.st_begin;
-        for (int i = 0; i < cnt; ++i, ++g) {
-          const int r = sg.st_begin + (i + sg.rot) % cnt;
-          const int s = g % NS;
-          if (g >= NS && !mbar_wait(empty + 8 * s, ((g / NS) - 1) & 1, abort_flag, p.status, ST_EMPTY)) { ok = false; break; }
-          mbar_expect_tx(full + 8 * s, p.h * 128);
-          tma_load_2d(base + s * C::STAGE, &tm_w, r * 128, sg.n0, full + 8 * s);
-        }
+      for (int g = 0; g < cnt; ++g) {
+        const int r = st_begin + (g + rot) % cnt, s = g % NS;
+        if (g >= NS && !mbar_wait(empty + 8 * s, ((g / NS) - 1) & 1, abort_flag, p.status, ST_EMPTY)) { drain_issued(full, NS, g); break; }
+        mbar_expect_tx(full + 8 * s, p.h * 128);
+        tma_load_2d(base + s * C::STAGE, &tm_w, r * 128, n0, full + 8 * s);
       }
-      if (!ok) drain_issued(full, NS, g);
     }
   } else if (warp == 2) {
     // ---- activation producer: the NTOK term rows of the same 128 k ----
     if (elect_one()) {
       tma_prefetch_desc(&tm_x);
       grid_dep_wait();
-      int g = 0;
-      bool ok = true;
-      while (ok && next_segment(sg)) {
-        const int cnt = sg.st_end - sg.st_begin;
-        for (int i = 0; i < cnt; ++i, ++g) {
-          const int r = sg.st_begin + (i + sg.rot) % cnt;
-          const int s = g % NS;
-          if (g >= NS && !mbar_wait(empty + 8 * s, ((g / NS) - 1) & 1, abort_flag, p.status, ST_EMPTY)) { ok = false; break; }
-          mbar_expect_tx(full + 8 * s, C::X_BYTES);
-          tma_load_2d(base + s * C::STAGE + C::W_BYTES, &tm_x, r * 128, 0, full + 8 * s);
-        }
+      for (int g = 0; g < cnt; ++g) {
+        const int r = st_begin + (g + rot) % cnt, s = g % NS;
+        if (g >= NS && !mbar_wait(empty + 8 * s, ((g / NS) - 1) & 1, abort_flag, p.status, ST_EMPTY)) { drain_issued(full, NS, g); break; }
+        mbar_expect_tx(full + 8 * s, C::X_BYTES);
+        tma_load_2d(base + s * C::STAGE + C::W_BYTES, &tm_x, r * 128, 0, full + 8 * s);
       }
-      if (!ok) drain_issued(full, NS, g);
     }
   } else if (warp == 1) {
     // ---- MMA issuer ----
     if (elect_one()) {
       const uint32_t idesc = instr_desc(p.e5m2 ? 1u : 0u, 0u, 128, NTOK);
       bool ok = true;
-      int g = 0, si = 0;
-      while (ok && next_segment(sg)) {
-        const int buf = si & 1;
-        if (si >= 2) { ok = mbar_wait(accum_empty + 8 * buf, ((si >> 1) - 1) & 1, abort_flag, p.status, ST_ACCEMPTY); if (!ok) break; }
-        const uint32_t d = tmem + buf * C::ACC_COLS;
 #pragma unroll 1
-        for (int r = sg.st_begin; r < sg.st_end; ++r, ++g) {
-          const int s = g % NS;
-          ok = mbar_wait(full + 8 * s, (g / NS) & 1, abort_flag, p.status, ST_FULL);
-          if (!ok) break;
-          tc_fence_after();
-          const uint64_t da = smem_desc_sw128(base + s * C::STAGE);
-          const uint64_t db = smem_desc_sw128(base + s * C::STAGE + C::W_BYTES);
-          mma_f8(d, da, db, idesc, r > sg.st_begin ? 1u : 0u);
-          mma_f8(d, da + 2, db + 2, idesc, 1u);
-          mma_f8(d, da + 4, db + 4, idesc, 1u);
-          mma_f8(d, da + 6, db + 6, idesc, 1u);
-          tc_commit(empty + 8 * s);
-        }
-        if (ok) tc_commit(accum_full + 8 * buf);
-        ++si;
+      for (int g = 0; g < cnt; ++g) {
+        const int s = g % NS;
+        ok = mbar_wait(full + 8 * s, (g / NS) & 1, abort_flag, p.status, ST_FULL);
+        if (!ok) break;
+        tc_fence_after();
+        const uint64_t da = smem_desc_sw128(base + s * C::STAGE);
+        const uint64_t db = smem_desc_sw128(base + s * C::STAGE + C::W_BYTES);
+        mma_f8(tmem, da, db, idesc, g > 0 ? 1u : 0u);
+        mma_f8(tmem, da + 2, db + 2, idesc, 1u);
+        mma_f8(tmem, da + 4, db + 4, idesc, 1u);
+        mma_f8(tmem, da + 6, db + 6, idesc, 1u);
+        tc_commit(empty + 8 * s);
       }
+      if (ok) tc_commit(accum_full);
     }
   } else {
     // ---- epilogue: warps 3..6, lane quadrant = warp & 3; a thread owns one weight row ----
     const int quad = warp & 3, rowi = quad * 32 + lane;
     uint16_t* outp = reinterpret_cast<uint16_t*>(p.out);
-    bool ok = true;
-    int si = 0, fixn = 0;
-    while (ok && next_segment(sg)) {
-      const int buf = si & 1;
-      ok = mbar_wait_warp(accum_full + 8 * buf, (si >> 1) & 1, abort_flag, p.status, ST_ACCUM);
-      if (!ok) break;
+    const bool leader = warp == 3 && lane == 0;
+    if (part && leader) {
+      grid_dep_wait();                             // the scratch may be an earlier launch's until then; activations come no sooner
+      arrivals_open(p.arrivals + strip, p.tag, p.epoch);
+    }
+    __syncwarp();
+    bool ok = mbar_wait_warp(accum_full, 0, abort_flag, p.status, ST_ACCUM);
+    if (ok) {
       tc_fence_after();
-      const int n = sg.n0 + rowi;
+      const int n = n0 + rowi;
       const int nn = n < p.N ? n : p.N - 1;
       const float sw = load_scalar(p.scale, p.scale_per_channel ? nn : 0, p.scale_dtype);
-      const uint32_t trow = tmem + ((uint32_t)(quad * 32) << 16) + buf * C::ACC_COLS;
-      float* const my_part = p.partials + ((size_t)(blockIdx.x * 2 + sg.slot) * p.Mp) * 128 + rowi;
+      const uint32_t trow = tmem + ((uint32_t)(quad * 32) << 16);
+      auto part_of = [&](int cta) { return p.partials + ((size_t)cta * p.Mp) * 128 + rowi; };
+      float* const my_part = part_of(blockIdx.x);
       auto write_out = [&](const float (&v)[8], int m0) {
         // token scales of this block of eight: one load per lane, past L1 (it may still hold the previous call's
         // scales at this address), handed round the warp by shuffle
@@ -232,62 +192,47 @@ umma_w8_direct_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_con
           v[i] = __uint_as_float(a[i]) + __uint_as_float(b[i]) * 0.0625f;
           if (p.NT == 3) v[i] += __uint_as_float(c[i]) * 0.00390625f;
         }
-        if (!sg.part) {
+        if (!part) {
           write_out(v, m0);
         } else {
 #pragma unroll
           for (int i = 0; i < 8; ++i) __stcg(my_part + (m0 + i) * 128, v[i]);
         }
       }
-      tc_fence_before();
-      mbar_arrive(accum_empty + 8 * buf);          // the MMAs of the segment after next may overwrite this accumulator
-      if (sg.part) {
-        const int64_t U = p.units, G = gridDim.x;
-        const int64_t us = (int64_t)sg.strip * p.sps, ue = us + p.sps - 1;
-        const int b_lo = (int)(((us + 1) * G + U - 1) / U) - 1, b_hi = (int)(((ue + 1) * G + U - 1) / U) - 1;
+      if (part) {
         mbar_arrive(fix_bar);          // hands this thread's partial sums to the leader, whose fence orders them before the count
-        ok = mbar_wait_warp(fix_bar, fixn & 1, abort_flag, p.status, ST_FIXUP); ++fixn;
-        if (!ok) break;
-        if (threadIdx.x == 3 * 32) {
-          __threadfence();                             // orders the partial sums of all 128 threads before the count
-          const int old = atomicAdd(p.counters + sg.strip, 1);
-          const int last = old == b_hi - b_lo;
-          if (last) p.counters[sg.strip] = 0;        // every contributor has arrived: ready for the next launch
-          *last_flag = last;
+        ok = mbar_wait_warp(fix_bar, 0, abort_flag, p.status, ST_FIXUP);
+        if (ok) {
+          if (leader) {
+            __threadfence();                           // orders the partial sums of all 128 threads before the count
+            *last_flag = arrivals_last(p.arrivals + strip, p.sps - 1);
+          }
+          mbar_arrive(fix_bar);
+          ok = mbar_wait_warp(fix_bar, 1, abort_flag, p.status, ST_FIXUP);
         }
-        mbar_arrive(fix_bar);
-        ok = mbar_wait_warp(fix_bar, fixn & 1, abort_flag, p.status, ST_FIXUP); ++fixn;
-        if (!ok) break;
-        if (*last_flag) {
+        if (ok && *last_flag) {
           __threadfence();
 #pragma unroll 1
           for (int m0 = 0; m0 < p.M; m0 += 8) {
-            float v[8];
+            // the sums of all pieces, four at most, in flight at once: a trip through L2 per eight tokens, not one per piece
+            float t[4][8], v[8];
+#pragma unroll
+            for (int q = 0; q < 4; ++q) {
+              const float* src = part_of(strip * p.sps + min(q, p.sps - 1));
+#pragma unroll
+              for (int i = 0; i < 8; ++i) t[q][i] = __ldcg(src + (m0 + i) * 128);
+            }
 #pragma unroll
             for (int i = 0; i < 8; ++i) v[i] = 0.f;
-            // all contributors' loads in flight at once: a trip through L2 per eight tokens, not one per contributor
-#pragma unroll 1
-            for (int b0 = b_lo; b0 <= b_hi; b0 += 4) {
-              float t[4][8];
 #pragma unroll
-              for (int q = 0; q < 4; ++q) {
-                const int b = min(b0 + q, b_hi);
-                const int64_t bu0 = (int64_t)b * U / G;
-                const float* src = p.partials + ((size_t)(b * 2 + (bu0 >= us ? 0 : 1)) * p.Mp) * 128 + rowi;
+            for (int q = 0; q < 4; ++q)
+              if (q < p.sps)
 #pragma unroll
-                for (int i = 0; i < 8; ++i) t[q][i] = __ldcg(src + (m0 + i) * 128);
-              }
-#pragma unroll
-              for (int q = 0; q < 4; ++q)
-                if (b0 + q <= b_hi)
-#pragma unroll
-                  for (int i = 0; i < 8; ++i) v[i] += t[q][i];
-            }
+                for (int i = 0; i < 8; ++i) v[i] += t[q][i];
             write_out(v, m0);
           }
         }
       }
-      ++si;
     }
   }
   tc_fence_before();
@@ -313,24 +258,9 @@ static int sm_count() {
   return sms[dev];
 }
 
-static int* w8d_counter_bank() {
-  static thread_local int* basep[16] = {nullptr};
-  static std::atomic<unsigned> next_bank{0};
-  int dev = 0;
-  cudaGetDevice(&dev);
-  if (dev < 0 || dev >= 16) return nullptr;
-  if (!basep[dev]) {
-    void* p = nullptr;
-    if (cudaGetSymbolAddress(&p, g_w8d_counters) != cudaSuccess) return nullptr;
-    basep[dev] = reinterpret_cast<int*>(p);
-  }
-  return basep[dev] + (size_t)(next_bank.fetch_add(1, std::memory_order_relaxed) % W8D_BANKS) * W8D_MAX_STRIPS;
-}
-
-// fp32 partial sums: [up to two CTAs per SM][2 slots][M rounded up to 8][128 rows]
-size_t umma_w8_direct_partial_bytes(int64_t M) {
-  return (size_t)sm_count() * 2 * 2 * (size_t)((M + 7) / 8 * 8) * 128 * sizeof(float);
-}
+// [a CTA per SM at most][M rounded up to 8][128 rows] fp32 partial sums, then a count per strip
+static size_t sum_bytes(int64_t M) { return (size_t)sm_count() * (size_t)((M + 7) / 8 * 8) * 128 * sizeof(float); }
+size_t umma_w8_direct_partial_bytes(int64_t M) { return sum_bytes(M) + (size_t)sm_count() * sizeof(Arrivals); }
 
 // Rows per strip (a multiple of 8 up to 128) that minimise the rows the busiest SM has to stream when the
 // strips are dealt out evenly; ties go to the taller strip.
@@ -389,11 +319,15 @@ int umma_w8_direct_linear(const UmmaW8DirectArgs& a, cudaStream_t st) {
   const int strips = (a.N + p.h - 1) / p.h;
   rc = make_tmap_2d(&tw, CU_TENSOR_MAP_DATA_TYPE_UINT8, 1, a.w, a.N, a.K, (uint64_t)a.K, p.h, 128, CU_TENSOR_MAP_SWIZZLE_128B);
   if (rc) return rc;
-  p.ust = cut ? (nst + pieces - 1) / pieces : nst; p.sps = (nst + p.ust - 1) / p.ust; p.units = strips * p.sps;
+  p.ust = cut ? (nst + pieces - 1) / pieces : nst; p.sps = (nst + p.ust - 1) / p.ust;
   p.partials = reinterpret_cast<float*>(a.partials);
-  p.counters = cut ? w8d_counter_bank() : nullptr;
-  if (cut && !p.counters) return B2Q_ERR_CUDA;
-  const int grid = p.units;
+  if (cut) {
+    p.arrivals = reinterpret_cast<Arrivals*>(reinterpret_cast<uint8_t*>(a.partials) + sum_bytes(a.M));
+    p.tag = arrivals_tag();
+    p.epoch = arrivals_epoch();
+    if (!p.epoch) return B2Q_ERR_CUDA;
+  }
+  const int grid = strips * p.sps;
   const bool overlap = tls().overlap_mode > 0;     // always directly behind its own pre-pass
   const bool deep = grid <= sms && ntok <= 128;
   if (deep) switch (ntok) {
@@ -414,9 +348,7 @@ int umma_w8_direct_linear(const UmmaW8DirectArgs& a, cudaStream_t st) {
 int w8d_reset_state() {
   void* p = nullptr;
   if (cudaGetSymbolAddress(&p, g_w8d_status) != cudaSuccess) return B2Q_ERR_CUDA;
-  if (cudaMemset(p, 0, sizeof(int)) != cudaSuccess) return B2Q_ERR_CUDA;
-  if (cudaGetSymbolAddress(&p, g_w8d_counters) != cudaSuccess) return B2Q_ERR_CUDA;
-  return cuda_status(cudaMemset(p, 0, sizeof(int) * W8D_BANKS * W8D_MAX_STRIPS));
+  return cuda_status(cudaMemset(p, 0, sizeof(int)));
 }
 int w8d_read_status(int* out) { return cuda_status(cudaMemcpyFromSymbol(out, g_w8d_status, sizeof(int))); }
 

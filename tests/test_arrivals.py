@@ -7,7 +7,7 @@ import re
 import pytest
 
 CSRC = os.path.join(os.path.dirname(os.path.dirname(os.path.abspath(__file__))), "llm-scaler_b200", "csrc")
-SOURCES = ["w4_stream.cu", "umma_w4.cu"]
+SOURCES = ["w4_stream.cu", "umma_w4.cu", "umma_w8_direct.cu"]
 BITS = 10
 MAX = (1 << BITS) - 1
 

@@ -54,7 +54,8 @@ class Linear:
 # kernel, force, kind, M, N, K; the scratch holds partial sums for each of them
 CUT = [("w4_stream", 7, "int4", 1, 2048, 16384), ("w4_stream", 7, "int4", 8, 520, 8192), ("w4_stream", 7, "int4", 5, 57344, 512),
        ("umma_w4", 2, "int4", 16, 2048, 14336), ("umma_w4", 2, "int4", 40, 520, 14336), ("umma_w4", 2, "int4", 64, 40960, 4096), ("umma_w4", 2, "int4", 100, 8192, 28672),
-       ("umma_w4", 2, "block", 27, 8192, 14336), ("umma_w4", 2, "block", 64, 1000, 14336)]
+       ("umma_w4", 2, "block", 27, 8192, 14336), ("umma_w4", 2, "block", 64, 1000, 14336),
+       ("umma_w8_direct", 0, "fp8", 20, 5120, 13824), ("umma_w8_direct", 0, "fp8", 33, 520, 8192), ("umma_w8_direct", 0, "fp8", 64, 9400, 14336)]
 
 
 @pytest.mark.parametrize("name,force,kind,M,N,K", CUT)
