@@ -446,10 +446,11 @@ B2Q_API int b2q_moe_forward_fp8(const b2q_moe_fp8* args, void* workspace, size_t
 /* Code of the first bounded device-side wait that expired since the library was loaded
  * (0 = none).  Synchronises the device; meant for tests and post-mortems.       */
 B2Q_API int b2q_device_status(int* out);
-/* Clears that code on the current device: the status words of every kernel family, and the arrival
- * counters of strips cut between CTAs (a CTA that gave up never delivered its arrival, so a stale
- * counter would make a later launch finish that strip early).  Synchronises the device first; call
- * it with no launch of this library in flight, once per device that reported a code.           */
+/* Clears that code on the current device: the status words of every kernel family.  It also invalidates
+ * the arrival counts of strips cut between CTAs, which lie in the callers' scratch: a CTA that gave up
+ * never delivered its arrival, and a replay of its graph would finish that strip early.  Synchronises
+ * the device first; call it with no launch of this library in flight, once per device that reported a
+ * code.                                                                                        */
 B2Q_API int b2q_device_status_reset(void);
 /* Self-test of the bounded waits: launches one CTA that waits, with a limit of about a millisecond,
  * on a barrier nobody arrives on.  The wait gives up, records `code` (> 0) as the device status and

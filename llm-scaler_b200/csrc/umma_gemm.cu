@@ -643,9 +643,9 @@ int w8a8_reset_state();
 int w8d_reset_state();
 int w4i_reset_state();
 
-// Clears, on the current device, the status word of every tcgen05 kernel family and the arrival counters of cut
-// strips.  A CTA that gave up on a wait never delivered its arrival, so its strip's counter is left non-zero and the
-// next launch that takes the same bank would finish that strip one arrival early: status and counters go together.
+// Clears, on the current device, the status word of every tcgen05 kernel family, and changes the word that the tags of arrival counts
+// are mixed with.  A CTA that gave up on a wait never delivered its arrival, so its strip's count is left non-zero, and a
+// replay of the same graph would finish that strip one arrival early: status and counts go together.
 // The device must be idle (the call synchronises it first).
 int umma_reset_status() {
   int* p = status_ptr();

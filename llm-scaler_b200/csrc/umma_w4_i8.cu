@@ -22,18 +22,16 @@
 //
 // Reference counterpart: esimd_gemv_int4 / esimd_gemm_int4_pgrp
 // (vllm/custom-esimd-kernels-vllm/csrc/xpu/esimd_kernels/gemv_int4.h, gemm_int4_pgrp.h), GGML N-major weights.
-#include <atomic>
 #include "umma_gemm.cuh"
 #include "sm100.cuh"
 #include "smallm.cuh"   // lds128
+#include "arrivals.cuh"
 
 namespace b2q {
 
 using namespace sm100;
 
 __device__ int g_w4i_status = 0;
-constexpr int W4I_BANKS = 64, W4I_MAX_STRIPS = 2048;
-__device__ int g_w4i_counters[W4I_BANKS * W4I_MAX_STRIPS];
 
 namespace w4i {
 enum { ST_RAWFULL = 401, ST_RAWEMPTY = 402, ST_XFULL = 403, ST_XEMPTY = 404, ST_AFULL = 405, ST_AEMPTY = 406,
@@ -65,7 +63,8 @@ struct W4IParams {
   uint32_t xor_mask;                 // 0x88888888 for two's-complement nibbles
   int h;                             // weight rows per strip
   int sps, ust, units;               // units per strip, raw stages per unit, units in total
-  float* partials; int* counters;
+  float* partials;                   // [grid][2 slots][16][128] fp32 sums of cut strips
+  Arrivals* arrivals; Arrivals tag; const Arrivals* epoch;      // [strips]
   int* status;
 };
 
@@ -247,6 +246,10 @@ umma_w4_i8_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constan
     int gc = 0, fixn = 0;
     bool ok = true;
     grid_dep_wait();                                   // reads what the pre-pass wrote (activation sums, token scales)
+    if (p.arrivals && warp == 4) {                     // only a run's ends can be cut strips
+      if (lane < 2 && u1 > u0) arrivals_open(p.arrivals + (lane ? u1 - 1 : u0) / p.sps, p.tag, p.epoch);
+      __syncwarp();
+    }
     while (ok && next_segment(sg)) {
       const int n = sg.n0 + rowi;
       const int nn = n < p.N ? n : p.N - 1;
@@ -342,10 +345,7 @@ umma_w4_i8_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constan
         if (!ok) break;
         if (threadIdx.x == 4 * 32) {
           __threadfence();
-          const int old = atomicAdd(p.counters + sg.strip, 1);
-          const int last = old == b_hi - b_lo;
-          if (last) p.counters[sg.strip] = 0;
-          *last_flag = last;
+          *last_flag = arrivals_last(p.arrivals + sg.strip, b_hi - b_lo);
         }
         mbar_arrive(fix_bar);
         ok = mbar_wait_warp(fix_bar, fixn & 1, abort_flag, p.status, ST_FIXUP); ++fixn;
@@ -387,24 +387,11 @@ static int w4i_sm_count() {
   return sms[dev];
 }
 
-static int* w4i_counter_bank() {
-  static thread_local int* basep[16] = {nullptr};
-  static std::atomic<unsigned> next_bank{0};
-  int dev = 0;
-  cudaGetDevice(&dev);
-  if (dev < 0 || dev >= 16) return nullptr;
-  if (!basep[dev]) {
-    void* p = nullptr;
-    if (cudaGetSymbolAddress(&p, g_w4i_counters) != cudaSuccess) return nullptr;
-    basep[dev] = reinterpret_cast<int*>(p);
-  }
-  return basep[dev] + (size_t)(next_bank.fetch_add(1, std::memory_order_relaxed) % W4I_BANKS) * W4I_MAX_STRIPS;
-}
-
 // term rows of the activation buffer: three terms x (M rounded up to 8), as a legal MMA N
 int umma_w4_i8_rows(int64_t M) { return M <= 8 ? 32 : 64; }
 
-// fp32 partial sums of cut strips: [two CTAs per SM][2 slots][16][128]
+// fp32 partial sums of cut strips: [two CTAs per SM][2 slots][16][128].  The last CTA's run ends with the last strip, so what it has behind
+// its first segment are whole strips: its second slot holds the arrival counts.
 size_t umma_w4_i8_partial_bytes() { return (size_t)w4i_sm_count() * 2 * 2 * 16 * 128 * sizeof(float); }
 
 static int w4i_pick_strip_rows(int N, int sms) {
@@ -446,15 +433,18 @@ int umma_w4_i8_linear(const UmmaW4I8Args& a, cudaStream_t st) {
   if (cudaGetSymbolAddress(&sym, g_w4i_status) != cudaSuccess) return B2Q_ERR_CUDA;
   p.status = reinterpret_cast<int*>(sym);
   const int sms = w4i_sm_count(), slots = 2 * sms, nst = (a.K + 255) / 256;
-  const bool cut = ((a.N + 127) / 128) * 2 <= sms && a.partials && a.partial_bytes >= umma_w4_i8_partial_bytes() &&
-                   (a.N + 127) / 128 <= W4I_MAX_STRIPS;
+  const bool cut = ((a.N + 127) / 128) * 2 <= sms && a.partials && a.partial_bytes >= umma_w4_i8_partial_bytes() && slots <= ARRIVALS_MAX;
   p.h = cut ? 128 : w4i_pick_strip_rows(a.N, sms);
   const int strips = (a.N + p.h - 1) / p.h;
   p.ust = cut ? 1 : nst; p.sps = cut ? nst : 1; p.units = strips * p.sps;
   p.partials = reinterpret_cast<float*>(a.partials);
-  p.counters = cut ? w4i_counter_bank() : nullptr;
-  if (cut && !p.counters) return B2Q_ERR_CUDA;
   const int grid = cut ? (p.units < slots ? p.units : slots) : strips;
+  if (cut) {
+    p.arrivals = reinterpret_cast<Arrivals*>(p.partials + (size_t)(2 * grid - 1) * 16 * 128);
+    p.tag = arrivals_tag();
+    p.epoch = arrivals_epoch();
+    if (!p.epoch) return B2Q_ERR_CUDA;
+  }
   CUtensorMap tw, tx;
   int rc = make_tmap_2d(&tw, CU_TENSOR_MAP_DATA_TYPE_UINT8, 1, a.w, a.N, a.K / 2, (uint64_t)a.K / 2, p.h, 128, CU_TENSOR_MAP_SWIZZLE_128B);
   if (rc) return rc;
@@ -468,9 +458,7 @@ int umma_w4_i8_linear(const UmmaW4I8Args& a, cudaStream_t st) {
 int w4i_reset_state() {
   void* p = nullptr;
   if (cudaGetSymbolAddress(&p, g_w4i_status) != cudaSuccess) return B2Q_ERR_CUDA;
-  if (cudaMemset(p, 0, sizeof(int)) != cudaSuccess) return B2Q_ERR_CUDA;
-  if (cudaGetSymbolAddress(&p, g_w4i_counters) != cudaSuccess) return B2Q_ERR_CUDA;
-  return cuda_status(cudaMemset(p, 0, sizeof(int) * W4I_BANKS * W4I_MAX_STRIPS));
+  return cuda_status(cudaMemset(p, 0, sizeof(int)));
 }
 int w4i_read_status(int* out) { return cuda_status(cudaMemcpyFromSymbol(out, g_w4i_status, sizeof(int))); }
 

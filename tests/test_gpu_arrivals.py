@@ -55,7 +55,8 @@ class Linear:
 CUT = [("w4_stream", 7, "int4", 1, 2048, 16384), ("w4_stream", 7, "int4", 8, 520, 8192), ("w4_stream", 7, "int4", 5, 57344, 512),
        ("umma_w4", 2, "int4", 16, 2048, 14336), ("umma_w4", 2, "int4", 40, 520, 14336), ("umma_w4", 2, "int4", 64, 40960, 4096), ("umma_w4", 2, "int4", 100, 8192, 28672),
        ("umma_w4", 2, "block", 27, 8192, 14336), ("umma_w4", 2, "block", 64, 1000, 14336),
-       ("umma_w8_direct", 0, "fp8", 20, 5120, 13824), ("umma_w8_direct", 0, "fp8", 33, 520, 8192), ("umma_w8_direct", 0, "fp8", 64, 9400, 14336)]
+       ("umma_w8_direct", 0, "fp8", 20, 5120, 13824), ("umma_w8_direct", 0, "fp8", 33, 520, 8192), ("umma_w8_direct", 0, "fp8", 64, 9400, 14336),
+       ("umma_w4_i8", 5, "int4", 8, 2048, 14336), ("umma_w4_i8", 5, "int4", 16, 8200, 1024)]
 
 
 @pytest.mark.parametrize("name,force,kind,M,N,K", CUT)
@@ -132,3 +133,26 @@ def test_streams_and_graphs_side_by_side(e, name, force, kind, M, N, K):
         for lin, ref in zip(lins, refs):
             assert torch.equal(lin.out, ref)
     assert e._lib.device_status() == 0
+
+
+def test_reset_invalidates_counts_that_are_half_full(e):
+    """What a launch leaves behind in which a wait ran out, and a replay of its graph finds: counts with its own tag and an arrival too many.
+    After the reset they are nobody's.  (The tag is read off the counts of strips that one CTA has alone: opened, and never added to.)"""
+    e.set_force_kernel(7)
+    M, N, K = 5, 57344, 512
+    lin = Linear(e, "int4", M, N, K, 6)
+    graph = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(graph):
+        lin.run()
+    graph.replay()
+    ref = lin.out.clone()
+    grid = 2 * torch.cuda.get_device_properties(0).multi_processor_count
+    counts = lin.ws[2 * grid * 4096:2 * grid * 4096 + N // 128 * 4 * 8].view(torch.int64)
+    tags = counts[counts != 0].unique()
+    assert tags.numel() == 1 and int(tags[0]) & 1023 == 0
+    counts.fill_(int(tags[0]) + 1)
+    e._lib.device_status_reset()
+    lin.out.fill_(float("nan"))
+    graph.replay()
+    torch.cuda.synchronize()
+    assert torch.equal(lin.out, ref) and e._lib.device_status() == 0
