@@ -821,7 +821,13 @@ int b2q_moe_forward_int4(const b2q_moe_int4* a, void* workspace, size_t workspac
   if (rc) return rc;
   if (!a->w13 || !a->s13 || !a->w2 || !a->s2) return B2Q_ERR_NULL;
   if (shared && (!a->shared_s13 || !a->shared_w2 || !a->shared_s2 || !a->gate_w)) return B2Q_ERR_NULL;
+  // what the steps below would refuse on their own, before any of them is launched; gate_w is read 16 bytes at a time
+  auto known = [](int dtype) { return dtype >= 0 && dtype <= 2; };
+  if (!known(a->s13_dtype) || !known(a->s2_dtype) || (shared && (!known(a->shared_s13_dtype) || !known(a->shared_s2_dtype)))) return B2Q_ERR_DTYPE;
+  if (a->layout < 0 || a->layout > 3 || (shared && (a->shared_layout < 0 || a->shared_layout > 3))) return B2Q_ERR_LAYOUT;
   if ((H % 128) != 0 || (I % 128) != 0 || (shared && (Is <= 0 || (Is % 128) != 0))) return B2Q_ERR_SHAPE;
+  if (!aligned16(a->w13) || !aligned16(a->w2) || (shared && (!aligned16(a->shared_w13) || !aligned16(a->shared_w2) || !aligned16(a->gate_w))))
+    return B2Q_ERR_ALIGN;
   if (T == 0) return B2Q_OK;
   cudaStream_t st = (cudaStream_t)stream;
   const MoeParts p = moe_parts(workspace, T, E, k, H, I, Is);
@@ -888,6 +894,8 @@ int b2q_moe_forward_fp8(const b2q_moe_fp8* a, void* workspace, size_t workspace_
   int rc = moe_check(a->x, a->logits, a->act_dtype, a->logits_dtype, T, a->E, a->top_k, H, I, a->out, workspace, workspace_bytes, need);
   if (rc) return rc;
   if (!a->w13 || !a->s13 || !a->w2 || !a->s2) return B2Q_ERR_NULL;
+  if (a->fp8_format != B2Q_E4M3 && a->fp8_format != B2Q_E5M2) return B2Q_ERR_DTYPE;
+  if (!aligned16(a->w13) || !aligned16(a->w2)) return B2Q_ERR_ALIGN;
   if (T == 0) return B2Q_OK;
   cudaStream_t st = (cudaStream_t)stream;
   const MoeParts p = moe_parts(workspace, T, E, k, H, I, 0);

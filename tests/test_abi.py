@@ -153,3 +153,40 @@ def test_cpp_op_library_loads_and_registers_the_dense_linears(lib_built):
     with pytest.raises((RuntimeError, NotImplementedError)):
         torch.ops.custom_esimd_kernels_vllm.esimd_gemv_int4(x, torch.zeros(8, 64, dtype=torch.uint8), torch.zeros(8, 1, dtype=torch.bfloat16),
                                                             torch.zeros(1, 8, dtype=torch.bfloat16))
+
+
+def _expert_layer(L, kind):
+    """Arguments of a whole expert layer at addresses that nothing reads: every call below is refused, and refused before a launch."""
+    at = iter(range(1 << 20, 1 << 30, 1 << 12))
+    if kind == "fp8":
+        a = L.MoeFp8(T=1, E=8, top_k=2, H=128, I=128)
+        names = ("x", "logits", "w13", "s13", "w2", "s2", "out")
+    else:
+        a = L.MoeInt4(T=1, E=8, top_k=2, H=128, I=128, shared_I=128)
+        names = ("x", "logits", "w13", "s13", "w2", "s2", "shared_w13", "shared_s13", "shared_w2", "shared_s2", "gate_w", "out")
+    for n in names:
+        setattr(a, n, next(at))
+    call = getattr(L.lib, "b2q_moe_forward_" + kind)
+    return a, lambda: call(a, 1 << 30, 1 << 30, None)
+
+
+@pytest.mark.parametrize("kind,pointer", [("int4", n) for n in ("x", "out", "w13", "w2", "shared_w13", "shared_w2", "gate_w")]
+                         + [("fp8", n) for n in ("x", "out", "w13", "w2")])
+@pytest.mark.parametrize("off", [2, 8])
+def test_expert_layers_refuse_what_is_not_aligned(lib_built, kind, pointer, off):
+    from custom_esimd_kernels_vllm import _lib as L
+    a, call = _expert_layer(L, kind)
+    setattr(a, pointer, getattr(a, pointer) + off)
+    before = L.launch_count()
+    assert call() == -4 and L.launch_count() == before
+
+
+@pytest.mark.parametrize("kind,field,value,code", [("int4", "s13_dtype", 3, -3), ("int4", "s2_dtype", -1, -3), ("int4", "shared_s13_dtype", 3, -3),
+                                                   ("int4", "shared_s2_dtype", 7, -3), ("int4", "layout", 4, -5), ("int4", "shared_layout", -1, -5),
+                                                   ("fp8", "fp8_format", 2, -3)])
+def test_expert_layers_refuse_types_and_layouts_they_do_not_know(lib_built, kind, field, value, code):
+    from custom_esimd_kernels_vllm import _lib as L
+    a, call = _expert_layer(L, kind)
+    setattr(a, field, value)
+    before = L.launch_count()
+    assert call() == code and L.launch_count() == before
