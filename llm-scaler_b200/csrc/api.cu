@@ -242,7 +242,7 @@ static int linear_int4_core(const void* x, int act_dtype, int64_t ldx, const voi
     return umma_w4_i8_linear(ia, st);
   }
   // up to eight tokens, weights worth streaming: w4_stream.cu (w4_stream_preferred has the line and both sides of it)
-  if (!peer && !kmajor && (force == 7 ? M <= W4_STREAM_MAX_TOK : force == 0 && w4_stream_preferred(M, N, K))) {
+  if (!peer && !kmajor && (force == 7 ? M <= W4_STREAM_MAX_TOK : force == 0 && w4_stream_preferred(M, N, K, workspace, workspace ? workspace_bytes : 0))) {
     W4StreamArgs sa{};
     sa.x = x; sa.ldx = ldx; sa.bf16 = act_dtype == B2Q_BF16;
     sa.w = w; sa.layout = w_layout; sa.scale = scale; sa.scale_dtype = scale_dtype; sa.s_stride_n = s_stride_n; sa.s_stride_g = s_stride_g;

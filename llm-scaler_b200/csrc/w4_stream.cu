@@ -564,12 +564,16 @@ static int launch_scale(int sd, bool gated, const CUtensorMap& tw, const CUtenso
   return sd == B2Q_BF16 ? launch_gated<BF16, B2Q_BF16>(gated, tw, tw2, p, grid, overlap, st) : launch_gated<BF16, B2Q_F16>(gated, tw, tw2, p, grid, overlap, st);
 }
 
-bool w4_stream_preferred(int64_t M, int64_t N, int64_t K) {
+static bool room(const W4SPlan& pl, const void* partials, size_t bytes) { return partials && aligned16(partials) && bytes >= pl.partial_bytes; }
+
+bool w4_stream_preferred(int64_t M, int64_t N, int64_t K, const void* partials, size_t partial_bytes) {
   if (M > W4_STREAM_MAX_TOK) return false;
   const double k = (double)K / 1024.0;
   const int64_t slots = 3 * (int64_t)sm_count(), rounds = ((N + 15) / 16 + slots - 1) / slots;
   const double there = 1.0 + (double)rounds * (0.9 + 1.38 * k) * (1.0 + 0.02 * (double)(M - 1));
-  const double here = 9.5 + 0.1e-6 * (double)N * (double)K + 0.2 * k;
+  const W4SPlan pl = plan(N, K);
+  const double whole = 4.0 + (double)((pl.strips + 2 * sm_count() - 1) / (2 * sm_count())) * pl.sps;
+  const double here = pl.cut && !room(pl, partials, partial_bytes) ? whole : 9.5 + 0.1e-6 * (double)N * (double)K + 0.2 * k;
   return here < 0.97 * there;
 }
 
@@ -620,7 +624,7 @@ int w4_stream_linear(const W4StreamArgs& a, cudaStream_t st) {
   int64_t work = (int64_t)p.strips * (grouped ? a.tile_cap : 1);
   if (!grouped) {
     const W4SPlan pl = plan(a.N, a.K);
-    if (pl.cut && a.partials && aligned16(a.partials) && a.partial_bytes >= pl.partial_bytes) {
+    if (pl.cut && room(pl, a.partials, a.partial_bytes)) {
       p.units = pl.strips * pl.sps; p.partials = reinterpret_cast<float4*>(a.partials);
       p.arrivals = reinterpret_cast<Arrivals*>(reinterpret_cast<uint8_t*>(a.partials) + sum_bytes(pl.grid)); p.tag = arrivals_tag(); p.epoch = arrivals_epoch();
       if (!p.epoch) return B2Q_ERR_CUDA;

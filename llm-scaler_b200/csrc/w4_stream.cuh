@@ -29,7 +29,9 @@ size_t w4_stream_partial_bytes(int64_t M, int64_t N, int64_t K);
 // come in rounds of three CTAs per SM that take their time for all of k.  By a fitted cost of both in us; one / eight tokens, there and
 // here: 4096 x 4096 8.3 / 8.8 and 13.4, 5888 x 5888 10.0 / 11.3 and 13.9, 10240 x 4096 14.2 / 15.5 and 15.1, but 7168 x 4224 14.3 / 17.3
 // and 13.4, 28672 x 1024 13.0 / 13.9 and 11.5, 2048 x 16384 26.8 / 30.7 and 17.4, 10240 x 8192 27.2 / 30.5 and 17.9.
-bool w4_stream_preferred(int64_t M, int64_t N, int64_t K);
+// Strips that should be cut, with no room for their partial sums, stay whole, about 1 us per stage: one / eight tokens, there and here, 2048 x
+// 16384 25.6 / 29.9 and 38.8 / 44.1, 8192 x 8192 25.1 / 29.2 and 30.7 / 34.7, but 57344 x 8192 101 / 136 and 68 / 73, 24576 x 4096 24.9 and 18.9.
+bool w4_stream_preferred(int64_t M, int64_t N, int64_t K, const void* partials, size_t partial_bytes);
 
 // Grouped launches of the expert pipeline: up to four rows per expert on average; from about six on tiles of eight tokens repeat too
 // much of the decoding.  Whole pass in us against the tcgen05 kernel behind its pre-passes, 128 experts of 2048 x 768, top-8, at 1 / 16 /

@@ -100,3 +100,24 @@ def test_dispatch_takes_it_where_the_other_kernel_needs_more_rounds(e):
         out = torch.empty(M, N, dtype=torch.bfloat16, device=DEV)
         e.esimd_gemm_int4_pgrp(x.to(DEV), w.to(DEV), s.to(DEV), out)
         assert e.last_kernel() == name
+
+
+def test_without_room_for_partial_sums_the_other_kernel_takes_strips_that_should_be_cut(e):
+    """Scratch is the caller's choice in the C ABI: none, less than asked for, unaligned.  37888 x 1024 is whole strips in any case, and so
+    many strips as 24576 x 4096 has are better off whole than there."""
+    L = e._lib
+    for M, N, K, without in ((1, 2048, 16384, "smallm"), (8, 8192, 8192, "smallm"), (1, 37888, 1024, "w4_stream"), (1, 24576, 4096, "w4_stream")):
+        x, q, w, s = _inputs(M, N, K, torch.bfloat16, torch.bfloat16)
+        x, wd, sd = x.to(DEV), w.to(DEV), s.to(DEV)
+        need = L.lib.b2q_linear_workspace_bytes(M, N, K)
+        ws = torch.empty(need + 16, dtype=torch.uint8, device=DEV)
+        outs = []
+        e.set_force_kernel(0)
+        for ptr, size, room in ((ws.data_ptr(), need, True), (None, 0, False), (ws.data_ptr(), 4096, False), (ws.data_ptr() + 8, need, False)):
+            out = torch.empty(M, N, dtype=torch.bfloat16, device=DEV)
+            rc = L.lib.b2q_linear_int4(x.data_ptr(), L.BF16, K, wd.data_ptr(), L.W4_NMAJOR, sd.data_ptr(), L.BF16, K // 128, 1, out.data_ptr(), N, M, N, K, 128,
+                                       ptr, size, torch.cuda.current_stream().cuda_stream)
+            assert rc == 0 and e.last_kernel() == ("w4_stream" if room else without), (N, K, size)
+            outs.append(out)
+        for out in outs:
+            _close(out, _exact(x.cpu(), q, s), torch.bfloat16)
