@@ -147,14 +147,20 @@ at::Tensor fp8_blockscale(const at::Tensor& input, const at::Tensor& weight, con
   return linear_fp8(input, weight, weight_scale, output, B2Q_SCALE_BLOCK128, -1, -1);
 }
 
-// out[:rows] = silu(gate) * up of input[:rows] (custom_esimd_kernels_vllm/_register.py: _moe_silu_mul over _impl.silu_mul)
+// out[:rows] = silu(gate) * up of input[:rows] (custom_esimd_kernels_vllm/_register.py: _moe_silu_mul over _impl.silu_mul).  The output is
+// written row behind row: a flat buffer or rows of N_half, and room for all of them.
 at::Tensor moe_silu_mul(const at::Tensor& input, at::Tensor output, int64_t N_gate_up, int64_t N_half, int64_t total_rows) {
   TORCH_CHECK(N_gate_up == 2 * N_half, "N_gate_up must be 2 * N_half");
-  require_cuda({&input});
-  const at::Tensor in = input.slice(0, 0, total_rows), out = output.slice(0, 0, total_rows);
-  TORCH_CHECK(in.dim() == 2 && in.is_contiguous(), "gate_up must be contiguous [rows, 2I]");
+  require_cuda({&input, &output});
+  TORCH_CHECK(total_rows >= 0, "total_rows must not be negative");
+  TORCH_CHECK(input.dim() == 2 && input.size(1) == N_gate_up, "gate_up must be [rows, N_gate_up]");
+  const at::Tensor in = input.slice(0, 0, total_rows);
+  TORCH_CHECK(in.is_contiguous(), "gate_up must be contiguous [rows, 2I]");
+  TORCH_CHECK(output.device() == in.device() && output.scalar_type() == in.scalar_type(), "output must have gate_up's device and type");
+  TORCH_CHECK(output.dim() >= 1 && output.is_contiguous() && (output.dim() == 1 || output.size(-1) == N_half) && output.numel() >= in.size(0) * N_half,
+              "output must be contiguous rows of N_half, at least as many as are computed");
   const c10::cuda::CUDAGuard guard(in.device());
-  check(b2q_silu_mul(in.data_ptr(), out.data_ptr(), act_dtype(in), in.size(0), in.size(1) / 2,
+  check(b2q_silu_mul(in.data_ptr(), output.data_ptr(), act_dtype(in), in.size(0), N_half,
                      c10::cuda::getCurrentCUDAStream(in.device().index()).stream()));
   return output;
 }

@@ -191,8 +191,20 @@ def _moe_scatter(hidden_states, router_top_value, sorted_token_ids, scattered_hi
 
 def _moe_silu_mul(input, output, N_gate_up, N_half, total_rows):
     I._chk(N_gate_up == 2 * N_half, "N_gate_up must be 2 * N_half")
-    I.silu_mul(input[:total_rows], output[:total_rows])
+    L.require_cuda(input, output)
+    I.silu_mul(_silu_rows(input, output, N_gate_up, N_half, total_rows), output)
     return output
+
+
+def _silu_rows(input, output, N_gate_up, N_half, total_rows):
+    """The rows of input to activate.  The output is written row behind row: a flat buffer or rows of N_half, and room for all of them."""
+    I._chk(total_rows >= 0, "total_rows must not be negative")
+    I._chk(input.dim() == 2 and input.shape[1] == N_gate_up, "gate_up must be [rows, N_gate_up]")
+    rows = input[:total_rows]
+    I._chk(output.device == rows.device and output.dtype == rows.dtype, "output must have gate_up's device and type")
+    I._chk(output.dim() >= 1 and output.is_contiguous() and (output.dim() == 1 or output.shape[-1] == N_half)
+           and output.numel() >= rows.shape[0] * N_half, "output must be contiguous rows of N_half, at least as many as are computed")
+    return rows
 
 
 def _moe_gather(moe_output, topk_ids, scattered_weights, final_hidden, K, topk, T):

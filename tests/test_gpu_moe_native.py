@@ -131,3 +131,27 @@ def test_logits_without_a_maximum_route_nowhere(e):
             e.set_force_kernel(0)
         assert torch.equal(out, ref) if kernel == 2 else torch.allclose(out, ref, rtol=1e-2, atol=1e-2)
         assert (out[2] == 0).all()
+
+
+@pytest.mark.parametrize("native", [True, False])
+def test_silu_mul_refuses_outputs_it_would_write_beyond(e, native):
+    """The C++ op and the Python one behind it: the same outputs are taken and refused, with nothing launched for the latter."""
+    from custom_esimd_kernels_vllm import _register as R
+    from test_host_logic import _outputs
+    op = torch.ops.custom_esimd_kernels_vllm.esimd_moe_silu_mul if native else R._moe_silu_mul
+    x = torch.randn(6, 64, device=DEV).to(torch.bfloat16)
+    ref = None
+    for out, fits in _outputs(torch.bfloat16, DEV):
+        before = e._lib.launch_count()
+        if fits:
+            got = op(x, out, 64, 32, 4).reshape(-1)[:128]
+            ref = got if ref is None else ref
+            assert torch.equal(got, ref) and e._lib.launch_count() == before + 1
+        else:
+            with pytest.raises((RuntimeError, NotImplementedError)):
+                op(x, out, 64, 32, 4)
+            assert e._lib.launch_count() == before
+    for args in ((x, x[:, :32].contiguous(), 64, 32, -1), (x, x, 128, 64, 4)):
+        with pytest.raises(RuntimeError):
+            op(*args)
+    assert op(x, torch.zeros(6, 32, dtype=torch.bfloat16, device=DEV), 64, 32, 100).shape == (6, 32)

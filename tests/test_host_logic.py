@@ -54,3 +54,26 @@ def test_python_repack_helpers_match_oracle(impl):
     w, ids = torch.rand(5, 2), torch.randint(0, 4, (5, 2), dtype=torch.int32)
     rows, wts, per = e.precompute_moe_route(w, ids, 4)     # CPU tensors take the torch fallback
     assert per.sum() == 10 and rows.numel() == 10
+
+
+def _outputs(dtype, device):
+    """Outputs of esimd_moe_silu_mul for 4 of 6 rows of [6, 64], and whether they hold what is written."""
+    z = lambda *s, **k: torch.zeros(*s, dtype=k.get("dtype", dtype), device=k.get("device", device))
+    return [(z(4, 32), True), (z(6, 32), True), (z(128), True), (z(2, 2, 32), True),
+            (z(3, 32), False), (z(127), False), (z(4, 16), False), (z(4, 64), False), (z(4, 64)[:, :32], False), (z(8, 32)[::2], False),
+            (z(4, 32, dtype=torch.float32), False), (z(4, 32, device="meta" if device == "cpu" else "cpu"), False)]
+
+
+def test_silu_mul_takes_outputs_that_hold_every_row(impl):
+    from custom_esimd_kernels_vllm import _register as R
+    x = torch.zeros(6, 64, dtype=torch.bfloat16)
+    for out, fits in _outputs(torch.bfloat16, "cpu"):
+        if fits:
+            assert R._silu_rows(x, out, 64, 32, 4).shape == (4, 64)
+        else:
+            with pytest.raises(RuntimeError):
+                R._silu_rows(x, out, 64, 32, 4)
+    for args in ((x, x[:, :32].contiguous(), 64, 32, -1), (x, x, 128, 64, 4), (x[0], x, 64, 32, 4)):
+        with pytest.raises(RuntimeError):
+            R._silu_rows(*args)
+    assert R._silu_rows(x, torch.zeros(6, 32, dtype=torch.bfloat16), 64, 32, 100).shape == (6, 64)      # no more rows than there are
