@@ -434,6 +434,7 @@ w4_stream_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constant
         for (int i2 = 0; i2 < 2; ++i2)
           asm volatile("st.shared.v4.f32 [%0], {%1,%2,%3,%4};" ::"r"(red + 512 * i2), "f"(acc[i2][0]), "f"(acc[i2][1]), "f"(acc[i2][2]), "f"(acc[i2][3]) : "memory");
       if (lane == 0) pair_ok[2 * w + turn] = ok;
+      __syncwarp();
       asm volatile("bar.sync %0, 64;" ::"r"(1 + w) : "memory");
       ok = pair_ok[2 * w] && pair_ok[2 * w + 1];
       if (turn == 0)

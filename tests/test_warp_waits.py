@@ -52,3 +52,29 @@ def test_copies_in_flight_are_waited_for(name):
         producers = sum(bool(re.search(r"\btma_load_2d(_pair)?\(", part)) for part in text.split("if (elect_one()) {")[1:])
         assert text.count("drain_issued(") == producers
         assert ("cp_async_arrive(" in text) == ("cp_async_wait_all()" in text)
+
+
+def _unconverged_barriers(text):
+    """Line numbers of aligned block barriers in front of which, since the last statement that a whole warp executes together, only
+    some of its lanes did something."""
+    text = re.sub(r"//[^\n]*", "", text)
+    found = []
+    for m in re.finditer(r'asm volatile\("bar\.sync', text):
+        before = text[:m.start()]
+        lanes = max((x.end() for x in re.finditer(r"\bif \((?:\w+ && )?lane (?:==|<) \w+\)", before)), default=-1)
+        together = max((x.end() for x in re.finditer(r"__syncwarp\(\)|__syncthreads\(\)|_sync\(0x|mbar_wait_warp\w*\(|bar\.sync", before)), default=-1)
+        if lanes > together:
+            found.append(text.count("\n", 0, m.start()) + 1)
+    return found
+
+
+def test_the_reader_sees_lanes_on_their_own():
+    assert _unconverged_barriers('if (lane == 0) a = b;\n__syncwarp();\nasm volatile("bar.sync 1, 64;");') == []
+    assert _unconverged_barriers('__syncwarp();\nif (lane == 0) a = b;\nasm volatile("bar.sync 1, 64;");') == [3]
+
+
+@pytest.mark.parametrize("name", sorted(f for f in os.listdir(CSRC) if f.endswith((".cu", ".cuh"))))
+def test_whole_warps_meet_at_aligned_barriers(name):
+    """bar.sync is the aligned form: all lanes of a warp have to execute it together."""
+    with open(os.path.join(CSRC, name)) as f:
+        assert _unconverged_barriers(f.read()) == []
