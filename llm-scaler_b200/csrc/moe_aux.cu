@@ -22,11 +22,20 @@ __device__ __forceinline__ int32_t ld_shared_word(const int32_t* p) {
   asm volatile("ld.global.s32 %0, [%1];" : "=r"(v) : "l"(p) : "memory");
   return v;
 }
+// Sixteen bytes in the same way; every thread reads its own, so ordering against other loads and stores is left to the compiler.
+__device__ __forceinline__ uint4 ld_shared_vec(const void* p) {
+  uint4 v;
+  asm volatile("ld.global.v4.u32 {%0,%1,%2,%3}, [%4];" : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w) : "l"(p));
+  return v;
+}
+__device__ __forceinline__ unsigned short ld_shared_u16(const void* p) {
+  unsigned short h;
+  asm volatile("ld.global.u16 %0, [%1];" : "=h"(h) : "l"(p));
+  return h;
+}
 __device__ __forceinline__ float ld_shared_scalar(const void* p, int64_t i, int dt) {
   if (dt == B2Q_F32) return __int_as_float(ld_shared_word(reinterpret_cast<const int32_t*>(p) + i));
-  unsigned short h;
-  asm volatile("ld.global.u16 %0, [%1];" : "=h"(h) : "l"(reinterpret_cast<const unsigned short*>(p) + i) : "memory");
-  return scalar_from_raw(h, dt);
+  return scalar_from_raw(ld_shared_u16(reinterpret_cast<const unsigned short*>(p) + i), dt);
 }
 __device__ __forceinline__ float load_scalar_cg(const void* p, int64_t i, int dt) {
   if (dt == B2Q_F32) return __ldcg(reinterpret_cast<const float*>(p) + i);
@@ -805,15 +814,15 @@ __global__ void act_prep_kernel(const void* __restrict__ x, int64_t ldx, const i
   if (!release_early) grid_dep_release();
   const int64_t r = blockIdx.x;
   // the launch covers the caller's upper bound of rows; the number actually routed here is only known on the device
-  if (n_valid && r >= *n_valid) return;
-  const int64_t srow = idx ? (int64_t)(idx[r] / div) : r;
+  if (n_valid && r >= ld_shared_word(n_valid)) return;
+  const int64_t srow = idx ? (int64_t)(ld_shared_word(idx + r) / div) : r;
   const uint16_t* row = reinterpret_cast<const uint16_t*>(x) + srow * ldx;
   // eight consecutive source values of the row as floats that are exactly representable in the source type
   auto load8 = [&](int k, float* f) {
-    const uint4 v = *reinterpret_cast<const uint4*>(row + k);
+    const uint4 v = ld_shared_vec(row + k);
     const T* e = reinterpret_cast<const T*>(&v);
     if constexpr (GATED) {
-      const uint4 u = *reinterpret_cast<const uint4*>(row + K + k);
+      const uint4 u = ld_shared_vec(row + K + k);
       const T* ue = reinterpret_cast<const T*>(&u);
 #pragma unroll
       for (int j = 0; j < 8; ++j) {
@@ -888,16 +897,16 @@ __global__ void __launch_bounds__(256) act_prep_warp_kernel(const void* __restri
   if (!release_early) grid_dep_release();
   const int lane = threadIdx.x & 31;
   const int64_t r = (int64_t)blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
-  if (r >= rows || (n_valid && r >= *n_valid)) return;
-  const int64_t srow = idx ? (int64_t)(idx[r] / div) : r;
+  if (r >= rows || (n_valid && r >= ld_shared_word(n_valid))) return;
+  const int64_t srow = idx ? (int64_t)(ld_shared_word(idx + r) / div) : r;
   const uint16_t* row = reinterpret_cast<const uint16_t*>(x) + srow * ldx;
   const int iters = K >> 8;
   uint4 raw[MAXI], up[GATED ? MAXI : 1];
 #pragma unroll
   for (int i = 0; i < MAXI; ++i)
     if (i < iters) {
-      raw[i] = *reinterpret_cast<const uint4*>(row + (i * 32 + lane) * 8);
-      if constexpr (GATED) up[i] = *reinterpret_cast<const uint4*>(row + K + (i * 32 + lane) * 8);
+      raw[i] = ld_shared_vec(row + (i * 32 + lane) * 8);
+      if constexpr (GATED) up[i] = ld_shared_vec(row + K + (i * 32 + lane) * 8);
     }
   float amax = 0.f;
 #pragma unroll
@@ -1012,7 +1021,7 @@ __global__ void act_split_fp8_kernel(const void* __restrict__ x, int64_t ldx, ui
   };
   float amax = 0.f;
   for (int k = threadIdx.x * 8; k < K; k += blockDim.x * 8) {
-    const uint4 v = *reinterpret_cast<const uint4*>(row + k);
+    const uint4 v = ld_shared_vec(row + k);
     const uint16_t* e = reinterpret_cast<const uint16_t*>(&v);
 #pragma unroll
     for (int j = 0; j < 8; ++j) amax = fmaxf(amax, fabsf(to_f(e[j])));
@@ -1029,7 +1038,7 @@ __global__ void act_split_fp8_kernel(const void* __restrict__ x, int64_t ldx, ui
   if (threadIdx.x == 0) inv_scale[r] = 1.0f / sc;
   constexpr int NT = IN_BF16 ? 2 : 3;
   for (int k = threadIdx.x * 8; k < K; k += blockDim.x * 8) {
-    const uint4 v = *reinterpret_cast<const uint4*>(row + k);
+    const uint4 v = ld_shared_vec(row + k);
     const uint16_t* e = reinterpret_cast<const uint16_t*>(&v);
     uint8_t t[NT][8];
 #pragma unroll
@@ -1089,7 +1098,7 @@ __global__ void act_split_i8_kernel(const void* __restrict__ x, int64_t ldx, int
   };
   float amax = 0.f;
   for (int k = threadIdx.x * 8; k < K; k += blockDim.x * 8) {
-    const uint4 v = *reinterpret_cast<const uint4*>(row + k);
+    const uint4 v = ld_shared_vec(row + k);
     const uint16_t* e = reinterpret_cast<const uint16_t*>(&v);
 #pragma unroll
     for (int j = 0; j < 8; ++j) amax = fmaxf(amax, fabsf(to_f(e[j])));
@@ -1119,7 +1128,7 @@ __global__ void act_split_i8_kernel(const void* __restrict__ x, int64_t ldx, int
     const int k = k0 + threadIdx.x * 8;
     float part = 0.f;
     if (k < K) {
-      const uint4 v = *reinterpret_cast<const uint4*>(row + k);
+      const uint4 v = ld_shared_vec(row + k);
       const uint16_t* e = reinterpret_cast<const uint16_t*>(&v);
       int8_t t[3][8];
 #pragma unroll
@@ -1203,9 +1212,9 @@ __global__ void __launch_bounds__(512) resadd_rmsnorm_kernel(const void* __restr
   const int k0 = threadIdx.x * 8, step = blockDim.x * 8;
   uint4 rv[NC], hv[NC], wv[NC];
   auto fetch = [&](int k, uint4& a, uint4& b, uint4& c) {
-    a = *reinterpret_cast<const uint4*>(res + k);
-    if (h) b = *reinterpret_cast<const uint4*>(h + k);
-    c = *reinterpret_cast<const uint4*>(w + k);
+    a = ld_shared_vec(res + k);
+    if (h) b = ld_shared_vec(h + k);
+    c = ld_shared_vec(w + k);
   };
   auto value = [&](const uint4& a, const uint4& b, float (&v)[8]) {
     const T* re = reinterpret_cast<const T*>(&a);
@@ -1254,7 +1263,7 @@ __global__ void __launch_bounds__(512) resadd_rmsnorm_kernel(const void* __restr
     if (h) *reinterpret_cast<uint4*>(res + k) = so;
     *reinterpret_cast<uint4*>(out + k) = no;
     if (out2) {
-      const uint4 w2v = *reinterpret_cast<const uint4*>(w2 + k);
+      const uint4 w2v = ld_shared_vec(w2 + k);
       const T* w2e = reinterpret_cast<const T*>(&w2v);
 #pragma unroll
       for (int j = 0; j < 8; ++j) ne[j] = Act<BF16>::from_f(v[j] * inv * Act<BF16>::to_f(w2e[j]));
@@ -1307,8 +1316,8 @@ __global__ void resadd_norm_split_fp8_kernel(const void* __restrict__ hidden, vo
   const T* w = reinterpret_cast<const T*>(weight);
   T* out = reinterpret_cast<T*>(normed) + r * K;
   auto load8 = [&](int k, float* v) {
-    const uint4 rv = *reinterpret_cast<const uint4*>(res + k);
-    const uint4 hv = *reinterpret_cast<const uint4*>(h + k);
+    const uint4 rv = ld_shared_vec(res + k);
+    const uint4 hv = ld_shared_vec(h + k);
     const T* re = reinterpret_cast<const T*>(&rv);
     const T* he = reinterpret_cast<const T*>(&hv);
 #pragma unroll
@@ -1343,7 +1352,7 @@ __global__ void resadd_norm_split_fp8_kernel(const void* __restrict__ hidden, vo
   for (int k = threadIdx.x * 8; k < K; k += blockDim.x * 8) {
     float v[8];
     load8(k, v);
-    const uint4 wv = *reinterpret_cast<const uint4*>(w + k);
+    const uint4 wv = ld_shared_vec(w + k);
     const T* we = reinterpret_cast<const T*>(&wv);
     uint4 so, no;
     T* se = reinterpret_cast<T*>(&so);
@@ -1424,15 +1433,16 @@ __global__ void gated_rmsnorm_kernel(const void* __restrict__ x, const void* __r
   const T* zr = reinterpret_cast<const T*>(z) + (int64_t)row * V;
   const T* w = reinterpret_cast<const T*>(weight);
   T* o = reinterpret_cast<T*>(out) + (int64_t)row * V;
+  auto in = [](const T* p) { return scalar_from_raw(ld_shared_u16(p), BF16 ? B2Q_BF16 : B2Q_F16); };
   float ss = 0.f;
-  for (int k = lane; k < V; k += 32) { const float v = Act<BF16>::to_f(xr[k]); ss = fmaf(v, v, ss); }
+  for (int k = lane; k < V; k += 32) { const float v = in(xr + k); ss = fmaf(v, v, ss); }
 #pragma unroll
   for (int off = 16; off > 0; off >>= 1) ss += __shfl_xor_sync(0xffffffffu, ss, off);
   const float inv = rsqrtf(ss / (float)V + eps);
   for (int k = lane; k < V; k += 32) {
-    const float g = Act<BF16>::to_f(zr[k]);
+    const float g = in(zr + k);
     const float silu = g / (1.f + __expf(-g));
-    o[k] = Act<BF16>::from_f(Act<BF16>::to_f(xr[k]) * inv * Act<BF16>::to_f(w[k]) * silu);
+    o[k] = Act<BF16>::from_f(in(xr + k) * inv * in(w + k) * silu);
   }
 }
 

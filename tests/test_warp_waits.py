@@ -78,3 +78,26 @@ def test_whole_warps_meet_at_aligned_barriers(name):
     """bar.sync is the aligned form: all lanes of a warp have to execute it together."""
     with open(os.path.join(CSRC, name)) as f:
         assert _unconverged_barriers(f.read()) == []
+
+
+def _read_only_loads(text):
+    """In kernels that begin while the one in front is running: places where a const __restrict__ pointer is read by a plain
+    dereference, which the compiler may turn into a load by the read-only path."""
+    text, found = re.sub(r"//[^\n]*", "", text), []
+    for m in re.finditer(r"__global__ (.*?)\n}\n", text, re.S):
+        body = m.group(1)
+        if re.search(r"grid_dep_wait\(\)|dep_enter\(\)", body):
+            for d in re.finditer(r"\*reinterpret_cast<const uint[24]\*>\((?!out \+|t\[|&)|\*n_valid|\bidx\[|\b[xz]r\[|\bw\[k\]", body):
+                found.append(text.count("\n", 0, m.start(1) + d.start()) + 1)
+    return found
+
+
+def test_the_reader_sees_plain_dereferences():
+    assert _read_only_loads("__global__ void f(const void* __restrict__ x) {\n  dep_enter();\n  a = *reinterpret_cast<const uint4*>(row + k);\n}\n") == [3]
+    assert _read_only_loads("__global__ void f(const void* __restrict__ x) {\n  dep_enter();\n  a = ld_shared_vec(row + k);\n}\n") == []
+
+
+def test_kernels_that_start_early_read_their_inputs_by_ordinary_loads():
+    """The read-only path promises that nothing is written while the kernel runs, and these run while their inputs are written."""
+    with open(os.path.join(CSRC, "moe_aux.cu")) as f:
+        assert _read_only_loads(f.read()) == []
