@@ -310,8 +310,7 @@ w4_stream_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constant
           ok = mbar_wait_warp(empty + 8 * s, par, abort_flag, p.status, ST_XEMPTY);
           if (!ok) break;
           // The counts of the CTA's cut strips, which only a run's ends can be, are opened before the first segment's last stage is
-          // handed to the warps that will add to them; behind the first stages, as the trip to DRAM would hold these up (decoder layer
-          // of one token 126.4 us that way, 126.0 here, 125.2 with counts that nobody has to open).
+          // handed to the warps that will add to them; behind the first stages, which would otherwise wait for the trip to DRAM.
           if (open && (i == RS || st + XW >= sg.nst)) {
             if (lane < 2 * BLOCKS) arrivals_open(p.arrivals + ((lane & 1) ? cur.u1 - 1 : cur.u0) / p.sps * BLOCKS + (lane >> 1), p.tag, p.epoch);
             open = false;

@@ -129,9 +129,9 @@ def test_rejects_shapes_outside_the_contract(L):
 
 
 @pytest.mark.parametrize("M,N,K,kmajor", [
-    (64, 2048, 4096, False), (16, 8192, 14336, False), (40, 5120, 2560, True),     # strips cut along k: partial sums, then delivery
-    (33, 18944, 512, False),                                                       # one whole strip per SM
-    (64, 37888, 512, False), (48, 40960, 768, False),                              # 256-row strips, whole and cut
+    (64, 2048, 14336, False), (16, 8192, 14336, False), (40, 5120, 8192, True),    # strips cut along k: partial sums, then delivery
+    (64, 2048, 4096, False), (40, 5120, 2560, True), (33, 18944, 512, False),      # whole strips, one per SM at most
+    (64, 37888, 512, False), (48, 40960, 768, False), (48, 40960, 4096, False),    # 256-row strips: whole, whole with two rounds, cut
 ])
 @pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16])
 @pytest.mark.parametrize("scratch", [True, False])                                 # without it the two-CTA kernel delivers

@@ -258,10 +258,10 @@ def test_bounded_wait_gives_up_and_reports(e):
     and the context is still usable for the next launch."""
     L = e._lib
     assert L.device_status() == 0
-    # a decode launch whose strips are cut along K (few strips, many SMs): it relies on the arrival counters that the
-    # reset below clears together with the status words of every kernel family
-    qb, sb = _int4(2048, 4096, torch.bfloat16, 5)
-    xb = torch.randn(40, 4096, generator=torch.Generator().manual_seed(5)).to(torch.bfloat16).to(DEV)
+    # a decode launch whose strips are cut along K (few strips, many SMs): it relies on arrival counts, whose tags the reset
+    # below changes together with the status words of every kernel family
+    qb, sb = _int4(2048, 14336, torch.bfloat16, 5)
+    xb = torch.randn(40, 14336, generator=torch.Generator().manual_seed(5)).to(torch.bfloat16).to(DEV)
     wb, sbd = int4.pack_nmajor_u8(qb).to(DEV), sb.to(DEV)
     before = torch.empty(40, 2048, dtype=torch.bfloat16, device=DEV)
     e.esimd_gemm_int4_pgrp(xb, wb, sbd, before)

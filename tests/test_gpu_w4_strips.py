@@ -42,7 +42,8 @@ def _check(out, ref, what, rounding=2.0 ** -8):
 @pytest.mark.parametrize("scale_dtype", [torch.bfloat16, torch.float16, torch.float32])
 @pytest.mark.parametrize("M,N,K", [
     (1, 128, 128), (16, 136, 384), (17, 1000, 1024),     # one tile; ragged strip; odd group count; aligned scale fetch
-    (33, 520, 2560), (64, 2048, 4096),                   # 64-token tile, cut strips
+    (33, 520, 2560), (64, 2048, 4096),                   # 64-token tile
+    (33, 520, 14336), (64, 2048, 14336),                 # cut strips, the last of them ragged; without rest
     (65, 300, 1280), (128, 1032, 2048),                  # 128-token tile, one of them
     (129, 384, 640), (400, 2184, 1152),                  # several token tiles, odd group counts
 ])
@@ -60,7 +61,17 @@ def test_tile_and_group_edges(e, M, N, K, scale_dtype):
     assert e._lib.device_status() == 0
 
 
-@pytest.mark.parametrize("M,N,K", [(16, 8192, 14336), (64, 8192, 14336), (64, 38016, 2048), (100, 10240, 8192), (700, 8192, 2048),
+def test_the_strips_called_cut_are_cut(e):
+    """Scratch beyond the pre-pass's part is asked for where strips are cut."""
+    up = lambda n: (n + 255) // 256 * 256
+    for M, N, K in ((33, 520, 14336), (64, 2048, 14336), (64, 8192, 14336), (64, 38016, 8192), (100, 4096, 14336), (128, 12288, 14336), (96, 520, 8192)):
+        assert e._lib.lib.b2q_linear_workspace_bytes(M, N, K) > up(2 * M * K) + up(4 * M), (M, N, K)
+    for M, N, K in ((17, 1032, 8192), (60, 1000, 14336)):
+        tok = 32 if M <= 32 else 64
+        assert e._lib.lib.b2q_linear_fp8_workspace_bytes(M, N, K) >= up(2 * M * K) + up(4 * M) + 2 * ((N + 127) // 128) * 128 * tok * 4, (M, N, K)
+
+
+@pytest.mark.parametrize("M,N,K", [(16, 8192, 14336), (64, 8192, 14336), (64, 38016, 2048), (64, 38016, 8192), (100, 10240, 8192), (700, 8192, 2048),
                                    (100, 4096, 14336), (128, 12288, 14336), (96, 520, 8192)])    # 128-token tiles cut into equal pieces, over the whole grid, ragged
 def test_many_segments_repeat_bit_for_bit(e, M, N, K):
     x, w, s, ref = _case(M, N, K, torch.bfloat16, 7)
@@ -77,7 +88,8 @@ def test_many_segments_repeat_bit_for_bit(e, M, N, K):
 
 
 @pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16])
-@pytest.mark.parametrize("M,N,K", [(1, 128, 128), (16, 200, 384), (17, 1032, 640), (33, 2048, 1152), (64, 8192, 5120), (27, 17408, 5120)])
+@pytest.mark.parametrize("M,N,K", [(1, 128, 128), (16, 200, 384), (17, 1032, 640), (33, 2048, 1152), (64, 8192, 5120), (27, 17408, 5120),
+                                   (17, 1032, 8192), (60, 1000, 14336)])              # cut strips, the last of them ragged
 def test_block_scaled_fp8_strips(e, M, N, K, dtype):
     """The e4m3 form of the kernel: a weight times its fp32 block scale is rounded to fp16 once, as above; with fp16
     output the tolerance is 2^-11 for the output's rounding and the same 2^-9 of a typical column for the weights'."""
