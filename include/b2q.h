@@ -164,7 +164,11 @@ B2Q_API int b2q_quantize_fp8(const void* w, int w_dtype, int64_t ldw, void* wq, 
  * over several CTAs per strip of rows so that they still occupy every SM; the partial sums are added in
  * a fixed order, so results are bit-reproducible from run to run.  Scratch that holds the rewritten
  * activations (M * K * 2 + M * 4 bytes, each part rounded up to 256) but not the partial sums keeps the
- * pre-pass; strips then stay whole.                                                              */
+ * pre-pass; strips then stay whole.
+ * M <= 8 on N-major nibbles needs no rewritten activations and scales fp32 sums, so every scale is exact there; its
+ * scratch holds partial sums only.
+ * Scratch is read and written until the call's last kernel has completed: calls that may run at the same time (streams,
+ * graphs) each need their own.  What it holds before a call does not matter, and nothing of a call stays outside it.   */
 B2Q_API size_t b2q_linear_workspace_bytes(int64_t M, int64_t N, int64_t K);
 B2Q_API int b2q_linear_int4(const void* x, int act_dtype, int64_t ldx,
                     const void* w, int w_layout,
@@ -179,7 +183,9 @@ B2Q_API int b2q_linear_int4(const void* x, int act_dtype, int64_t ldx,
  * fp8_GEMM_pert.h:4030-4075, fp8_GEMM_blockscale.h:64-223).
  * w is [N, K] one byte per element, row-major.  Activation stays 16-bit
  * (w8a16); e4m3 decode is exact including subnormals.  K % 16 == 0.
- * workspace is optional (NULL / 0 allowed).  With at least
+ * workspace is optional (NULL / 0 allowed), and the call's own like b2q_linear_int4's.  M <= 16 runs, where that is the
+ * faster choice by size, type and scale mode, in one launch without any scratch: the weights become exact 16-bit
+ * values, meet the activations as they are, and the scales are applied in fp32.  Otherwise, with at least
  * b2q_linear_fp8_workspace_bytes() of scratch:
  *  - M <= 64 with per-channel or per-tensor scales runs on the 8-bit tensor-core path: the weights are
  *    used as stored and every activation row is rewritten as 2^e times a sum of two (bf16) or three
@@ -204,9 +210,9 @@ B2Q_API int b2q_linear_fp8(const void* x, int act_dtype, int64_t ldx,
  * scaled_resadd_norm_gemv_fp8.h:70-95):
  *   v = (hidden + residual) * scalar;  residual <- v;  normed_out <- v * rsqrt(mean(v^2) + eps) * norm_weight;
  *   out = normed_out * dequant(W)^T            (normed_out as stored, i.e. rounded to act_dtype).
- * hidden, residual, normed_out are contiguous [M, K], norm_weight [K]; the rest as b2q_linear_fp8.  On the decode
- * path (M <= 64, per-channel or per-tensor scale, scratch given) the norm runs inside the GEMV's own activation
- * pre-pass: two launches in all (pre-pass, GEMV) instead of three; elsewhere the norm is its own launch.          */
+ * hidden, residual, normed_out are contiguous [M, K], norm_weight [K]; the rest as b2q_linear_fp8.  Two launches where
+ * the linear needs no pre-pass (norm, linear), and on the 8-bit path (M <= 64, per-channel or per-tensor scale, scratch
+ * given), where the norm runs inside the pre-pass; three elsewhere.                                               */
 B2Q_API int b2q_resadd_norm_linear_fp8(const void* hidden, void* residual, const void* norm_weight, void* normed_out,
                                float eps, float scalar, int act_dtype, const void* w, int fp8_format,
                                const void* scale, int scale_dtype, int scale_mode, void* out, int64_t ldo,

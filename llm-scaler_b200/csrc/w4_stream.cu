@@ -10,7 +10,7 @@
 //   next 8        decode, MMA, output: 32 rows of the strip each, every other stage
 // What it replaces (smallm.cuh, one CTA per 16-row strip) loaded scales and activations from global memory for every 128 k, fed
 // one chain of eight dependent MMAs with them and waited for both.  57344 x 8192, one / eight tokens: 102 / 132 us there, 54 / 57
-// here (fp16), with the same ring and no decode 41 us.  What the difference is made of: nibble conversion 10 us, MMAs 3.
+// here (fp16).  Probes of the same ring, none of them kept: no decode 41 us, nibble conversion adds 10, MMAs 3.
 // What was found on the way, same shape, one token:
 // * 72 KB of ring per SM instead of 128: 48 us without any decode.
 // * An MMA takes some 80 cycles to deliver and a group's eight can only be chained (their sum is scaled in fp32): hence two tiles
@@ -22,6 +22,7 @@
 //
 // Work: strips of 128 rows x stages of 256 k.  Dense launches give every CTA an equal run of stages; a strip cut between CTAs is
 // summed, block by block, by whoever delivers last, in CTA order: nobody waits, and the result does not depend on who that is.
+// Who comes last is counted in the caller's scratch (arrivals.cuh).
 // Grouped launches walk (tile, strip) pairs.  GATED: a strip is 64 gate rows and the 64 up rows that go with them, paired in
 // one thread's accumulators, and the output is silu(gate) * up.
 //
