@@ -465,7 +465,8 @@ B2Q_API int b2q_selftest_bounded_wait(int code, int* gave_up, void* stream);
 
 /* Kernel selection override for benchmarking: 0 = automatic, 1 = the mma.sync streaming kernel,
  * 2 = the tcgen05 kernel with 16-bit operands, 3 = the same without activation pre-pass,
- * 4 = the same with one CTA per strip (no strip cutting), 5 = INT4 decode on the int8 MMA,
+ * 4 = the same with one CTA per strip (no strip cutting), 5 = INT4 decode on the int8 MMA (its scratch is asked for
+ * while the override is set),
  * 6 = the CTA-pair (cta_group::2) variant of the W8A8 GEMM, 7 = the INT4 decode streaming kernel, 8 = the FP8 streaming
  * kernel of up to sixteen tokens. */
 B2Q_API void b2q_set_force_kernel(int which);

@@ -317,7 +317,8 @@ int b2q_linear_int4_allreduce(const void* x, int act_dtype, int64_t ldx, const v
 }
 
 size_t b2q_linear_workspace_bytes(int64_t M, int64_t N, int64_t K) {
-  const size_t a = ws_prep_bytes(M, K) + umma_w4_partial_bytes(M, N, K), b = ws_i8_bytes(M, K), c = w4_stream_partial_bytes(M, N, K);
+  const size_t a = ws_prep_bytes(M, K) + umma_w4_partial_bytes(M, N, K), b = w4_stream_partial_bytes(M, N, K);
+  const size_t c = tls().force_kernel == 5 ? ws_i8_bytes(M, K) : 0;      // the int8 path is taken on request only
   return a > b ? (a > c ? a : c) : (b > c ? b : c);
 }
 size_t b2q_linear_fp8_workspace_bytes(int64_t M, int64_t N, int64_t K) {

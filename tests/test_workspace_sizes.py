@@ -53,3 +53,26 @@ def test_int4_short_k_is_not_cut_for_128_token_tiles(lib):
                 assert lib.b2q_linear_workspace_bytes(M, N, K) == _prep(M, K)
         assert lib.b2q_linear_workspace_bytes(M, 4096, 14336) - _prep(M, 14336) == 2 * 4 * 32 * 128 * 128 * 4      # four equal pieces
         assert lib.b2q_linear_workspace_bytes(M, 8192, 28672) - _prep(M, 28672) == 2 * SMS * 128 * 128 * 4         # the whole grid
+
+
+@pytest.mark.parametrize("M", [1, 8, 9, 16])
+@pytest.mark.parametrize("N,K", [(4096, 4096), (8192, 28672), (57344, 8192)])
+def test_int4_few_rows_ask_for_what_can_be_used(lib, M, N, K):
+    """The pre-pass with two slots of 128 rows per SM behind it (K-major weights), or two slots of eight tokens for each of two CTAs per SM
+    and four counts per strip; the int8 path's term rows only while that path is asked for."""
+    most = max(_prep(M, K) + 2 * SMS * 128 * 16 * 4, 2 * 2 * SMS * 128 * 8 * 4 + (N + 127) // 128 * 4 * 8)
+    assert _prep(M, K) <= lib.b2q_linear_workspace_bytes(M, N, K) <= most
+    lib.b2q_set_force_kernel(5)
+    try:
+        assert lib.b2q_linear_workspace_bytes(M, N, K) > 4 << 20
+    finally:
+        lib.b2q_set_force_kernel(0)
+
+
+@pytest.mark.parametrize("M", [1, 20, 64])
+def test_fp8_partial_sums_of_cut_strips_are_one_slot_per_sm(lib, M):
+    """Term rows in e4m3 (three per fp16 token, in the MMA's steps), scales, and [SMs][M in eights][128] fp32 with a count per strip."""
+    rows = next(r for r in (16, 32, 64, 128, 256) if r >= 3 * ((M + 7) // 8 * 8))
+    K = 13824
+    assert lib.b2q_linear_fp8_workspace_bytes(M, 5120, K) <= max(_up(rows * K) + _up(4 * M) + SMS * ((M + 7) // 8 * 8) * 128 * 4 + SMS * 8,
+                                                                 _prep(M, K) + 2 * SMS * 128 * 64 * 4)
