@@ -34,6 +34,15 @@ __device__ __forceinline__ void fence_proxy_async() { asm volatile("fence.proxy.
 __device__ __forceinline__ void mbar_arrive(uint32_t bar) {
   asm volatile("{\n\t.reg .b64 st;\n\tmbarrier.arrive.shared::cta.b64 st, [%0];\n\t}" ::"r"(bar) : "memory");
 }
+// One arrival for a warp that is done reading a stage by ordinary loads.  The fence is what makes it wait for them: without it the
+// last load of a stage could still be on its way, past the arrival, when the next copy landed (INT4 streaming kernel, dense with K =
+// 1024: the last sixteen bytes of a row belonged to the next strip in up to 3 of 100 launches).  Kernels whose loads feed a tensor-memory
+// store that they wait for need no fence.
+__device__ __forceinline__ void mbar_arrive_read(uint32_t bar) {
+  asm volatile("fence.acq_rel.cta;" ::: "memory");
+  __syncwarp();
+  if ((threadIdx.x & 31) == 0) mbar_arrive(bar);
+}
 __device__ __forceinline__ void mbar_expect_tx(uint32_t bar, uint32_t bytes) {
   asm volatile("{\n\t.reg .b64 st;\n\tmbarrier.arrive.expect_tx.shared::cta.b64 st, [%0], %1;\n\t}" ::"r"(bar), "r"(bytes)
                : "memory");

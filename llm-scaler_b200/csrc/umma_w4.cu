@@ -783,8 +783,7 @@ umma_w4_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constant__
           as += C::A_ROUND; if (as >= S) { as -= S; apar ^= 1u; }
         }
         if (!ok) break;
-        __syncwarp();
-        if (WT != WT_W8 && elected) mbar_arrive(sc_empty + 8 * ss);
+        if (WT != WT_W8) mbar_arrive_read(sc_empty + 8 * ss);
         __syncwarp();
         if (++ss == C::SCS) { ss = 0; spar ^= 1u; }
       }

@@ -415,15 +415,13 @@ w4_stream_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constant
                 acc[i2][2] += sb * (u[i2][2] + v[i2][2]); acc[i2][3] += sb * (u[i2][3] + v[i2][3]);
               }
             }
-            __syncwarp();
-            if (lane == 0) mbar_arrive(empty + 8 * s);
+            mbar_arrive_read(empty + 8 * s);
           }
           if (++s == RS) { s = 0; par ^= 1u; }
         }
         if (!ok) break;
         j = 0;
-        __syncwarp();
-        if (lane == 0) mbar_arrive(sc_empty + 8 * ss);
+        mbar_arrive_read(sc_empty + 8 * ss);
         if (++ss == SCS) { ss = 0; spar ^= 1u; }
       }
       // The block's two warps add up; the first delivers.  They meet twice, so that the buffer is free again before the next

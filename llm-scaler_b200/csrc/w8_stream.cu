@@ -257,8 +257,7 @@ __global__ void __launch_bounds__(w8s::THREADS, 2) w8_stream_kernel(const __grid
         else if (w < C::KG) step(std::integral_constant<int, 4>{});
         else step(std::integral_constant<int, H - 4>{});
       }
-      __syncwarp();
-      if (lane == 0) mbar_arrive(empty + 8 * s);
+      mbar_arrive_read(empty + 8 * s);
       if (++s == p.ns) { s = 0; par ^= 1u; }
     }
     // The warps of a group add up.  All meet twice, so that the buffer is free again before the next pass, and go on only if none

@@ -155,3 +155,22 @@ def test_silu_mul_refuses_outputs_it_would_write_beyond(e, native):
         with pytest.raises(RuntimeError):
             op(*args)
     assert op(x, torch.zeros(6, 32, dtype=torch.bfloat16, device=DEV), 64, 32, 100).shape == (6, 32)
+
+
+@pytest.mark.parametrize("H", [640, 768, 1024])
+def test_expert_decode_repeats_bit_for_bit(e, H):
+    """Many launches of several short segments per CTA: stages that are handed back to the producer too early show as a row of one tile
+    that differs now and then."""
+    g = torch.Generator(device=DEV).manual_seed(H)
+    T, E, k, Ii, dtype = 128, 64, 8, 384, torch.float16
+    x, logits = torch.randn(T, H, generator=g, device=DEV).to(dtype), torch.randn(T, E, generator=g, device=DEV).to(dtype)
+    (w13, s13), (w2, s2) = _int4(g, E, N=2 * Ii, K=H, dtype=dtype), _int4(g, E, N=H, K=Ii, dtype=dtype)
+    (gu, gus), (dn, dns) = _int4(g, N=2 * Ii, K=H, dtype=dtype), _int4(g, N=H, K=Ii, dtype=dtype)
+    gate = (torch.randn(1, H, generator=g, device=DEV) / H ** 0.5).to(dtype)
+    gus, dns = gus.t().contiguous(), dns.t().contiguous()
+    e.set_force_kernel(7)
+    try:
+        outs = [e.moe_forward_full_int4(x, logits, w13, s13, gu, gus, w2, s2, dn, dns, gate, k, 1, E, True) for _ in range(400)]
+    finally:
+        e.set_force_kernel(0)
+    assert len({o.cpu().numpy().tobytes() for o in outs}) == 1

@@ -121,3 +121,26 @@ def test_without_room_for_partial_sums_the_other_kernel_takes_strips_that_should
             outs.append(out)
         for out in outs:
             _close(out, _exact(x.cpu(), q, s), torch.bfloat16)
+
+
+@pytest.mark.parametrize("K", [1024, 512, 768])
+def test_a_stage_is_read_before_it_is_overwritten(e, K):
+    """Three strips per CTA, a nibble of its own for each, and tokens that each see one group: what a stage loses to the copy that follows it,
+    in whichever of many launches, is another strip's value.  (Whole strips: no scratch.)"""
+    L = e._lib
+    per = 2 * torch.cuda.get_device_properties(0).multi_processor_count
+    N, G = per * 3 * 128, K // 128
+    nib = (torch.arange(per * 3, device=DEV) // per * 4 + 3).repeat_interleave(128)
+    word = sum(nib << (4 * j) for j in range(8))
+    w = torch.where(word >= 2 ** 31, word - 2 ** 32, word).to(torch.int32)[:, None].expand(N, K // 8).contiguous()
+    s, x = torch.ones(N, G, device=DEV, dtype=torch.float16), torch.zeros(G, K, device=DEV, dtype=torch.float16)
+    for m in range(G):
+        x[m, m * 128:(m + 1) * 128] = 1
+    ref = ((nib - 8) * 128).to(torch.float16).expand(G, N)
+    out = torch.empty(G, N, device=DEV, dtype=torch.float16)
+    wrong = 0
+    for _ in range(500):
+        assert L.lib.b2q_linear_int4(x.data_ptr(), L.F16, K, w.data_ptr(), L.W4_NMAJOR, s.data_ptr(), L.F16, G, 1, out.data_ptr(), N, G, N, K, 128, None, 0,
+                                     torch.cuda.current_stream().cuda_stream) == 0
+        wrong += not torch.equal(out, ref)
+    assert e.last_kernel() == "w4_stream" and wrong == 0

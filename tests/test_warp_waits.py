@@ -101,3 +101,29 @@ def test_kernels_that_start_early_read_their_inputs_by_ordinary_loads():
     """The read-only path promises that nothing is written while the kernel runs, and these run while their inputs are written."""
     with open(os.path.join(CSRC, "moe_aux.cu")) as f:
         assert _read_only_loads(f.read()) == []
+
+
+# Stages that warps read by ordinary loads, and that somebody overwrites after their arrival.  The loads of the tcgen05 kernels' raw
+# stages feed tensor-memory stores that are waited for in front of the arrival.
+READ_STAGES = {"w4_stream.cu": ["empty", "sc_empty"], "w8_stream.cu": ["empty"], "umma_w4.cu": ["sc_empty"]}
+
+
+@pytest.mark.parametrize("name", sorted(READ_STAGES))
+def test_a_stage_is_released_behind_its_loads(name):
+    """mbar_arrive() alone lets the last loads of a stage pass the arrival; mbar_arrive_read() fences them."""
+    with open(os.path.join(CSRC, name)) as f:
+        text = re.sub(r"//[^\n]*", "", f.read())
+    for bar in READ_STAGES[name]:
+        assert len(re.findall(r"\bmbar_arrive_read\(%s \+" % bar, text)) == 1
+        assert not re.search(r"\bmbar_arrive\(%s \+" % bar, text)
+    with open(os.path.join(CSRC, "sm100.cuh")) as f:
+        body = re.search(r"void mbar_arrive_read\(uint32_t bar\) \{(.*?)\n\}", f.read(), re.S).group(1)
+    assert body.index("fence.acq_rel.cta") < body.index("__syncwarp()") < body.index("mbar_arrive(bar)")
+
+
+@pytest.mark.parametrize("name", ["umma_gemm.cu", "umma_w4.cu", "umma_w4_i8.cu"])
+def test_raw_stages_are_released_behind_the_stores_that_they_feed(name):
+    with open(os.path.join(CSRC, name)) as f:
+        text = re.sub(r"//[^\n]*", "", f.read())
+    at = text.index("mbar_arrive(raw_empty +")
+    assert max(text.rfind("lds128(", 0, at), text.rfind("lds32(", 0, at)) < text.rfind("tmem_st_wait()", 0, at)
