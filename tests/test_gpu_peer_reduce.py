@@ -129,9 +129,9 @@ def test_rejects_shapes_outside_the_contract(L):
 
 
 @pytest.mark.parametrize("M,N,K,kmajor", [
-    (64, 2048, 14336, False), (16, 8192, 14336, False), (40, 5120, 8192, True),    # strips cut along k: partial sums, then delivery
-    (64, 2048, 4096, False), (40, 5120, 2560, True), (33, 18944, 512, False),      # whole strips, one per SM at most
-    (64, 37888, 512, False), (48, 40960, 768, False), (48, 40960, 4096, False),    # 256-row strips: whole, whole with two rounds, cut
+    (64, 2048, 4096, False), (16, 8192, 14336, False), (40, 5120, 2560, True),     # strips cut along k: partial sums, then delivery
+    (33, 18944, 512, False),                                                       # one whole strip per SM
+    (64, 37888, 512, False), (48, 40960, 768, False),                              # 256-row strips, whole and cut
 ])
 @pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16])
 @pytest.mark.parametrize("scratch", [True, False])                                 # without it the two-CTA kernel delivers
@@ -168,3 +168,12 @@ def test_gemm_epilogue_delivers_its_strips(L, M, N, K, kmajor, dtype, scratch):
         assert v.value == 0 and L.device_status() == 0
     finally:
         L.lib.b2q_comm_destroy(comm)
+
+
+@pytest.mark.parametrize("M,N,K,kmajor", [(64, 2048, 14336, False), (40, 5120, 8192, True), (48, 40960, 4096, False)])
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16])
+@pytest.mark.parametrize("scratch", [True, False])
+def test_gemm_epilogue_delivers_cut_strips(L, M, N, K, kmajor, dtype, scratch):
+    """The same where k is long enough for strips to be cut, N-major, K-major and 256 rows high: partial sums, then delivery."""
+    assert L.lib.b2q_linear_workspace_bytes(M, N, K) >= 2 * M * K + 4 * M + 2 * 64 * 64 * 4      # partial sums behind the pre-pass's part
+    test_gemm_epilogue_delivers_its_strips(L, M, N, K, kmajor, dtype, scratch)

@@ -258,10 +258,10 @@ def test_bounded_wait_gives_up_and_reports(e):
     and the context is still usable for the next launch."""
     L = e._lib
     assert L.device_status() == 0
-    # a decode launch whose strips are cut along K (few strips, many SMs): it relies on arrival counts, whose tags the reset
-    # below changes together with the status words of every kernel family
-    qb, sb = _int4(2048, 14336, torch.bfloat16, 5)
-    xb = torch.randn(40, 14336, generator=torch.Generator().manual_seed(5)).to(torch.bfloat16).to(DEV)
+    # a decode launch whose strips are cut along K (few strips, many SMs): it relies on the arrival counters that the
+    # reset below clears together with the status words of every kernel family
+    qb, sb = _int4(2048, 4096, torch.bfloat16, 5)
+    xb = torch.randn(40, 4096, generator=torch.Generator().manual_seed(5)).to(torch.bfloat16).to(DEV)
     wb, sbd = int4.pack_nmajor_u8(qb).to(DEV), sb.to(DEV)
     before = torch.empty(40, 2048, dtype=torch.bfloat16, device=DEV)
     e.esimd_gemm_int4_pgrp(xb, wb, sbd, before)
@@ -279,3 +279,19 @@ def test_bounded_wait_gives_up_and_reports(e):
     e.esimd_gemm_int4_pgrp(x.to(DEV), int4.pack_nmajor_u8(q).to(DEV), s.to(DEV), out)
     assert_close(out, int4.linear(x, q, s), what="launch after an expired wait")
     assert L.device_status() == 0
+
+
+def test_cut_strips_around_the_reset(e):
+    """A decode launch whose strips are cut along K relies on arrival counts, whose tags the reset changes together with the status words
+    of every kernel family: the same bits before and after it."""
+    L = e._lib
+    q, s = _int4(2048, 14336, torch.bfloat16, 5)
+    x = torch.randn(40, 14336, generator=torch.Generator().manual_seed(5)).to(torch.bfloat16)
+    outs = [torch.empty(40, 2048, dtype=torch.bfloat16, device=DEV) for _ in range(2)]
+    xd, w, sd = x.to(DEV), int4.pack_nmajor_u8(q).to(DEV), s.to(DEV)
+    e.esimd_gemm_int4_pgrp(xd, w, sd, outs[0])
+    assert L.selftest_bounded_wait(code=778) is True and L.device_status() == 778
+    L.device_status_reset()
+    e.esimd_gemm_int4_pgrp(xd, w, sd, outs[1])
+    assert torch.equal(*outs) and L.device_status() == 0
+    assert_close(outs[1], int4.linear(x, q, s), what="cut-strip launch after the reset")

@@ -42,8 +42,7 @@ def _check(out, ref, what, rounding=2.0 ** -8):
 @pytest.mark.parametrize("scale_dtype", [torch.bfloat16, torch.float16, torch.float32])
 @pytest.mark.parametrize("M,N,K", [
     (1, 128, 128), (16, 136, 384), (17, 1000, 1024),     # one tile; ragged strip; odd group count; aligned scale fetch
-    (33, 520, 2560), (64, 2048, 4096),                   # 64-token tile
-    (33, 520, 14336), (64, 2048, 14336),                 # cut strips, the last of them ragged; without rest
+    (33, 520, 2560), (64, 2048, 4096),                   # 64-token tile, cut strips
     (65, 300, 1280), (128, 1032, 2048),                  # 128-token tile, one of them
     (129, 384, 640), (400, 2184, 1152),                  # several token tiles, odd group counts
 ])
@@ -61,6 +60,13 @@ def test_tile_and_group_edges(e, M, N, K, scale_dtype):
     assert e._lib.device_status() == 0
 
 
+@pytest.mark.parametrize("scale_dtype", [torch.bfloat16, torch.float16, torch.float32])
+@pytest.mark.parametrize("M,N,K", [(33, 520, 14336), (64, 2048, 14336)])
+def test_cut_tile_edges(e, M, N, K, scale_dtype):
+    """Long k, where cuts pay: the last strip ragged; without rest."""
+    test_tile_and_group_edges(e, M, N, K, scale_dtype)
+
+
 def test_the_strips_called_cut_are_cut(e):
     """Scratch beyond the pre-pass's part is asked for where strips are cut."""
     up = lambda n: (n + 255) // 256 * 256
@@ -71,7 +77,7 @@ def test_the_strips_called_cut_are_cut(e):
         assert e._lib.lib.b2q_linear_fp8_workspace_bytes(M, N, K) >= up(2 * M * K) + up(4 * M) + 2 * ((N + 127) // 128) * 128 * tok * 4, (M, N, K)
 
 
-@pytest.mark.parametrize("M,N,K", [(16, 8192, 14336), (64, 8192, 14336), (64, 38016, 2048), (64, 38016, 8192), (100, 10240, 8192), (700, 8192, 2048),
+@pytest.mark.parametrize("M,N,K", [(16, 8192, 14336), (64, 8192, 14336), (64, 38016, 2048), (100, 10240, 8192), (700, 8192, 2048),
                                    (100, 4096, 14336), (128, 12288, 14336), (96, 520, 8192)])    # 128-token tiles cut into equal pieces, over the whole grid, ragged
 def test_many_segments_repeat_bit_for_bit(e, M, N, K):
     x, w, s, ref = _case(M, N, K, torch.bfloat16, 7)
@@ -87,9 +93,13 @@ def test_many_segments_repeat_bit_for_bit(e, M, N, K):
     assert e._lib.device_status() == 0
 
 
+def test_many_cut_segments_of_256_rows_repeat_bit_for_bit(e):
+    """Ragged strips of 256 rows, cut."""
+    test_many_segments_repeat_bit_for_bit(e, 64, 38016, 8192)
+
+
 @pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16])
-@pytest.mark.parametrize("M,N,K", [(1, 128, 128), (16, 200, 384), (17, 1032, 640), (33, 2048, 1152), (64, 8192, 5120), (27, 17408, 5120),
-                                   (17, 1032, 8192), (60, 1000, 14336)])              # cut strips, the last of them ragged
+@pytest.mark.parametrize("M,N,K", [(1, 128, 128), (16, 200, 384), (17, 1032, 640), (33, 2048, 1152), (64, 8192, 5120), (27, 17408, 5120)])
 def test_block_scaled_fp8_strips(e, M, N, K, dtype):
     """The e4m3 form of the kernel: a weight times its fp32 block scale is rounded to fp16 once, as above; with fp16
     output the tolerance is 2^-11 for the output's rounding and the same 2^-9 of a typical column for the weights'."""
@@ -109,6 +119,13 @@ def test_block_scaled_fp8_strips(e, M, N, K, dtype):
             _check(out, ref, (M, N, K), 2.0 ** -8 if dtype == torch.bfloat16 else 2.0 ** -11)
         assert torch.equal(out, first)
     assert e._lib.device_status() == 0
+
+
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16])
+@pytest.mark.parametrize("M,N,K", [(17, 1032, 8192), (60, 1000, 14336)])
+def test_block_scaled_fp8_cut_strips(e, M, N, K, dtype):
+    """The last of the cut strips ragged."""
+    test_block_scaled_fp8_strips(e, M, N, K, dtype)
 
 
 @pytest.mark.parametrize("rows", [(1, 0, 3, 16, 2), (40, 17, 0, 31, 33), (64, 65, 130, 1, 40)])

@@ -11,7 +11,7 @@ import re
 import pytest
 
 CSRC = os.path.join(os.path.dirname(os.path.dirname(os.path.abspath(__file__))), "llm-scaler_b200", "csrc")
-KERNELS = sorted(f for f in os.listdir(CSRC) if re.match(r"umma_.*\.cu$|w\d_stream\.cu$", f))
+KERNELS = sorted(f for f in os.listdir(CSRC) if f.startswith("umma_") and f.endswith(".cu"))
 
 
 def _per_lane_waits(text):
@@ -51,7 +51,20 @@ def test_copies_in_flight_are_waited_for(name):
         # one drain per elected producer, one wait behind asynchronous copies that arrive on a barrier
         producers = sum(bool(re.search(r"\btma_load_2d(_pair)?\(", part)) for part in text.split("if (elect_one()) {")[1:])
         assert text.count("drain_issued(") == producers
-        assert ("cp_async_arrive(" in text) == ("cp_async_wait_all()" in text or "cp.async.wait_all" in text)
+        assert ("cp_async_arrive(" in text) == ("cp_async_wait_all()" in text)
+
+
+STREAMS = ["w4_stream.cu", "w8_stream.cu"]
+
+
+@pytest.mark.parametrize("name", STREAMS)
+def test_streaming_kernels_wait_together_and_for_their_copies(name):
+    with open(os.path.join(CSRC, name)) as f:
+        source = f.read()
+    assert _per_lane_waits(source) == []
+    for text in source.split("__global__ ")[1:]:
+        assert text.count("drain_issued(") == sum("tma_load_2d(" in part for part in text.split("if (elect_one()) {")[1:]) == 1
+        assert "cp_async_arrive(" in text and "cp.async.wait_all" in text
 
 
 def _unconverged_barriers(text):
