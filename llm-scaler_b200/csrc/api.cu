@@ -242,13 +242,13 @@ static int linear_int4_core(const void* x, int act_dtype, int64_t ldx, const voi
     return umma_w4_i8_linear(ia, st);
   }
   // up to eight tokens, weights worth streaming: w4_stream.cu (w4_stream_preferred has the line and both sides of it)
-  if (!peer && !kmajor && (force == 7 ? M <= W4_STREAM_MAX_TOK : force == 0 && w4_stream_preferred(M, N, K, workspace, workspace ? workspace_bytes : 0))) {
+  if (!peer && !kmajor && M <= W4_STREAM_MAX_TOK && (force == 7 || force == 0)) {
     W4StreamArgs sa{};
     sa.x = x; sa.ldx = ldx; sa.bf16 = act_dtype == B2Q_BF16;
     sa.w = w; sa.layout = w_layout; sa.scale = scale; sa.scale_dtype = scale_dtype; sa.s_stride_n = s_stride_n; sa.s_stride_g = s_stride_g;
     sa.out = out; sa.ldo = ldo; sa.M = (int)M; sa.N = (int)N; sa.K = (int)K; sa.tile = (int)M;
     sa.partials = workspace; sa.partial_bytes = workspace ? workspace_bytes : 0;
-    if (w4_stream_supported(sa)) return w4_stream_linear(sa, st);
+    if (w4_stream_supported(sa) && (force == 7 || w4_stream_preferred(sa))) return w4_stream_linear(sa, st);
   }
   // The tcgen05 kernel is flat in M up to 64 and the only one for K-major layouts and prefill.
   // small weights at small M: one launch of the streaming kernel beats pre-pass + GEMM (16 / 32 tokens: 1024 x 1024 3.5 / 5.4

@@ -565,14 +565,26 @@ static int launch_scale(int sd, bool gated, const CUtensorMap& tw, const CUtenso
 
 static bool room(const W4SPlan& pl, const void* partials, size_t bytes) { return partials && aligned16(partials) && bytes >= pl.partial_bytes; }
 
-bool w4_stream_preferred(int64_t M, int64_t N, int64_t K, const void* partials, size_t partial_bytes) {
+// bytes of a row's scales per asynchronous copy: 16 or 4, 0 = element by element
+static int scale_bytes(const void* scale, int dtype, int64_t stride_n, int64_t stride_g, int groups) {
+  const int esz = dtype_bytes(dtype);
+  const uintptr_t at = reinterpret_cast<uintptr_t>(scale);
+  if (stride_g != 1) return 0;
+  if ((groups * esz) % 16 == 0 && (stride_n * esz) % 16 == 0 && (at & 15u) == 0) return 16;
+  return (groups * esz) % 4 == 0 && (stride_n * esz) % 4 == 0 && (at & 3u) == 0 ? 4 : 0;
+}
+
+bool w4_stream_preferred(const W4StreamArgs& a) {
+  const int64_t M = a.M, N = a.N, K = a.K;
   if (M > W4_STREAM_MAX_TOK) return false;
   const double k = (double)K / 1024.0;
   const int64_t slots = 3 * (int64_t)sm_count(), rounds = ((N + 15) / 16 + slots - 1) / slots;
   const double there = 1.0 + (double)rounds * (0.9 + 1.38 * k) * (1.0 + 0.02 * (double)(M - 1));
   const W4SPlan pl = plan(N, K);
   const double whole = 4.0 + (double)((pl.strips + 2 * sm_count() - 1) / (2 * sm_count())) * pl.sps;
-  const double here = pl.cut && !room(pl, partials, partial_bytes) ? whole : 9.5 + 0.1e-6 * (double)N * (double)K + 0.2 * k;
+  const double contributors = pl.cut ? (double)pl.grid / pl.strips : 1.0, sums = contributors > 10.0 ? 0.23 * (contributors - 10.0) : 0.0;
+  const double narrow = scale_bytes(a.scale, a.scale_dtype, a.s_stride_n, a.s_stride_g, a.K / 128) == 16 ? 0.0 : 1.0;
+  const double here = (pl.cut && !room(pl, a.partials, a.partial_bytes) ? whole : 9.5 + 0.1e-6 * (double)N * (double)K + 0.2 * k + sums) + narrow;
   return here < 0.97 * there;
 }
 
@@ -592,16 +604,8 @@ int w4_stream_linear(const W4StreamArgs& a, cudaStream_t st) {
   if (rc) return rc;
   W4SParams p{};
   p.x = a.x; p.ldx = a.ldx;
-  const int esz = dtype_bytes(a.scale_dtype), G = a.K / 128;
-  auto scales = [&](const void* sp, int64_t sn, int64_t sg) {
-    W4SParams::Scales sc{sp, sn, sg, 0};
-    const uintptr_t at = reinterpret_cast<uintptr_t>(sp);
-    if (sg == 1) {
-      if ((G * esz) % 16 == 0 && (sn * esz) % 16 == 0 && (at & 15u) == 0) sc.vec = 16;
-      else if ((G * esz) % 4 == 0 && (sn * esz) % 4 == 0 && (at & 3u) == 0) sc.vec = 4;
-    }
-    return sc;
-  };
+  const int G = a.K / 128;
+  auto scales = [&](const void* sp, int64_t sn, int64_t sg) { return W4SParams::Scales{sp, sn, sg, scale_bytes(sp, a.scale_dtype, sn, sg, G)}; };
   p.sc = scales(a.scale, a.s_stride_n, a.s_stride_g);
   p.s_expert_elems = (int64_t)a.N * G;
   p.shared_e = -1;

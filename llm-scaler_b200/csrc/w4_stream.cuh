@@ -31,7 +31,11 @@ size_t w4_stream_partial_bytes(int64_t M, int64_t N, int64_t K);
 // and 13.4, 28672 x 1024 13.0 / 13.9 and 11.5, 2048 x 16384 26.8 / 30.7 and 17.4, 10240 x 8192 27.2 / 30.5 and 17.9.
 // Strips that should be cut, with no room for their partial sums, stay whole, about 1 us per stage: one / eight tokens, there and here, 2048 x
 // 16384 25.6 / 29.9 and 38.8 / 44.1, 8192 x 8192 25.1 / 29.2 and 30.7 / 34.7, but 57344 x 8192 101 / 136 and 68 / 73, 24576 x 4096 24.9 and 18.9.
-bool w4_stream_preferred(int64_t M, int64_t N, int64_t K, const void* partials, size_t partial_bytes);
+// Few strips are cut into many pieces, and whoever comes last adds up all of a strip's sums: 0.23 us per contributor beyond ten.  Scales that
+// cannot be fetched 16 bytes at a time: 1 us more.  By 655 launches of N = 64 .. 57344 and K = 1024 .. 28672, seven of them 2 to 7 % slower by
+// the rule than on the other side, against over a hundred by up to 49 % without these two.  One token, there and here: 1024 x 8192 12.3 and 17.9, 512 x 8192
+// 11.7 and 17.4, 256 x 16384 25.2 and 28.3, but 1024 x 16384 26.2 and 20.0, 512 x 28672 46.7 and 32.7; seven tokens, 69 groups, 2128 x 8832 15.5 and 19.2.
+bool w4_stream_preferred(const W4StreamArgs& a);
 
 // Grouped launches of the expert pipeline: up to four rows per expert on average; from about six on tiles of eight tokens repeat too
 // much of the decoding.  Whole pass in us against the tcgen05 kernel behind its pre-passes, 128 experts of 2048 x 768, top-8, at 1 / 16 /

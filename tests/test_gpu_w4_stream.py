@@ -102,6 +102,17 @@ def test_dispatch_takes_it_where_the_other_kernel_needs_more_rounds(e):
         assert e.last_kernel() == name
 
 
+def test_dispatch_counts_the_sums_of_strips_cut_into_many_pieces(e):
+    """Few rows and long k: some thirty contributors to a strip cost more than the other kernel's one round takes."""
+    e.set_force_kernel(0)
+    for M, N, K, name in ((1, 1024, 8192, "smallm"), (8, 512, 8192, "smallm"), (1, 256, 16384, "smallm"), (7, 2128, 8832, "smallm"), (1, 1024, 16384, "w4_stream"), (4, 512, 28672, "w4_stream")):
+        x, q, w, s = _inputs(M, N, K, torch.bfloat16, torch.bfloat16)
+        out = torch.empty(M, N, dtype=torch.bfloat16, device=DEV)
+        e.esimd_gemm_int4_pgrp(x.to(DEV), w.to(DEV), s.to(DEV), out)
+        assert e.last_kernel() == name, (M, N, K)
+        _close(out, _exact(x, q, s), torch.bfloat16)
+
+
 def test_without_room_for_partial_sums_the_other_kernel_takes_strips_that_should_be_cut(e):
     """Scratch is the caller's choice in the C ABI: none, less than asked for, unaligned.  37888 x 1024 is whole strips in any case, and so
     many strips as 24576 x 4096 has are better off whole than there."""
