@@ -995,6 +995,10 @@ int umma_w4_prep_linear(const UmmaW4Args& a, cudaStream_t st) {
 // (512 x 12288 x 5120, block scales, 75 against 73 us).  128 x 17408 x 5120, block scales: 56 -> 36 us, 1221 x 4680 x 2048 43 -> 37;
 // 4001 x 17408 x 5120 stays where it was, 587 us against 645 here.  So do up to 4 Mi weights at up to 128 tokens, although they
 // would gain up to 5 us (100 x 2048 x 2048, block scales: 17.6 against 13.1): test_gpu_w4_strips.py names the kernel of such a call.
+// Up to k of 512 the MMAs no longer hide the output's way out, the less so where its rows are not 16-byte aligned: 1 us more per round
+// against the 256-token tiles, 3 where unaligned, 1 with longer k.  3000 x 1466 x 128, per tensor, 12.8 against 9.1 us there, 151 x 12072 x 256 12.5
+// against 10.5, 217 x 16422 x 640, block scales, 17.1 against 14.1.  Over 462 launches of N = 64 .. 28672, K = 128 .. 2560 and 65 to 4096 tokens, half of
+// them unaligned, 16 that the rule takes are 2 to 9 % slower here; without this term 59 were, by up to 49 %.
 static bool w8_strips_pay(const UmmaW8Args& a) {
   if (a.M <= 128 && (int64_t)a.N * a.K <= (4 << 20)) return false;
   const int sms = sm_count();
@@ -1002,7 +1006,8 @@ static bool w8_strips_pay(const UmmaW8Args& a) {
   const double k = a.K / 1024.0;
   const bool block = a.scale_mode == B2Q_SCALE_BLOCK128;
   auto rounds = [](int64_t work, int64_t slots) { return (double)((work + slots - 1) / slots); };
-  const double here = (block ? 4.67 : 5.93) + rounds(strips * ((a.M + 127) / 128), sms) * (block ? 1.16 + 4.08 * k : 0.74 + 3.31 * k);
+  const double stores = aligned16(a.out) && (a.ldo % 8) == 0 ? (a.K <= 512 && a.M > 128 ? 1.0 : 0.0) : (a.K <= 512 ? 3.0 : 1.0);
+  const double here = (block ? 4.67 : 5.93) + rounds(strips * ((a.M + 127) / 128), sms) * (stores + (block ? 1.16 + 4.08 * k : 0.74 + 3.31 * k));
   const double there = a.M <= 128 ? (block ? 2.98 : 3.57) + rounds(strips, 2 * (int64_t)sms) * (block ? 2.98 + 6.26 * k : 3.57 + 4.18 * k)
                                   : (block ? 1.30 : 1.70) + rounds(strips * ((a.M + 255) / 256), sms) * (block ? 8.92 + 5.56 * k : 8.39 + 5.36 * k);
   return here < 0.95 * there;

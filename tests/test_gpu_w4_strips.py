@@ -237,6 +237,26 @@ def test_fp8_dense_above_64_tokens_strips(e, M, N, K, mode, dtype):
     assert e._lib.device_status() == 0
 
 
+@pytest.mark.parametrize("M,N,K,mode,kernel", [(217, 16422, 640, "block", "umma_wo"), (217, 16424, 640, "block", "umma_w4"), (1611, 1890, 768, "tensor", "umma_wo"),
+                                               (1611, 1896, 768, "tensor", "umma_w4"), (151, 12072, 256, "tensor", "umma_wo")])
+def test_fp8_dense_above_64_tokens_short_k_route_by_alignment(e, M, N, K, mode, kernel):
+    """Rows of output that are not 16-byte aligned, and their aligned neighbours (tolerance as above)."""
+    g = torch.Generator(device=DEV).manual_seed(M + N + K)
+    w = (torch.randn(N, K, generator=g, device=DEV) * 96).clamp_(-448, 448).to(torch.float8_e4m3fn)
+    x = torch.randn(M, K, generator=g, device=DEV).to(torch.bfloat16)
+    s = (0.5 + torch.rand(*(((N + 127) // 128, K // 128) if mode == "block" else (1,)), generator=g, device=DEV)) / 4096
+    full = s.double().repeat_interleave(128, 0)[:N].repeat_interleave(128, 1) if mode == "block" else s.double()
+    ref = x.double() @ (w.double() * full).T
+    out = torch.full((M, N), float("nan"), dtype=torch.bfloat16, device=DEV)
+    if mode == "block":
+        e.esimd_gemm_fp8_blockscale(x, w, s, out)
+    else:
+        e.esimd_gemm_fp8_pert(x, w, s, out)
+    assert e.last_kernel() == kernel
+    assert float((out.double() - ref).norm() / ref.norm()) < 2.0 ** -8
+    assert e._lib.device_status() == 0
+
+
 @pytest.mark.parametrize("E,rows,N,K", [
     (3, (60, 0, 33), 1096, 640),                       # 64-token tiles, short strips: few pieces
     (2, (129, 200), 520, 1152),                        # 128-token tiles, short strips
