@@ -1189,15 +1189,15 @@ int act_split_i8(const void* x, bool in_bf16, int64_t ldx, void* xq, float* inv_
 // skips the add and leaves the residual untouched, and a second weight writes a second normalised row from the same
 // 1/rms (esimd_norm_gemv_norm_fp16, csrc/xpu/esimd_kernels/norm_gemv_norm_fp16.h:56-98).
 //
-// Latency-bound (a row or a few): a thread's first two chunks of eight stay in registers between the sum and the output, so inputs and
-// weight are fetched once and together (K up to 8192, beyond that the rest is read again); every thread adds up the warps' sums
-// itself.  Where the weights of the next kernel may be fetched at any time (overlap mode 2) that kernel may start at once.
+// A row's inputs are read twice, the second time from L1, and 32 registers let two CTAs of 1024 threads share an SM: 8192 x 4096 46 us, 78 with the
+// inputs held in registers in between; 2048 x 8192 27 us, 40 with 34 registers; a few rows take the same either way.  Where the weights of the next kernel may be fetched at any time (overlap mode 2) that kernel may start at once.
 template <bool BF16>
-__global__ void __launch_bounds__(512) resadd_rmsnorm_kernel(const void* __restrict__ hidden, void* __restrict__ residual, const void* __restrict__ weight,
+__global__ void __launch_bounds__(1024, 2) resadd_rmsnorm_kernel(const void* __restrict__ hidden, void* __restrict__ residual, const void* __restrict__ weight,
                                       void* __restrict__ normed, const void* __restrict__ weight2, void* __restrict__ normed2,
                                       int K, float eps, float scalar, int release_early) {
   using T = typename Act<BF16>::T;
   __shared__ float red[32];
+  __shared__ float inv_sh;
   if (release_early) grid_dep_release();
   grid_dep_wait();
   if (!release_early) grid_dep_release();
@@ -1208,50 +1208,43 @@ __global__ void __launch_bounds__(512) resadd_rmsnorm_kernel(const void* __restr
   const T* w2 = reinterpret_cast<const T*>(weight2);
   T* out = reinterpret_cast<T*>(normed) + r * K;
   T* out2 = normed2 ? reinterpret_cast<T*>(normed2) + r * K : nullptr;
-  constexpr int NC = 2;
-  const int k0 = threadIdx.x * 8, step = blockDim.x * 8;
-  uint4 rv[NC], hv[NC], wv[NC];
-  auto fetch = [&](int k, uint4& a, uint4& b, uint4& c) {
-    a = ld_shared_vec(res + k);
-    if (h) b = ld_shared_vec(h + k);
-    c = ld_shared_vec(w + k);
-  };
-  auto value = [&](const uint4& a, const uint4& b, float (&v)[8]) {
-    const T* re = reinterpret_cast<const T*>(&a);
-    const T* he = reinterpret_cast<const T*>(&b);
+  auto load8 = [&](int k, float (&v)[8]) {
+    const uint4 rv = ld_shared_vec(res + k);
+    const T* re = reinterpret_cast<const T*>(&rv);
+    if (h) {
+      const uint4 hv = ld_shared_vec(h + k);
+      const T* he = reinterpret_cast<const T*>(&hv);
 #pragma unroll
-    for (int j = 0; j < 8; ++j) v[j] = h ? (Act<BF16>::to_f(he[j]) + Act<BF16>::to_f(re[j])) * scalar : Act<BF16>::to_f(re[j]);
-  };
+      for (int j = 0; j < 8; ++j) v[j] = (Act<BF16>::to_f(he[j]) + Act<BF16>::to_f(re[j])) * scalar;
+    } else {
 #pragma unroll
-  for (int i = 0; i < NC; ++i)
-    if (k0 + i * step < K) fetch(k0 + i * step, rv[i], hv[i], wv[i]);
+      for (int j = 0; j < 8; ++j) v[j] = Act<BF16>::to_f(re[j]);
+    }
+  };
   float ss = 0.f;
-  auto square = [&](const uint4& a, const uint4& b) {
+  for (int k = threadIdx.x * 8; k < K; k += blockDim.x * 8) {
     float v[8];
-    value(a, b, v);
+    load8(k, v);
 #pragma unroll
     for (int j = 0; j < 8; ++j) ss = fmaf(v[j], v[j], ss);
-  };
-#pragma unroll
-  for (int i = 0; i < NC; ++i)
-    if (k0 + i * step < K) square(rv[i], hv[i]);
-  for (int k = k0 + NC * step; k < K; k += step) {
-    uint4 a, b, c;
-    fetch(k, a, b, c);
-    square(a, b);
   }
 #pragma unroll
   for (int o = 16; o > 0; o >>= 1) ss += __shfl_xor_sync(0xffffffffu, ss, o);
   if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = ss;
   __syncthreads();
-  float t = 0.f;
-  for (int i = 0; i < (int)(blockDim.x >> 5); ++i) t += red[i];
-  const float inv = rsqrtf(t / (float)K + eps);
+  if (threadIdx.x == 0) {
+    float t = 0.f;
+    for (int i = 0; i < (int)(blockDim.x >> 5); ++i) t += red[i];
+    inv_sh = rsqrtf(t / (float)K + eps);
+  }
+  __syncthreads();
+  const float inv = inv_sh;
   // only now is the residual overwritten, each element by the thread that read it
-  auto deliver = [&](int k, const uint4& a, const uint4& b, const uint4& c) {
+  for (int k = threadIdx.x * 8; k < K; k += blockDim.x * 8) {
     float v[8];
-    value(a, b, v);
-    const T* we = reinterpret_cast<const T*>(&c);
+    load8(k, v);
+    const uint4 wv = ld_shared_vec(w + k);
+    const T* we = reinterpret_cast<const T*>(&wv);
     uint4 so, no;
     T* se = reinterpret_cast<T*>(&so);
     T* ne = reinterpret_cast<T*>(&no);
@@ -1269,14 +1262,6 @@ __global__ void __launch_bounds__(512) resadd_rmsnorm_kernel(const void* __restr
       for (int j = 0; j < 8; ++j) ne[j] = Act<BF16>::from_f(v[j] * inv * Act<BF16>::to_f(w2e[j]));
       *reinterpret_cast<uint4*>(out2 + k) = no;
     }
-  };
-#pragma unroll
-  for (int i = 0; i < NC; ++i)
-    if (k0 + i * step < K) deliver(k0 + i * step, rv[i], hv[i], wv[i]);
-  for (int k = k0 + NC * step; k < K; k += step) {
-    uint4 a, b, c;
-    fetch(k, a, b, c);
-    deliver(k, a, b, c);
   }
 }
 
@@ -1284,7 +1269,7 @@ int resadd_rmsnorm(const void* hidden, void* residual, const void* weight, void*
                    bool bf16, int64_t M, int K, float eps, float scalar, cudaStream_t st) {
   if (M == 0) return B2Q_OK;
   int threads = (K / 8 + 31) / 32 * 32;
-  threads = threads > 512 ? 512 : (threads < 32 ? 32 : threads);      // room beside a CTA of the kernels around it
+  threads = threads > 1024 ? 1024 : (threads < 32 ? 32 : threads);
   const bool overlap = tls().overlap_mode > 0;
   cudaError_t e;
   if (bf16) e = launch_overlapped(resadd_rmsnorm_kernel<true>, dim3((unsigned)M), dim3(threads), 0, st, overlap, hidden, residual, weight, normed, weight2, normed2, K, eps, scalar, tls().overlap_mode == 2 ? 1 : 0);

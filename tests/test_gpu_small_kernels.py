@@ -1,0 +1,49 @@
+"""The small kernels between the linears at the edges of what a thread fetches at once: rows of a norm beyond what one pass of a CTA holds, many
+rows, experts that leave a lane's last logits empty.  Against fp64; the output is rounded once, 2^-9 of an element in bf16, 2^-12 in
+fp16, and the fp32 sums in front of it are exact to some 2^-18: twice the rounding in all."""
+import os
+import re
+
+import pytest
+import torch
+
+from gpu_util import DEV
+
+pytestmark = pytest.mark.gpu
+TOL = {torch.bfloat16: 2.0 ** -8, torch.float16: 2.0 ** -11}
+
+
+@pytest.fixture(scope="module")
+def impl():
+    from custom_esimd_kernels_vllm import _impl
+    return _impl
+
+
+def _close(out, ref, dtype):
+    err = (out.double() - ref).abs() - TOL[dtype] * ref.abs() - (2.0 ** -24 if dtype == torch.float16 else 0.0)
+    assert float(err.max()) <= 0, float(err.max())
+
+
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16])
+@pytest.mark.parametrize("M,K", [(1, 8), (3, 1032), (700, 4096), (2, 8192), (5, 8200), (300, 16392)])
+def test_residual_norm(impl, dtype, M, K):
+    g = torch.Generator(device=DEV).manual_seed(M + K)
+    h, r, w, w2 = (torch.randn(*s, generator=g, device=DEV).to(dtype) for s in ((M, K), (M, K), (K,), (K,)))
+    v = h.float() + r.float()
+    n = v.double() * (v.double().pow(2).mean(1, keepdim=True) + 1e-6).rsqrt()
+    res, out, out2 = r.clone(), torch.empty_like(r), torch.empty_like(r)
+    impl.resadd_rmsnorm(h, res, w, out, 1e-6)
+    assert torch.equal(res, v.to(dtype))
+    _close(out, n * w.double(), dtype)
+    v = r.double()
+    n = v * (v.pow(2).mean(1, keepdim=True) + 1e-6).rsqrt()
+    impl.rmsnorm_fused(None, r, 1.0, w, out, w2, out2, 1e-6)
+    _close(out, n * w.double(), dtype)
+    _close(out2, n * w2.double(), dtype)
+
+
+def test_two_blocks_of_norm_rows_share_an_sm():
+    src = os.path.join(os.path.dirname(os.path.dirname(os.path.abspath(__file__))), "llm-scaler_b200", "csrc", "moe_aux.cu")
+    with open(src) as f:
+        text = f.read()
+    assert re.search(r"__launch_bounds__\(1024, 2\) resadd_rmsnorm_kernel\(", text) and "threads > 1024 ? 1024" in text[text.index("int resadd_rmsnorm("):]
