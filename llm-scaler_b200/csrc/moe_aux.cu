@@ -1418,17 +1418,34 @@ __global__ void gated_rmsnorm_kernel(const void* __restrict__ x, const void* __r
   const T* zr = reinterpret_cast<const T*>(z) + (int64_t)row * V;
   const T* w = reinterpret_cast<const T*>(weight);
   T* o = reinterpret_cast<T*>(out) + (int64_t)row * V;
-  auto in = [](const T* p) { return scalar_from_raw(ld_shared_u16(p), BF16 ? B2Q_BF16 : B2Q_F16); };
+  auto value = [](unsigned short raw) { return scalar_from_raw(raw, BF16 ? B2Q_BF16 : B2Q_F16); };
+  // A lane's first eight elements of all three are fetched together (V up to 256; beyond that one by one, x again in the second pass).  One by one:
+  // 16 x 256 4.6 us, now 2.7.
+  constexpr int NC = 8;
+  unsigned short xc[NC], zc[NC], wc[NC];
+#pragma unroll
+  for (int i = 0; i < NC; ++i)
+    if (lane + 32 * i < V) xc[i] = ld_shared_u16(xr + lane + 32 * i);
+#pragma unroll
+  for (int i = 0; i < NC; ++i)
+    if (lane + 32 * i < V) { zc[i] = ld_shared_u16(zr + lane + 32 * i); wc[i] = ld_shared_u16(w + lane + 32 * i); }
   float ss = 0.f;
-  for (int k = lane; k < V; k += 32) { const float v = in(xr + k); ss = fmaf(v, v, ss); }
+#pragma unroll
+  for (int i = 0; i < NC; ++i)
+    if (lane + 32 * i < V) { const float v = value(xc[i]); ss = fmaf(v, v, ss); }
+  for (int k = lane + 32 * NC; k < V; k += 32) { const float v = value(ld_shared_u16(xr + k)); ss = fmaf(v, v, ss); }
 #pragma unroll
   for (int off = 16; off > 0; off >>= 1) ss += __shfl_xor_sync(0xffffffffu, ss, off);
   const float inv = rsqrtf(ss / (float)V + eps);
-  for (int k = lane; k < V; k += 32) {
-    const float g = in(zr + k);
+  auto deliver = [&](int k, unsigned short xv, unsigned short zv, unsigned short wv) {
+    const float g = value(zv);
     const float silu = g / (1.f + __expf(-g));
-    o[k] = Act<BF16>::from_f(in(xr + k) * inv * in(w + k) * silu);
-  }
+    o[k] = Act<BF16>::from_f(value(xv) * inv * value(wv) * silu);
+  };
+#pragma unroll
+  for (int i = 0; i < NC; ++i)
+    if (lane + 32 * i < V) deliver(lane + 32 * i, xc[i], zc[i], wc[i]);
+  for (int k = lane + 32 * NC; k < V; k += 32) deliver(k, ld_shared_u16(xr + k), ld_shared_u16(zr + k), ld_shared_u16(w + k));
 }
 
 int gated_rmsnorm(const void* x, const void* z, const void* weight, void* out, bool bf16, int rows, int V, float eps, cudaStream_t st) {

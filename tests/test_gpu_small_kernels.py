@@ -47,3 +47,13 @@ def test_two_blocks_of_norm_rows_share_an_sm():
     with open(src) as f:
         text = f.read()
     assert re.search(r"__launch_bounds__\(1024, 2\) resadd_rmsnorm_kernel\(", text) and "threads > 1024 ? 1024" in text[text.index("int resadd_rmsnorm("):]
+
+
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16])
+@pytest.mark.parametrize("rows,V", [(1, 8), (3, 128), (5, 250), (700, 256), (2, 264), (9, 520)])
+def test_gated_norm(impl, dtype, rows, V):
+    g = torch.Generator(device=DEV).manual_seed(rows + V)
+    x, z, w = (torch.randn(*s, generator=g, device=DEV).to(dtype) for s in ((rows, V), (rows, V), (V,)))
+    xd, zd = x.double(), z.double()
+    ref = xd * (xd.pow(2).mean(1, keepdim=True) + 1e-6).rsqrt() * w.double() * zd / (1 + (-zd).exp())
+    _close(impl.gated_rmsnorm(x, z, w, 1e-6).view(rows, V), ref, dtype)
