@@ -42,6 +42,21 @@ __device__ __forceinline__ float load_scalar_cg(const void* p, int64_t i, int dt
   return scalar_from_raw(__ldcg(reinterpret_cast<const unsigned short*>(p) + i), dt);
 }
 
+// A lane's logits of a token, experts lane, lane + 32, ..., -inf beyond E: all of them requested before any is looked at (512 experts, 16
+// tokens, top-10: 5.7 us, 8.3 with a wait for each).
+template <int N> __device__ __forceinline__ void load_logits(const void* p, int64_t at, int lane, int E, int dt, float (&v)[N]) {
+  uint32_t raw[N];
+  if (dt == B2Q_F32) {
+#pragma unroll
+    for (int j = 0; j < N; ++j) raw[j] = __ldcg(reinterpret_cast<const unsigned int*>(p) + at + min(lane + 32 * j, E - 1));
+  } else {
+#pragma unroll
+    for (int j = 0; j < N; ++j) raw[j] = __ldcg(reinterpret_cast<const unsigned short*>(p) + at + min(lane + 32 * j, E - 1));
+  }
+#pragma unroll
+  for (int j = 0; j < N; ++j) v[j] = lane + 32 * j < E ? scalar_from_raw(raw[j], dt) : -INFINITY;
+}
+
 // ---------------------------------------------------------------------------
 // softmax -> top-k -> renormalise.  One warp per token; lane l owns experts
 // l, l+32, ... so loads are coalesced.  Selection order and tie rule follow
@@ -58,12 +73,9 @@ __global__ void moe_topk_kernel(const void* __restrict__ logits, int ldt, int64_
   if (tok >= T) return;
   float v[PER_LANE];
   float mx = -INFINITY;
+  load_logits(logits, tok * E, lane, E, ldt, v);
 #pragma unroll
-  for (int j = 0; j < PER_LANE; ++j) {
-    const int e = lane + 32 * j;
-    v[j] = e < E ? load_scalar_cg(logits, tok * E + e, ldt) : -INFINITY;
-    mx = fmaxf(mx, v[j]);
-  }
+  for (int j = 0; j < PER_LANE; ++j) mx = fmaxf(mx, v[j]);
 #pragma unroll
   for (int o = 16; o > 0; o >>= 1) mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, o));
   float sum = 0.f;
@@ -315,12 +327,9 @@ __global__ void __launch_bounds__(1024) moe_route_fused_kernel(const void* __res
   for (int tok = warp; tok < T; tok += 32) {
     float v[PER_LANE];
     float mx = -INFINITY;
+    load_logits(logits, (int64_t)tok * E, lane, E, ldt, v);
 #pragma unroll
-    for (int j = 0; j < PER_LANE; ++j) {
-      const int e = lane + 32 * j;
-      v[j] = e < E ? load_scalar_cg(logits, (int64_t)tok * E + e, ldt) : -INFINITY;
-      mx = fmaxf(mx, v[j]);
-    }
+    for (int j = 0; j < PER_LANE; ++j) mx = fmaxf(mx, v[j]);
 #pragma unroll
     for (int o = 16; o > 0; o >>= 1) mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, o));
     float sum = 0.f;

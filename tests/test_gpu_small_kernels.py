@@ -57,3 +57,17 @@ def test_gated_norm(impl, dtype, rows, V):
     xd, zd = x.double(), z.double()
     ref = xd * (xd.pow(2).mean(1, keepdim=True) + 1e-6).rsqrt() * w.double() * zd / (1 + (-zd).exp())
     _close(impl.gated_rmsnorm(x, z, w, 1e-6).view(rows, V), ref, dtype)
+
+
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16, torch.float32])
+@pytest.mark.parametrize("T,E,k", [(1, 1, 1), (3, 33, 5), (9, 100, 8), (300, 255, 6), (2, 512, 10), (5, 1000, 32)])
+def test_topk_of_distinct_logits(impl, dtype, T, E, k):
+    """Logits a sixteenth apart (in bf16 some are equal: the lowest index first), in any order: the same experts in the same order, weights as their softmax."""
+    g = torch.Generator(device=DEV).manual_seed(T + E)
+    order = torch.stack([torch.randperm(E, generator=g, device=DEV) for _ in range(T)])
+    logits = ((order - E // 2) / 16.0).to(dtype)
+    wts, ids = impl.moe_topk(logits, k, True, weight_dtype=torch.float32)
+    ref = torch.sort(logits.double(), dim=1, descending=True, stable=True)
+    assert torch.equal(ids.long(), ref.indices[:, :k])
+    p = ref.values[:, :k].softmax(1)
+    assert float(((wts.double() - p).abs() / p).max()) < 2.0 ** -16
