@@ -71,3 +71,20 @@ def test_topk_of_distinct_logits(impl, dtype, T, E, k):
     assert torch.equal(ids.long(), ref.indices[:, :k])
     p = ref.values[:, :k].softmax(1)
     assert float(((wts.double() - p).abs() / p).max()) < 2.0 ** -16
+
+
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16])
+@pytest.mark.parametrize("T,H", [(1, 8), (149, 2048), (3, 8200), (256, 16384)])
+def test_shared_gate(impl, dtype, T, H):
+    """Fewer rows than SMs and more, behind kernels that write its inputs, several in a row on one stream."""
+    g = torch.Generator(device=DEV).manual_seed(T + H)
+    x, gate, sh, ro = (torch.randn(*s, generator=g, device=DEV).to(dtype) for s in ((T, H), (1, H), (T, H), (T, H)))
+    gate /= H ** 0.5
+    ref = ro.double() + torch.sigmoid(x.double() @ gate.double().T) * sh.double()
+    for _ in range(3):
+        buf = torch.empty_like(sh)
+        impl.silu_mul(torch.cat([torch.full_like(sh, 30.0), sh / 30.0], 1), buf)      # silu(30) = 30 in either type
+        a = (sh / 30.0).double() * 30.0
+        out = impl.moe_shared_gate_add(x, gate, buf, ro)
+        lim = TOL[dtype] * (ro.double().abs() + 2 * a.abs()) + 2.0 ** -20
+        assert bool(((out.double() - (ref + torch.sigmoid(x.double() @ gate.double().T) * (a - sh.double()))).abs() <= lim).all())
