@@ -1208,7 +1208,9 @@ int act_split_i8(const void* x, bool in_bf16, int64_t ldx, void* xq, float* inv_
 // 1/rms (esimd_norm_gemv_norm_fp16, csrc/xpu/esimd_kernels/norm_gemv_norm_fp16.h:56-98).
 //
 // A row's inputs are read twice, the second time from L1, and 32 registers let two CTAs of 1024 threads share an SM: 8192 x 4096 46 us, 78 with the
-// inputs held in registers in between; 2048 x 8192 27 us, 40 with 34 registers; a few rows take the same either way.  Where the weights of the next kernel may be fetched at any time (overlap mode 2) that kernel may start at once.
+// inputs held in registers in between; 2048 x 8192 27 us, 40 with 34 registers.
+// Where the weights of the next kernel may be fetched at any time (overlap mode 2) that kernel may start at once, as long as there is at most a row
+// per SM (dep_enter).
 template <bool BF16>
 __global__ void __launch_bounds__(1024, 2) resadd_rmsnorm_kernel(const void* __restrict__ hidden, void* __restrict__ residual, const void* __restrict__ weight,
                                       void* __restrict__ normed, const void* __restrict__ weight2, void* __restrict__ normed2,
@@ -1283,15 +1285,99 @@ __global__ void __launch_bounds__(1024, 2) resadd_rmsnorm_kernel(const void* __r
   }
 }
 
+// The same for few rows of K up to 8192, a chain of latencies: a thread's two chunks of eight stay in registers between the sum and the output, so
+// that inputs and weight are fetched once and together, and every thread adds up the warps' sums itself.  FP8 layer of three tokens, two
+// norms: 70.5 us, 71.2 with the kernel above; 64 x 8192 3.4 us, 3.2 there.
+template <bool BF16>
+__global__ void __launch_bounds__(512) resadd_rmsnorm_few_kernel(const void* __restrict__ hidden, void* __restrict__ residual, const void* __restrict__ weight,
+                                      void* __restrict__ normed, const void* __restrict__ weight2, void* __restrict__ normed2,
+                                      int K, float eps, float scalar, int release_early) {
+  using T = typename Act<BF16>::T;
+  __shared__ float red[32];
+  if (release_early) grid_dep_release();
+  grid_dep_wait();
+  if (!release_early) grid_dep_release();
+  const int64_t r = blockIdx.x;
+  const T* h = hidden ? reinterpret_cast<const T*>(hidden) + r * K : nullptr;
+  T* res = reinterpret_cast<T*>(residual) + r * K;
+  const T* w = reinterpret_cast<const T*>(weight);
+  const T* w2 = reinterpret_cast<const T*>(weight2);
+  T* out = reinterpret_cast<T*>(normed) + r * K;
+  T* out2 = normed2 ? reinterpret_cast<T*>(normed2) + r * K : nullptr;
+  constexpr int NC = 2;
+  const int k0 = threadIdx.x * 8, step = blockDim.x * 8;
+  uint4 rv[NC], hv[NC], wv[NC];
+#pragma unroll
+  for (int i = 0; i < NC; ++i)
+    if (k0 + i * step < K) {
+      rv[i] = ld_shared_vec(res + k0 + i * step);
+      if (h) hv[i] = ld_shared_vec(h + k0 + i * step);
+      wv[i] = ld_shared_vec(w + k0 + i * step);
+    }
+  auto value = [&](int i, float (&v)[8]) {
+    const T* re = reinterpret_cast<const T*>(&rv[i]);
+    const T* he = reinterpret_cast<const T*>(&hv[i]);
+#pragma unroll
+    for (int j = 0; j < 8; ++j) v[j] = h ? (Act<BF16>::to_f(he[j]) + Act<BF16>::to_f(re[j])) * scalar : Act<BF16>::to_f(re[j]);
+  };
+  float ss = 0.f;
+#pragma unroll
+  for (int i = 0; i < NC; ++i)
+    if (k0 + i * step < K) {
+      float v[8];
+      value(i, v);
+#pragma unroll
+      for (int j = 0; j < 8; ++j) ss = fmaf(v[j], v[j], ss);
+    }
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) ss += __shfl_xor_sync(0xffffffffu, ss, o);
+  if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = ss;
+  __syncthreads();
+  float t = 0.f;
+  for (int i = 0; i < (int)(blockDim.x >> 5); ++i) t += red[i];
+  const float inv = rsqrtf(t / (float)K + eps);
+  // only now is the residual overwritten, each element by the thread that read it
+#pragma unroll
+  for (int i = 0; i < NC; ++i) {
+    const int k = k0 + i * step;
+    if (k >= K) break;
+    float v[8];
+    value(i, v);
+    const T* we = reinterpret_cast<const T*>(&wv[i]);
+    uint4 so, no;
+    T* se = reinterpret_cast<T*>(&so);
+    T* ne = reinterpret_cast<T*>(&no);
+#pragma unroll
+    for (int j = 0; j < 8; ++j) {
+      se[j] = Act<BF16>::from_f(v[j]);
+      ne[j] = Act<BF16>::from_f(v[j] * inv * Act<BF16>::to_f(we[j]));
+    }
+    if (h) *reinterpret_cast<uint4*>(res + k) = so;
+    *reinterpret_cast<uint4*>(out + k) = no;
+    if (out2) {
+      const uint4 w2v = ld_shared_vec(w2 + k);
+      const T* w2e = reinterpret_cast<const T*>(&w2v);
+#pragma unroll
+      for (int j = 0; j < 8; ++j) ne[j] = Act<BF16>::from_f(v[j] * inv * Act<BF16>::to_f(w2e[j]));
+      *reinterpret_cast<uint4*>(out2 + k) = no;
+    }
+  }
+}
+
 int resadd_rmsnorm(const void* hidden, void* residual, const void* weight, void* normed, const void* weight2, void* normed2,
                    bool bf16, int64_t M, int K, float eps, float scalar, cudaStream_t st) {
   if (M == 0) return B2Q_OK;
+  const bool few = M <= 16 && K <= 8192;
   int threads = (K / 8 + 31) / 32 * 32;
-  threads = threads > 1024 ? 1024 : (threads < 32 ? 32 : threads);
-  const bool overlap = tls().overlap_mode > 0;
-  cudaError_t e;
-  if (bf16) e = launch_overlapped(resadd_rmsnorm_kernel<true>, dim3((unsigned)M), dim3(threads), 0, st, overlap, hidden, residual, weight, normed, weight2, normed2, K, eps, scalar, tls().overlap_mode == 2 ? 1 : 0);
-  else e = launch_overlapped(resadd_rmsnorm_kernel<false>, dim3((unsigned)M), dim3(threads), 0, st, overlap, hidden, residual, weight, normed, weight2, normed2, K, eps, scalar, tls().overlap_mode == 2 ? 1 : 0);
+  const int most = few ? 512 : 1024;                                  // few: room beside a CTA of the kernels around it
+  threads = threads > most ? most : (threads < 32 ? 32 : threads);
+  const int mode = tls().overlap_mode;
+  auto go = [&](auto kern) {
+    return launch_overlapped(kern, dim3((unsigned)M), dim3(threads), 0, st, mode > 0, hidden, residual, weight, normed, weight2, normed2, K, eps, scalar,
+                             mode == 2 && M <= 148 ? 1 : 0);
+  };
+  const cudaError_t e = bf16 ? (few ? go(resadd_rmsnorm_few_kernel<true>) : go(resadd_rmsnorm_kernel<true>))
+                             : (few ? go(resadd_rmsnorm_few_kernel<false>) : go(resadd_rmsnorm_kernel<false>));
   note_launch("resadd_rmsnorm");
   return e == cudaSuccess ? launch_status() : B2Q_ERR_CUDA;
 }

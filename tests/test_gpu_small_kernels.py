@@ -1,9 +1,6 @@
 """The small kernels between the linears at the edges of what a thread fetches at once: rows of a norm beyond what one pass of a CTA holds, many
 rows, experts that leave a lane's last logits empty.  Against fp64; the output is rounded once, 2^-9 of an element in bf16, 2^-12 in
 fp16, and the fp32 sums in front of it are exact to some 2^-18: twice the rounding in all."""
-import os
-import re
-
 import pytest
 import torch
 
@@ -25,7 +22,7 @@ def _close(out, ref, dtype):
 
 
 @pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16])
-@pytest.mark.parametrize("M,K", [(1, 8), (3, 1032), (700, 4096), (2, 8192), (5, 8200), (300, 16392)])
+@pytest.mark.parametrize("M,K", [(1, 8), (3, 1032), (700, 4096), (2, 8192), (5, 8200), (300, 16392), (16, 8192), (17, 8192), (16, 4104)])
 def test_residual_norm(impl, dtype, M, K):
     g = torch.Generator(device=DEV).manual_seed(M + K)
     h, r, w, w2 = (torch.randn(*s, generator=g, device=DEV).to(dtype) for s in ((M, K), (M, K), (K,), (K,)))
@@ -40,13 +37,6 @@ def test_residual_norm(impl, dtype, M, K):
     impl.rmsnorm_fused(None, r, 1.0, w, out, w2, out2, 1e-6)
     _close(out, n * w.double(), dtype)
     _close(out2, n * w2.double(), dtype)
-
-
-def test_two_blocks_of_norm_rows_share_an_sm():
-    src = os.path.join(os.path.dirname(os.path.dirname(os.path.abspath(__file__))), "llm-scaler_b200", "csrc", "moe_aux.cu")
-    with open(src) as f:
-        text = f.read()
-    assert re.search(r"__launch_bounds__\(1024, 2\) resadd_rmsnorm_kernel\(", text) and "threads > 1024 ? 1024" in text[text.index("int resadd_rmsnorm("):]
 
 
 @pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16])
